@@ -481,17 +481,15 @@ int run_pipeline(elas_handle* h, const uint8_t* img0, const uint8_t* img1, float
     auto mark = [&](int i) -> cudaError_t {
         return h->timing ? cudaEventRecordWithFlags(h->ev[i], st, ev_flags) : cudaSuccess;
     };
-    CK(cudaMemsetAsync(h->err, 0, sizeof(unsigned), st));
-    CK(mark(ELAS_TIME_DESCRIPTOR));
-    CK(launch_descriptor(img0, img1, h->desc0, h->desc1, W, H, st));
-    n += 1;
-    CK(mark(ELAS_TIME_SUPPORT));
     const uint32_t* bins = nullptr;
     h->pn_used = h->prop && H >= 4 && W >= 4 && g.cw > 0 && g.ch > 0;
+    CK(mark(ELAS_TIME_DESCRIPTOR));
+    CK(launch_descriptor(img0, img1, h->desc0, h->desc1, W, H, h->err, h->pn_used ? h->pn_stats : nullptr, st));
+    n += 1;
+    CK(mark(ELAS_TIME_SUPPORT));
     if (h->pn_used) {
         rc = ensure_pn(h, g);
         if (rc != ELAS_OK) return rc;
-        CK(cudaMemsetAsync(h->pn_stats, 0, 4 * sizeof(int32_t), st));
         CK(pn::launch_features(h->desc0, h->desc1, h->pn_in, W, H, st));
         CK(pn::launch_infer(h->pw, h->pn_in, h->pn_a0, h->pn_a1, h->pn_out, H / 4, W / 4, h->num_sms, h->err, st));
         CK(pn::launch_topk(h->pn_out, h->pn_bins, H / 4, W / 4, g.cw, g.ch, g.step, g.D, st));
@@ -509,8 +507,9 @@ int run_pipeline(elas_handle* h, const uint8_t* img0, const uint8_t* img1, float
     // beside the Delaunay and prior stages and joins before dense matching
     // (recorded as graph edges inside a capture).  With stage timing on it
     // runs in line, so that the stage marks keep their meaning.
-    // The direct prior paint also needs zeroed prior maps, which the side
-    // stream clears meanwhile; the join then comes before the prior stage.
+    // The prior paint also needs zeroed prior maps (direct) or tile counts
+    // (tiled), which the side stream clears meanwhile; the join therefore
+    // comes before the prior stage.
     const bool fork = !h->timing;
     const bool tiled = (h->test_flags & ELAS_TEST_PRIOR_TILED) != 0 ||
                        ((h->test_flags & ELAS_TEST_PRIOR_DIRECT) == 0 && (long long)W * H >= PRIOR_TILED_MIN_PIXELS);
@@ -524,6 +523,8 @@ int run_pipeline(elas_handle* h, const uint8_t* img0, const uint8_t* img1, float
         if (!tiled) {
             CK(cudaMemsetAsync(h->prior0, 0, size_t(W) * H * sizeof(uint32_t), h->side));
             CK(cudaMemsetAsync(h->prior1, 0, size_t(W) * H * sizeof(uint32_t), h->side));
+        } else {
+            CK(cudaMemsetAsync(h->ptiles.cnt, 0, 2 * (prior_tile_count(g) + 1) * sizeof(int32_t), h->side));
         }
         CK(cudaEventRecordWithFlags(h->side_join, h->side, 0));
     } else {
@@ -541,7 +542,7 @@ int run_pipeline(elas_handle* h, const uint8_t* img0, const uint8_t* img1, float
     if (fork) CK(cudaStreamWaitEvent(st, h->side_join, 0));
     CK(launch_prior(h->del[0].tri, h->del[1].tri, h->del[0].ctr, h->del[1].ctr, h->del[0].Tmax, h->can, h->uvd,
                     h->rast, h->ptiles, h->prior0, h->prior1, g, prior_shift(g, dp), g.D + dp.plane_radius + 1,
-                    h->num_sms, h->err, st, &n, tiled, fork && !tiled,
+                    h->num_sms, h->err, st, &n, tiled, fork,
                     (h->test_flags & ELAS_TEST_PRIOR_SMALL_BINS) ? 2 : PT_BIN));
     int shape = 512;
     rc = dense_threads_for(h, g, dp, st, &n, &shape);
@@ -566,7 +567,8 @@ int run_pipeline(elas_handle* h, const uint8_t* img0, const uint8_t* img1, float
     float* dev_outs[2] = {host_out ? h->out0 : out0, host_out ? h->out1 : out1};   // device partners of tmp
     float* start[2];
     for (int k = 0; k < 2; ++k) start[k] = from_tmp && k < nviews ? h->tmp[k] : outs[k];
-    CK(launch_lr(h->raw0, h->raw1, h->lr0, h->lr1, start[0], start[1], g, p.lr_threshold, st, sub));
+    CK(launch_lr(h->raw0, h->raw1, h->lr0, h->lr1, start[0], start[1], h->roots[0], h->roots[1], g, p.lr_threshold, st,
+                 sub));
     n += 1;
     CK(mark(ELAS_TIME_POST));
     PostViews pv;

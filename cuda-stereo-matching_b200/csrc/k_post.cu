@@ -568,7 +568,6 @@ cudaError_t launch_post(PostViews pv, int nviews, const Geom& g, const DevParams
     // with the tile filter following, speckle removal is applied as it loads
     const bool fuse = post_fuses_speckle(p, median, adaptive_mean);
     if (p.speckle_size > 0) {
-        for (int k = 0; k < nviews; ++k) cudaMemsetAsync(pv.roots[k], 0, sizeof(int32_t), st);
         const dim3 tiles((W + SPK_T - 1) / SPK_T, (H + SPK_T - 1) / SPK_T, nviews);
         launch_k(k_spk_tile, tiles, dim3(SPK_T, SPK_ROWS), 0, st, pv, W, H, p.speckle_sim_threshold);
         const long long border = (long long)H * (tiles.x - 1) + (long long)W * (tiles.y - 1);

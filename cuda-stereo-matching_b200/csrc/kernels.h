@@ -52,8 +52,10 @@ struct DelDev {
     uint32_t Hmax;         // power of two
 };
 
+// Also zeroes the error word and, where given, the four proposal counters
+// (a memset node of its own costs 3-5 us on a pair's critical path).
 cudaError_t launch_descriptor(const uint8_t* img0, const uint8_t* img1, uint4* desc0, uint4* desc1,
-                              int W, int H, cudaStream_t st);
+                              int W, int H, unsigned* err, int32_t* stats, cudaStream_t st);
 
 // bins (nullable): packed learned search sets per candidate; then stats[0]
 // counts candidates the proposal settled and stats[1] those that fell back
@@ -100,7 +102,8 @@ size_t prior_overflow_capacity(const Geom& g, int Tmax);
 // rast: scratch of 2 * Tmax * raster_bytes() for the per-triangle set-up.
 // tiled: paint tile by tile in shared memory (tl used) instead of with
 // global atomics into the zeroed prior; the same bytes either way.
-// zeroed: (direct paint) the caller has zeroed both priors already.
+// zeroed: the caller has zeroed what the paint adds to already (direct:
+// both priors; tiled: the tile counts).
 // bin_cap: (tiled paint) entries used of each tile's bin (tests lower it so
 // that the overflow list is used).
 cudaError_t launch_prior(const int32_t* tri0, const int32_t* tri1, const int32_t* ctr0, const int32_t* ctr1,
@@ -123,14 +126,16 @@ cudaError_t launch_dense(const uint4* desc0, const uint4* desc1, const uint32_t*
                          const DevParams& p, int pshift, unsigned* err, cudaStream_t st, int threads, int sub = 0,
                          bool force_bitset = false);
 
-// L/R check into o0/o1 and, where c0 is not null, also into c0/c1
-cudaError_t launch_lr(const float* d0, const float* d1, float* o0, float* o1, float* c0, float* c1, const Geom& g,
-                      int lr_threshold, cudaStream_t st, int sub);
+// L/R check into o0/o1 and, where c0 is not null, also into c0/c1; zeroes
+// the lengths of both views' roots lists (r0, r1) for the speckle filter.
+cudaError_t launch_lr(const float* d0, const float* d1, float* o0, float* o1, float* c0, float* c1, int32_t* r0,
+                      int32_t* r1, const Geom& g, int lr_threshold, cudaStream_t st, int sub);
 
 // Buffers of the post-filter chain, per view: the filters ping-pong between
 // cur and nxt (the chain starts in cur; the result is copied to out if it
 // does not end there); lab/root/sz are union-find scratch (W*H int32 each),
-// roots the list of tile-local roots (W*H + 1 int32).
+// roots the list of tile-local roots (W*H + 1 int32; its length, the first
+// entry, zeroed by launch_lr).
 struct PostViews {
     float* cur[2];
     float* nxt[2];
