@@ -10,7 +10,7 @@
 //   gap       rows, then columns: a run of <= ipol_gap_width invalid pixels
 //             between valid a and b becomes (a+b)/2 if |a-b| <= 3 else
 //             min(a,b).  Widths up to 8 run inside the fused tile kernel,
-//             wider gaps as one thread per line.
+//             wider gaps as a row pass and a column pass.
 //   mean      5x5 weighted mean of valid pixels, w = 1/(1+(d_q-d_p)^2).
 //   median    lower median of the valid pixels of the 3x3 window.
 #include <cuda_runtime.h>
@@ -351,25 +351,110 @@ __global__ void k_uf_apply(float* D, const int32_t* __restrict__ root, const int
     if (r >= 0 && sz[r] < min_size) D[i] = -1.0f;
 }
 
-// horizontal = 1: one thread per row; 0: one thread per column (used for
-// gap widths too large for the per-pixel search).
-__global__ void k_gap(PostViews pv, int W, int H, int gap, int horizontal) {
+// Gaps wider than the tile filter's halo, rows then columns.  A run of
+// invalid pixels between valid a and b is filled from a and b alone, which
+// no fill changes, so every pixel can look for its two ends by itself: in a
+// bit mask of the line's valid pixels kept in shared memory (32 pixels a
+// word, empty words skipped).  Bound by latency (a handful of dependent
+// loads a pixel); one thread walking a whole line in order took 1089 us for
+// the rows (and 16 for the speckle pass before them) and 348 us for the
+// columns of a 1242x375 pair, this pair of kernels 13 us each.
+__device__ __forceinline__ float gap_value(float a, float b) {
+    return fabsf(a - b) <= 3.0f ? __fmul_rn(0.5f, __fadd_rn(a, b)) : fminf(a, b);
+}
+
+// One CTA per row: cur -> nxt, applying the speckle decision of k_spk_apply
+// on the way in when spk_min > 0 (no separate pass).
+constexpr int GAP_THREADS = 256;
+__global__ void __launch_bounds__(GAP_THREADS) k_gap_rows(PostViews pv, int W, int gap, int spk_min) {
     grid_dep_wait();
-    float* D = pv.cur[blockIdx.z];
-    int l = blockIdx.x * blockDim.x + threadIdx.x;
-    int lines = horizontal ? H : W, len = horizontal ? W : H;
-    if (l >= lines) return;
-    size_t base = horizontal ? size_t(l) * W : size_t(l);
-    size_t stride = horizontal ? 1 : size_t(W);
-    int k = 0;
-    while (k < len) {
-        if (D[base + k * stride] >= 0) { ++k; continue; }
-        int k0 = k;
-        while (k < len && D[base + k * stride] < 0) ++k;
-        if (k0 > 0 && k < len && k - k0 <= gap) {
-            float a = D[base + (k0 - 1) * stride], b = D[base + k * stride];
-            float f = fabsf(a - b) <= 3.0f ? __fmul_rn(0.5f, __fadd_rn(a, b)) : fminf(a, b);
-            for (int q = k0; q < k; ++q) D[base + q * stride] = f;
+    extern __shared__ uint32_t mask[];          // (W + 31) / 32 words
+    const int view = blockIdx.z, lane = threadIdx.x & 31;
+    const size_t base = size_t(blockIdx.x) * W;
+    const float* __restrict__ src = pv.cur[view] + base;
+    float* __restrict__ dst = pv.nxt[view] + base;
+    const int32_t* __restrict__ lab = pv.lab[view] + base;
+    const int32_t* __restrict__ sz = pv.sz[view];
+    const int32_t* __restrict__ acc = pv.root[view];
+    const int nw = (W + 31) / 32;
+    for (int x0 = threadIdx.x & ~31; x0 < W; x0 += GAP_THREADS) {
+        const int x = x0 + lane;
+        float d = x < W ? src[x] : -1.0f;
+        if (spk_min > 0 && x < W) {
+            const int l = lab[x];
+            if (d >= 0 && acc[-sz[l] - 1] < spk_min) d = -1.0f;
+        }
+        const unsigned m = __ballot_sync(0xffffffffu, d >= 0);
+        if (lane == 0) mask[x0 >> 5] = m;
+        if (d >= 0) dst[x] = d;
+    }
+    __syncthreads();
+    for (int x0 = threadIdx.x & ~31; x0 < W; x0 += GAP_THREADS) {
+        const int x = x0 + lane;
+        const unsigned m = mask[x0 >> 5];
+        if (x >= W || ((m >> lane) & 1u)) continue;
+        unsigned below = m & ((1u << lane) - 1u), above = m & ~((2u << lane) - 1u);
+        int wl = x0 >> 5, wh = wl;
+        while (!below && wl > 0) below = mask[--wl];
+        while (!above && wh + 1 < nw) above = mask[++wh];
+        float f = -1.0f;
+        if (below && above) {
+            const int lo = 32 * wl + 31 - __clz(below), hi = 32 * wh + __ffs(above) - 1;
+            if (hi - lo - 1 <= gap) f = gap_value(src[lo], src[hi]);
+        }
+        dst[x] = f;
+    }
+}
+
+// One CTA per 32 columns, a warp per 32 rows at a time (lane = column):
+// src -> dst, in place when they are the same.
+constexpr int GAP_COL_WARPS = 16;
+__global__ void __launch_bounds__(32 * GAP_COL_WARPS) k_gap_cols(PostViews pv, int W, int H, int gap) {
+    grid_dep_wait();
+    extern __shared__ uint32_t mask[];          // [(H + 31) / 32][32]
+    const int view = blockIdx.z, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int x = blockIdx.x * 32 + lane, nb = (H + 31) / 32;
+    const float* src = pv.cur[view] + x;
+    float* dst = pv.nxt[view] + x;
+    const bool in = x < W, copy = src != dst;
+    for (int b = warp; b < nb; b += GAP_COL_WARPS) {
+        const int n = min(32, H - 32 * b);
+        uint32_t bits = 0;
+#pragma unroll 8
+        for (int r = 0; r < n; ++r) {
+            const float d = in ? src[size_t(32 * b + r) * W] : -1.0f;
+            bits |= d >= 0 ? 1u << r : 0u;
+        }
+        mask[32 * b + lane] = bits;
+    }
+    __syncthreads();
+    if (!in) return;
+    for (int b = warp; b < nb; b += GAP_COL_WARPS) {
+        const int n = min(32, H - 32 * b);
+        const uint32_t bits = mask[32 * b + lane];
+        int lo = -1;                            // the last valid row before the current one
+        for (int w = b - 1; w >= 0 && lo < 0; --w)
+            if (const uint32_t m = mask[32 * w + lane]) lo = 32 * w + 31 - __clz(m);
+        bool open = false;                      // inside a run whose fill value f is known
+        float f = -1.0f;
+        for (int r = 0; r < n; ++r) {
+            const size_t at = size_t(32 * b + r) * W;
+            if ((bits >> r) & 1u) {
+                lo = 32 * b + r;
+                open = false;
+                if (copy) dst[at] = src[at];
+                continue;
+            }
+            if (!open) {
+                open = true;
+                f = -1.0f;
+                int hi = -1;
+                if (const uint32_t m = bits >> r) hi = 32 * b + r + __ffs(m) - 1;
+                for (int w = b + 1; w < nb && hi < 0; ++w)
+                    if (const uint32_t m = mask[32 * w + lane]) hi = 32 * w + __ffs(m) - 1;
+                if (lo >= 0 && hi >= 0 && hi - lo - 1 <= gap) f = gap_value(src[size_t(lo) * W], src[size_t(hi) * W]);
+            }
+            if (copy || f >= 0) dst[at] = f;
         }
     }
 }
@@ -392,7 +477,7 @@ __device__ __forceinline__ float gap_fill(const float* line, int stride, int k, 
             if (line[j * stride] >= 0) { hi = k + j; break; }
     if (lo >= 0 && hi >= 0 && hi - lo - 1 <= gap) {
         float a = line[-(k - lo) * stride], b = line[(hi - k) * stride];
-        return fabsf(a - b) <= 3.0f ? __fmul_rn(0.5f, __fadd_rn(a, b)) : fminf(a, b);
+        return gap_value(a, b);
     }
     return c;
 }
@@ -578,7 +663,7 @@ cudaError_t launch_post(PostViews pv, int nviews, const Geom& g, const DevParams
         // SM walks it (idle CTAs cost their launch; measured against four)
         launch_k(k_spk_count, dim3(imin(gn, num_sms), 1, nviews), 256, 0, st, pv, n, err);
         launched += 3;
-        if (!fuse) {
+        if (!fuse && p.ipol_gap_width <= PGMAX) {
             launch_k(k_spk_apply, dim3(gn, 1, nviews), 256, 0, st, pv, n, p.speckle_size);
             flip();
             launched += 1;
@@ -587,9 +672,20 @@ cudaError_t launch_post(PostViews pv, int nviews, const Geom& g, const DevParams
     const int gap = p.ipol_gap_width;
     const int spk = fuse ? p.speckle_size : 0;
     const bool tile_gap = gap > 0 && gap <= PGMAX;
-    if (gap > PGMAX) {   // wide gaps: serial scans per line, in place
-        launch_k(k_gap, dim3((H + 127) / 128, 1, nviews), 128, 0, st, pv, W, H, gap, 1);
-        launch_k(k_gap, dim3((W + 127) / 128, 1, nviews), 128, 0, st, pv, W, H, gap, 0);
+    if (gap > PGMAX) {   // wide gaps: cur -> nxt by rows, then by columns
+        launch_k(k_gap_rows, dim3(H, 1, nviews), GAP_THREADS, size_t((W + 31) / 32) * sizeof(uint32_t), st, pv, W, gap,
+                 p.speckle_size);
+        flip();
+        // in place before the tile filter; as the chain's last pass straight
+        // into the final buffers
+        PostViews pc = pv;
+        const bool last = !adaptive_mean && !median;
+        for (int k = 0; k < 2; ++k) pc.nxt[k] = last ? pv.out[k] : pv.cur[k];
+        allow_smem(k_gap_cols);
+        launch_k(k_gap_cols, dim3((W + 31) / 32, 1, nviews), 32 * GAP_COL_WARPS,
+                 size_t((H + 31) / 32) * 32 * sizeof(uint32_t), st, pc, W, H, gap);
+        if (last)
+            for (int k = 0; k < nviews; ++k) pv.cur[k] = pv.out[k];
         launched += 2;
     }
     if (tile_gap || adaptive_mean || median) {

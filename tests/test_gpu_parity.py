@@ -149,6 +149,21 @@ def test_post_filters_individually(elas, filt):
     run_and_compare(elas, L, R, p, check_triangle=False)
 
 
+@pytest.mark.parametrize("width,height,gap,speckle,median", [(97, 61, 9, 0, False), (64, 64, 40, 20, False),
+                                                             (333, 31, 5000, 0, True), (160, 225, 33, 50, True)])
+def test_wide_gap_sizes(elas, width, height, gap, speckle, median):
+    """Gaps wider than the tile filter takes, at widths and heights around
+    the 32-pixel words of the row and column passes: as the chain's last
+    pass and before the median, with and without speckle removal."""
+    L, R, _, _ = eb.synth_pair(3, 31, width=width, height=height, disp_max=24)
+    p = eb.params_reference()
+    p.disp_max = 24
+    p.ipol_gap_width = gap
+    p.speckle_size = speckle
+    p.filter_median = median
+    run_and_compare(elas, L, R, p, check_triangle=False)
+
+
 def test_constructor_default_parameters(elas):
     """Elas::parameters() defaults (support_threshold 0.95, gamma 5, sradius 3,
     ipol_gap_width 5000, median on)."""
