@@ -203,3 +203,55 @@ def test_topk_bins_match_float64_scores(preset, seed):
             if len(got):
                 worst = max(worst, float(np.max(np.abs(gs - es) / tol)))
     assert worst <= 1.0, worst
+
+
+@pytest.mark.parametrize("shift", [0, 1])
+@pytest.mark.parametrize("nimg,hd,wd", [(1, 1, 1), (2, 8, 32), (3, 9, 33), (2, 5, 31), (1, 17, 65)])
+def test_training_convolutions_at_tile_edges(torch, nimg, hd, wd, shift):
+    """Forward, input, weight and bias gradients of one layer around the
+    kernels' tile sizes (8 x 32 and 4 x 32 cells) and with buffers off a
+    16-byte boundary (shift floats), against float64.  A sum of n products
+    in fp32, in any order, is off by at most n * 2^-23 of the sum of their
+    magnitudes."""
+    F = torch.nn.functional
+    gen = torch.Generator().manual_seed(1000 * hd + wd + shift)
+
+    def buf(n, data=None):
+        t = torch.zeros(n + 4, device="cuda")[shift:shift + n]
+        if data is not None:
+            t.copy_(data.reshape(-1))
+        return t
+
+    ch, taps = po.CH, po.TAPS
+    x, dy = (torch.randn((nimg, hd, wd, ch), generator=gen) for _ in range(2))
+    w, b = torch.randn((taps, ch, ch), generator=gen) * 0.1, torch.randn(ch, generator=gen)
+    n = x.numel()
+    dx_, dy_, dw_, db_ = buf(n, x), buf(n, dy), buf(w.numel(), w), buf(ch, b)
+    y, gx, gw, gb, scratch = buf(n), buf(n), buf(w.numel()), buf(ch), buf(w.numel())
+    eb.pn_conv_forward(dx_.data_ptr(), dw_.data_ptr(), db_.data_ptr(), y.data_ptr(), nimg, hd, wd, True)
+    eb.pn_conv_backward(dx_.data_ptr(), y.data_ptr(), dw_.data_ptr(), dy_.data_ptr(), gx.data_ptr(), gw.data_ptr(),
+                        gb.data_ptr(), scratch.data_ptr(), nimg, hd, wd, True)
+    torch.cuda.synchronize()
+
+    def conv(v, k):                       # v [n][h][w][ci], k [tap][ci][co]
+        k = k.view(3, 3, ch, ch).permute(3, 2, 0, 1)
+        return F.conv2d(v.permute(0, 3, 1, 2), k, padding=1).permute(0, 2, 3, 1)
+
+    xd, wd_, got = x.double(), w.double(), y.cpu().double().view(x.shape)
+    ref = conv(xd, wd_) + b.double()
+    mag = conv(xd.abs(), wd_.abs()) + b.double().abs()
+    assert bool(((got - ref.clamp(min=0)).abs() <= (taps * ch + 1) * 2.0 ** -23 * mag).all())
+    g = torch.where(got > 0, dy.double(), torch.zeros_like(got))     # the ReLU mask the kernels used
+    flip = wd_.flip(0).transpose(1, 2)
+    assert bool(((gx.cpu().double().view(x.shape) - conv(g, flip)).abs()
+                 <= taps * ch * 2.0 ** -23 * conv(g.abs(), flip.abs())).all())
+
+    def wgrad(v, u):
+        p = F.pad(v, (0, 0, 1, 1, 1, 1))
+        return torch.stack([torch.einsum("nhwi,nhwo->io", p[:, t // 3:t // 3 + hd, t % 3:t % 3 + wd], u)
+                            for t in range(taps)])
+
+    cells = nimg * hd * wd
+    assert bool(((gw.cpu().double().view(w.shape) - wgrad(xd, g)).abs()
+                 <= cells * 2.0 ** -23 * wgrad(xd.abs(), g.abs())).all())
+    assert bool(((gb.cpu().double() - g.sum((0, 1, 2))).abs() <= cells * 2.0 ** -23 * g.abs().sum((0, 1, 2))).all())
