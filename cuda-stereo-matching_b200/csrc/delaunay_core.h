@@ -357,6 +357,28 @@ HD bool star_better(int ip, uint32_t pp, int iq, uint32_t pq, int ia, uint32_t p
     return side > 0 ? inside_sos_p(ip, pp, iq, pq, ia, pa, ib, pb) : inside_sos_p(ip, pp, ia, pa, iq, pq, ib, pb);
 }
 
+// star_better for side > 0 with a and b known to lie strictly left of p->q,
+// by the centres of their circles on the bisector of p and q: with u = q - p
+// a point s (relative to p) has its centre at t = (|s|^2 - u.s) / cross(u, s)
+// (up to a common scale), and b is inside a's circle when its t is smaller.
+// Numerators stay below 2^31 and denominators below 2^30 at the coordinate
+// limits of orient_p, so the cross products are exact in int64.  Equal
+// centres (four co-circular points) go by the perturbation: the lowest
+// index decides as in inside_sos_p, where d = b, and a's own barycentric
+// coordinate is positive as b lies left of p->q.
+HD bool star_better_left(int ip, uint32_t pp, int iq, uint32_t pq, int ia, uint32_t pa, int ib, uint32_t pb) {
+    const int32_t ux = dx_p(pq, pp), uy = dy_p(pq, pp);
+    const int32_t ax = dx_p(pa, pp), ay = dy_p(pa, pp), bx = dx_p(pb, pp), by = dy_p(pb, pp);
+    const int32_t ca = ux * ay - uy * ax, cb = ux * by - uy * bx;
+    const int32_t na = ax * ax + ay * ay - (ux * ax + uy * ay), nb = bx * bx + by * by - (ux * bx + uy * by);
+    const int64_t l = int64_t(nb) * ca, r = int64_t(na) * cb;
+    if (l != r) return l < r;
+    const int m = imin(imin(ip, iq), imin(ia, ib));
+    if (m == ib) return true;
+    if (m == ia) return false;
+    return (m == ip ? orient_p(pb, pq, pa) : orient_p(pp, pb, pa)) < 0;
+}
+
 // Is b strictly on the walk's side of p->q?
 HD bool star_side(uint32_t pp, uint32_t pq, uint32_t pb, int side) {
     const int64_t o = orient_p(pp, pq, pb);
@@ -419,33 +441,29 @@ HD bool circle_inside(uint32_t pp, uint32_t pq, uint32_t pr, int R, const int32_
            side_ok(-BY1, -CY, RD, V2);
 }
 
-// Search policy of the star walk.  A search first takes a point's window,
-// the points with |x - px|, |y - py| <= R0, staged once per point (up to
-// STAR_CAP of them), and then squares of doubling half-size Rs
-// (star_square) around p until its answer is proven:
-//  * nearest neighbour at distance d: proven once d <= Rs; if the first
-//    square with a candidate does not prove it, the square of half-size d
-//    holds the answer and is searched last;
-//  * next neighbour r: proven once its circle passes circle_within(Rs).
-//    When the circle reaches no further than 2 Rs, the part of the circle
-//    through p, q, r inside the box is searched instead of the next square
-//    (the answer's circle on that side of p->q nests inside it, so the
-//    answer lies there).  A near-collinear r has a huge circle although the
-//    answer is often just outside the window: growing the square finds it
-//    at a small cost where the circle would cover much of the box.
-// A square covering the box holds every point, so its answer is final (and
-// "none" proves a hull edge).
-constexpr int STAR_CAP = 512;
+// When a star is proven.  With every point of the square of half-size R
+// around p at hand, the nearest neighbour at distance d is certain once
+// d <= R and the next neighbour r after q once circle_inside(R) holds for p,
+// q, r: monotone in R, and certain in any case once the square covers the
+// box of all points (which also proves a hull edge).  A search over growing
+// squares starts at half-size R0 and doubles it until its answer is
+// certain; the number of doublings a star needs is therefore a property of
+// the star, whatever points were looked at to find it.  The sequential
+// emulation searches that way (its window keeps every point, STAR_CAP); the
+// device finds the star from fewer points and counts the same doublings.
+constexpr int STAR_CAP = 1 << 30;
 
 // The window's half-size R0 of a problem: 3.5 mean point spacings (the
-// square root of the box area per point), within [16, 128] pixels.  Most
-// stars then need no second search (a smaller window makes most steps
-// search again, a larger one makes every step scan more points).  Exact
-// double operations: the same value on the host and the device.
+// square root of the box area per point), within [16, 128] pixels: the
+// largest such r with 4 r^2 n <= 49 area.  Most stars are then proven by
+// the window (a smaller one proves fewer, a larger one holds more points
+// than a step should look at).
 HD int star_r0(const int32_t* box, int n) {
-    const double area = double(box[2] - box[0] + 1) * double(box[3] - box[1] + 1);
-    const double r = 3.5 * sqrt(area / double(n > 0 ? n : 1));
-    return r < 16.0 ? 16 : (r > 128.0 ? 128 : int(r));
+    const int64_t area = int64_t(box[2] - box[0] + 1) * (box[3] - box[1] + 1);
+    int r = 16;
+    for (int st = 64; st > 0; st >>= 1)
+        if (r + st <= 128 && 4LL * (r + st) * (r + st) * (n > 0 ? n : 1) <= 49 * area) r += st;
+    return r;
 }
 constexpr int STAR_NB = 256;      // neighbours of one point on each side of its start
 

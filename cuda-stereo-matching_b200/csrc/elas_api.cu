@@ -265,8 +265,8 @@ size_t layout(elas_handle* h, const Geom& g, char* base) {
         D.ctr = (int32_t*)take(16 * 4);
         D.pxy = (uint32_t*)take(nmax * 4);
         D.sxy = (uint32_t*)take(nmax * 4);
-        D.ne_y = (int32_t*)take(rows * 4);
-        D.rinfo = (int4*)take(rows * 16);
+        D.xb = (int32_t*)take(rows * ((size_t(g.W) + 7) / 8 + 1) * 4);
+        D.far = (int32_t*)take(DelDev::FAR_REC * nmax * 4);
         D.tcnt = (int32_t*)take(nmax * 4);
         D.toff = (int32_t*)take(nmax * 4);
         D.sown = (int32_t*)take(24 * nmax * 4);
@@ -274,7 +274,6 @@ size_t layout(elas_handle* h, const Geom& g, char* base) {
         D.hnext = (int32_t*)take(nmax * 4);
         D.hprev = (int32_t*)take(nmax * 4);
         D.box = (int32_t*)take(32);
-        D.ylut = (int32_t*)take((size_t(g.H) + 2) * 4);
         D.hkey = (unsigned long long*)take(hmax * 8);
         D.hcnt = (int32_t*)take(hmax * 4);
         D.hval = (int32_t*)take(2 * hmax * 4);
@@ -535,9 +534,9 @@ int run_pipeline(elas_handle* h, const uint8_t* img0, const uint8_t* img1, float
                        h->flip_round_limit > 0 ||
                        ((h->test_flags & ELAS_TEST_DELAUNAY_STARS) == 0 &&
                         (long long)W * H > DELAUNAY_STARS_MAX_PIXELS);
-    CK(launch_delaunay(h->del[0], h->del[1], h->row_off, g.ch + corners, g.cw * g.ch + 6 * corners, H, h->num_sms,
-                       h->cluster_size, h->err, st, &n, flips, (h->test_flags & ELAS_TEST_FLIP_GLOBAL) != 0,
-                       h->flip_round_limit));
+    CK(launch_delaunay(h->del[0], h->del[1], h->row_off, g.ch + corners, g.cw * g.ch + 6 * corners, W, H,
+                       g.step, corners ? g.ch : -1, h->num_sms, h->cluster_size, h->err, st, &n, flips,
+                       (h->test_flags & ELAS_TEST_FLIP_GLOBAL) != 0, h->flip_round_limit));
     CK(mark(ELAS_TIME_PRIOR));
     if (fork) CK(cudaStreamWaitEvent(st, h->side_join, 0));
     CK(launch_prior(h->del[0].tri, h->del[1].tri, h->del[0].ctr, h->del[1].ctr, h->del[0].Tmax, h->can, h->uvd,

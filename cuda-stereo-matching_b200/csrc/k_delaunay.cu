@@ -131,131 +131,213 @@ __device__ __forceinline__ void propose_owned(int h0, int h1, int32_t* ring, Opp
 // (keeps the lowest index), write the unique list to srt[row_off[r] ..]
 // (with the packed coordinates beside it in sxy) and its length to rcnt[r];
 // pxy[i] gets point i's packed coordinates, or PXY_NONE if it was dropped.
-__global__ void __launch_bounds__(512) k_rowsort(DelDev d0, DelDev d1, const int32_t* __restrict__ row_off,
-                                                 int nrows, unsigned* err) {
+// The left view's rows come sorted (the support list is in raster order;
+// only add_corners breaks it) and need no sort; up to ROW_RANK points every
+// thread counts the keys below its own (one pass without barriers, where a
+// bitonic sort of 64 keys has 21 stages with one each).
+// xbs > 0 (star construction): also the row's index by 8-pixel column
+// bucket, xb[r * xbs + k] = the position in srt of the row's first point at
+// or right of column 8 k (bucket 0 also holds the columns below 0, the last
+// entry is the row's end), with which the star searches find a column range
+// by two independent loads.
+constexpr int ROW_THREADS = 256;
+constexpr int ROW_RANK = 2 * ROW_THREADS;
+__global__ void __launch_bounds__(ROW_THREADS) k_rowsort(DelDev d0, DelDev d1, const int32_t* __restrict__ row_off,
+                                                         int nrows, int xbs, unsigned* err) {
     grid_dep_wait();
-    __shared__ unsigned long long key[SORT_CAP];
-    __shared__ int keep[SORT_CAP];
+    // x biased to 16 bits (the right view's corner points of add_corners
+    // lie left of x = 0) above the 12-bit position in the row
+    __shared__ uint32_t key[SORT_CAP];
+    __shared__ int cx[SORT_CAP];        // x of the points kept
+    __shared__ int wcnt[ROW_THREADS / 32 + 1];
     const DelDev& D = blockIdx.y ? d1 : d0;
-    const int r = blockIdx.x;
+    const int r = blockIdx.x, tid = threadIdx.x;
     if (r >= nrows) return;
     const int b = row_off[r], n = row_off[r + 1] - b;
     if (n > SORT_CAP) {
-        if (threadIdx.x == 0) { set_err(err, ERRF_BOUNDS); D.rcnt[r] = 0; }
+        if (tid == 0) { set_err(err, ERRF_BOUNDS); D.rcnt[r] = 0; }
+        for (int k = tid; k < xbs; k += ROW_THREADS) D.xb[size_t(r) * xbs + k] = b;
         return;
     }
     int np = 1;
     while (np < n) np <<= 1;
-    for (int i = threadIdx.x; i < np; i += blockDim.x)
-        // x with its sign bit flipped orders signed coordinates as unsigned keys
-        // (the right view's corner points of add_corners lie left of x = 0)
-        key[i] = i < n ? (uint64_t(uint32_t(D.x[b + i]) ^ 0x80000000u) << 32 | uint32_t(b + i)) : ~0ull;
+    for (int i = tid; i < np; i += ROW_THREADS)
+        key[i] = i < n ? uint32_t(D.x[b + i] + 32768) << 12 | uint32_t(i) : 0xffffffffu;
+    const int32_t yr = n > 0 ? D.y[b] : 0;      // the row's y
     __syncthreads();
-    for (int k = 2; k <= np; k <<= 1)
-        for (int j = k >> 1; j > 0; j >>= 1) {
-            for (int i = threadIdx.x; i < np; i += blockDim.x) {
-                int ixj = i ^ j;
-                if (ixj > i) {
-                    bool up = (i & k) == 0;
-                    unsigned long long a = key[i], c = key[ixj];
-                    if ((a > c) == up) { key[i] = c; key[ixj] = a; }
-                }
+    bool unsorted = false;
+    for (int i = tid + 1; i < n; i += ROW_THREADS) unsorted = unsorted || key[i] < key[i - 1];
+    if (__syncthreads_or(unsorted)) {
+        if (n <= ROW_RANK) {
+            const uint32_t k0 = tid < n ? key[tid] : 0u, k1 = tid + ROW_THREADS < n ? key[tid + ROW_THREADS] : 0u;
+            int r0 = 0, r1 = 0;
+            for (int j = 0; j < n; ++j) {
+                const uint32_t kj = key[j];
+                r0 += kj < k0;
+                r1 += kj < k1;
             }
             __syncthreads();
+            if (tid < n) key[r0] = k0;
+            if (tid + ROW_THREADS < n) key[r1] = k1;
+            __syncthreads();
+        } else {
+            for (int k = 2; k <= np; k <<= 1)
+                for (int j = k >> 1; j > 0; j >>= 1) {
+                    for (int i = tid; i < np; i += ROW_THREADS) {
+                        const int ixj = i ^ j;
+                        if (ixj > i) {
+                            const bool up = (i & k) == 0;
+                            const uint32_t a = key[i], c = key[ixj];
+                            if ((a > c) == up) { key[i] = c; key[ixj] = a; }
+                        }
+                    }
+                    __syncthreads();
+                }
         }
-    for (int i = threadIdx.x; i < n; i += blockDim.x)
-        keep[i] = (i == 0 || (key[i] >> 32) != (key[i - 1] >> 32)) ? 1 : 0;
-    __syncthreads();
-    // compaction: each warp counts its span, warp 0 turns the counts into offsets
-    __shared__ int wcnt[17];
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
-    const int span = (n + nw - 1) / nw;
+    }
+    // compaction: each warp counts its span, every thread sums the counts before its own
+    const int lane = tid & 31, warp = tid >> 5, nw = ROW_THREADS >> 5;
+    const int span = ((n + nw - 1) / nw + 31) & ~31;
+    const int w0 = imin(n, warp * span), w1 = imin(n, w0 + span);
+    auto kept = [&](int i) { return i == 0 || (key[i] >> 12) != (key[i - 1] >> 12); };
     int c = 0;
-    for (int i = warp * span + lane; i < min(n, (warp + 1) * span); i += 32) c += keep[i];
+    for (int i = w0 + lane; i < w1; i += 32) c += kept(i);
     c = __reduce_add_sync(0xffffffffu, c);
     if (lane == 0) wcnt[warp] = c;
     __syncthreads();
-    if (threadIdx.x == 0) {
-        int run = 0;
-        for (int w = 0; w < nw; ++w) { int t = wcnt[w]; wcnt[w] = run; run += t; }
-        wcnt[16] = run;
-        D.rcnt[r] = run;
+    int base = 0, nu = 0;
+#pragma unroll
+    for (int w = 0; w < nw; ++w) {
+        base += w < warp ? wcnt[w] : 0;
+        nu += wcnt[w];
     }
-    __syncthreads();
-    int base = wcnt[warp];
-    const int32_t yr = n > 0 ? D.y[b] : 0;      // the row's y
-    for (int i0 = warp * span; i0 < min(n, (warp + 1) * span); i0 += 32) {
-        int i = i0 + lane;
-        const bool in = i < min(n, (warp + 1) * span);
-        bool k = in && keep[i];
-        unsigned m = __ballot_sync(0xffffffffu, k);
+    if (tid == 0) D.rcnt[r] = nu;
+    for (int i0 = w0; i0 < w1; i0 += 32) {
+        const int i = i0 + lane;
+        const bool in = i < w1;
+        const bool k = in && kept(i);
+        const unsigned m = __ballot_sync(0xffffffffu, k);
         if (in) {
-            const int32_t idx = int32_t(key[i] & 0xffffffffu);
-            const uint32_t xy = pack_xy(int32_t(uint32_t(key[i] >> 32) ^ 0x80000000u), yr);
+            const int32_t idx = b + int32_t(key[i] & 0xfffu);
+            const uint32_t xy = pack_xy(int32_t(key[i] >> 12) - 32768, yr);
             // packed coordinates by point (the star searches), PXY_NONE for a dropped duplicate
             D.pxy[idx] = k ? xy : PXY_NONE;
             D.hnext[idx] = -1;
             D.hprev[idx] = -1;
             if (k) {
-                const int pos = b + base + __popc(m & ((1u << lane) - 1));
-                D.srt[pos] = idx;
-                D.sxy[pos] = xy;
+                const int pos = base + __popc(m & ((1u << lane) - 1));
+                D.srt[b + pos] = idx;
+                D.sxy[b + pos] = xy;
+                cx[pos] = px_of(xy);
             }
         }
         base += __popc(m);
     }
+    if (xbs == 0) return;
+    __syncthreads();
+    for (int k = tid; k < xbs; k += ROW_THREADS) {
+        int lo = 0, hi = nu;
+        if (k == 0) hi = 0;
+        if (k == xbs - 1) lo = nu;
+        while (lo < hi) {
+            const int mid = (lo + hi) >> 1;
+            if (cx[mid] < 8 * k) lo = mid + 1;
+            else hi = mid;
+        }
+        D.xb[size_t(r) * xbs + k] = b + lo;
+    }
 }
 
+// Lattice rows: row r lies at y = r * step; with add_corners the extra row
+// `crow` (-1: none) holds the corner points at y = H - 1.
+struct RowGeom {
+    int step, crow, H;
+    float inv;          // 1 / step
+    __device__ __forceinline__ int y(int r) const { return r == crow ? H - 1 : r * step; }
+    // floor(y / step): (y + 0.5) / step is at least 0.5 / step away from a
+    // whole number, far more than the rounding for y <= 16384
+    __device__ __forceinline__ int row(int y) const { return int((float(y) + 0.5f) * inv); }
+};
+
 // For the star construction, in the block of k_plan once the non-empty
-// rows (ne, with their y in ney, both in shared memory) are known: the
-// table ylut (y -> first non-empty row at or below y, for y in [0, H]),
-// the box of all points (box[0..3]) and the window half-size (box[4],
-// star_r0), and the hull boundary (hnext / hprev of every boundary point;
-// the rows' extreme points are staged in shared memory and each decided by
-// hull_on_chain).  roff and cnt: the rows' offsets and unique counts, also
-// in shared memory.
+// rows (ne, with their y in ney, both in shared memory) are known: the box
+// of all points (box[0..3]) and the window half-size (box[4], star_r0), and
+// the hull boundary (hnext / hprev of every boundary point).  roff and cnt:
+// the rows' offsets and unique counts, also in shared memory.  The rows'
+// extreme points are staged in shared memory; HULL_LANES lanes decide one of
+// them together (hull_on_chain's two minima over the other rows, each lane
+// every HULL_LANES-th row, then merged), both chains at once.
+constexpr int HULL_LANES = 8;
 __device__ void star_setup(const DelDev& D, const int32_t* roff, const int32_t* cnt, const int32_t* ne,
-                           const int32_t* ney, int R, int H, int npts, uint32_t* xyf, uint32_t* xyl, int32_t* lstk,
-                           int32_t* rstk, int* ws) {
-    __shared__ int box_s[4];
-    const int tid = threadIdx.x, nt = blockDim.x;
+                           const int32_t* ney, int R, int npts, uint32_t* xyf, uint32_t* xyl, int32_t* lstk,
+                           int32_t* rstk, int32_t* flag, int* ws) {
+    __shared__ int box_s[2];
+    const int tid = threadIdx.x, nt = blockDim.x, lane = tid & 31;
     if (tid == 0) {
         box_s[0] = INT_MAX;
-        box_s[2] = INT_MIN;
+        box_s[1] = INT_MIN;
     }
     __syncthreads();
-    for (int s = tid; s <= R; s += nt) {
-        const int lo = s ? ney[s - 1] + 1 : 0, hi = s < R ? ney[s] : H;
-        for (int v = lo; v <= hi && v <= H; ++v) D.ylut[v] = s;
-    }
-    for (int s = tid; s < R; s += nt) {
-        const int r = ne[s], b = roff[r];
-        const uint32_t f = D.sxy[b], l = D.sxy[b + cnt[r] - 1];
-        xyf[s] = f;
-        xyl[s] = l;
-        atomicMin(&box_s[0], px_of(f));
-        atomicMax(&box_s[2], px_of(l));
+    for (int s0 = tid - lane; s0 < R; s0 += nt) {
+        const int s = s0 + lane;
+        int x0 = INT_MAX, x1 = INT_MIN;
+        if (s < R) {
+            const int r = ne[s], b = roff[r];
+            const uint32_t f = D.sxy[b], l = D.sxy[b + cnt[r] - 1];
+            xyf[s] = f;
+            xyl[s] = l;
+            flag[s] = 0;
+            x0 = px_of(f);
+            x1 = px_of(l);
+        }
+        x0 = __reduce_min_sync(0xffffffffu, x0);
+        x1 = __reduce_max_sync(0xffffffffu, x1);
+        if (lane == 0) {
+            atomicMin(&box_s[0], x0);
+            atomicMax(&box_s[1], x1);
+        }
     }
     __syncthreads();
-    if (tid == 0) {
-        const int32_t b[4] = {R ? box_s[0] : 0, R ? ney[0] : 0, R ? box_s[2] : 0, R ? ney[R - 1] : 0};
+    if (tid == nt - 1) {
+        const int32_t b[4] = {R ? box_s[0] : 0, R ? ney[0] : 0, R ? box_s[1] : 0, R ? ney[R - 1] : 0};
         for (int k = 0; k < 4; ++k) D.box[k] = b[k];
         D.box[4] = star_r0(b, npts);
     }
     if (R < 2) return;
-    // the chains, decided point by point and compacted in row order
+    // flag[i]: bit 0 on the left chain, bit 16 on the right one
+    const int hl = tid % HULL_LANES;
+    for (int it = tid / HULL_LANES; it < ((2 * R + 3) & ~3); it += nt / HULL_LANES) {   // whole warps
+        const int side = it & 1, i = imin(it >> 1, R - 1);
+        const uint32_t* xy = side ? xyl : xyf;
+        const uint32_t c = xy[i];
+        const int sg = side ? -1 : 1;
+        int32_t n0 = 1, e0 = 0, n1 = 1, e1 = 0;         // rows above and below; 1/0: +infinity
+#pragma unroll 4
+        for (int j = hl; j < R; j += HULL_LANES) {
+            const int32_t x = sg * dx_p(xy[j], c), y = dy_p(xy[j], c);
+            if (y < 0 && (e0 == 0 || x * e0 < n0 * -y)) { n0 = x; e0 = -y; }
+            if (y > 0 && (e1 == 0 || x * e1 < n1 * y)) { n1 = x; e1 = y; }
+        }
+#pragma unroll
+        for (int o = 1; o < HULL_LANES; o <<= 1) {
+            const int32_t m0 = __shfl_xor_sync(0xffffffffu, n0, o), f0 = __shfl_xor_sync(0xffffffffu, e0, o);
+            const int32_t m1 = __shfl_xor_sync(0xffffffffu, n1, o), f1 = __shfl_xor_sync(0xffffffffu, e1, o);
+            if (f0 != 0 && (e0 == 0 || m0 * e0 < n0 * f0)) { n0 = m0; e0 = f0; }
+            if (f1 != 0 && (e1 == 0 || m1 * e1 < n1 * f1)) { n1 = m1; e1 = f1; }
+        }
+        if (hl == 0 && it < 2 * R && (e0 == 0 || e1 == 0 || n0 * e1 + n1 * e0 >= 0))
+            atomicOr(&flag[i], side ? 1 << 16 : 1);
+    }
+    __syncthreads();
     int nl = 0, nr = 0;
     for (int b = 0; b < R; b += nt) {
-        const int i = b + tid;
-        const int fl = i < R && hull_on_chain(0, R, xyf, i) ? 1 : 0;
-        const int fr = i < R && hull_on_chain(1, R, xyl, i) ? 1 : 0;
-        int tl_ = 0, tr_ = 0;
-        const int pl = block_scan(fl, ws, &tl_);
-        const int pr = block_scan(fr, ws, &tr_);
-        if (fl) lstk[nl + pl] = i;
-        if (fr) rstk[nr + pr] = i;
-        nl += tl_;
-        nr += tr_;
+        const int i = b + tid, f = i < R ? flag[i] : 0;
+        int tot = 0;
+        const int pos = block_scan(f, ws, &tot);        // both chains' counts in one scan (below 2^16 each)
+        if (f & 0xffff) lstk[nl + (pos & 0xffff)] = i;
+        if (f >> 16) rstk[nr + (pos >> 16)] = i;
+        nl += tot & 0xffff;
+        nr += tot >> 16;
     }
     __syncthreads();
     const int tl = cnt[ne[0]], bl = cnt[ne[R - 1]];
@@ -268,20 +350,21 @@ __device__ void star_setup(const DelDev& D, const int32_t* roff, const int32_t* 
         return D.srt[roff[r] + (last ? cnt[r] - 1 : pos)];
     };
     for (int j = tid; j < C; j += nt) {
-        const int v = at(j);
-        D.hnext[v] = at(j + 1 == C ? 0 : j + 1);
-        D.hprev[v] = at(j == 0 ? C - 1 : j - 1);
+        const int v = at(j), a = at(j + 1 == C ? 0 : j + 1), b = at(j == 0 ? C - 1 : j - 1);
+        D.hnext[v] = a;
+        D.hprev[v] = b;
     }
 }
 
-// Non-empty rows (list, and their y for the star searches), then either the
-// star set-up (stars) or the strip offsets (flips).  One 1024-thread block
-// per problem; the per-row arrays are staged in shared memory (8 arrays of
-// nrows entries).  ctr[7] = 1 when the strip plan holds (two non-empty rows
-// at least, strips and pockets within Tmax); the strips and pockets are then
-// built by k_strips, which also sets the triangle count ctr[0].
+// Non-empty rows, then either the star set-up (stars) or the strip offsets
+// (flips).  One 1024-thread block per problem; the per-row arrays are staged
+// in shared memory (PLAN_ARRAYS arrays of nrows entries).  ctr[7] = 1 when
+// the strip plan holds (two non-empty rows at least, strips and pockets
+// within Tmax); the strips and pockets are then built by k_strips, which
+// also sets the triangle count ctr[0].
+constexpr int PLAN_ARRAYS = 9;
 __global__ void __launch_bounds__(1024) k_plan(DelDev d0, DelDev d1, const int32_t* __restrict__ row_off,
-                                               int nrows, int H, int flips, unsigned* err) {
+                                               int nrows, RowGeom rg, int flips, unsigned* err) {
     grid_dep_wait();
     __shared__ int ws[33];
     extern __shared__ int32_t psm[];
@@ -291,35 +374,32 @@ __global__ void __launch_bounds__(1024) k_plan(DelDev d0, DelDev d1, const int32
     int32_t* ney = psm + 3 * nrows;
     DelDev D = blockIdx.x ? d1 : d0;
     const int tid = threadIdx.x, nt = blockDim.x;
-    for (int r = tid; r < nrows; r += nt) {
-        roff[r] = row_off[r];
-        cnt[r] = D.rcnt[r];
-    }
-    __syncthreads();
+    const int npts = row_off[nrows];
     int R = 0, total = 0;
     // non-empty rows in order
     for (int r0 = 0; r0 < nrows; r0 += nt) {
         const int r = r0 + tid;
-        const int f = (r < nrows && cnt[r] > 0) ? 1 : 0;
+        int f = 0;
+        if (r < nrows) {
+            const int c = D.rcnt[r];
+            roff[r] = row_off[r];
+            cnt[r] = c;
+            f = c > 0 ? 1 : 0;
+        }
         const int pos = block_scan(f, ws, &total);
-        if (f) ne[R + pos] = r;
+        if (f) {
+            ne[R + pos] = r;
+            ney[R + pos] = rg.y(r);
+            if (flips) D.ne[R + pos] = r;
+        }
         R += total;
     }
     __syncthreads();
-    for (int s = tid; s < R; s += nt) {
-        const int r = ne[s];
-        const int y = D.y[roff[r]];
-        ney[s] = y;
-        D.ne[s] = r;
-        D.ne_y[s] = y;
-        D.rinfo[s] = make_int4(y, roff[r], cnt[r], 0);
-    }
-    __syncthreads();
-    const int npts = row_off[nrows];
     int off = 0;
     if (!flips) {
-        star_setup(D, roff, cnt, ne, ney, R, H, npts, reinterpret_cast<uint32_t*>(psm + 4 * nrows),
-                   reinterpret_cast<uint32_t*>(psm + 5 * nrows), psm + 6 * nrows, psm + 7 * nrows, ws);
+        star_setup(D, roff, cnt, ne, ney, R, npts, reinterpret_cast<uint32_t*>(psm + 4 * nrows),
+                   reinterpret_cast<uint32_t*>(psm + 5 * nrows), psm + 6 * nrows, psm + 7 * nrows, psm + 8 * nrows,
+                   ws);
     } else {
         // strip s between ne[s] and ne[s+1] holds cnt[ne[s]] + cnt[ne[s+1]] - 2 triangles
         for (int s0 = 0; s0 < R - 1; s0 += nt) {
@@ -341,149 +421,262 @@ __global__ void __launch_bounds__(1024) k_plan(DelDev d0, DelDev d1, const int32
         D.ctr[9] = npts;  // support points (vertex ids) of the problem
         D.ctr[4] = 0;    // flip rounds and flips (the flip kernels set them)
         D.ctr[5] = 0;
-        D.ctr[11] = 0;   // star construction: overflow pool cursor, searches beyond the window, windows grown
+        D.ctr[10] = 0;   // points left to k_star_far
+        D.ctr[11] = 0;   // star construction: overflow pool cursor, (unused), window doublings
         D.ctr[12] = 0;
         D.ctr[13] = 0;
     }
 }
 
 // ---------------------------------------------------------------------------
-// Star construction (delaunay_core.h, star_walk): one warp per point finds
-// the point's Delaunay neighbours directly, with no initial triangulation
-// and no flips.  Candidates come from the rows (ne_y gives each non-empty
-// row's y; a row's points are sorted by x with their packed coordinates in
-// sxy), gathered into shared memory per window; every search is a warp-wide
-// minimum under the star order, so its answer does not depend on how the
-// lanes split the candidates.
+// Star construction (delaunay_core.h, star_walk): every point's Delaunay
+// neighbours are found directly, with no initial triangulation and no
+// flips.  Every search is a minimum under a strict total order, so its
+// answer does not depend on how threads split the candidates, nor on which
+// points beyond the necessary ones were looked at.
+//
+// Bound by latency: a walk is a chain of some ten dependent steps, and the
+// slowest point's chain is the construction's time.  Nine points in ten have
+// their whole star within a small square, the others border large empty
+// regions and need points from far away.  Hence two kernels:
+//   * k_star, a warp per point: the candidates are the at most 64 points
+//     nearest around p, two per lane in registers, gathered once (a square
+//     of half-size R0, smaller where points are dense, larger where they are
+//     sparse).  The walk runs to its end on these alone, in fp32 (exact at
+//     such distances), then each lane proves one triangle.  A star that is
+//     not proven goes to a list.
+//   * k_star_far, a CTA per listed point: the certain triangles are kept,
+//     every other step looks at every point of the view.
+// One warp per point for everything, with a staged window and searches of
+// growing squares, took 54 us at 1242x375 and 399 us with the corner points
+// of add_corners; the two kernels 11 + 20 and 12 + 51 us.
 
 constexpr int STAR_WARPS = 8;      // points in flight per CTA
 constexpr int STAR_SLOT = 12;      // owned triangles kept in a point's own slot; more go to the pool
-
-// The star order as a float key: for the edge p->q (u = q - p) and a
-// candidate s (relative to p) strictly on the walk's side, the centre of
-// the circle through p, q, s lies at q/2 + t (-uy, ux) with
-// t = (|s|^2 - u.s) / (2 cross(u, s)); the next neighbour has the smallest
-// t on the left and the largest on the right, i.e. the smallest
-// (|s|^2 - u.s) / |cross(u, s)| on either side.  Numerator and denominator
-// are exact in int32 (below 2^31 at the coordinate limits of orient_p);
-// the key carries at most three roundings (two conversions, one division of
-// at most 2 ulp), a relative error below 4e-7, so keys further apart than
-// 4e-6 of the larger order their points correctly and closer ones are
-// compared exactly.
-__device__ __forceinline__ bool star_key(int32_t ux, int32_t uy, int32_t sx, int32_t sy, int side, float* key) {
-    const int32_t cr = ux * sy - uy * sx;           // orient(p, q, s)
-    if (side > 0 ? cr <= 0 : cr >= 0) return false;
-    const int32_t num = sx * sx + sy * sy - (ux * sx + uy * sy);
-    *key = __fdividef(__int2float_rn(num), __int2float_rn(cr > 0 ? cr : -cr));
-    return true;
-}
+constexpr int STAR_LANE = 2;       // candidates per lane
+constexpr int STAR_CAND = 32 * STAR_LANE;
+constexpr int FAR_REC = DelDev::FAR_REC;   // ints of a listed point's record: point, counts, proofs, neighbours
 
 struct StarSmem {
-    int32_t cid[STAR_CAP];         // the point's window: point index
-    uint32_t cxy[STAR_CAP];        // and packed coordinates
-    int32_t ccw[STAR_NB];          // the walk's two neighbour lists
-    int32_t cw[STAR_NB];
+    int32_t nb[STAR_NB];           // the star's neighbours in counter-clockwise order
+    uint32_t nxy[STAR_NB];
 };
 
-__device__ __forceinline__ unsigned long long warp_min_u64(unsigned long long v) {
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-        const unsigned long long w = __shfl_xor_sync(0xffffffffu, v, o);
-        v = w < v ? w : v;
-    }
-    return v;
+struct StarEdge {                  // the walk's current edge p -> q
+    int p, q;
+    uint32_t pp, pq;
+    int32_t ux, uy;
+};
+struct StarBest {                  // best next neighbour so far (i < 0: none)
+    int i;
+    uint32_t xy;
+    float k;
+};
+
+// The star order as a float key: for the edge p->q (u = q - p) and a
+// candidate s (relative to p) strictly left of it, the centre of the circle
+// through p, q, s lies at q/2 + t (-uy, ux) with t = (|s|^2 - u.s) /
+// (2 cross(u, s)); the next neighbour has the smallest t.  Numerator and
+// denominator are exact in int32 (below 2^31 at the coordinate limits of
+// orient_p); the key carries at most three roundings (two conversions, one
+// division of at most 2 ulp), a relative error below 4e-7, so keys further
+// apart than 4e-6 of the larger order their points correctly and closer
+// ones are compared exactly.
+constexpr float STAR_KEY_TOL = 4e-6f;
+
+// Out of line: rarely reached and long, and the kernels' chains wait for
+// instruction fetches as well as for data.
+__device__ __noinline__ bool star_exact(int p, uint32_t pp, int q, uint32_t pq, int a, uint32_t axy, int b,
+                                        uint32_t bxy) {
+    return star_better_left(p, pp, q, pq, a, axy, b, bxy);
 }
 
-// Every point of a region, spread evenly over the warp's lanes: each lane
-// takes a row (ylut gives the rows of the region's y range, rinfo each
-// row's y, first position and count in one 16-byte load), finds the
-// row's column ranges (one, or two beside a ring's hole) by binary search
-// in the row's sorted coordinates, and the ranges of 32 rows are then dealt
-// out one point per lane (a lane finds the row of its point by a binary
-// search over the lanes' offsets).
-// take(index, packed xy, k) receives each point with its running number k.
-template <class Take>
-__device__ void star_stream(const DelDev& D, const int32_t* __restrict__ row_off, const StarRegion& g,
-                            const int32_t* box, int lane, Take&& take) {
-    if (g.y0 > g.y1) return;
-    const int s0 = D.ylut[g.y0], s1 = D.ylut[g.y1 + 1];
-    int done = 0;
-    // positions [lo, hi) of the row's sorted points with x in [x0, x1]
-    auto range = [&](const uint32_t* xs, int cnt, int32_t x0, int32_t x1, int* b, int* n) {
-        int l = 0, h = cnt;
-        while (l < h) {
-            const int mid = (l + h) >> 1;
-            if (px_of(xs[mid]) < x0) l = mid + 1;
-            else h = mid;
+__device__ __forceinline__ void star_take(const StarEdge& e, StarBest& best, int s, uint32_t sxy) {
+    const int32_t sx = dx_p(sxy, e.pp), sy = dy_p(sxy, e.pp);
+    const int32_t cr = e.ux * sy - e.uy * sx;           // orient(p, q, s)
+    if (cr <= 0) return;
+    const float k = __fdividef(__int2float_rn(sx * sx + sy * sy - (e.ux * sx + e.uy * sy)), __int2float_rn(cr));
+    if (best.i >= 0) {
+        const float tol = STAR_KEY_TOL * fmaxf(fabsf(best.k), fabsf(k));
+        if (k > best.k + tol) return;
+        if (k >= best.k - tol &&
+            (sxy == best.xy || !star_exact(e.p, e.pp, e.q, e.pq, best.i, best.xy, s, sxy)))
+            return;
+    }
+    best.i = s;
+    best.xy = sxy;
+    best.k = k;
+}
+
+// The minimum over the lanes' bests, in every lane: the smallest key (one
+// reduction over order-preserving key bits), then the lanes within the
+// keys' rounding of it one by one, exactly.  A lane's other candidates need
+// no look: each is worse than its lane's best.
+__device__ __forceinline__ void star_reduce(const StarEdge& e, StarBest& best, int lane) {
+    const uint32_t kb = __float_as_uint(best.k);
+    const uint32_t u = best.i < 0 ? 0xffffffffu : ((kb & 0x80000000u) ? ~kb : (kb | 0x80000000u));
+    const uint32_t umin = __reduce_min_sync(0xffffffffu, u);
+    if (umin == 0xffffffffu) return;            // no lane holds a candidate
+    const int wl = __ffs(__ballot_sync(0xffffffffu, u == umin)) - 1;
+    StarBest w;
+    w.i = __shfl_sync(0xffffffffu, best.i, wl);
+    w.xy = __shfl_sync(0xffffffffu, best.xy, wl);
+    w.k = __shfl_sync(0xffffffffu, best.k, wl);
+    const bool tie = best.i >= 0 && best.xy != w.xy &&
+                     fabsf(best.k - w.k) <= STAR_KEY_TOL * fmaxf(fabsf(best.k), fabsf(w.k));
+    for (unsigned m = __ballot_sync(0xffffffffu, tie); m; m &= m - 1) {
+        const int j = __ffs(m) - 1;
+        const int ci = __shfl_sync(0xffffffffu, best.i, j);
+        const uint32_t cxy = __shfl_sync(0xffffffffu, best.xy, j);
+        const float ck = __shfl_sync(0xffffffffu, best.k, j);
+        if (cxy != w.xy && star_exact(e.p, e.pp, e.q, e.pq, w.i, w.xy, ci, cxy)) {
+            w.i = ci;
+            w.xy = cxy;
+            w.k = ck;
         }
-        const int lb = l;
-        h = cnt;
-        while (l < h) {
-            const int mid = (l + h) >> 1;
-            if (px_of(xs[mid]) <= x1) l = mid + 1;
-            else h = mid;
-        }
-        *b = lb;
-        *n = l - lb;
+    }
+    best = w;
+}
+
+// circle_inside in 64-bit floats, for the few triangles that need it (its
+// dependent 64-bit operations take over a thousand cycles).
+__device__ __noinline__ bool star_proven(uint32_t pp, uint32_t pq, uint32_t pr, int R, const int32_t* box) {
+    return circle_inside(pp, pq, pr, R, box);
+}
+
+// In fp32: 1 when the whole circle through p, q and r lies in the square of
+// half-size R by more than the rounding, -1 when it leaves it by more than
+// the rounding, 0 otherwise.  With |q|, |r| <= 2 rho, |q - r| >= 1 the centre
+// is off by less than 5e-7 rho^2 (two products of a coordinate and a squared
+// length, each rounded once, over the exact determinant) and the rest by
+// 1e-6 of the extent.
+__device__ __forceinline__ int star_circle_fits(uint32_t pp, uint32_t pq, uint32_t pr, int R) {
+    const int32_t qx = dx_p(pq, pp), qy = dy_p(pq, pp), rx = dx_p(pr, pp), ry = dy_p(pr, pp);
+    const float q2 = float(qx * qx + qy * qy), r2 = float(rx * rx + ry * ry);
+    const float d = 2.0f * float(qx * ry - qy * rx);
+    const float cx = __fdividef(float(ry) * q2 - float(qy) * r2, d);
+    const float cy = __fdividef(float(qx) * r2 - float(rx) * q2, d);
+    const float rho2 = cx * cx + cy * cy;
+    const float ext = fmaxf(fabsf(cx), fabsf(cy)) + sqrtf(rho2);
+    const float mg = 0.25f + 2e-6f * ext + 1e-6f * rho2;
+    return ext + mg <= float(R) ? 1 : (ext - mg > float(R) ? -1 : 0);
+}
+// circle_inside: a circle that leaves the square can only be proven by its
+// part inside the box of all points, which needs a square that reaches past
+// the box (rim).
+__device__ __forceinline__ bool star_inside(uint32_t pp, uint32_t pq, uint32_t pr, int R, bool rim,
+                                            const int32_t* box) {
+    const int fit = star_circle_fits(pp, pq, pr, R);
+    return fit > 0 || ((fit == 0 || rim) && star_proven(pp, pq, pr, R, box));
+}
+
+// One row's points between columns x0 and x1 (and at most seven columns
+// more on either side, the buckets' width): first position and count.
+__device__ __forceinline__ void star_cols(const DelDev& D, int xbs, int row, int x0, int x1, int* b, int* n) {
+    const int32_t* xb = D.xb + size_t(row) * xbs;
+    *b = xb[imin(imax(x0 >> 3, 0), xbs - 2)];
+    *n = xb[imin(imax(x1 >> 3, 0), xbs - 2) + 1] - *b;
+}
+
+__device__ __forceinline__ int warp_excl_scan(int n, int lane) {
+    int incl = n;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const int y = __shfl_up_sync(0xffffffffu, incl, o);
+        if (lane >= o) incl += y;
+    }
+    return incl - n;
+}
+
+__device__ __forceinline__ float redux_min_f32(float v) {
+    float r;
+    asm volatile("redux.sync.min.f32 %0, %1, 0xffffffff;" : "=f"(r) : "f"(v));
+    return r;
+}
+
+// Store the owned triangles of p's star (a warp; the nt triangles of the
+// list nb of deg neighbours of which p is the smallest vertex): their number
+// in tcnt[p], their vertex pairs in p's slot, or in the pool when more than
+// STAR_SLOT.
+__device__ __forceinline__ void star_output(const DelDev& D, int p, const int32_t* nb, int deg, int nt, int lane,
+                                            unsigned* err) {
+    auto owned = [&](int i, int* a, int* c) {
+        if (i >= nt) return false;
+        *a = nb[i];
+        *c = nb[i + 1 == deg ? 0 : i + 1];
+        return p < *a && p < *c;
     };
-    for (int sb = s0; sb < s1; sb += 32) {
-        const int srow = sb + lane;
-        int b = 0, n0 = 0, b1 = 0, n1 = 0;
-        if (srow < s1) {
-            const int4 ri = D.rinfo[srow];      // y, first position, unique points
-            int32_t x0, x1, x2, x3;
-            g.cols2(ri.x, box, &x0, &x1, &x2, &x3);
-            if (x0 <= x1 || x2 <= x3) {
-                const int base = ri.y, cnt = ri.z;
-                const uint32_t* xs = D.sxy + base;
-                if (x0 <= x1) {
-                    range(xs, cnt, x0, x1, &b, &n0);
-                    b += base;
-                }
-                if (x2 <= x3) {
-                    range(xs, cnt, x2, x3, &b1, &n1);
-                    b1 += base;
-                }
-            }
-        }
-        const int n = n0 + n1;
-        int incl = n;
-#pragma unroll
-        for (int o = 1; o < 32; o <<= 1) {
-            const int y = __shfl_up_sync(0xffffffffu, incl, o);
-            if (lane >= o) incl += y;
-        }
-        const int tot = __shfl_sync(0xffffffffu, incl, 31), excl = incl - n;
-        for (int kb = 0; kb < tot; kb += 32) {
-            const int k = kb + lane;
-            int j = 0;
-#pragma unroll
-            for (int st = 16; st > 0; st >>= 1) {
-                const int c = j + st;
-                const int e = __shfl_sync(0xffffffffu, excl, c & 31);
-                if (c < 32 && e <= k) j = c;
-            }
-            const int jb = __shfl_sync(0xffffffffu, b, j), je = __shfl_sync(0xffffffffu, excl, j);
-            const int jn0 = __shfl_sync(0xffffffffu, n0, j), jb1 = __shfl_sync(0xffffffffu, b1, j);
-            if (k < tot) {
-                const int o = k - je;
-                const int pos = o < jn0 ? jb + o : jb1 + (o - jn0);
-                take(D.srt[pos], D.sxy[pos], done + k);
-            }
-        }
-        done += tot;
+    int a = 0, c = 0;
+    bool o = owned(lane, &a, &c);
+    unsigned bal = __ballot_sync(0xffffffffu, o);
+    int own = __popc(bal);
+    for (int t = 32; t < nt; t += 32) {
+        int a2, c2;
+        own += __popc(__ballot_sync(0xffffffffu, owned(t + lane, &a2, &c2)));
     }
+    int32_t* dst = D.sown + size_t(p) * 2 * STAR_SLOT;
+    if (own > STAR_SLOT) {
+        int base = 0;
+        if (lane == 0) base = atomicAdd(&D.ctr[11], own);
+        base = __shfl_sync(0xffffffffu, base, 0);
+        if (base + own > D.Tmax) {
+            if (lane == 0) set_err(err, ERRF_BOUNDS);
+            own = 0;
+        } else {
+            if (lane == 0) dst[0] = base;
+            dst = D.spool + 2 * size_t(base);
+        }
+    }
+    if (own > 0) {
+        int pos = 0;
+        for (int t = 0;;) {
+            if (o) {
+                const int j = pos + __popc(bal & ((1u << lane) - 1u));
+                *reinterpret_cast<int2*>(dst + 2 * j) = make_int2(a, c);
+            }
+            t += 32;
+            if (t >= nt) break;
+            pos += __popc(bal);
+            o = owned(t + lane, &a, &c);
+            bal = __ballot_sync(0xffffffffu, o);
+        }
+    }
+    if (lane == 0) D.tcnt[p] = own;
 }
 
-// Grid-stride over (point, view) with one warp per point: the star
-// (star_walk with the two-phase searches of the search policy), its owned
-// triangles (p the smallest vertex) counted into tcnt[p] and stored as
-// vertex pairs in p's slot (or in the pool when more than STAR_SLOT).
-// Three CTAs per SM (80 registers a thread): measured faster at 1242x375
-// than four (64 registers, more spills) and than two (no spills, but the
-// points no longer fit one wave).
-__global__ void __launch_bounds__(STAR_WARPS * 32, 3) k_star(DelDev d0, DelDev d1,
-                                                           const int32_t* __restrict__ row_off, unsigned* err) {
+// The doublings of the window's half-size R0 until the square proves p's
+// whole star (what a search by growing squares would have made), by a warp:
+// its nt triangles of the deg neighbours at nxy, the start at squared
+// distance qd2 (0: a hull point's successor, which needs no proof) and, with
+// `open`, a hull edge that only a square over the whole box proves.  Lane =
+// item * 4 + level: eight items at four sizes at a time, as a test in 64-bit
+// floats takes over a thousand cycles.
+__device__ int star_doublings(const DelDev& D, uint32_t pp, const uint32_t* nxy, int deg, int nt, uint32_t qd2,
+                              bool open, int lane) {
+    const int px = px_of(pp), py = py_of(pp);
+    int most = 0;
+    for (int t = 0; t <= nt; t += 8) {
+        const int i = t + (lane >> 2);
+        for (int l0 = 0;; l0 += 4) {
+            const int R = D.box[4] << (l0 + (lane & 3));
+            const bool w = px - R <= D.box[0], n = py - R <= D.box[1], e = px + R >= D.box[2], s = py + R >= D.box[3];
+            bool pass = (w && n && e && s) || i > nt;
+            if (!pass)
+                pass = i == nt ? !open && qd2 <= uint32_t(R) * uint32_t(R)
+                               : star_inside(pp, nxy[i], nxy[i + 1 == deg ? 0 : i + 1], R, w || n || e || s, D.box);
+            const unsigned nib = (__ballot_sync(0xffffffffu, pass) >> (lane & 28)) & 15u;
+            if (nib) most = imax(most, l0 + __ffs(nib) - 1);
+            if (__all_sync(0xffffffffu, nib != 0u)) break;
+        }
+    }
+    return __reduce_max_sync(0xffffffffu, most);
+}
+
+// Grid-stride over (point, view) with one warp per point: the star from the
+// points around p, stored if it is proven, else p joins the list of
+// k_star_far.
+__global__ void __launch_bounds__(STAR_WARPS * 32, 3) k_star(DelDev d0, DelDev d1, int nrows, RowGeom rg, int xbs,
+                                                             unsigned* err) {
     grid_dep_wait();
     __shared__ StarSmem smem[STAR_WARPS];
     // blockIdx.x is the view, so that the two views' first blocks (the ones
@@ -500,253 +693,327 @@ __global__ void __launch_bounds__(STAR_WARPS * 32, 3) k_star(DelDev d0, DelDev d
             if (lane == 0) D.tcnt[p] = 0;
             continue;
         }
-        const int px = px_of(pp), py = py_of(pp);
         const int hn = D.hnext[p], hp = D.hprev[p];
-        int circles = 0, squares = 0;
-        // phase 1: the window, staged once (streamed again by each search if it holds more than STAR_CAP)
-        const StarRegion win = star_square_region(pp, R0, box);
-        int K = 0;
-        star_stream(D, row_off, win, box, lane, [&](int32_t s, uint32_t sxy, int k) {
-            if (k < STAR_CAP) {
-                sm.cid[k] = s;
-                sm.cxy[k] = sxy;
-            }
-            K = k + 1;
-        });
-        K = __reduce_max_sync(0xffffffffu, K);
-        __syncwarp();
-        const bool staged = K <= STAR_CAP;
-        // the window grows (and stays grown for the point's later searches)
-        // while its rings fit behind the staged points
-        int Rw = R0;
-        bool ring_full = !staged;
-        auto grow = [&](auto&& take) {
-            ++squares;
-            int T = 0;
-            star_stream(D, row_off, star_ring_region(pp, Rw, box), box, lane, [&](int32_t s, uint32_t sxy, int k) {
-                take(s, sxy);
-                if (K + k < STAR_CAP) {
-                    sm.cid[K + k] = s;
-                    sm.cxy[K + k] = sxy;
-                }
-                T = k + 1;
-            });
-            T = __reduce_max_sync(0xffffffffu, T);
-            __syncwarp();
-            if (K + T > STAR_CAP) {
-                ring_full = true;
-                return false;
-            }
-            K += T;
-            Rw *= 2;
-            return true;
-        };
-        auto window = [&](auto&& take) {
-            if (staged) {
-                for (int k = lane; k < K; k += 32) take(sm.cid[k], sm.cxy[k]);
-            } else {
-                star_stream(D, row_off, win, box, lane, [&](int32_t s, uint32_t sxy, int) { take(s, sxy); });
-            }
-        };
+        const uint32_t hnxy = hn >= 0 ? D.pxy[hn] : PXY_NONE, hpxy = hp >= 0 ? D.pxy[hp] : PXY_NONE;
+        const int px = px_of(pp), py = py_of(pp);
         auto covers = [&](int Rs) {
             return px - Rs <= box[0] && px + Rs >= box[2] && py - Rs <= box[1] && py + Rs >= box[3];
         };
-        // coordinates of the walk's start (q0) and of the last neighbour
-        // found, so a step need not load its edge's far end again
-        int c0 = hn, c1 = -1;
-        uint32_t x0c = hn >= 0 ? D.pxy[hn] : 0u, x1c = 0u;
-        auto nearest = [&]() -> int {
-            unsigned long long best = ~0ull;
-            uint32_t nxy = 0;
-            auto take = [&](int32_t s, uint32_t sxy) {
-                if (s == p) return;
-                const int32_t dx = dx_p(sxy, pp), dy = dy_p(sxy, pp);
-                const unsigned long long key = uint64_t(uint32_t(dx * dx + dy * dy)) << 32 | uint32_t(s);
-                if (key < best) {
-                    best = key;
-                    nxy = sxy;
-                }
-            };
-            auto take3 = [&](int32_t s, uint32_t sxy, int) { take(s, sxy); };
-            auto finish = [&]() {
-                const unsigned long long g = warp_min_u64(best);
-                const int wl = __ffs(__ballot_sync(0xffffffffu, best == g)) - 1;
-                nxy = __shfl_sync(0xffffffffu, nxy, wl < 0 ? 0 : wl);
-                best = g;
-            };
-            window(take);
-            finish();
-            for (int Rs = Rw;;) {
-                const uint64_t d2 = best >> 32;
-                if (best != ~0ull && d2 <= uint64_t(Rs) * uint64_t(Rs)) break;
-                if (covers(Rs)) break;
-                if (Rs == Rw && !ring_full) {
-                    Rs = grow(take) ? Rw : 2 * Rs;
-                    finish();
-                    continue;
-                }
-                if (best != ~0ull) {
-                    // the nearest lies within distance sqrt(d2): the square of that half-size
-                    int d = int(sqrt(double(d2)));
-                    while (uint64_t(d) * uint64_t(d) < d2) ++d;
-                    ++circles;
-                    best = ~0ull;
-                    star_stream(D, row_off, star_square_region(pp, d, box), box, lane, take3);
-                    finish();
-                    break;
-                }
-                Rs = star_square(Rs);
-                ++squares;
-                star_stream(D, row_off, star_square_region(pp, Rs, box), box, lane, take3);
-                finish();
-            }
-            if (best == ~0ull) return -1;
-            c0 = int(uint32_t(best));
-            x0c = nxy;
-            return c0;
-        };
-        auto next = [&](int q, int side) -> int {
-            const uint32_t pq = q == c1 ? x1c : (q == c0 ? x0c : D.pxy[q]);
-            const int32_t ux = dx_p(pq, pp), uy = dy_p(pq, pp);
-            int bi = -1;
-            uint32_t bxy = 0;
-            float bk = 0.0f;
-            // b replaces a (keys ka, kb) under the star order: decided by the
-            // keys when they differ by more than their rounding can explain,
-            // else exactly (star_better)
-            auto wins = [&](float ka, int a, uint32_t axy, float kb, int b, uint32_t bxy2) {
-                const float m = 4e-6f * fmaxf(fabsf(ka), fabsf(kb));
-                if (kb < ka - m) return true;
-                if (kb > ka + m) return false;
-                return star_better(p, pp, q, pq, a, axy, b, bxy2, side);
-            };
-            auto take = [&](int32_t s, uint32_t sxy) {
-                float k;
-                if (!star_key(ux, uy, dx_p(sxy, pp), dy_p(sxy, pp), side, &k)) return;
-                if (bi < 0 || wins(bk, bi, bxy, k, s, sxy)) {
-                    bi = s;
-                    bxy = sxy;
-                    bk = k;
-                }
-            };
-            auto take3 = [&](int32_t s, uint32_t sxy, int) { take(s, sxy); };
-            // Minimum under the star order over the lanes' bests.  Fast path:
-            // the smallest key (one reduction over order-preserving key
-            // bits), final unless another lane's best lies within the keys'
-            // rounding of it; then a butterfly decides exactly (the order is
-            // strict and total, so every lane ends with the same point).  A
-            // lane's other candidates need no look: each is worse than its
-            // lane's best, which the winner beats.
-            auto reduce = [&]() {
-                const uint32_t kb = __float_as_uint(bk);
-                const uint32_t u = bi < 0 ? 0xffffffffu : ((kb & 0x80000000u) ? ~kb : (kb | 0x80000000u));
-                const uint32_t umin = __reduce_min_sync(0xffffffffu, u);
-                if (umin == 0xffffffffu) return;            // no lane holds a candidate
-                const int wl = __ffs(__ballot_sync(0xffffffffu, u == umin)) - 1;
-                const int wi = __shfl_sync(0xffffffffu, bi, wl);
-                const uint32_t wxy = __shfl_sync(0xffffffffu, bxy, wl);
-                const float wk = __shfl_sync(0xffffffffu, bk, wl);
-                const bool tie = bi >= 0 && bi != wi && fabsf(bk - wk) <= 4e-6f * fmaxf(fabsf(bk), fabsf(wk));
-                if (__ballot_sync(0xffffffffu, tie) == 0u) {
-                    bi = wi;
-                    bxy = wxy;
-                    bk = wk;
-                    return;
-                }
-#pragma unroll
-                for (int o = 16; o > 0; o >>= 1) {
-                    const int oi = __shfl_xor_sync(0xffffffffu, bi, o);
-                    const uint32_t oxy = __shfl_xor_sync(0xffffffffu, bxy, o);
-                    const float ok = __shfl_xor_sync(0xffffffffu, bk, o);
-                    if (oi >= 0 && oi != bi && (bi < 0 || wins(bk, bi, bxy, ok, oi, oxy))) {
-                        bi = oi;
-                        bxy = oxy;
-                        bk = ok;
+        // The candidates: the points of a square of half-size r (a lane per
+        // row), r found from R0 by the points it holds.
+        int r = R0, b = 0, n = 0, K = 0;
+        bool shrunk = false, trusted = true;
+        for (int it = 0;; ++it) {
+            // the rows from py - r to py + r (and the corners' extra row when it may be one of them)
+            const int s0 = imin(rg.row(imax(py - r, 0) + rg.step - 1), nrows - 1);
+            const int s1 = rg.crow >= 0 && py + r >= rg.H - 1 ? nrows : imin(rg.row(py + r) + 1, nrows);
+            n = 0;
+            if (s1 - s0 <= 32) {
+                if (s0 + lane < s1) {
+                    star_cols(D, xbs, s0 + lane, px - r, px + r, &b, &n);
+                    if (r <= 8) {               // the buckets' width counts here
+                        while (n > 0 && px_of(D.sxy[b]) < px - r) { ++b; --n; }
+                        while (n > 0 && px_of(D.sxy[b + n - 1]) > px + r) --n;
                     }
                 }
-            };
-            window(take);
-            reduce();
-            for (int Rs = Rw;;) {
-                if (bi >= 0 && circle_inside(pp, pq, bxy, Rs, box)) break;
-                if (covers(Rs)) break;
-                if (Rs == Rw && !ring_full) {
-                    Rs = grow(take) ? Rw : 2 * Rs;
-                    reduce();
-                    continue;
+                K = __reduce_add_sync(0xffffffffu, n);
+            } else {
+                K = STAR_CAND + 1;
+            }
+            if (K > STAR_CAND) {
+                if (it >= 24 || r <= 2) { trusted = false; break; }
+                const int rs = s1 - s0 > 32 ? r * 3 / 5 : int(float(r) * sqrtf(44.0f / float(K)));
+                r = imax(2, imin(rs, r - 1));
+                shrunk = true;
+            } else if (K < 20 && !shrunk && it < 3 && !covers(r)) {
+                r *= 2;
+            } else {
+                break;
+            }
+        }
+        // dealt out over the lanes, two slots each (slot = lane + 32 c): the
+        // rows' positions are laid end to end in shared memory
+        int cid[STAR_LANE];
+        uint32_t cxy[STAR_LANE];
+        float fx[STAR_LANE], fy[STAR_LANE], fn[STAR_LANE];     // relative to p; squared length, 0 for p and empty slots
+        {
+            const int excl = warp_excl_scan(n, lane);
+            if (!trusted) K = n = 0;
+            for (int i = 0; i < n; ++i) sm.nb[excl + i] = b + i;
+            __syncwarp();
+#pragma unroll
+            for (int c = 0; c < STAR_LANE; ++c) {
+                const int k = lane + 32 * c;
+                const bool in = k < K;
+                const int pos = in ? sm.nb[k] : 0;
+                cid[c] = in ? D.srt[pos] : -1;
+                cxy[c] = in ? D.sxy[pos] : pp;
+                const int dx = dx_p(cxy[c], pp), dy = dy_p(cxy[c], pp);
+                fx[c] = float(dx);
+                fy[c] = float(dy);
+                fn[c] = float(dx * dx + dy * dy);
+            }
+            __syncwarp();
+        }
+        auto slot_of = [&](uint32_t xy) {       // the candidates' slot of a point, -1: not among them
+            const unsigned m0 = __ballot_sync(0xffffffffu, cid[0] >= 0 && cxy[0] == xy);
+            const unsigned m1 = __ballot_sync(0xffffffffu, cid[1] >= 0 && cxy[1] == xy);
+            return m0 ? __ffs(m0) - 1 : (m1 ? 31 + __ffs(m1) : -1);
+        };
+        auto id_at = [&](int slot) { return __shfl_sync(0xffffffffu, slot & 32 ? cid[1] : cid[0], slot & 31); };
+        auto xy_at = [&](int slot) { return __shfl_sync(0xffffffffu, slot & 32 ? cxy[1] : cxy[0], slot & 31); };
+        const bool whole = trusted && covers(r);
+        // the square reaches past the box of all points: a circle that leaves
+        // the square may still be proven by its part inside the box
+        const bool rim = px - r < box[0] || px + r > box[2] || py - r < box[1] || py + r > box[3];
+        // The walk's start.  A hull point whose successor is not among the
+        // candidates cannot be finished here; it walks from its nearest
+        // neighbour for the record's sake.
+        int q0slot = hn >= 0 ? slot_of(hnxy) : -1;
+        const bool adrift = hn >= 0 && q0slot < 0;
+        if (q0slot < 0) {
+            // nearest neighbour, the lowest index among equals
+            const float l0 = fn[0] > 0.0f ? fn[0] : INFINITY, l1 = fn[1] > 0.0f ? fn[1] : INFINITY;
+            const float lm = redux_min_f32(fminf(l0, l1));
+            if (lm < INFINITY && (whole || lm <= float(r * r))) {
+                const int i0 = l0 == lm ? cid[0] : INT_MAX, i1 = l1 == lm ? cid[1] : INT_MAX;
+                const int q0 = __reduce_min_sync(0xffffffffu, imin(i0, i1));
+                const unsigned m0 = __ballot_sync(0xffffffffu, i0 == q0), m1 = __ballot_sync(0xffffffffu, i1 == q0);
+                q0slot = m0 ? __ffs(m0) - 1 : 31 + __ffs(m1);
+            }
+        }
+        // The walk on the candidates: lane i keeps neighbour i (up to 32).
+        // Coordinates within the square are small enough (r stays below
+        // 2048) that cross products and numerators are exact in fp32, so a
+        // step is two keys, one reduction and a vote.
+        int m = 0, nb = 0;                  // neighbours listed; the lane's: its slot, then its index
+        bool closed = false, full = false;
+        if (q0slot >= 0 && trusted) {
+            const int hpslot = hp >= 0 ? slot_of(hpxy) : -1;
+            int slot = q0slot;
+            for (;;) {
+                if (lane == m) nb = slot;
+                ++m;
+                if (m > 1 && slot == hpslot) { full = !adrift; break; }
+                if (m == 32) break;
+                const float ux = __shfl_sync(0xffffffffu, slot & 32 ? fx[1] : fx[0], slot & 31);
+                const float uy = __shfl_sync(0xffffffffu, slot & 32 ? fy[1] : fy[0], slot & 31);
+                float k[STAR_LANE];
+#pragma unroll
+                for (int c = 0; c < STAR_LANE; ++c) {
+                    const float cr = ux * fy[c] - uy * fx[c];
+                    const float num = fn[c] - (ux * fx[c] + uy * fy[c]);
+                    k[c] = cr > 0.0f ? __fdividef(num, cr) : INFINITY;
                 }
-                int need = 0;
-                if (bi >= 0) circle_within(pp, pq, bxy, Rs, box, &need);
-                if (bi >= 0 && need <= 2 * Rs) {
-                    ++circles;
-                    star_stream(D, row_off, star_circle_region(pp, pq, bxy, box), box, lane, take3);
-                    reduce();
+                const float km = redux_min_f32(fminf(k[0], k[1]));
+                if (km == INFINITY) break;
+                const float lim = km + 2.0f * STAR_KEY_TOL * fabsf(km);
+                unsigned m0 = __ballot_sync(0xffffffffu, k[0] <= lim), m1 = __ballot_sync(0xffffffffu, k[1] <= lim);
+                int ws = m0 ? __ffs(m0) - 1 : 31 + __ffs(m1);
+                if (__popc(m0) + __popc(m1) > 1) {
+                    // equal within the keys' rounding: exactly, one by one
+                    const int q = id_at(slot);
+                    const uint32_t pq = xy_at(slot);
+                    if (m0) m0 &= m0 - 1;
+                    else m1 &= m1 - 1;
+                    int wi = id_at(ws);
+                    uint32_t wxy = xy_at(ws);
+                    while (m0 | m1) {
+                        const int cs = m0 ? __ffs(m0) - 1 : 31 + __ffs(m1);
+                        if (m0) m0 &= m0 - 1;
+                        else m1 &= m1 - 1;
+                        const int ci = id_at(cs);
+                        const uint32_t cx = xy_at(cs);
+                        if (star_exact(p, pp, q, pq, wi, wxy, ci, cx)) { ws = cs; wi = ci; wxy = cx; }
+                    }
+                }
+                slot = ws;
+                if (slot == q0slot) { closed = full = hn < 0; break; }
+            }
+        }
+        // every triangle's proof at once
+        uint32_t nxy, sure;
+        {
+            const int li = nb & 31;
+            const int i0 = __shfl_sync(0xffffffffu, cid[0], li), i1 = __shfl_sync(0xffffffffu, cid[1], li);
+            const uint32_t x0 = __shfl_sync(0xffffffffu, cxy[0], li), x1 = __shfl_sync(0xffffffffu, cxy[1], li);
+            const bool up = (nb & 32) != 0;
+            nb = up ? i1 : i0;
+            nxy = up ? x1 : x0;
+            const uint32_t next = __shfl_sync(0xffffffffu, nxy, lane + 1 == m ? 0 : lane + 1);
+            const int nt = star_tris(m, closed);
+            const bool in = lane < nt;
+            sure = __ballot_sync(0xffffffffu, in && (whole || star_inside(pp, nxy, next, r, rim, D.box)));
+            full = full && sure == (nt >= 32 ? 0xffffffffu : (1u << nt) - 1u);
+        }
+        if (full) {
+            sm.nb[lane] = nb;
+            sm.nxy[lane] = nxy;
+            __syncwarp();
+            const int nt = star_tris(m, closed);
+            if (r > R0) {
+                const uint32_t q = __shfl_sync(0xffffffffu, nxy, 0);
+                const int dx = dx_p(q, pp), dy = dy_p(q, pp);
+                const uint32_t qd2 = hn >= 0 ? 0u : uint32_t(dx * dx + dy * dy);
+                const int g = star_doublings(D, pp, sm.nxy, m, nt, qd2, false, lane);
+                if (lane == 0 && g) atomicAdd(&D.ctr[13], g);
+            }
+            star_output(D, p, sm.nb, m, nt, lane, err);
+        } else {
+            // what is known of the star goes along: the neighbours listed and which triangles are certain
+            int at = 0;
+            if (lane == 0) at = atomicAdd(&D.ctr[10], 1);
+            at = __shfl_sync(0xffffffffu, at, 0);
+            int32_t* rec = D.far + size_t(at) * FAR_REC;
+            const int known = m <= FAR_REC - 3 ? m : 0;
+            if (lane == 0) {
+                rec[0] = p;
+                rec[1] = known | (closed ? 1 << 8 : 0) | (adrift ? 1 << 9 : 0);
+                rec[2] = int32_t(sure);
+            }
+            if (lane < known) rec[3 + lane] = nb;
+        }
+        __syncwarp();
+    }
+}
+
+// The minimum of a step over the CTA's lanes, in every thread: per warp,
+// then over the warps' results in `part`, which the caller alternates
+// between two arrays from step to step (so one barrier a step is enough).
+template <class Reduce, class T>
+__device__ __forceinline__ void star_cta_min(T& v, T* part, int lane, int warp, int nwarps, const T& none,
+                                             Reduce reduce) {
+    reduce(v);
+    if (lane == 0) part[warp] = v;
+    __syncthreads();
+    v = lane < nwarps ? part[lane] : none;
+    reduce(v);
+}
+
+// The listed points, a CTA each: a certain triangle of the record is taken
+// as it is; every other step starts from a guess (the record's next
+// neighbour, or none) and looks at every point of the view; only if one is
+// better than the guess are the threads' results merged.  A thread keeps its
+// first FAR_KEEP points in registers.  Looking at fewer points was slower
+// each time (at 1242x375, against 21 us): only the rows that the guess's
+// circle reaches 27, in them only the columns inside it 48, every point
+// tested against the circle first 24, as the instructions that choose
+// lengthen a step more than the points left out shorten it.
+constexpr int FAR_THREADS = 512, FAR_KEEP = 8;
+__global__ void __launch_bounds__(FAR_THREADS, 2) k_star_far(DelDev d0, DelDev d1, unsigned* err) {
+    grid_dep_wait();
+    constexpr int NW = FAR_THREADS / 32;
+    __shared__ StarSmem sm;
+    __shared__ StarBest part[2][NW];
+    __shared__ uint2 near[NW];
+    const DelDev& D = blockIdx.x ? d1 : d0;
+    const int count = D.ctr[10], N = D.ctr[9], R = D.ctr[6];
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    if (int(blockIdx.y) >= count) return;
+    uint32_t keep[FAR_KEEP];
+#pragma unroll
+    for (int k = 0; k < FAR_KEEP; ++k) {
+        const int i = tid + k * FAR_THREADS;
+        keep[k] = i < N ? D.pxy[i] : PXY_NONE;
+    }
+    int flip = 0;
+    for (int q = blockIdx.y; q < count; q += gridDim.y) {
+        const int32_t* rec = D.far + size_t(q) * FAR_REC;
+        const int p = rec[0], lm = rec[1] & 0xff;
+        const bool lclosed = ((rec[1] >> 8) & 1) != 0, adrift = ((rec[1] >> 9) & 1) != 0;
+        const uint32_t sure = uint32_t(rec[2]);
+        const int lz = lane < lm ? rec[3 + lane] : -1;
+        const uint32_t lzxy = lz >= 0 ? D.pxy[lz] : PXY_NONE;
+        const uint32_t pp = D.pxy[p];
+        const int hn = D.hnext[p], hp = D.hprev[p];
+        const uint32_t hpxy = hp >= 0 ? D.pxy[hp] : PXY_NONE;
+        int q0 = lm > 0 && !adrift ? __shfl_sync(0xffffffffu, lz, 0) : hn;
+        __syncthreads();                        // the previous point is done with
+        if (q0 < 0) {
+            // nearest neighbour, the lowest index among equals
+            uint2 best = make_uint2(0xffffffffu, 0xffffffffu);     // squared distance, index
+            for (int i = tid; i < N; i += FAR_THREADS) {
+                const uint32_t xy = D.pxy[i];
+                if (xy == PXY_NONE || i == p) continue;
+                const int dx = dx_p(xy, pp), dy = dy_p(xy, pp);
+                const uint32_t d = uint32_t(dx * dx + dy * dy);
+                if (d < best.x) best = make_uint2(d, uint32_t(i));
+            }
+            star_cta_min(best, near, lane, warp, NW, make_uint2(0xffffffffu, 0xffffffffu), [](uint2& v) {
+                const uint32_t d = __reduce_min_sync(0xffffffffu, v.x);
+                v.y = __reduce_min_sync(0xffffffffu, v.x == d ? v.y : 0xffffffffu);
+                v.x = d;
+            });
+            q0 = int(best.y);                   // -1: no other point
+        }
+        int m = 0;
+        uint32_t qd2 = 0;
+        bool closed = false, open = false, ok = true;
+        if (q0 >= 0) {
+            const uint32_t q0xy = D.pxy[q0];
+            if (tid == 0) { sm.nb[0] = q0; sm.nxy[0] = q0xy; }
+            m = 1;
+            StarEdge e{p, q0, pp, q0xy, dx_p(q0xy, pp), dy_p(q0xy, pp)};
+            if (hn < 0) qd2 = uint32_t(e.ux * e.ux + e.uy * e.uy);
+            int j = lm > 0 && !adrift ? 0 : -1; // the current neighbour's place in the record (-1: not in it)
+            for (;;) {
+                StarBest best{-1, 0u, 0.0f};
+                const int jn = j < 0 ? -1 : (j + 1 < lm ? j + 1 : (lclosed ? 0 : -1));
+                const int gi = __shfl_sync(0xffffffffu, lz, jn < 0 ? 0 : jn);
+                const uint32_t gxy = __shfl_sync(0xffffffffu, lzxy, jn < 0 ? 0 : jn);
+                if (jn >= 0 && ((sure >> j) & 1u) != 0u) {
+                    best.i = gi;
+                    best.xy = gxy;
+                } else {
+                    if (jn >= 0) star_take(e, best, gi, gxy);
+                    const int guess = best.i;
+#pragma unroll
+                    for (int k = 0; k < FAR_KEEP; ++k)
+                        if (keep[k] != PXY_NONE) star_take(e, best, tid + k * FAR_THREADS, keep[k]);
+#pragma unroll 1
+                    for (int i = tid + FAR_KEEP * FAR_THREADS; i < N; i += FAR_THREADS) {
+                        const uint32_t xy = D.pxy[i];
+                        if (xy != PXY_NONE) star_take(e, best, i, xy);
+                    }
+                    if (__syncthreads_or(best.i != guess)) {
+                        star_cta_min(best, part[flip], lane, warp, NW, StarBest{-1, 0u, 0.0f},
+                                     [&](StarBest& v) { star_reduce(e, v, lane); });
+                        flip ^= 1;
+                    }
+                }
+                if (best.i < 0) {
+                    open = true;                // a hull edge
+                    ok = hn >= 0 || R < 2;
                     break;
                 }
-                Rs = star_square(Rs);
-                ++squares;
-                star_stream(D, row_off, star_half_region(pp, pq, side, Rs, box), box, lane, take3);
-                reduce();
-            }
-            if (bi >= 0) {
-                c1 = bi;
-                x1c = bxy;
-            }
-            return bi;
-        };
-        int m = 0, k = 0;
-        bool closed = false;
-        const bool ok = star_walk(hn, hp, nearest, next, sm.ccw, sm.cw, STAR_NB, &m, &k, &closed);
-        __syncwarp();
-        int own = 0;
-        const int deg = m + k, nt = ok ? star_tris(deg, closed) : 0;
-        for (int b = 0; b < nt; b += 32) {
-            const int i = b + lane;
-            bool o = false;
-            if (i < nt) {
-                const int a = star_at(sm.ccw, m, sm.cw, k, i), c = star_at(sm.ccw, m, sm.cw, k, i + 1 == deg ? 0 : i + 1);
-                o = p < a && p < c;
-            }
-            own += __popc(__ballot_sync(0xffffffffu, o));
-        }
-        int32_t* dst = D.sown + size_t(p) * 2 * STAR_SLOT;
-        if (own > STAR_SLOT) {
-            int base = 0;
-            if (lane == 0) base = atomicAdd(&D.ctr[11], own);
-            base = __shfl_sync(0xffffffffu, base, 0);
-            if (base + own > D.Tmax) {
-                if (lane == 0) set_err(err, ERRF_BOUNDS);
-                own = 0;
-            } else {
-                if (lane == 0) dst[0] = base;
-                dst = D.spool + 2 * size_t(base);
+                if (best.xy == q0xy) {
+                    closed = ok = hn < 0;
+                    break;
+                }
+                if (m >= STAR_NB) {
+                    ok = false;
+                    break;
+                }
+                if (tid == 0) { sm.nb[m] = best.i; sm.nxy[m] = best.xy; }
+                ++m;
+                if (best.xy == hpxy) break;
+                j = __ffs(__ballot_sync(0xffffffffu, lzxy == best.xy)) - 1;
+                e.q = best.i;
+                e.pq = best.xy;
+                e.ux = dx_p(best.xy, pp);
+                e.uy = dy_p(best.xy, pp);
             }
         }
-        if (!ok && lane == 0) set_err(err, ERRF_BOUNDS);
-        int pos = 0;
-        for (int b = 0; b < nt && own > 0; b += 32) {
-            const int i = b + lane;
-            bool o = false;
-            int a = 0, c = 0;
-            if (i < nt) {
-                a = star_at(sm.ccw, m, sm.cw, k, i);
-                c = star_at(sm.ccw, m, sm.cw, k, i + 1 == deg ? 0 : i + 1);
-                o = p < a && p < c;
+        __syncthreads();
+        if (warp == 0) {
+            const int nt = ok ? star_tris(m, closed) : 0;
+            const int g = star_doublings(D, pp, sm.nxy, m, nt, qd2, open, lane);
+            if (lane == 0) {
+                if (g) atomicAdd(&D.ctr[13], g);
+                if (!ok) set_err(err, ERRF_BOUNDS);
             }
-            const unsigned bal = __ballot_sync(0xffffffffu, o);
-            if (o) {
-                const int j = pos + __popc(bal & ((1u << lane) - 1u));
-                dst[2 * j] = a;
-                dst[2 * j + 1] = c;
-            }
-            pos += __popc(bal);
+            star_output(D, p, sm.nb, m, nt, lane, err);
         }
-        if (lane == 0) {
-            D.tcnt[p] = own;
-            if (circles) atomicAdd(&D.ctr[12], circles);
-            if (squares) atomicAdd(&D.ctr[13], squares);
-        }
-        __syncwarp();
     }
 }
 
@@ -1574,19 +1841,22 @@ int cluster_size_for_flip() {
     return 0;
 }
 
-cudaError_t launch_delaunay(DelDev& d0, DelDev& d1, const int32_t* row_off, int nrows, int nmax, int H, int num_sms,
-                            int csize, unsigned* err, cudaStream_t st, int* nlaunch, bool flips,
-                            bool force_global, int round_limit) {
-    launch_k(k_rowsort, dim3(nrows, 2), 512, 0, st, d0, d1, row_off, nrows, err);
-    const size_t plan_smem = size_t(32) * nrows;
+cudaError_t launch_delaunay(DelDev& d0, DelDev& d1, const int32_t* row_off, int nrows, int nmax, int W, int H,
+                            int step, int crow, int num_sms, int csize, unsigned* err, cudaStream_t st,
+                            int* nlaunch, bool flips, bool force_global, int round_limit) {
+    const int xbs = flips ? 0 : (W + 7) / 8 + 1;
+    launch_k(k_rowsort, dim3(nrows, 2), ROW_THREADS, 0, st, d0, d1, row_off, nrows, xbs, err);
+    const size_t plan_smem = size_t(PLAN_ARRAYS) * sizeof(int32_t) * nrows;
+    const RowGeom rg{step, crow, H, 1.0f / float(step)};
     allow_smem(k_plan);
-    launch_k(k_plan, 2, 1024, plan_smem, st, d0, d1, row_off, nrows, H, flips ? 1 : 0, err);
+    launch_k(k_plan, 2, 1024, plan_smem, st, d0, d1, row_off, nrows, rg, flips ? 1 : 0, err);
     if (!flips) {
         launch_k(k_star, dim3(2, imax(1, imin((nmax + STAR_WARPS - 1) / STAR_WARPS, 6 * num_sms))), STAR_WARPS * 32,
-                 0, st, d0, d1, row_off, err);
+                 0, st, d0, d1, nrows, rg, xbs, err);
+        launch_k(k_star_far, dim3(2, imax(1, imin(nmax, 2 * num_sms))), FAR_THREADS, 0, st, d0, d1, err);
         launch_k(k_star_emit, dim3(imax(1, (nmax + EMIT_THREADS - 1) / EMIT_THREADS), 2), EMIT_THREADS, 0, st, d0, d1,
                  err);
-        if (nlaunch) *nlaunch += 4;
+        if (nlaunch) *nlaunch += 5;
         return cudaGetLastError();
     }
     // the pocket walk's chain and stack (2 sides x (index, x, y, 4-int stack

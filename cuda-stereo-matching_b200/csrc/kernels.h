@@ -30,12 +30,12 @@ struct DelDev {
     int32_t* cflips;       // cluster kernel: per-CTA flips      [16 * 6 * 4096]
     int32_t* ctr;          // [16]: 0 triangles, 1 strip triangles, 4 flip rounds, 5 flips,
                            //       6 non-empty rows, 8 handled by the cluster kernel, 9 points,
-                           //       11 star pool cursor, 12 star windows grown,
-                           //       13 star searches over every point
+                           //       10 points of far, 11 star pool cursor, 12 unused (0),
+                           //       13 window doublings that prove the stars
     uint32_t* pxy;         // [Nmax] packed coordinates by point (PXY_NONE: dropped duplicate)
     uint32_t* sxy;         // [Nmax] packed coordinates beside srt
-    int32_t* ne_y;         // [rows] y of each non-empty row
-    int4* rinfo;           // [rows] non-empty row: y, first position in srt, unique points
+    int32_t* xb;           // [rows][(W + 7) / 8 + 1] first sorted position at or right of each 8-pixel column
+    int32_t* far;          // [Nmax][FAR_REC] points whose star the window does not prove, with what it found
     int32_t* tcnt;         // [Nmax] triangles owned by each point (star construction)
     int32_t* toff;         // [Nmax] their offsets in tri
     int32_t* sown;         // [24*Nmax] owned triangles' vertex pairs, per point
@@ -43,11 +43,11 @@ struct DelDev {
     int32_t* hnext;        // [Nmax] successor on the hull boundary (-1: interior point)
     int32_t* hprev;        // [Nmax] predecessor on the hull boundary
     int32_t* box;          // [8] x0, y0, x1, y1 of all points, [4] star window half-size
-    int32_t* ylut;         // [H+2] y -> first non-empty row at or below y
     unsigned long long* hkey;  // [Hmax]
     int32_t* hcnt;         // [Hmax]
     int32_t* hval;         // [2*Hmax]
     int32_t* hslot;        // [3*Tmax]
+    static constexpr int FAR_REC = 32;
     int Tmax;
     uint32_t Hmax;         // power of two
 };
@@ -76,10 +76,11 @@ cudaError_t launch_grid(const int32_t* can, uint32_t* tmp0, uint32_t* tmp1, uint
 // and Lawson edge flips instead; then force_global flips every problem with
 // the global-memory kernel (tests) and round_limit > 0 caps the flip rounds
 // (ERRF_FLIP_LIMIT when hit).  Both give the same triangles (the unique
-// triangulation under the perturbation), in different list orders.
-cudaError_t launch_delaunay(DelDev& d0, DelDev& d1, const int32_t* row_off, int nrows, int nmax, int H, int num_sms,
-                            int cluster_size, unsigned* err, cudaStream_t st, int* nlaunch, bool flips = false,
-                            bool force_global = false, int round_limit = 0);
+// triangulation under the perturbation), in different list orders.  Lattice
+// row r lies at y = r * step, the corners' row crow (-1: none) at y = H - 1.
+cudaError_t launch_delaunay(DelDev& d0, DelDev& d1, const int32_t* row_off, int nrows, int nmax, int W, int H,
+                            int step, int crow, int num_sms, int cluster_size, unsigned* err, cudaStream_t st,
+                            int* nlaunch, bool flips = false, bool force_global = false, int round_limit = 0);
 // Largest cluster (16 or 8 CTAs) with two co-resident copies for the flip
 // kernel, or 0 if none fits.
 int cluster_size_for_flip();
