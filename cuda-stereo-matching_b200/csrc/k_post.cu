@@ -15,6 +15,7 @@
 //   median    lower median of the valid pixels of the 3x3 window.
 #include <cuda_runtime.h>
 #include <mutex>
+#include <type_traits>
 #include "../../include/elas_b200.h"
 #include "common.cuh"
 #include "launch.cuh"
@@ -459,178 +460,249 @@ __global__ void __launch_bounds__(32 * GAP_COL_WARPS) k_gap_cols(PostViews pv, i
     }
 }
 
-// Gap interpolation (rows, then columns), adaptive mean and median in one
-// pass over a 32x32 output tile, every intermediate in shared memory.  The
-// input region carries a halo of G + 3 for gaps up to G (the column pass
-// needs the row pass G rows away, the mean 2 more, the median 1 more).
-// Each stage is computed exactly as its separate kernel (k_gap_px,
-// k_mean_median) does.
-constexpr int PT = 32, PGMAX = 8;
-__device__ __forceinline__ float gap_fill(const float* line, int stride, int k, int len, int gap, float c) {
-    // line[k*stride] is the pixel; positions < 0 or >= len are outside the image
-    if (c >= 0) return c;
-    int lo = -1, hi = -1;
-    for (int j = 1; j <= gap && k - j >= 0; ++j)
-        if (line[-j * stride] >= 0) { lo = k - j; break; }
-    if (lo >= 0)
-        for (int j = 1; j <= gap && k + j < len; ++j)
-            if (line[j * stride] >= 0) { hi = k + j; break; }
-    if (lo >= 0 && hi >= 0 && hi - lo - 1 <= gap) {
-        float a = line[-(k - lo) * stride], b = line[(hi - k) * stride];
-        return gap_value(a, b);
-    }
-    return c;
+// 3-value and 9-value medians.  A column of three sorted rows of three gives
+// the median of nine: the middle one of the largest low, the middle middle
+// and the smallest high.
+__device__ __forceinline__ float med3(float a, float b, float c) {
+    return fmaxf(fminf(a, b), fminf(fmaxf(a, b), c));
+}
+struct Tri { float lo, mid, hi; };
+__device__ __forceinline__ Tri sort3(float a, float b, float c) {
+    const float l = fminf(a, b), h = fmaxf(a, b);
+    return {fminf(l, c), fmaxf(l, fminf(h, c)), fmaxf(h, c)};
+}
+__device__ __forceinline__ float med9(const Tri& p, const Tri& q, const Tri& r) {
+    return med3(fmaxf(fmaxf(p.lo, q.lo), r.lo), med3(p.mid, q.mid, r.mid), fminf(fminf(p.hi, q.hi), r.hi));
 }
 
-// 9-input sorting network (25 compare-exchanges, depth 7; checked by the
-// 0-1 principle on all 512 binary inputs).
-template <int I, int J>
-__device__ __forceinline__ void cex(float (&a)[9]) {
-    const float x = a[I], y = a[J];
-    a[I] = fminf(x, y);
-    a[J] = fmaxf(x, y);
-}
-__device__ __forceinline__ void sort9(float (&a)[9]) {
-    cex<0, 3>(a); cex<1, 7>(a); cex<2, 5>(a); cex<4, 8>(a); cex<0, 7>(a); cex<2, 4>(a); cex<3, 8>(a);
-    cex<5, 6>(a); cex<0, 2>(a); cex<1, 3>(a); cex<4, 5>(a); cex<7, 8>(a); cex<1, 4>(a); cex<3, 6>(a);
-    cex<5, 7>(a); cex<0, 1>(a); cex<2, 4>(a); cex<3, 5>(a); cex<6, 8>(a); cex<2, 3>(a); cex<4, 5>(a);
-    cex<6, 7>(a); cex<1, 2>(a); cex<3, 4>(a); cex<5, 6>(a);
+// Speckle decision, gap interpolation (rows, then columns), adaptive mean
+// and median in one pass over a tile of PT_OW x (4 R - 2) output pixels, every
+// intermediate in shared memory.  The input region carries a halo of G + 3
+// for gaps up to G (the column pass needs the row pass G rows away, the mean
+// 2 more, the median 1 more).  Eight warps: two side by side over 64
+// columns, four strips of R rows (the mean's region is 64 x 4 R: whole
+// warps).
+//
+// Bound by instruction issue and the shared-memory pipe, so each stage keeps
+// what neighbouring pixels share in registers:
+//   load    a warp loads whole rows and, as it knows their valid pixels from
+//           ballots, fills the row gaps at once: run lengths come from the
+//           bits on either side.  Fills are written in place (only invalid
+//           pixels are written, only valid ones read).  The column pass
+//           does the same with the rows' bit masks.
+//   mean    a thread walks down a column with the 5 x 5 window in registers
+//           (five loads a pixel instead of 25).  Every value is a multiple
+//           of 1/4 (integer disparities, halves from the row gaps, quarters
+//           from the column gaps) in [0, disp_max], so v * 16 + 2^23 is exact
+//           and the difference of two such floats' bits is the byte offset
+//           of the pair's weight 1 / (1 + (d_q - d_p)^2), made once by the
+//           same correctly rounded operations as the direct formula: an add
+//           and a load a weight.  The table covers differences of either
+//           sign; invalid pixels get bits so far up that they meet the
+//           zeros behind it, and a weight of 0 leaves both sums as they are.
+//   median  a thread walks down a column with three sorted rows of three;
+//           only a window with invalid pixels sorts for itself.
+// A thread per pixel for each stage took 314 us at 2880x1988 (D 0-511) and 37
+// at 1242x375; this form 221 and 28.
+constexpr int PGMAX = 8, PT_OW = 62, POST_THREADS = 256;
+constexpr uint32_t MAGIC_F32 = 0x4b000000u;     // bits of 2^23
+// weights of the mean: entries -4 D .. 8 D + 1 of the difference in quarters
+inline size_t post_weights(int D) { return 12 * size_t(D) + 2; }
+__device__ __forceinline__ float lds_f32(uint32_t addr) {
+    float v;
+    asm("ld.shared.f32 %0, [%1];" : "=f"(v) : "r"(addr));
+    return v;
 }
 
-// Adaptive-mean weights.  Every value the mean reads is a multiple of 1/4
-// (integer disparities, halves from the row gap pass, quarters from the
-// column pass) in [0, disp_max], so with the key K = 4 * d the weight of a
-// valid pair is WT[|K_q - K_p|], WT[j] = 1 / (1 + (j/4)^2) made by the same
-// correctly rounded operations as the direct formula, for j <= 4 disp_max.
-// Invalid pixels get a key far away from every valid one, which lands on
-// the table's last entry, weight 0: an invalid neighbour adds 0 to both
-// sums (bit for bit the same as skipping it).  The table has
-// 4 disp_max + 2 entries.  The neighbour's value is read back from its key
-// (K / 4 is exact for these quarters), so the 5x5 window loads one array.
-constexpr int K_INVALID = 1 << 20;
+// Tiles of 30 rows from this many per SM on, of 14 rows below.
+constexpr int POST_TALL_TILES = 2;
 
-// spk_min > 0: the input is the L/R result before speckle removal, and
-// every loaded pixel goes through the speckle decision of k_spk_apply
-// (segments smaller than spk_min become invalid) on the way in.
-// Persistent: each CTA builds the weight table once and walks 32x32 tiles
-// of both views with a stride of the grid size.
-constexpr int POST_THREADS = 512;    // threads of a tile-filter CTA (measured against 256 and 1024)
-template <int G, bool GAP, bool MEAN, bool MEDIAN, int NT>
-__global__ void __launch_bounds__(NT, 2048 / NT) k_post_tile(PostViews pv, int W, int H, int gap, int spk_min,
-                                                             int wt_n, int nviews) {
+template <int G, bool GAP, bool MEAN, bool MEDIAN, int R>
+__global__ void __launch_bounds__(POST_THREADS, MEAN ? 3 : 4) k_post_tile(PostViews pv, int W, int H, int gap,
+                                                                          int spk_min, int D, int nviews) {
     grid_dep_wait();
-    constexpr int PHALO = G + 3, PS = PT + 2 * PHALO;   // S tile side
-    extern __shared__ float WT[];               // wt_n weights when MEAN
-    __shared__ float S[PS][PS];                 // input, halo PHALO
-    __shared__ float G2[PS][PT + 6];            // after the row pass: columns [-3, 35)
-    __shared__ float V[PT + 6][PT + 6];         // after the column pass: [-3, 35)^2
-    __shared__ int K[MEAN ? PT + 6 : 1][PT + 6];   // mean keys of V
-    __shared__ float M[PT + 2][PT + 2];         // after the mean: [-1, 33)^2
-    const int tid = threadIdx.x;
+    constexpr int OW = PT_OW, OH = 4 * R - 2, HALO = G + 3, SW = OW + 2 * HALO, SH = OH + 2 * HALO;
+    constexpr int NSEG = (SW + 31) / 32, NWARP = POST_THREADS / 32;
+    static_assert(NSEG == 3 && OW + 2 == 64, "three ballots a row, two warps over the mean's columns");
+    extern __shared__ float WT[];               // weights when MEAN
+    __shared__ float S[SH][SW];                 // the input region, gaps filled in place
+    __shared__ uint32_t msk[SH][NSEG];          // its valid pixels after the row pass
+    __shared__ float M[MEAN && MEDIAN ? OH + 2 : 1][OW + 2];    // after the mean: [-1, OW + 1) x [-1, OH + 1)
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const float OUT = -2.0f;                    // outside the image (never valid, never filled)
     if (MEAN)
-        for (int j = tid; j < wt_n; j += NT) {
-            const float q = float(j) * 0.25f;
-            WT[j] = j < wt_n - 1 ? __frcp_rn(__fmaf_rn(q, q, 1.0f)) : 0.0f;
+        for (int j = tid; j < 12 * D + 2; j += POST_THREADS) {
+            const float q = float(j - 4 * D) * 0.25f;
+            WT[j] = j <= 8 * D ? __frcp_rn(__fmaf_rn(q, q, 1.0f)) : 0.0f;
         }
-    const int tiles_x = (W + PT - 1) / PT, tiles_y = (H + PT - 1) / PT, per_view = tiles_x * tiles_y;
+    const uint32_t wt0 = MEAN ? smem_u32(WT) + 16u * uint32_t(D) : 0u;      // the weight of difference 0
+    const uint32_t kinv = MAGIC_F32 + 4u * uint32_t(8 * D + 1);             // bits of an invalid pixel
+    const int tiles_x = (W + OW - 1) / OW, tiles_y = (H + OH - 1) / OH, per_view = tiles_x * tiles_y;
     for (int tile = blockIdx.x; tile < nviews * per_view; tile += gridDim.x) {
-        const int view = tile / per_view, tv = tile - view * per_view;
-        const float* __restrict__ src = pv.cur[view];
-        float* __restrict__ dst = pv.nxt[view];
-        const int u0 = (tv % tiles_x) * PT, v0 = (tv / tiles_x) * PT;
-        const int32_t* __restrict__ lab = pv.lab[view];
-        const int32_t* __restrict__ sz = pv.sz[view];
-        const int32_t* __restrict__ acc = pv.root[view];
-        __syncthreads();                        // the previous tile (and the table) is done with
-        // The speckle decision of k_spk_apply: the local root lab[j] holds
-        // -(global root + 1) in its size slot, whose segment size is
-        // acc[global root].  The value and lab[j] are loaded together, so each
-        // pixel waits on three dependent loads, and the loop is unrolled so that
-        // two pixels' chains overlap.
+        const bool second = tile >= per_view;
+        const int tv = second ? tile - per_view : tile;
+        const float* __restrict__ src = second ? pv.cur[1] : pv.cur[0];
+        float* __restrict__ dst = second ? pv.nxt[1] : pv.nxt[0];
+        const int32_t* __restrict__ lab = second ? pv.lab[1] : pv.lab[0];
+        const int32_t* __restrict__ sz = second ? pv.sz[1] : pv.sz[0];
+        const int32_t* __restrict__ acc = second ? pv.root[1] : pv.root[0];
+        const int u0 = (tv % tiles_x) * OW, v0 = (tv / tiles_x) * OH;
+        if (!(MEAN && MEDIAN)) __syncthreads();     // the previous tile's last stage read S
+        // Load, speckle decision and row gaps.  The decision is k_spk_apply's:
+        // the local root lab[j] holds -(global root + 1) in its size slot,
+        // whose segment size is acc[global root]; the value and the label are
+        // loaded together and two rows' chains overlap.
 #pragma unroll 2
-        for (int i = tid; i < PS * PS; i += NT) {
-            int r = i / PS, c = i % PS;
-            int x = u0 - PHALO + c, y = v0 - PHALO + r;
-            float d = OUT;
-            if (x >= 0 && x < W && y >= 0 && y < H) {
-                const size_t j = size_t(y) * W + x;
-                d = src[j];
-                if (spk_min > 0) {
-                    const int l = lab[j];
-                    if (d >= 0 && acc[-sz[l] - 1] < spk_min) d = -1.0f;   // a valid pixel has l >= 0
+        for (int r = warp; r < SH; r += NWARP) {
+            const int y = v0 - HALO + r;
+            float d[NSEG];
+            int l[NSEG];
+            uint32_t m[NSEG + 2];
+#pragma unroll
+            for (int k = 0; k < NSEG; ++k) {
+                const int c = 32 * k + lane, x = u0 - HALO + c;
+                const bool in = c < SW && x >= 0 && x < W && y >= 0 && y < H;
+                const size_t j = size_t(in ? y : 0) * W + (in ? x : 0);
+                d[k] = in ? src[j] : OUT;
+                l[k] = spk_min > 0 && in ? lab[j] : -1;
+            }
+            if (spk_min > 0) {
+#pragma unroll
+                for (int k = 0; k < NSEG; ++k) l[k] = d[k] >= 0 ? sz[l[k]] : 0;     // a valid pixel has a label
+#pragma unroll
+                for (int k = 0; k < NSEG; ++k)
+                    if (d[k] >= 0 && acc[-l[k] - 1] < spk_min) d[k] = -1.0f;
+            }
+            m[0] = m[NSEG + 1] = 0;
+#pragma unroll
+            for (int k = 0; k < NSEG; ++k) {
+                m[k + 1] = __ballot_sync(0xffffffffu, d[k] >= 0);
+                if (32 * k + lane < SW) S[r][32 * k + lane] = d[k];
+            }
+            if (GAP) {
+                __syncwarp();
+                uint32_t after[NSEG];
+#pragma unroll
+                for (int k = 0; k < NSEG; ++k) {
+                    after[k] = m[k + 1];
+                    if (__any_sync(0xffffffffu, d[k] < 0 && d[k] != OUT)) {
+                        const int c = 32 * k + lane;
+                        // bit 31: the pixel to the left; bit 0: the one to the right
+                        const uint32_t lf = __funnelshift_r(m[k], m[k + 1], lane);
+                        const uint32_t rt = __funnelshift_rc(m[k + 1], m[k + 2], lane + 1);
+                        const int dl = __clz(lf) + 1, dr = rt ? __ffs(rt) : 33;     // 33: none within 32
+                        const bool fill = d[k] < 0 && dl <= gap && dr <= gap && dl + dr - 1 <= gap;
+                        if (fill) S[r][c] = gap_value(S[r][c - dl], S[r][c + dr]);
+                        after[k] = __ballot_sync(0xffffffffu, d[k] >= 0 || fill);
+                    }
+                }
+                if (lane < NSEG) msk[r][lane] = lane == 0 ? after[0] : (lane == 1 ? after[1] : after[2]);
+            }
+        }
+        __syncthreads();
+        if (GAP) {
+            // column gaps of [-3, OW + 3) x [-3, OH + 3)
+            for (int r = HALO - 3 + warp; r < HALO + OH + 3; r += NWARP) {
+                const int y = v0 - HALO + r;
+                if (y < 0 || y >= H) continue;
+#pragma unroll
+                for (int k = 0; k < NSEG; ++k) {
+                    const int c = 32 * k + lane, x = u0 - HALO + c;
+                    const bool wanted = c >= HALO - 3 && c < HALO + OW + 3 && x >= 0 && x < W;
+                    const bool inv = wanted && !((msk[r][k] >> lane) & 1u);
+                    if (!__any_sync(0xffffffffu, inv)) continue;
+                    int dl = 0, dr = 0;
+#pragma unroll
+                    for (int j = G; j >= 1; --j) {
+                        if ((msk[r - j][k] >> lane) & 1u) dl = j;
+                        if ((msk[r + j][k] >> lane) & 1u) dr = j;
+                    }
+                    if (inv && dl && dr && dl + dr - 1 <= gap) S[r][c] = gap_value(S[r - dl][c], S[r + dr][c]);
                 }
             }
-            S[r][c] = d;
+            __syncthreads();
         }
-        __syncthreads();
-        // row pass on rows [-PHALO, 32+PHALO), columns [-3, 35)
-        for (int i = tid; i < PS * (PT + 6); i += NT) {
-            int r = i / (PT + 6), c = i % (PT + 6);
-            int x = u0 - 3 + c;
-            float val = S[r][c + PHALO - 3];
-            if (GAP && val != OUT && val < 0) val = gap_fill(&S[r][c + PHALO - 3], 1, x, W, gap, val);
-            G2[r][c] = val;
-        }
-        __syncthreads();
-        // column pass on [-3, 35)^2
-        for (int i = tid; i < (PT + 6) * (PT + 6); i += NT) {
-            int r = i / (PT + 6), c = i % (PT + 6);
-            int y = v0 - 3 + r;
-            float val = G2[r + PHALO - 3][c];
-            if (GAP && val != OUT && val < 0) val = gap_fill(&G2[r + PHALO - 3][c], PT + 6, y, H, gap, val);
-            V[r][c] = val;
-            if (MEAN) K[r][c] = val >= 0 ? __float2int_rn(val * 4.0f) : K_INVALID;
-        }
-        __syncthreads();
-        // mean on [-1, 33)^2, in the oracle's (dy, dx) order: num by fma, den by add
-        for (int i = tid; i < (PT + 2) * (PT + 2); i += NT) {
-            int r = i / (PT + 2), c = i % (PT + 2);
-            float dp = V[r + 2][c + 2];
-            float out = dp;
-            if (MEAN && dp >= 0) {
-                const int kp = K[r + 2][c + 2];
+        const int col = 32 * (warp & 1) + lane, row0 = R * (warp >> 1);
+        if (MEAN) {
+            // mean at column col - 1, rows row0 - 1 .., in the oracle's (dy, dx)
+            // order: num by fma, den by add
+            float v[5][5];
+            uint32_t q[5][5];
+            auto load = [&](int slot, int r) {
+#pragma unroll
+                for (int c = 0; c < 5; ++c) {
+                    v[slot][c] = S[HALO - 3 + r][HALO - 3 + col + c];
+                    q[slot][c] = v[slot][c] >= 0 ? __float_as_uint(fmaf(v[slot][c], 16.0f, 8388608.0f)) : kinv;
+                }
+            };
+#pragma unroll
+            for (int r = 0; r < 4; ++r) load(r, row0 + r);
+#pragma unroll
+            for (int i = 0; i < R; ++i) {
+                load((i + 4) % 5, row0 + i + 4);
+                const float vp = v[(i + 2) % 5][2];
+                const uint32_t base = wt0 - (vp >= 0 ? q[(i + 2) % 5][2] : MAGIC_F32);
                 float num = 0.0f, den = 0.0f;
 #pragma unroll
-                for (int dy = -2; dy <= 2; ++dy)
+                for (int dy = 0; dy < 5; ++dy)
 #pragma unroll
-                    for (int dx = -2; dx <= 2; ++dx) {
-                        const int kq = K[r + 2 + dy][c + 2 + dx];
-                        const float dq = __int2float_rn(kq) * 0.25f;
-                        const int j = min(abs(kq - kp), wt_n - 1);
-                        const float w = WT[j];
-                        num = __fmaf_rn(w, dq, num);
+                    for (int dx = 0; dx < 5; ++dx) {
+                        const int s = (i + dy) % 5;
+                        const float w = dy == 2 && dx == 2 ? 1.0f : lds_f32(base + q[s][dx]);
+                        num = __fmaf_rn(w, v[s][dx], num);
                         den = __fadd_rn(den, w);
                     }
-                out = __fdiv_rn(num, den);
-            }
-            M[r][c] = out;
-        }
-        __syncthreads();
-        for (int o = tid; o < PT * PT; o += NT) {
-            int ty = o / PT, tx = o % PT;
-            int u = u0 + tx, v = v0 + ty;
-            if (u < W && v < H) {
-                float c = M[ty + 1][tx + 1];
-                float out = c;
-                if (MEDIAN && c >= 0) {
-                    // invalid neighbours sort last as +inf; the lower median of the
-                    // n valid values is then element (n-1)/2 (all in registers)
-                    float a[9];
-                    int n = 0;
-#pragma unroll
-                    for (int k = 0; k < 9; ++k) {
-                        float q = M[ty + k / 3][tx + k % 3];
-                        n += q >= 0 ? 1 : 0;
-                        a[k] = q >= 0 ? q : INFINITY;
-                    }
-                    sort9(a);
-                    const int m = (n - 1) >> 1;     // n >= 1 (the centre), so m in [0, 4]
-                    out = a[0];
-#pragma unroll
-                    for (int k = 1; k < 5; ++k) out = m == k ? a[k] : out;
+                const float out = vp >= 0 ? __fdiv_rn(num, den) : vp;
+                if (MEDIAN) {
+                    M[row0 + i][col] = out;
+                } else {
+                    const int u = u0 + col - 1, y = v0 + row0 + i - 1;
+                    if (col >= 1 && col <= OW && u < W && row0 + i >= 1 && row0 + i <= OH && y < H)
+                        dst[size_t(y) * W + u] = out;
                 }
-                dst[size_t(v) * W + u] = out;
+            }
+            if (MEDIAN) __syncthreads();
+        }
+        if (MEDIAN || !MEAN) {
+            // output column col, rows row0 ..; row r of the window's column
+            auto at = [&](int r, int c) { return MEAN ? M[r][c] : S[HALO - 1 + r][HALO - 1 + c]; };
+            const int u = u0 + col;
+            if (col < OW && u < W) {
+                Tri t[3];
+                float mid[3];                   // the window's middle column
+                auto load = [&](int slot, int r) {
+                    mid[slot] = at(r, col + 1);
+                    if (MEDIAN) t[slot] = sort3(at(r, col), mid[slot], at(r, col + 2));
+                };
+                load(0, row0);
+                load(1, row0 + 1);
+#pragma unroll
+                for (int i = 0; i < R; ++i) {
+                    const int y = v0 + row0 + i;
+                    if (row0 + i >= OH || y >= H) break;
+                    load((i + 2) % 3, row0 + i + 2);
+                    const float c = mid[(i + 1) % 3];
+                    float out = c;
+                    if (MEDIAN && c >= 0) {
+                        if (fminf(fminf(t[0].lo, t[1].lo), t[2].lo) >= 0) {
+                            out = med9(t[0], t[1], t[2]);
+                        } else {
+                            // n < 9 valid values: their lower median is the median of
+                            // nine when the invalid ones count as the lowest and the
+                            // highest value in turn
+                            float a[9];
+                            bool low = true;
+#pragma unroll
+                            for (int k = 0; k < 9; ++k) {
+                                const float w = at(row0 + i + k / 3, col + k % 3);
+                                a[k] = w >= 0 ? w : (low ? -INFINITY : INFINITY);
+                                low = low != (w < 0);
+                            }
+                            out = med9(sort3(a[0], a[1], a[2]), sort3(a[3], a[4], a[5]), sort3(a[6], a[7], a[8]));
+                        }
+                    }
+                    dst[size_t(y) * W + u] = out;
+                }
             }
         }
     }
@@ -695,33 +767,40 @@ cudaError_t launch_post(PostViews pv, int nviews, const Geom& g, const DevParams
         for (int k = 0; k < nviews; ++k) direct = direct && pv.out[k] != pv.cur[k];
         if (direct)
             for (int k = 0; k < nviews; ++k) pv.nxt[k] = pv.out[k];
-        const int tiles = ((W + PT - 1) / PT) * ((H + PT - 1) / PT) * nviews;
-        const int grid = imax(1, imin(tiles, (2048 / POST_THREADS) * num_sms));
-        const int wt_n = 4 * g.D + 2;
-        const size_t smem = adaptive_mean ? size_t(wt_n) * sizeof(float) : 0;
+        const size_t smem = adaptive_mean ? post_weights(g.D) * sizeof(float) : 0;
         const int key = (tile_gap ? 4 : 0) | (adaptive_mean ? 2 : 0) | (median ? 1 : 0);
-        auto go = [&](auto kern) {
+        auto go = [&](auto kern, int oh) {
             if (smem) allow_smem(kern);
-            launch_k(kern, grid, POST_THREADS, smem, st, pv, W, H, gap, spk, wt_n, nviews);
+            const int tiles = ((W + PT_OW - 1) / PT_OW) * ((H + oh - 1) / oh) * nviews;
+            const int ctas = (adaptive_mean ? 3 : 4) * num_sms;     // resident at once
+            launch_k(kern, imax(1, imin(tiles, ctas)), POST_THREADS, smem, st, pv, W, H, gap, spk, g.D, nviews);
         };
-        if (!tile_gap || gap <= 3) {   // halo 6
-            switch (key) {
-            case 1: go(k_post_tile<3, false, false, true, POST_THREADS>); break;
-            case 2: go(k_post_tile<3, false, true, false, POST_THREADS>); break;
-            case 3: go(k_post_tile<3, false, true, true, POST_THREADS>); break;
-            case 4: go(k_post_tile<3, true, false, false, POST_THREADS>); break;
-            case 5: go(k_post_tile<3, true, false, true, POST_THREADS>); break;
-            case 6: go(k_post_tile<3, true, true, false, POST_THREADS>); break;
-            default: go(k_post_tile<3, true, true, true, POST_THREADS>); break;
+        // R rows a strip (see k_post_tile): tall tiles repeat less of their
+        // halo, flat ones spread a small image over more SMs
+        auto pick = [&](auto r) {
+            constexpr int R = decltype(r)::value, OH = 4 * R - 2;
+            if (!tile_gap || gap <= 3) {   // halo 6
+                switch (key) {
+                case 1: go(k_post_tile<3, false, false, true, R>, OH); break;
+                case 2: go(k_post_tile<3, false, true, false, R>, OH); break;
+                case 3: go(k_post_tile<3, false, true, true, R>, OH); break;
+                case 4: go(k_post_tile<3, true, false, false, R>, OH); break;
+                case 5: go(k_post_tile<3, true, false, true, R>, OH); break;
+                case 6: go(k_post_tile<3, true, true, false, R>, OH); break;
+                default: go(k_post_tile<3, true, true, true, R>, OH); break;
+                }
+            } else {                       // gaps 4..8: halo 11
+                switch (key) {
+                case 4: go(k_post_tile<PGMAX, true, false, false, R>, OH); break;
+                case 5: go(k_post_tile<PGMAX, true, false, true, R>, OH); break;
+                case 6: go(k_post_tile<PGMAX, true, true, false, R>, OH); break;
+                default: go(k_post_tile<PGMAX, true, true, true, R>, OH); break;
+                }
             }
-        } else {                       // gaps 4..8: halo 11
-            switch (key) {
-            case 4: go(k_post_tile<PGMAX, true, false, false, POST_THREADS>); break;
-            case 5: go(k_post_tile<PGMAX, true, false, true, POST_THREADS>); break;
-            case 6: go(k_post_tile<PGMAX, true, true, false, POST_THREADS>); break;
-            default: go(k_post_tile<PGMAX, true, true, true, POST_THREADS>); break;
-            }
-        }
+        };
+        const long long tall = (long long)((W + PT_OW - 1) / PT_OW) * ((H + 29) / 30) * nviews;
+        if (tall >= POST_TALL_TILES * num_sms) pick(std::integral_constant<int, 8>{});
+        else pick(std::integral_constant<int, 4>{});
         flip();
         launched += 1;
     }
