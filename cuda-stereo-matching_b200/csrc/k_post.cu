@@ -503,7 +503,7 @@ __device__ __forceinline__ float med9(const Tri& p, const Tri& q, const Tri& r) 
 //   median  a thread walks down a column with three sorted rows of three;
 //           only a window with invalid pixels sorts for itself.
 // A thread per pixel for each stage took 314 us at 2880x1988 (D 0-511) and 37
-// at 1242x375; this form 221 and 28.
+// at 1242x375; this form 207 and 25.
 constexpr int PGMAX = 8, PT_OW = 62, POST_THREADS = 256;
 constexpr uint32_t MAGIC_F32 = 0x4b000000u;     // bits of 2^23
 // weights of the mean: entries -4 D .. 8 D + 1 of the difference in quarters
@@ -513,9 +513,6 @@ __device__ __forceinline__ float lds_f32(uint32_t addr) {
     asm("ld.shared.f32 %0, [%1];" : "=f"(v) : "r"(addr));
     return v;
 }
-
-// Tiles of 30 rows from this many per SM on, of 14 rows below.
-constexpr int POST_TALL_TILES = 2;
 
 template <int G, bool GAP, bool MEAN, bool MEDIAN, int R>
 __global__ void __launch_bounds__(POST_THREADS, MEAN ? 3 : 4) k_post_tile(PostViews pv, int W, int H, int gap,
@@ -551,20 +548,24 @@ __global__ void __launch_bounds__(POST_THREADS, MEAN ? 3 : 4) k_post_tile(PostVi
         // Load, speckle decision and row gaps.  The decision is k_spk_apply's:
         // the local root lab[j] holds -(global root + 1) in its size slot,
         // whose segment size is acc[global root]; the value and the label are
-        // loaded together and two rows' chains overlap.
+        // loaded together and two rows' chains overlap (four: no faster).
+        const int x0 = u0 - HALO + lane;
+        uint32_t cols = 0;                      // bit k: column x0 + 32 k is in the region and the image
+#pragma unroll
+        for (int k = 0; k < NSEG; ++k)
+            cols |= 32 * k + lane < SW && x0 + 32 * k >= 0 && x0 + 32 * k < W ? 1u << k : 0u;
 #pragma unroll 2
         for (int r = warp; r < SH; r += NWARP) {
             const int y = v0 - HALO + r;
+            const bool row = y >= 0 && y < H;
+            const ptrdiff_t at = ptrdiff_t(row ? y : 0) * W + x0;
             float d[NSEG];
             int l[NSEG];
             uint32_t m[NSEG + 2];
 #pragma unroll
             for (int k = 0; k < NSEG; ++k) {
-                const int c = 32 * k + lane, x = u0 - HALO + c;
-                const bool in = c < SW && x >= 0 && x < W && y >= 0 && y < H;
-                const size_t j = size_t(in ? y : 0) * W + (in ? x : 0);
-                d[k] = in ? src[j] : OUT;
-                l[k] = spk_min > 0 && in ? lab[j] : -1;
+                d[k] = row && ((cols >> k) & 1u) ? src[at + 32 * k] : OUT;
+                l[k] = spk_min > 0 && row && ((cols >> k) & 1u) ? lab[at + 32 * k] : -1;
             }
             if (spk_min > 0) {
 #pragma unroll
@@ -585,7 +586,8 @@ __global__ void __launch_bounds__(POST_THREADS, MEAN ? 3 : 4) k_post_tile(PostVi
 #pragma unroll
                 for (int k = 0; k < NSEG; ++k) {
                     after[k] = m[k + 1];
-                    if (__any_sync(0xffffffffu, d[k] < 0 && d[k] != OUT)) {
+                    // nothing to fill in a full word, nor (gaps up to 8) in an empty one
+                    if (m[k + 1] != 0u && m[k + 1] != 0xffffffffu) {
                         const int c = 32 * k + lane;
                         // bit 31: the pixel to the left; bit 0: the one to the right
                         const uint32_t lf = __funnelshift_r(m[k], m[k + 1], lane);
@@ -641,18 +643,21 @@ __global__ void __launch_bounds__(POST_THREADS, MEAN ? 3 : 4) k_post_tile(PostVi
             for (int i = 0; i < R; ++i) {
                 load((i + 4) % 5, row0 + i + 4);
                 const float vp = v[(i + 2) % 5][2];
-                const uint32_t base = wt0 - (vp >= 0 ? q[(i + 2) % 5][2] : MAGIC_F32);
-                float num = 0.0f, den = 0.0f;
+                float out = vp;
+                if (__any_sync(0xffffffffu, vp >= 0)) {
+                    const uint32_t base = wt0 - (vp >= 0 ? q[(i + 2) % 5][2] : MAGIC_F32);
+                    float num = 0.0f, den = 0.0f;
 #pragma unroll
-                for (int dy = 0; dy < 5; ++dy)
+                    for (int dy = 0; dy < 5; ++dy)
 #pragma unroll
-                    for (int dx = 0; dx < 5; ++dx) {
-                        const int s = (i + dy) % 5;
-                        const float w = dy == 2 && dx == 2 ? 1.0f : lds_f32(base + q[s][dx]);
-                        num = __fmaf_rn(w, v[s][dx], num);
-                        den = __fadd_rn(den, w);
-                    }
-                const float out = vp >= 0 ? __fdiv_rn(num, den) : vp;
+                        for (int dx = 0; dx < 5; ++dx) {
+                            const int s = (i + dy) % 5;
+                            const float w = dy == 2 && dx == 2 ? 1.0f : lds_f32(base + q[s][dx]);
+                            num = __fmaf_rn(w, v[s][dx], num);
+                            den = __fadd_rn(den, w);
+                        }
+                    if (vp >= 0) out = __fdiv_rn(num, den);
+                }
                 if (MEDIAN) {
                     M[row0 + i][col] = out;
                 } else {
@@ -769,14 +774,17 @@ cudaError_t launch_post(PostViews pv, int nviews, const Geom& g, const DevParams
             for (int k = 0; k < nviews; ++k) pv.nxt[k] = pv.out[k];
         const size_t smem = adaptive_mean ? post_weights(g.D) * sizeof(float) : 0;
         const int key = (tile_gap ? 4 : 0) | (adaptive_mean ? 2 : 0) | (median ? 1 : 0);
+        const int ctas = (adaptive_mean ? 3 : 4) * num_sms;     // resident at once
+        auto tiles_of = [&](int oh) { return ((W + PT_OW - 1) / PT_OW) * ((H + oh - 1) / oh) * nviews; };
         auto go = [&](auto kern, int oh) {
             if (smem) allow_smem(kern);
-            const int tiles = ((W + PT_OW - 1) / PT_OW) * ((H + oh - 1) / oh) * nviews;
-            const int ctas = (adaptive_mean ? 3 : 4) * num_sms;     // resident at once
-            launch_k(kern, imax(1, imin(tiles, ctas)), POST_THREADS, smem, st, pv, W, H, gap, spk, g.D, nviews);
+            launch_k(kern, imax(1, imin(tiles_of(oh), ctas)), POST_THREADS, smem, st, pv, W, H, gap, spk, g.D, nviews);
         };
-        // R rows a strip (see k_post_tile): tall tiles repeat less of their
-        // halo, flat ones spread a small image over more SMs
+        // R rows a strip (see k_post_tile): the height for which the rounds of
+        // resident CTAs take the least, a round costing about 24 rows more
+        // than the 4 R it computes (halo, table, latency: 10, 12.5 and 14 us
+        // for R = 4, 5 and 8).  1242x375: two rounds of R = 8 28 us, two of
+        // R = 5 25; 960x540: three of R = 4 30, two of R = 8 27.6.
         auto pick = [&](auto r) {
             constexpr int R = decltype(r)::value, OH = 4 * R - 2;
             if (!tile_gap || gap <= 3) {   // halo 6
@@ -798,8 +806,12 @@ cudaError_t launch_post(PostViews pv, int nviews, const Geom& g, const DevParams
                 }
             }
         };
-        const long long tall = (long long)((W + PT_OW - 1) / PT_OW) * ((H + 29) / 30) * nviews;
-        if (tall >= POST_TALL_TILES * num_sms) pick(std::integral_constant<int, 8>{});
+        auto cost = [&](int r) { return (tiles_of(4 * r - 2) + ctas - 1) / ctas * (4 * r + 24); };
+        int best = 8;
+        for (int r : {5, 4})
+            if (cost(r) < cost(best)) best = r;
+        if (best == 8) pick(std::integral_constant<int, 8>{});
+        else if (best == 5) pick(std::integral_constant<int, 5>{});
         else pick(std::integral_constant<int, 4>{});
         flip();
         launched += 1;
