@@ -60,6 +60,7 @@ struct elas_handle {
     int32_t* root[2] = {nullptr, nullptr};       // union-find roots per view
     int32_t* usize[2] = {nullptr, nullptr};      // segment sizes per view
     int32_t* roots[2] = {nullptr, nullptr};      // tile-local roots of the speckle labelling per view
+    int32_t* tick = nullptr;                     // speckle border tickets of both views
     unsigned* err = nullptr;
     unsigned* err_host = nullptr;   // pinned copy of the error word (read back after each host-buffer call)
 
@@ -304,6 +305,7 @@ size_t layout(elas_handle* h, const Geom& g, char* base) {
         h->usize[k] = (int32_t*)take(px * 4);
         h->roots[k] = (int32_t*)take(px * 4 + 4);
     }
+    h->tick = (int32_t*)take(2 * post_tickets(g.W, g.H) * 4);
     h->err = (unsigned*)take(64);
     return off;
 }
@@ -461,11 +463,11 @@ void free_pn(elas_handle* h) {
     if (h->pw.b) cudaFree(h->pw.b);
 }
 
-// host_out: out0/out1 are device-mapped pinned host memory.  Every
-// intermediate then stays in device memory and only the last pass of each
-// view writes there, so the results cross PCIe while that pass computes.
+// out0/out1 may be device-mapped pinned host memory: every intermediate stays
+// in device memory and only the last pass of each view writes there, so the
+// results cross PCIe while that pass computes.
 int run_pipeline(elas_handle* h, const uint8_t* img0, const uint8_t* img1, float* out0, float* out1, int W, int H,
-                 cudaStream_t st, bool host_out = false) {
+                 cudaStream_t st) {
     const elas_params& p = h->params;
     Geom g = geom_of(W, H, p);
     DevParams dp = dev_params(p);
@@ -482,8 +484,15 @@ int run_pipeline(elas_handle* h, const uint8_t* img0, const uint8_t* img1, float
     };
     const uint32_t* bins = nullptr;
     h->pn_used = h->prop && H >= 4 && W >= 4 && g.cw > 0 && g.ch > 0;
+    // subsampling: dense, L/R and post-filters on every second row and column
+    const int sub = p.subsampling ? 1 : 0;
+    Geom go = g;
+    go.W = W >> sub;
+    go.H = H >> sub;
+    const PairZero zero{h->err, h->pn_used ? h->pn_stats : nullptr, {h->roots[0], h->roots[1]}, h->tick,
+                        dp.speckle_size > 0 ? int(2 * post_tickets(go.W, go.H)) : 0};
     CK(mark(ELAS_TIME_DESCRIPTOR));
-    CK(launch_descriptor(img0, img1, h->desc0, h->desc1, W, H, h->err, h->pn_used ? h->pn_stats : nullptr, st));
+    CK(launch_descriptor(img0, img1, h->desc0, h->desc1, W, H, zero, st));
     n += 1;
     CK(mark(ELAS_TIME_SUPPORT));
     if (h->pn_used) {
@@ -547,40 +556,41 @@ int run_pipeline(elas_handle* h, const uint8_t* img0, const uint8_t* img1, float
     rc = dense_threads_for(h, g, dp, st, &n, &shape);
     if (rc != ELAS_OK) return rc;
     CK(mark(ELAS_TIME_DENSE));
-    // subsampling: dense, L/R and post-filters on every second row and column
-    const int sub = p.subsampling ? 1 : 0;
-    Geom go = g;
-    go.W = W >> sub;
-    go.H = H >> sub;
     CK(launch_dense(h->desc0, h->desc1, h->prior0, h->prior1, h->grid0, h->grid1, h->raw0, h->raw1, g, dp,
                     prior_shift(g, dp), h->err, st, shape, sub, (h->test_flags & ELAS_TEST_DENSE_BITSET) != 0));
     n += 1;
     CK(mark(ELAS_TIME_LR));
-    // The checked maps also land where the post-filter chain starts: in the
-    // outputs, or, when the chain's first pass cannot work in place (speckle
-    // removal applied inside the tile filter), in the scratch maps, so that
-    // the last pass writes the outputs.
+    // The post-filters start from the checked maps and write the outputs in
+    // their last pass; a view without post-filters gets them from the check
+    // itself.  With speckle removal on both views the check is made by its
+    // first kernel (the L/R stage mark then covers nothing).
     const int nviews = p.postprocess_only_left ? 1 : 2;
-    const bool from_tmp = host_out || post_fuses_speckle(dp, p.filter_median, p.filter_adaptive_mean);
+    const bool post = post_any(dp, p.filter_median, p.filter_adaptive_mean);
+    const bool lr_in_post = dp.speckle_size > 0 && nviews == 2;
     float* outs[2] = {out0, out1};
-    float* dev_outs[2] = {host_out ? h->out0 : out0, host_out ? h->out1 : out1};   // device partners of tmp
-    float* start[2];
-    for (int k = 0; k < 2; ++k) start[k] = from_tmp && k < nviews ? h->tmp[k] : outs[k];
-    CK(launch_lr(h->raw0, h->raw1, h->lr0, h->lr1, start[0], start[1], h->roots[0], h->roots[1], g, p.lr_threshold, st,
-                 sub));
-    n += 1;
-    CK(mark(ELAS_TIME_POST));
-    PostViews pv;
-    for (int k = 0; k < 2; ++k) {
-        pv.cur[k] = start[k];
-        pv.nxt[k] = start[k] == dev_outs[k] ? h->tmp[k] : dev_outs[k];
-        pv.out[k] = outs[k];
-        pv.lab[k] = h->lab[k];
-        pv.root[k] = h->root[k];
-        pv.sz[k] = h->usize[k];
-        pv.roots[k] = h->roots[k];
+    if (!lr_in_post) {
+        CK(launch_lr(h->raw0, h->raw1, h->lr0, h->lr1, post ? nullptr : outs[0],
+                     post && nviews == 2 ? nullptr : outs[1], g, p.lr_threshold, st, sub));
+        n += 1;
     }
-    CK(launch_post(pv, nviews, go, dp, p.filter_median, p.filter_adaptive_mean, h->err, st, &n, h->num_sms));
+    CK(mark(ELAS_TIME_POST));
+    if (post) {
+        const LrInput lr{lr_in_post ? h->raw0 : nullptr, h->raw1, float(p.lr_threshold), sub ? 0.5f : 1.0f};
+        PostViews pv;
+        for (int k = 0; k < 2; ++k) {
+            pv.cur[k] = k ? h->lr1 : h->lr0;
+            pv.nxt[k] = h->tmp[k];
+            pv.out[k] = outs[k];
+            pv.lab[k] = h->lab[k];
+            pv.root[k] = h->root[k];
+            pv.sz[k] = h->usize[k];
+            pv.roots[k] = h->roots[k];
+            pv.tick[k] = h->tick + k * post_tickets(go.W, go.H);
+        }
+        int last_args = 0;
+        CK(launch_post(pv, lr, nviews, go, dp, p.filter_median, p.filter_adaptive_mean, h->err, st, &n, h->num_sms,
+                       &last_args));
+    }
     CK(mark(ELAS_TIME_COUNT));
     h->launches += n;
     h->have_last = true;
@@ -595,11 +605,11 @@ int run_pipeline(elas_handle* h, const uint8_t* img0, const uint8_t* img1, float
 // only launch the graph.  A caller that is itself capturing gets the plain
 // launches, which join its capture.
 int run_pipeline_graphed(elas_handle* h, const uint8_t* img0, const uint8_t* img1, float* out0, float* out1, int W,
-                         int H, cudaStream_t st, bool host_out = false) {
+                         int H, cudaStream_t st) {
     cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
     CK(cudaStreamIsCapturing(st, &cs));
     if (!h->use_graphs || cs != cudaStreamCaptureStatusNone)
-        return run_pipeline(h, img0, img1, out0, out1, W, H, st, host_out);
+        return run_pipeline(h, img0, img1, out0, out1, W, H, st);
     const Geom g = geom_of(W, H, h->params);
     int rc = ensure_workspace(h, g);
     if (rc != ELAS_OK) return rc;
@@ -610,7 +620,7 @@ int run_pipeline_graphed(elas_handle* h, const uint8_t* img0, const uint8_t* img
     std::vector<int64_t> sig = {int64_t(img0), int64_t(img1), int64_t(out0), int64_t(out1), W, H,
                                 int64_t(h->arena), int64_t(h->arena_bytes), int64_t(h->pn_in), int64_t(h->pn_bins),
                                 int64_t(h->pn_stats), h->timing ? 1 : 0, h->prop ? 1 : 0, h->prop_version,
-                                h->test_flags, h->flip_round_limit, host_out ? 1 : 0};
+                                h->test_flags, h->flip_round_limit};
     int64_t pw[sizeof(elas_params) / 8 + 1] = {};
     std::memcpy(pw, &h->params, sizeof(elas_params));
     for (int64_t x : pw) sig.push_back(x);
@@ -624,13 +634,13 @@ int run_pipeline_graphed(elas_handle* h, const uint8_t* img0, const uint8_t* img
     }
     if (sig != h->single_seen) {
         h->single_seen = sig;
-        return run_pipeline(h, img0, img1, out0, out1, W, H, st, host_out);
+        return run_pipeline(h, img0, img1, out0, out1, W, H, st);
     }
     if (!h->own_stream) CK(cudaStreamCreateWithFlags(&h->own_stream, cudaStreamNonBlocking));
     if (h->single_exec) { cudaGraphExecDestroy(h->single_exec); h->single_exec = nullptr; }
     const long long before = h->launches;
     CK(cudaStreamBeginCapture(h->own_stream, cudaStreamCaptureModeThreadLocal));
-    rc = run_pipeline(h, img0, img1, out0, out1, W, H, h->own_stream, host_out);
+    rc = run_pipeline(h, img0, img1, out0, out1, W, H, h->own_stream);
     cudaGraph_t graph = nullptr;
     cudaError_t e = cudaStreamEndCapture(h->own_stream, &graph);
     if (rc != ELAS_OK) { if (graph) cudaGraphDestroy(graph); return rc; }
@@ -977,7 +987,7 @@ int elas_b200_process(elas_handle* h, const uint8_t* left, const uint8_t* right,
     float* m1 = mapped_host(disp_left);
     float* m2 = mapped_host(disp_right);
     if (m1 && m2) {
-        rc = run_pipeline_graphed(h, h->img0, h->img1, m1, m2, W, H, st, true);
+        rc = run_pipeline_graphed(h, h->img0, h->img1, m1, m2, W, H, st);
         if (rc != ELAS_OK) return rc;
         return check_device_errors(h, st);
     }

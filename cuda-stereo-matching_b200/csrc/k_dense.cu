@@ -556,17 +556,13 @@ __global__ void __launch_bounds__(1024) k_dense(const uint4* __restrict__ desc0,
 // snapshot copies, src/Elas.cu:542-546).
 // scale = 0.5 on subsampled maps: a disparity (in full-resolution pixels)
 // moves d / 2 columns there.
-// The checked maps go to O1/O2 and, where given, also to C1/C2 (the
-// buffers the post-filters then work on in place).
+// The checked maps go to O1/O2 and, where given, also to C1 and C2 (the
+// result of a view without post-filters).
 __global__ void k_lr(const float* __restrict__ D1, const float* __restrict__ D2, float* __restrict__ O1,
                      float* __restrict__ O2, float* __restrict__ C1, float* __restrict__ C2,
-                     int32_t* __restrict__ r1, int32_t* __restrict__ r2, int W, int H, float thr, float scale) {
+                     int W, int H, float thr, float scale) {
     grid_dep_wait();
     int u = blockIdx.x * blockDim.x + threadIdx.x, v = blockIdx.y;
-    if (u == 0 && v == 0) {
-        *r1 = 0;
-        *r2 = 0;
-    }
     if (u >= W || v >= H) return;
     size_t a = size_t(v) * W + u;
     float d1 = D1[a], d2 = D2[a];
@@ -584,10 +580,8 @@ __global__ void k_lr(const float* __restrict__ D1, const float* __restrict__ D2,
     }
     O1[a] = o1;
     O2[a] = o2;
-    if (C1) {
-        C1[a] = o1;
-        C2[a] = o2;
-    }
+    if (C1) C1[a] = o1;
+    if (C2) C2[a] = o2;
 }
 
 }  // namespace
@@ -652,10 +646,10 @@ cudaError_t launch_dense(const uint4* desc0, const uint4* desc1, const uint32_t*
     return cudaGetLastError();
 }
 
-cudaError_t launch_lr(const float* d0, const float* d1, float* o0, float* o1, float* c0, float* c1, int32_t* r0,
-                      int32_t* r1, const Geom& g, int lr_threshold, cudaStream_t st, int sub) {
+cudaError_t launch_lr(const float* d0, const float* d1, float* o0, float* o1, float* c0, float* c1, const Geom& g,
+                      int lr_threshold, cudaStream_t st, int sub) {
     const int W = g.W >> sub, H = g.H >> sub;
-    launch_k(k_lr, dim3((W + 255) / 256, H), 256, 0, st, d0, d1, o0, o1, c0, c1, r0, r1, W, H, float(lr_threshold),
+    launch_k(k_lr, dim3((W + 255) / 256, H), 256, 0, st, d0, d1, o0, o1, c0, c1, W, H, float(lr_threshold),
              sub ? 0.5f : 1.0f);
     return cudaGetLastError();
 }

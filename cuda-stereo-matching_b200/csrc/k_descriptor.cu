@@ -57,13 +57,16 @@ __global__ void __launch_bounds__(256) k_descriptor(const uint8_t* __restrict__ 
                                                     const uint8_t* __restrict__ img1,
                                                     uint4* __restrict__ desc0,
                                                     uint4* __restrict__ desc1, int W, int H,
-                                                    unsigned* __restrict__ err, int32_t* __restrict__ stats) {
+                                                    PairZero z) {
     grid_dep_wait();
     // the first kernel of a pair clears the words that later ones only add to
-    if (threadIdx.x == 0 && blockIdx.x == 0 && blockIdx.y == 0 && blockIdx.z == 0) {
-        *err = 0u;
-        if (stats) stats[0] = stats[1] = stats[2] = stats[3] = 0;
+    const int cta = blockIdx.x + gridDim.x * (blockIdx.y + gridDim.y * blockIdx.z);
+    if (cta == 0 && threadIdx.x == 0) {
+        *z.err = 0u;
+        *z.roots[0] = *z.roots[1] = 0;
+        if (z.stats) z.stats[0] = z.stats[1] = z.stats[2] = z.stats[3] = 0;
     }
+    for (int i = cta * 256 + threadIdx.x; i < z.ntick; i += 256 * gridDim.x * gridDim.y * gridDim.z) z.tick[i] = 0;
     __shared__ __align__(16) uint8_t raw[VEC ? IH : 1][RW * 16];   // staged words of each tile row
     __shared__ int roff[IH];                              // byte of image column u0 - 3 within raw[r]
     __shared__ __align__(4) uint8_t im[IH][IWP];          // the tile, 0 outside the image
@@ -211,15 +214,15 @@ __global__ void __launch_bounds__(256) k_descriptor(const uint8_t* __restrict__ 
 }  // namespace
 
 cudaError_t launch_descriptor(const uint8_t* img0, const uint8_t* img1, uint4* desc0, uint4* desc1,
-                              int W, int H, unsigned* err, int32_t* stats, cudaStream_t st) {
+                              int W, int H, const PairZero& z, cudaStream_t st) {
     dim3 grid((W + TX - 1) / TX, (H + TY - 1) / TY, 2);
     static const bool vec_on = [] {
         const char* e = std::getenv("ELAS_B200_DESC_VEC");
         return !(e && e[0] == '0');
     }();
     const bool vec = vec_on && ((reinterpret_cast<uintptr_t>(img0) | reinterpret_cast<uintptr_t>(img1)) & 15) == 0;
-    if (vec) launch_k(k_descriptor<true>, grid, 256, 0, st, img0, img1, desc0, desc1, W, H, err, stats);
-    else launch_k(k_descriptor<false>, grid, 256, 0, st, img0, img1, desc0, desc1, W, H, err, stats);
+    if (vec) launch_k(k_descriptor<true>, grid, 256, 0, st, img0, img1, desc0, desc1, W, H, z);
+    else launch_k(k_descriptor<false>, grid, 256, 0, st, img0, img1, desc0, desc1, W, H, z);
     return cudaGetLastError();
 }
 

@@ -151,150 +151,194 @@ __device__ __forceinline__ void lunion(int* L, int a, int b) {
     }
 }
 
-// A CTA of 32 x 8 threads per 32x32 tile, each thread taking the tile rows
-// ty, ty + 8, ty + 16, ty + 24 (a warp holds one tile row at a time, for
-// the run ballots): eight such CTAs fit on an SM where a tile per
-// 1024-thread CTA fitted two, so the waits at the tile's barriers overlap
-// with other tiles' work.
-constexpr int SPK_ROWS = 8;
-constexpr int SPK_RPT = SPK_T / SPK_ROWS;
-__global__ void __launch_bounds__(SPK_T * SPK_ROWS) k_spk_tile(PostViews pv, int W, int H, float thr) {
-    grid_dep_wait();
-    __shared__ float S[SPK_T][SPK_T];
-    __shared__ int L[SPK_T * SPK_T];
-    __shared__ int C[SPK_T * SPK_T];
-    __shared__ int n_roots, base;
-    const int view = blockIdx.z;
-    const float* __restrict__ D = pv.cur[view];
-    const int tx = threadIdx.x, tid = threadIdx.y * SPK_T + tx;
-    const int x = blockIdx.x * SPK_T + tx;
-    float d[SPK_RPT], dl[SPK_RPT];
-    bool conn_l[SPK_RPT];
-#pragma unroll
-    for (int j = 0; j < SPK_RPT; ++j) {
-        const int ty = threadIdx.y + SPK_ROWS * j, t = ty * SPK_T + tx, y = blockIdx.y * SPK_T + ty;
-        const bool in = x < W && y < H;
-        d[j] = in ? D[size_t(y) * W + x] : -1.0f;
-        const bool valid = d[j] >= 0;
-        S[ty][tx] = d[j];
-        C[t] = 0;
-        // runs of the row: every pixel points at the first pixel of its run
-        dl[j] = __shfl_up_sync(0xffffffffu, d[j], 1);
-        conn_l[j] = valid && tx > 0 && dl[j] >= 0 && fabsf(d[j] - dl[j]) <= thr;
-        const unsigned starts = __ballot_sync(0xffffffffu, valid && !conn_l[j]);
-        const unsigned mine = starts & (0xffffffffu >> (31 - tx));
-        L[t] = valid ? ty * SPK_T + (31 - __clz(mine)) : t;
+// uf_find and uf_union on labels that other CTAs of the same launch wrote or
+// still link: loads go to L2 (a line in L1 may hold another tile's labels
+// from before).
+__device__ __forceinline__ int uf_find_l2(int32_t* lab, int x, unsigned* err) {
+    for (int it = 0; it < UF_LIMIT; ++it) {
+        const int p = __ldcg(lab + x);
+        if (p == x) return x;
+        const int gp = __ldcg(lab + p);
+        if (gp != p) __stcg(lab + x, gp);
+        x = p;
     }
-    if (tid == 0) n_roots = 0;
-    __syncthreads();
-    // vertical links; a link is implied when the left neighbours make the same one
-#pragma unroll
-    for (int j = 0; j < SPK_RPT; ++j) {
-        const int ty = threadIdx.y + SPK_ROWS * j, t = ty * SPK_T + tx;
-        if (d[j] >= 0 && ty + 1 < SPK_T) {
-            const float q = S[ty + 1][tx];
-            if (q >= 0 && fabsf(q - d[j]) <= thr) {
-                bool implied = false;
-                if (tx > 0) {
-                    const float ql = S[ty + 1][tx - 1];
-                    implied = conn_l[j] && ql >= 0 && fabsf(ql - q) <= thr && fabsf(ql - dl[j]) <= thr;
-                }
-                if (!implied) lunion(L, t, t + SPK_T);
-            }
-        }
+    atomicOr(err, ERRF_BOUNDS);
+    return x;
+}
+__device__ void uf_union_l2(int32_t* lab, int a, int b, unsigned* err) {
+    for (int it = 0; it < UF_LIMIT; ++it) {
+        int ra = uf_find_l2(lab, a, err), rb = uf_find_l2(lab, b, err);
+        if (ra == rb) return;
+        if (ra < rb) { int t = ra; ra = rb; rb = t; t = a; a = b; b = t; }
+        const int old = atomicCAS(&lab[ra], ra, rb);
+        if (old == ra) return;
+        a = old;
     }
-    __syncthreads();
-    // roots: the run heads (the only nodes of the forest) walk to their
-    // root and keep it; every pixel then reads its head's entry
-    int r[SPK_RPT];
-#pragma unroll
-    for (int j = 0; j < SPK_RPT; ++j) {
-        const int t = (threadIdx.y + SPK_ROWS * j) * SPK_T + tx;
-        r[j] = d[j] >= 0 && !conn_l[j] ? lfind(L, t) : -1;
-    }
-    __syncthreads();
-#pragma unroll
-    for (int j = 0; j < SPK_RPT; ++j)
-        if (d[j] >= 0 && !conn_l[j]) L[(threadIdx.y + SPK_ROWS * j) * SPK_T + tx] = r[j];
-    __syncthreads();
-#pragma unroll
-    for (int j = 0; j < SPK_RPT; ++j) {
-        const int t = (threadIdx.y + SPK_ROWS * j) * SPK_T + tx;
-        if (d[j] >= 0 && conn_l[j]) r[j] = L[L[t]];
-        // component sizes, one shared atomic per group of lanes with the same root
-        const unsigned peers = __match_any_sync(0xffffffffu, r[j]);
-        if (r[j] >= 0 && tx == __ffs(peers) - 1) atomicAdd(&C[r[j]], __popc(peers));
-    }
-    // the tile's local roots take consecutive list slots: one reservation per tile
-    int slot[SPK_RPT];
-#pragma unroll
-    for (int j = 0; j < SPK_RPT; ++j) {
-        const int ty = threadIdx.y + SPK_ROWS * j, t = ty * SPK_T + tx;
-        const bool is_root = x < W && blockIdx.y * SPK_T + ty < H && r[j] == t;
-        slot[j] = is_root ? atomicAdd(&n_roots, 1) : -1;
-    }
-    __syncthreads();
-    if (tid == 0) base = n_roots > 0 ? atomicAdd(pv.roots[view], n_roots) : 0;
-    __syncthreads();
-#pragma unroll
-    for (int j = 0; j < SPK_RPT; ++j) {
-        const int ty = threadIdx.y + SPK_ROWS * j, t = ty * SPK_T + tx, y = blockIdx.y * SPK_T + ty;
-        if (x < W && y < H) {
-            const size_t i = size_t(y) * W + x;
-            const int rx = blockIdx.x * SPK_T + (r[j] & (SPK_T - 1)), ry = blockIdx.y * SPK_T + (r[j] / SPK_T);
-            pv.lab[view][i] = r[j] >= 0 ? int(size_t(ry) * W + rx) : -1;
-            if (slot[j] >= 0) {         // a local root: its count, its segment-size slot, its list entry
-                pv.sz[view][i] = C[t];
-                pv.root[view][i] = 0;
-                pv.roots[view][1 + base + slot[j]] = int(i);
-            }
-        }
-    }
+    atomicOr(err, ERRF_BOUNDS);
 }
 
-// Links across tile borders: item k < H * (tx_n - 1) is row k % H of the
-// right border of tile column k / H; the rest are bottom borders, x
-// fastest.  Neighbouring lanes thus hold neighbouring pixel pairs of one
-// border, and a segment crossing it over many pixels makes the same union
-// (the same two tile-local roots) many times: a lane skips its union when
-// the lane before it holds the same connected pair (unions are idempotent,
-// so the segments are the same).
-__global__ void k_spk_border(PostViews pv, int W, int H, float thr, unsigned* err) {
+// The left/right check of one pixel (k_lr in k_dense.cu) with the other
+// view's map: the pixel it points at must hold the same disparity within
+// thr.  dir: -1 for the left view, +1 for the right one.
+__device__ __forceinline__ float lr_checked(float d, const float* __restrict__ other_row, int u, int W, float dir,
+                                            float scale, float thr) {
+    const float uw = float(u) + dir * (d * scale);
+    if (!(d >= 0 && uw >= 0 && uw < float(W))) return -1.0f;
+    return fabsf(other_row[int(uw)] - d) > thr ? -1.0f : d;
+}
+
+// A CTA of 32 x 8 threads per 32x32 tile, each thread taking the tile rows
+// ty, ty + 8, ty + 16, ty + 24 (a warp holds one tile row at a time).  Bound
+// by instruction issue and, on small images, by its chain of barriers, so
+// the nodes of the tile's forest are runs (connected pixels of one row, named
+// by their first pixel) and every decision about runs is made on ballots:
+// where runs start, which pixels continue one, which vertical links repeat
+// the one to their left.  Only run heads find roots and add their length;
+// the other pixels get their head's label by a shuffle.
+// LR: the input is the dense result of both views and the tile also makes
+// the left/right check, writing the checked map (cur) that the rest of the
+// chain reads, so no pass of its own runs.
+// Links across a tile's borders are made by whichever of the two tiles ends
+// last, found by a ticket per border (zeroed by an earlier kernel of the
+// pair): its four border warps each link one border, so no second pass over
+// the borders runs either.  Neighbouring lanes hold neighbouring pixel pairs,
+// and a segment crossing a border over many pixels makes the same union many
+// times: a lane skips its union when the lane before it holds the same
+// connected pair.
+// Check, tiles and borders as three kernels with a node per pixel: 3.7 + 15.6
+// + 9.0 us at 1242x375, 32 + 113 + 31 at 2880x1988; this kernel 21 and 136
+// (eight CTAs per SM; five: 25 and 182).
+constexpr int SPK_ROWS = 8;
+constexpr int SPK_RPT = SPK_T / SPK_ROWS;
+template <bool LR>
+__global__ void __launch_bounds__(SPK_T * SPK_ROWS, 8) k_spk_tile(PostViews pv, LrInput lr, int W, int H, float thr,
+                                                               unsigned* err) {
     grid_dep_wait();
-    const int view = blockIdx.z;
-    const float* __restrict__ D = pv.cur[view];
-    int32_t* lab = pv.lab[view];
-    const int txn = (W + SPK_T - 1) / SPK_T, tyn = (H + SPK_T - 1) / SPK_T;
-    const long long nr = (long long)H * (txn - 1), nb = (long long)W * (tyn - 1);
-    const int lane = threadIdx.x & 31;
-    // every lane of a warp runs the same trip count (the shuffle below)
-    const long long stride = (long long)gridDim.x * blockDim.x;
-    for (long long k0 = blockIdx.x * (long long)blockDim.x + (threadIdx.x & ~31); k0 < nr + nb; k0 += stride) {
-        const long long k = k0 + lane;
-        int a = -1, b = -1;
-        if (k < nr + nb) {
-            int x, y, x2, y2;
-            if (k < nr) {
-                y = int(k % H);
-                x = int(k / H) * SPK_T + SPK_T - 1;
-                x2 = x + 1; y2 = y;
-            } else {
-                const long long kb = k - nr;
-                x = int(kb % W);
-                y = int(kb / W) * SPK_T + SPK_T - 1;
-                x2 = x; y2 = y + 1;
+    __shared__ float S[SPK_T][SPK_T];
+    __shared__ int L[SPK_T * SPK_T];            // forest, at run heads only
+    __shared__ int C[SPK_T * SPK_T];            // pixel counts, at tile-local roots
+    __shared__ uint32_t starts[SPK_T], conts[SPK_T];    // per row: run heads; pixels connected to their left
+    __shared__ int n_roots, base;
+    const bool second = blockIdx.z != 0;
+    float* D = second ? pv.cur[1] : pv.cur[0];
+    int32_t* lab = second ? pv.lab[1] : pv.lab[0];
+    int32_t* tick = second ? pv.tick[1] : pv.tick[0];
+    const int tx = threadIdx.x, warp = threadIdx.y, tid = warp * SPK_T + tx;
+    const int x = blockIdx.x * SPK_T + tx, y0 = blockIdx.y * SPK_T;
+    const uint32_t upto = 0xffffffffu >> (31 - tx);     // this lane and the ones before it
+    float d[SPK_RPT];
+    uint32_t st[SPK_RPT], ct[SPK_RPT];
+#pragma unroll
+    for (int j = 0; j < SPK_RPT; ++j) {
+        const int y = y0 + warp + SPK_ROWS * j;
+        const bool in = x < W && y < H;
+        const size_t at = size_t(y) * W + x;
+        if (LR) {
+            d[j] = in ? (second ? lr.d1 : lr.d0)[at] : -1.0f;
+            if (in) {
+                d[j] = lr_checked(d[j], (second ? lr.d0 : lr.d1) + size_t(y) * W, x, W, second ? 1.0f : -1.0f,
+                                  lr.scale, lr.thr);
+                D[at] = d[j];
             }
-            const size_t i = size_t(y) * W + x, j = size_t(y2) * W + x2;
-            const float d = D[i], q = D[j];
-            if (d >= 0 && q >= 0 && fabsf(q - d) <= thr) {
-                a = lab[i];
-                b = lab[j];
+        } else {
+            d[j] = in ? D[at] : -1.0f;
+        }
+    }
+    if (tid == 0) n_roots = 0;
+#pragma unroll
+    for (int j = 0; j < SPK_RPT; ++j) {
+        const int ty = warp + SPK_ROWS * j, t = ty * SPK_T + tx;
+        const float dl = __shfl_up_sync(0xffffffffu, d[j], 1);
+        const bool valid = d[j] >= 0, cont = valid && tx > 0 && dl >= 0 && fabsf(d[j] - dl) <= thr;
+        st[j] = __ballot_sync(0xffffffffu, valid && !cont);
+        ct[j] = __ballot_sync(0xffffffffu, cont);
+        S[ty][tx] = d[j];
+        if (valid && !cont) {
+            L[t] = t;
+            C[t] = 0;
+        }
+        if (tx == 0) {
+            starts[ty] = st[j];
+            conts[ty] = ct[j];
+        }
+    }
+    __syncthreads();
+    // vertical links; one is implied when the left neighbours make the same
+#pragma unroll
+    for (int j = 0; j < SPK_RPT; ++j) {
+        const int ty = warp + SPK_ROWS * j;
+        if (ty + 1 == SPK_T) continue;
+        const float q = S[ty + 1][tx];
+        const uint32_t v = __ballot_sync(0xffffffffu, d[j] >= 0 && q >= 0 && fabsf(q - d[j]) <= thr);
+        const uint32_t first = v & ~((v << 1) & ct[j] & conts[ty + 1]);
+        if ((first >> tx) & 1u)
+            lunion(L, ty * SPK_T + 31 - __clz(st[j] & upto), (ty + 1) * SPK_T + 31 - __clz(starts[ty + 1] & upto));
+    }
+    __syncthreads();
+    // run heads find their root and add their run's length; the local roots
+    // take consecutive list slots
+    int r[SPK_RPT], slot[SPK_RPT];
+#pragma unroll
+    for (int j = 0; j < SPK_RPT; ++j) {
+        const int t = (warp + SPK_ROWS * j) * SPK_T + tx;
+        const bool head = (st[j] >> tx) & 1u;
+        r[j] = -1;
+        if (head) {
+            r[j] = lfind(L, t);
+            atomicAdd(&C[r[j]], __ffs(~((ct[j] >> tx) >> 1)));      // 1 + the pixels that continue it
+        }
+        const uint32_t roots = __ballot_sync(0xffffffffu, head && r[j] == t);
+        int b = 0;
+        if (tx == 0 && roots) b = atomicAdd(&n_roots, __popc(roots));
+        b = __shfl_sync(0xffffffffu, b, 0);
+        slot[j] = (roots >> tx) & 1u ? b + __popc(roots & (upto >> 1)) : -1;
+    }
+    __syncthreads();
+    if (tid == 0) base = n_roots > 0 ? atomicAdd(second ? pv.roots[1] : pv.roots[0], n_roots) : 0;
+    __syncthreads();
+#pragma unroll
+    for (int j = 0; j < SPK_RPT; ++j) {
+        const int ty = warp + SPK_ROWS * j, y = y0 + ty;
+        const uint32_t mine = st[j] & upto;
+        const int root = __shfl_sync(0xffffffffu, r[j], mine ? 31 - __clz(mine) : 0);
+        if (x < W && y < H) {
+            const size_t i = size_t(y) * W + x;
+            const int rx = blockIdx.x * SPK_T + (root & (SPK_T - 1)), ry = y0 + (root / SPK_T);
+            lab[i] = d[j] >= 0 ? int(size_t(ry) * W + rx) : -1;
+            if (slot[j] >= 0) {         // a local root: its count, its segment-size slot, its list entry
+                (second ? pv.sz[1] : pv.sz[0])[i] = C[ty * SPK_T + tx];
+                (second ? pv.root[1] : pv.root[0])[i] = 0;
+                (second ? pv.roots[1] : pv.roots[0])[1 + base + slot[j]] = int(i);
             }
         }
-        const int pa = __shfl_up_sync(0xffffffffu, a, 1), pb = __shfl_up_sync(0xffffffffu, b, 1);
-        const bool same = lane > 0 && pa == a && pb == b;
-        if (a >= 0 && !same) uf_union(lab, a, b, err);
     }
+    __syncthreads();
+    // borders: warps 0 and 1 the ones to the right and left, 2 and 3 those below and above
+    if (warp >= 4) return;
+    const int txn = gridDim.x, tyn = gridDim.y;
+    const bool vertical = warp < 2;
+    const int bx = blockIdx.x - (warp == 1), by = blockIdx.y - (warp == 3);     // the tile left of or above the border
+    if (bx < 0 || by < 0 || (vertical ? bx + 1 >= txn : by + 1 >= tyn)) return;
+    int before = 0;
+    if (tx == 0) {
+        __threadfence();                // this tile's labels before its ticket
+        before = atomicAdd(&tick[(vertical ? 0 : txn * tyn) + by * txn + bx], 1);
+        __threadfence();                // the other tile's labels after it
+    }
+    if (__shfl_sync(0xffffffffu, before, 0) == 0) return;       // the other tile is yet to end
+    const int xa = vertical ? bx * SPK_T + SPK_T - 1 : bx * SPK_T + tx;
+    const int ya = vertical ? by * SPK_T + tx : by * SPK_T + SPK_T - 1;
+    int a = -1, b = -1;
+    if (xa < W && ya < H) {
+        const size_t i = size_t(ya) * W + xa, k = i + (vertical ? 1 : W);
+        const float p = __ldcg(D + i), q = __ldcg(D + k);
+        if (p >= 0 && q >= 0 && fabsf(q - p) <= thr) {
+            a = __ldcg(lab + i);
+            b = __ldcg(lab + k);
+        }
+    }
+    const int pa = __shfl_up_sync(0xffffffffu, a, 1), pb = __shfl_up_sync(0xffffffffu, b, 1);
+    if (a >= 0 && !(tx > 0 && pa == a && pb == b)) uf_union_l2(lab, a, b, err);
 }
 
 // Sizes: every tile-local root (from the roots list) adds its count at its
@@ -715,33 +759,38 @@ __global__ void __launch_bounds__(POST_THREADS, MEAN ? 3 : 4) k_post_tile(PostVi
 
 }  // namespace
 
-bool post_fuses_speckle(const DevParams& p, bool median, bool adaptive_mean) {
-    const int gap = p.ipol_gap_width;
-    return p.speckle_size > 0 && gap <= PGMAX && (gap > 0 || adaptive_mean || median);
+bool post_any(const DevParams& p, bool median, bool adaptive_mean) {
+    return p.speckle_size > 0 || p.ipol_gap_width > 0 || median || adaptive_mean;
 }
 
-cudaError_t launch_post(PostViews pv, int nviews, const Geom& g, const DevParams& p, bool median,
-                        bool adaptive_mean, unsigned* err, cudaStream_t st, int* nlaunch, int num_sms) {
+size_t post_tickets(int W, int H) { return size_t(2) * ((W + SPK_T - 1) / SPK_T) * ((H + SPK_T - 1) / SPK_T); }
+
+cudaError_t launch_post(PostViews pv, const LrInput& lr, int nviews, const Geom& g, const DevParams& p, bool median,
+                        bool adaptive_mean, unsigned* err, cudaStream_t st, int* nlaunch, int num_sms, int* last_args) {
     const int W = g.W, H = g.H, n = W * H;
     int launched = 0;
     auto flip = [&]() {
         for (int k = 0; k < 2; ++k) { float* t = pv.cur[k]; pv.cur[k] = pv.nxt[k]; pv.nxt[k] = t; }
     };
+    // every chain's first pass works out of place, so the L/R map it starts
+    // from stays as it is; the tile filter, always the last pass, writes the
+    // final buffers
     // with the tile filter following, speckle removal is applied as it loads
-    const bool fuse = post_fuses_speckle(p, median, adaptive_mean);
+    const bool fuse = p.ipol_gap_width <= PGMAX && (p.ipol_gap_width > 0 || adaptive_mean || median);
     if (p.speckle_size > 0) {
         const dim3 tiles((W + SPK_T - 1) / SPK_T, (H + SPK_T - 1) / SPK_T, nviews);
-        launch_k(k_spk_tile, tiles, dim3(SPK_T, SPK_ROWS), 0, st, pv, W, H, p.speckle_sim_threshold);
-        const long long border = (long long)H * (tiles.x - 1) + (long long)W * (tiles.y - 1);
-        const int gb = int(border / 256 + 1 < 4096 ? border / 256 + 1 : 4096);
-        launch_k(k_spk_border, dim3(gb, 1, nviews), 256, 0, st, pv, W, H, p.speckle_sim_threshold, err);
+        launch_k(lr.d0 ? k_spk_tile<true> : k_spk_tile<false>, tiles, dim3(SPK_T, SPK_ROWS), 0, st, pv, lr, W, H,
+                 p.speckle_sim_threshold, err);
         const int gn = imax(1, imin(8 * 1024, (n + 255) / 256));
         // the roots list is far shorter than the image: a grid of one CTA per
         // SM walks it (idle CTAs cost their launch; measured against four)
         launch_k(k_spk_count, dim3(imin(gn, num_sms), 1, nviews), 256, 0, st, pv, n, err);
-        launched += 3;
+        launched += 2;
         if (!fuse && p.ipol_gap_width <= PGMAX) {
+            // the chain's only pass: straight into the final buffers
+            for (int k = 0; k < nviews; ++k) pv.nxt[k] = pv.out[k];
             launch_k(k_spk_apply, dim3(gn, 1, nviews), 256, 0, st, pv, n, p.speckle_size);
+            *last_args = 3;
             flip();
             launched += 1;
         }
@@ -761,17 +810,13 @@ cudaError_t launch_post(PostViews pv, int nviews, const Geom& g, const DevParams
         allow_smem(k_gap_cols);
         launch_k(k_gap_cols, dim3((W + 31) / 32, 1, nviews), 32 * GAP_COL_WARPS,
                  size_t((H + 31) / 32) * 32 * sizeof(uint32_t), st, pc, W, H, gap);
+        *last_args = 4;
         if (last)
             for (int k = 0; k < nviews; ++k) pv.cur[k] = pv.out[k];
         launched += 2;
     }
     if (tile_gap || adaptive_mean || median) {
-        // the tile pass is the chain's last: it writes the final buffers
-        // directly unless one of them is its own input
-        bool direct = true;
-        for (int k = 0; k < nviews; ++k) direct = direct && pv.out[k] != pv.cur[k];
-        if (direct)
-            for (int k = 0; k < nviews; ++k) pv.nxt[k] = pv.out[k];
+        for (int k = 0; k < nviews; ++k) pv.nxt[k] = pv.out[k];
         const size_t smem = adaptive_mean ? post_weights(g.D) * sizeof(float) : 0;
         const int key = (tile_gap ? 4 : 0) | (adaptive_mean ? 2 : 0) | (median ? 1 : 0);
         const int ctas = (adaptive_mean ? 3 : 4) * num_sms;     // resident at once
@@ -779,6 +824,7 @@ cudaError_t launch_post(PostViews pv, int nviews, const Geom& g, const DevParams
         auto go = [&](auto kern, int oh) {
             if (smem) allow_smem(kern);
             launch_k(kern, imax(1, imin(tiles_of(oh), ctas)), POST_THREADS, smem, st, pv, W, H, gap, spk, g.D, nviews);
+            *last_args = 7;
         };
         // R rows a strip (see k_post_tile): the height for which the rounds of
         // resident CTAs take the least, a round costing about 24 rows more
@@ -816,9 +862,6 @@ cudaError_t launch_post(PostViews pv, int nviews, const Geom& g, const DevParams
         flip();
         launched += 1;
     }
-    for (int k = 0; k < nviews; ++k)   // cudaMemcpyDefault: the final buffer may be mapped host memory
-        if (pv.cur[k] != pv.out[k])
-            cudaMemcpyAsync(pv.out[k], pv.cur[k], size_t(n) * sizeof(float), cudaMemcpyDefault, st);
     if (nlaunch) *nlaunch += launched;
     return cudaGetLastError();
 }

@@ -52,10 +52,18 @@ struct DelDev {
     uint32_t Hmax;         // power of two
 };
 
-// Also zeroes the error word and, where given, the four proposal counters
-// (a memset node of its own costs 3-5 us on a pair's critical path).
+// Also zeroes the words that later kernels of the pair only add to (memset
+// nodes of their own would cost 3-5 us each on a pair's critical path).
+struct PairZero {
+    unsigned* err;         // the error word
+    int32_t* stats;        // four proposal counters (nullable)
+    int32_t* roots[2];     // lengths of the speckle filter's roots lists
+    int32_t* tick;         // ntick border tickets of the speckle filter
+    int ntick;
+};
+constexpr int DESCRIPTOR_ARGS = 7;     // of its kernel: the images come first
 cudaError_t launch_descriptor(const uint8_t* img0, const uint8_t* img1, uint4* desc0, uint4* desc1,
-                              int W, int H, unsigned* err, int32_t* stats, cudaStream_t st);
+                              int W, int H, const PairZero& z, cudaStream_t st);
 
 // bins (nullable): packed learned search sets per candidate; then stats[0]
 // counts candidates the proposal settled and stats[1] those that fell back
@@ -127,16 +135,18 @@ cudaError_t launch_dense(const uint4* desc0, const uint4* desc1, const uint32_t*
                          const DevParams& p, int pshift, unsigned* err, cudaStream_t st, int threads, int sub = 0,
                          bool force_bitset = false);
 
-// L/R check into o0/o1 and, where c0 is not null, also into c0/c1; zeroes
-// the lengths of both views' roots lists (r0, r1) for the speckle filter.
-cudaError_t launch_lr(const float* d0, const float* d1, float* o0, float* o1, float* c0, float* c1, int32_t* r0,
-                      int32_t* r1, const Geom& g, int lr_threshold, cudaStream_t st, int sub);
+// L/R check into o0/o1 and, where given, also into c0 and c1 (arguments
+// LR_ARG_C0 and the next of its kernel's LR_ARGS).
+constexpr int LR_ARGS = 10, LR_ARG_C0 = 4;
+cudaError_t launch_lr(const float* d0, const float* d1, float* o0, float* o1, float* c0, float* c1, const Geom& g,
+                      int lr_threshold, cudaStream_t st, int sub);
 
-// Buffers of the post-filter chain, per view: the filters ping-pong between
-// cur and nxt (the chain starts in cur; the result is copied to out if it
-// does not end there); lab/root/sz are union-find scratch (W*H int32 each),
-// roots the list of tile-local roots (W*H + 1 int32; its length, the first
-// entry, zeroed by launch_lr).
+// Buffers of the post-filter chain, per view: it starts from the L/R map cur
+// (left as it is), keeps intermediate maps in nxt and ends in out (which
+// may be mapped host memory: it is only written, once).  lab/root/sz are
+// union-find scratch (W*H int32 each), roots the list of tile-local roots
+// (W*H + 1 int32; its length, the first entry, starts at 0), tick a ticket
+// per tile border (post_tickets int32, all 0 at the start).
 struct PostViews {
     float* cur[2];
     float* nxt[2];
@@ -145,16 +155,24 @@ struct PostViews {
     int32_t* root[2];
     int32_t* sz[2];
     int32_t* roots[2];
+    int32_t* tick[2];
+};
+// The dense maps, for a chain whose first kernel (the speckle tiles) also
+// makes the L/R check into cur; d0 null: cur holds the checked maps already.
+struct LrInput {
+    const float* d0;
+    const float* d1;
+    float thr, scale;
 };
 
-// True when launch_post applies the speckle result while loading the fused
-// tile filter instead of in a pass of its own; the filter chain then must
-// not start in the output buffer (it never writes in place), so the caller
-// starts it in pv.nxt.
-bool post_fuses_speckle(const DevParams& p, bool median, bool adaptive_mean);
+// Whether the parameters ask for any post-filter.
+bool post_any(const DevParams& p, bool median, bool adaptive_mean);
+size_t post_tickets(int W, int H);
 
-// Post-filters on nviews (1 or 2) disparity images.
-cudaError_t launch_post(PostViews pv, int nviews, const Geom& g, const DevParams& p, bool median, bool adaptive_mean,
-                        unsigned* err, cudaStream_t st, int* nlaunch, int num_sms);
+// Post-filters on nviews (1 or 2) disparity images.  last_args: the number
+// of arguments of the last kernel launched; its first one is a PostViews
+// whose nxt are the final buffers.
+cudaError_t launch_post(PostViews pv, const LrInput& lr, int nviews, const Geom& g, const DevParams& p, bool median,
+                        bool adaptive_mean, unsigned* err, cudaStream_t st, int* nlaunch, int num_sms, int* last_args);
 
 }  // namespace elas
