@@ -26,6 +26,19 @@
 
 using namespace elas;
 
+// A pair's caller buffers, and the kernel nodes of a captured pair that take
+// them: the descriptors read both images; the L/R check and the last
+// post-filter write the maps they are told to (null: neither of the two).
+struct PairBuffers {
+    const uint8_t *img0 = nullptr, *img1 = nullptr;
+    float *out0 = nullptr, *out1 = nullptr;
+};
+struct PairNodes {
+    cudaGraphNode_t desc = nullptr, lr = nullptr, post = nullptr;
+    bool lr_out[2] = {false, false};
+    int post_views = 0, post_args = 0;
+};
+
 struct elas_handle {
     elas_params params;
     int device = 0;
@@ -91,10 +104,14 @@ struct elas_handle {
     elas_handle* owner = nullptr;     // the user's handle, for a batch worker
 
     // single-pair CUDA graph: captured on the second call with the same
-    // signature (buffers, size, parameters, workspace), replayed after that
+    // signature (size, parameters, workspace), replayed after that with the
+    // call's own buffers
+    cudaGraph_t single_graph = nullptr;
     cudaGraphExec_t single_exec = nullptr;
     std::vector<int64_t> single_sig, single_seen;
     long long single_launches = 0;
+    PairNodes single_nodes;
+    PairBuffers single_io;            // what the graph's next launch reads and writes
 
     // learned support-point proposal (off until weights are set)
     bool prop = false;
@@ -463,11 +480,25 @@ void free_pn(elas_handle* h) {
     if (h->pw.b) cudaFree(h->pw.b);
 }
 
+// The node that the last launch on a capturing stream became.
+cudaError_t last_node(cudaStream_t st, cudaGraphNode_t* node) {
+    cudaStreamCaptureStatus cs;
+    const cudaGraphNode_t* deps = nullptr;
+    const cudaGraphEdgeData* edges = nullptr;
+    size_t n = 0;
+    const cudaError_t e = cudaStreamGetCaptureInfo_v3(st, &cs, nullptr, nullptr, &deps, &edges, &n);
+    if (e != cudaSuccess) return e;
+    if (n != 1) return cudaErrorUnknown;
+    *node = deps[0];
+    return cudaSuccess;
+}
+
 // out0/out1 may be device-mapped pinned host memory: every intermediate stays
 // in device memory and only the last pass of each view writes there, so the
-// results cross PCIe while that pass computes.
+// results cross PCIe while that pass computes.  nodes (inside a capture of
+// the single-pair graph): receives the nodes that take the caller's buffers.
 int run_pipeline(elas_handle* h, const uint8_t* img0, const uint8_t* img1, float* out0, float* out1, int W, int H,
-                 cudaStream_t st) {
+                 cudaStream_t st, PairNodes* nodes = nullptr) {
     const elas_params& p = h->params;
     Geom g = geom_of(W, H, p);
     DevParams dp = dev_params(p);
@@ -493,6 +524,7 @@ int run_pipeline(elas_handle* h, const uint8_t* img0, const uint8_t* img1, float
                         dp.speckle_size > 0 ? int(2 * post_tickets(go.W, go.H)) : 0};
     CK(mark(ELAS_TIME_DESCRIPTOR));
     CK(launch_descriptor(img0, img1, h->desc0, h->desc1, W, H, zero, st));
+    if (nodes) CK(last_node(st, &nodes->desc));
     n += 1;
     CK(mark(ELAS_TIME_SUPPORT));
     if (h->pn_used) {
@@ -572,6 +604,11 @@ int run_pipeline(elas_handle* h, const uint8_t* img0, const uint8_t* img1, float
         CK(launch_lr(h->raw0, h->raw1, h->lr0, h->lr1, post ? nullptr : outs[0],
                      post && nviews == 2 ? nullptr : outs[1], g, p.lr_threshold, st, sub));
         n += 1;
+        if (nodes) {
+            CK(last_node(st, &nodes->lr));
+            nodes->lr_out[0] = !post;
+            nodes->lr_out[1] = !(post && nviews == 2);
+        }
     }
     CK(mark(ELAS_TIME_POST));
     if (post) {
@@ -590,6 +627,11 @@ int run_pipeline(elas_handle* h, const uint8_t* img0, const uint8_t* img1, float
         int last_args = 0;
         CK(launch_post(pv, lr, nviews, go, dp, p.filter_median, p.filter_adaptive_mean, h->err, st, &n, h->num_sms,
                        &last_args));
+        if (nodes) {
+            CK(last_node(st, &nodes->post));
+            nodes->post_views = nviews;
+            nodes->post_args = last_args;
+        }
     }
     CK(mark(ELAS_TIME_COUNT));
     h->launches += n;
@@ -597,13 +639,65 @@ int run_pipeline(elas_handle* h, const uint8_t* img0, const uint8_t* img1, float
     return ELAS_OK;
 }
 
-// run_pipeline through a cached CUDA graph.  A call whose signature was
-// not seen before runs eagerly (it sizes the workspaces and tunes the dense
+void drop_single_graph(elas_handle* h) {
+    if (h->single_exec) cudaGraphExecDestroy(h->single_exec);
+    if (h->single_graph) cudaGraphDestroy(h->single_graph);
+    h->single_exec = nullptr;
+    h->single_graph = nullptr;
+}
+
+// Point the captured pair at these buffers: the nodes that take them get new
+// arguments (a microsecond or two on the host, only when a buffer changed),
+// which launches already under way do not see.
+int bind_buffers(elas_handle* h, const PairBuffers& io) {
+    const PairNodes& nd = h->single_nodes;
+    PairBuffers& now = h->single_io;
+    cudaKernelNodeParams p;
+    void* args[16];
+    auto fetch = [&](cudaGraphNode_t node, int n) {
+        const cudaError_t e = cudaGraphKernelNodeGetParams(node, &p);
+        if (e == cudaSuccess) std::copy(p.kernelParams, p.kernelParams + n, args);
+        p.kernelParams = args;
+        return e;
+    };
+    if (io.img0 != now.img0 || io.img1 != now.img1) {
+        const uint8_t *i0 = io.img0, *i1 = io.img1;
+        CK(fetch(nd.desc, DESCRIPTOR_ARGS));
+        args[0] = &i0;
+        args[1] = &i1;
+        CK(cudaGraphExecKernelNodeSetParams(h->single_exec, nd.desc, &p));
+    }
+    if (io.out0 != now.out0 || io.out1 != now.out1) {
+        float *o0 = io.out0, *o1 = io.out1;
+        if (nd.lr && (nd.lr_out[0] || nd.lr_out[1])) {
+            CK(fetch(nd.lr, LR_ARGS));
+            if (nd.lr_out[0]) args[LR_ARG_C0] = &o0;
+            if (nd.lr_out[1]) args[LR_ARG_C0 + 1] = &o1;
+            CK(cudaGraphExecKernelNodeSetParams(h->single_exec, nd.lr, &p));
+        }
+        if (nd.post) {
+            CK(fetch(nd.post, nd.post_args));
+            PostViews pv = *static_cast<PostViews*>(args[0]);     // the last pass writes pv.nxt
+            pv.nxt[0] = o0;
+            if (nd.post_views > 1) pv.nxt[1] = o1;
+            args[0] = &pv;
+            CK(cudaGraphExecKernelNodeSetParams(h->single_exec, nd.post, &p));
+        }
+    }
+    now = io;
+    return ELAS_OK;
+}
+
+// run_pipeline through a cached CUDA graph.  A call whose signature was not
+// seen before runs eagerly (it sizes the workspaces and tunes the dense
 // shape); the next call with the same signature is captured on the handle's
 // own stream (the caller's stream may be the legacy default stream, which
 // cannot be captured) and launched into the caller's stream; later calls
-// only launch the graph.  A caller that is itself capturing gets the plain
-// launches, which join its capture.
+// only launch the graph, after pointing it at their buffers, so programs
+// that cycle through frame buffers replay it too (with the buffers part of
+// the signature, a double-buffered 640x480 stream ran eagerly every time:
+// two pairs 340 us; now 281).  A caller that is itself capturing gets
+// the plain launches, which join its capture.
 int run_pipeline_graphed(elas_handle* h, const uint8_t* img0, const uint8_t* img1, float* out0, float* out1, int W,
                          int H, cudaStream_t st) {
     cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
@@ -617,14 +711,19 @@ int run_pipeline_graphed(elas_handle* h, const uint8_t* img0, const uint8_t* img
         rc = ensure_pn(h, g);
         if (rc != ELAS_OK) return rc;
     }
-    std::vector<int64_t> sig = {int64_t(img0), int64_t(img1), int64_t(out0), int64_t(out1), W, H,
-                                int64_t(h->arena), int64_t(h->arena_bytes), int64_t(h->pn_in), int64_t(h->pn_bins),
+    // images on 16-byte boundaries take another descriptor kernel
+    const int64_t aligned = ((reinterpret_cast<uintptr_t>(img0) | reinterpret_cast<uintptr_t>(img1)) & 15) == 0;
+    std::vector<int64_t> sig = {aligned, W, H, int64_t(h->arena), int64_t(h->arena_bytes), int64_t(h->pn_in),
+                                int64_t(h->pn_bins),
                                 int64_t(h->pn_stats), h->timing ? 1 : 0, h->prop ? 1 : 0, h->prop_version,
                                 h->test_flags, h->flip_round_limit};
     int64_t pw[sizeof(elas_params) / 8 + 1] = {};
     std::memcpy(pw, &h->params, sizeof(elas_params));
     for (int64_t x : pw) sig.push_back(x);
+    const PairBuffers io{img0, img1, out0, out1};
     if (h->single_exec && sig == h->single_sig) {
+        rc = bind_buffers(h, io);
+        if (rc != ELAS_OK) return rc;
         CK(cudaGraphLaunch(h->single_exec, st));
         h->g = g;   // what run_pipeline leaves behind for the stage dumps
         h->pn_used = h->prop && H >= 4 && W >= 4 && g.cw > 0 && g.ch > 0;
@@ -637,18 +736,20 @@ int run_pipeline_graphed(elas_handle* h, const uint8_t* img0, const uint8_t* img
         return run_pipeline(h, img0, img1, out0, out1, W, H, st);
     }
     if (!h->own_stream) CK(cudaStreamCreateWithFlags(&h->own_stream, cudaStreamNonBlocking));
-    if (h->single_exec) { cudaGraphExecDestroy(h->single_exec); h->single_exec = nullptr; }
+    drop_single_graph(h);
     const long long before = h->launches;
     CK(cudaStreamBeginCapture(h->own_stream, cudaStreamCaptureModeThreadLocal));
-    rc = run_pipeline(h, img0, img1, out0, out1, W, H, h->own_stream);
-    cudaGraph_t graph = nullptr;
-    cudaError_t e = cudaStreamEndCapture(h->own_stream, &graph);
-    if (rc != ELAS_OK) { if (graph) cudaGraphDestroy(graph); return rc; }
-    if (e != cudaSuccess) return cuda_fail(h, e, "cudaStreamEndCapture");
-    e = cudaGraphInstantiate(&h->single_exec, graph, 0);
-    cudaGraphDestroy(graph);
-    if (e != cudaSuccess) { h->single_exec = nullptr; return cuda_fail(h, e, "cudaGraphInstantiate"); }
+    PairNodes nodes;
+    rc = run_pipeline(h, img0, img1, out0, out1, W, H, h->own_stream, &nodes);
+    cudaError_t e = cudaStreamEndCapture(h->own_stream, &h->single_graph);
+    if (rc == ELAS_OK && e == cudaSuccess) e = cudaGraphInstantiate(&h->single_exec, h->single_graph, 0);
+    if (rc != ELAS_OK || e != cudaSuccess) {
+        drop_single_graph(h);
+        return rc != ELAS_OK ? rc : cuda_fail(h, e, "capturing the pair's graph");
+    }
     h->single_sig = sig;
+    h->single_nodes = nodes;
+    h->single_io = io;
     h->single_launches = h->launches - before;
     CK(cudaGraphLaunch(h->single_exec, st));
     return ELAS_OK;
@@ -921,7 +1022,7 @@ int elas_b200_destroy(elas_handle* h) {
     if (h->batch_start) cudaEventDestroy(h->batch_start);
     if (h->lat_start) cudaEventDestroy(h->lat_start);
     free_pn(h);
-    if (h->single_exec) cudaGraphExecDestroy(h->single_exec);
+    drop_single_graph(h);
     if (h->own_stream) cudaStreamDestroy(h->own_stream);
     if (h->side) cudaStreamDestroy(h->side);
     if (h->side_fork) cudaEventDestroy(h->side_fork);

@@ -241,6 +241,44 @@ def test_device_api_matches_host_api(elas):
     assert np.array_equal(o1.cpu().numpy(), h1) and np.array_equal(o2.cpu().numpy(), h2)
 
 
+@pytest.mark.parametrize("mode", ["filters", "plain", "left_only", "left_only_plain", "speckle", "wide_gap",
+                                  "wide_gap_median", "subsampled"])
+def test_graph_replays_follow_the_callers_buffers(elas, mode):
+    """A replayed pair reads and writes the buffers of its own call, whichever
+    kernels take them: three sets of buffers in turn (one off a 16-byte
+    boundary), new contents each round, against the host-buffer call of a
+    second handle."""
+    import torch
+
+    W, H, D = 160, 120, 47
+    p = eb.params_config(D, post=mode in ("filters", "left_only", "subsampled"))
+    p.postprocess_only_left = mode.startswith("left_only")
+    p.subsampling = mode == "subsampled"
+    if mode == "speckle":
+        p.speckle_size = 50
+    if mode.startswith("wide_gap"):
+        p.ipol_gap_width = 100
+        p.filter_median = mode == "wide_gap_median"
+    elas.set_params(p)
+    other = eb.Elas(p)
+    shape = elas.out_shape(W, H)
+    sets = [[torch.zeros(W * H + 16, dtype=torch.uint8, device="cuda")[o:o + W * H] for _ in range(2)]
+            + [torch.full(shape, 9.0, device="cuda") for _ in range(2)] for o in (0, 0, 5)]
+    try:
+        for k in range(9):
+            L, R, _, _ = eb.synth_pair(3, 60 + k, width=W, height=H, disp_max=D)
+            b = sets[k % 3]
+            b[0].copy_(torch.from_numpy(L.reshape(-1)))
+            b[1].copy_(torch.from_numpy(R.reshape(-1)))
+            torch.cuda.synchronize()
+            elas.process_device(b[0].data_ptr(), b[1].data_ptr(), b[2].data_ptr(), b[3].data_ptr(), W, H)
+            torch.cuda.synchronize()
+            h1, h2 = other.process(L, R)
+            assert np.array_equal(b[2].cpu().numpy(), h1) and np.array_equal(b[3].cpu().numpy(), h2), k
+    finally:
+        other.close()
+
+
 @pytest.mark.parametrize("shift", [1, 3])
 def test_device_api_unaligned_images(elas, shift):
     """Device images that do not start on a 16-byte boundary take the
