@@ -5,6 +5,7 @@
 //
 // Both views run as two independent problems inside the same launches:
 // problem 0 triangulates (u, v), problem 1 triangulates (u - d, v).
+#include <algorithm>
 #include <climits>
 #include <cooperative_groups.h>
 #include <type_traits>
@@ -266,16 +267,22 @@ struct RowGeom {
 // the rows' offsets and unique counts, also in shared memory.  The rows'
 // extreme points are staged in shared memory; HULL_LANES lanes decide one of
 // them together (hull_on_chain's two minima over the other rows, each lane
-// every HULL_LANES-th row, then merged), both chains at once.
-constexpr int HULL_LANES = 8;
+// a share of the rows, then merged), both chains at once: first against the
+// HULL_GROUP rows around it, then what is left (a third) against what is
+// left, as a point inside the hull is inside the hull of the points that
+// their own groups keep.  One SM does this, bound by instruction issue:
+// against all rows at once the kernel took 7.2 us for 73 rows and 17.4 for
+// 214, now 6.7 and 10.2.
+constexpr int HULL_LANES = 8, HULL_GROUP = 16;
 __device__ void star_setup(const DelDev& D, const int32_t* roff, const int32_t* cnt, const int32_t* ne,
                            const int32_t* ney, int R, int npts, uint32_t* xyf, uint32_t* xyl, int32_t* lstk,
                            int32_t* rstk, int32_t* flag, int* ws) {
-    __shared__ int box_s[2];
+    __shared__ int box_s[2], left[2];
     const int tid = threadIdx.x, nt = blockDim.x, lane = tid & 31;
     if (tid == 0) {
         box_s[0] = INT_MAX;
         box_s[1] = INT_MIN;
+        left[0] = left[1] = 0;
     }
     __syncthreads();
     for (int s0 = tid - lane; s0 < R; s0 += nt) {
@@ -306,15 +313,16 @@ __device__ void star_setup(const DelDev& D, const int32_t* roff, const int32_t* 
     if (R < 2) return;
     // flag[i]: bit 0 on the left chain, bit 16 on the right one
     const int hl = tid % HULL_LANES;
-    for (int it = tid / HULL_LANES; it < ((2 * R + 3) & ~3); it += nt / HULL_LANES) {   // whole warps
-        const int side = it & 1, i = imin(it >> 1, R - 1);
+    // hull_on_chain for row i of a side against n rows, row(k) the k-th
+    auto on_chain = [&](int side, int i, int n, auto row) {
         const uint32_t* xy = side ? xyl : xyf;
         const uint32_t c = xy[i];
         const int sg = side ? -1 : 1;
         int32_t n0 = 1, e0 = 0, n1 = 1, e1 = 0;         // rows above and below; 1/0: +infinity
-#pragma unroll 4
-        for (int j = hl; j < R; j += HULL_LANES) {
-            const int32_t x = sg * dx_p(xy[j], c), y = dy_p(xy[j], c);
+#pragma unroll 2
+        for (int k = hl; k < n; k += HULL_LANES) {
+            const uint32_t v = xy[row(k)];
+            const int32_t x = sg * dx_p(v, c), y = dy_p(v, c);
             if (y < 0 && (e0 == 0 || x * e0 < n0 * -y)) { n0 = x; e0 = -y; }
             if (y > 0 && (e1 == 0 || x * e1 < n1 * y)) { n1 = x; e1 = y; }
         }
@@ -325,8 +333,21 @@ __device__ void star_setup(const DelDev& D, const int32_t* roff, const int32_t* 
             if (f0 != 0 && (e0 == 0 || m0 * e0 < n0 * f0)) { n0 = m0; e0 = f0; }
             if (f1 != 0 && (e1 == 0 || m1 * e1 < n1 * f1)) { n1 = m1; e1 = f1; }
         }
-        if (hl == 0 && it < 2 * R && (e0 == 0 || e1 == 0 || n0 * e1 + n1 * e0 >= 0))
-            atomicOr(&flag[i], side ? 1 << 16 : 1);
+        return e0 == 0 || e1 == 0 || n0 * e1 + n1 * e0 >= 0;
+    };
+    for (int it = tid / HULL_LANES; it < ((2 * R + 3) & ~3); it += nt / HULL_LANES) {   // whole warps
+        const int side = it & 1, i = imin(it >> 1, R - 1), b = i & ~(HULL_GROUP - 1);
+        const bool on = on_chain(side, i, imin(HULL_GROUP, R - b), [&](int k) { return b + k; });
+        if (hl == 0 && it < 2 * R && on) (side ? rstk : lstk)[atomicAdd(&left[side], 1)] = i;
+    }
+    __syncthreads();
+    const int n0 = left[0], n1 = left[1];
+    for (int it = tid / HULL_LANES; it < ((n0 + n1 + 3) & ~3); it += nt / HULL_LANES) {
+        const int side = it >= n0 && n1 > 0, q = imin(it, n0 + n1 - 1) - (side ? n0 : 0);
+        const int32_t* rows = side ? rstk : lstk;
+        const int i = rows[q];
+        const bool on = on_chain(side, i, side ? n1 : n0, [&](int k) { return rows[k]; });
+        if (hl == 0 && it < n0 + n1 && on) atomicOr(&flag[i], side ? 1 << 16 : 1);
     }
     __syncthreads();
     int nl = 0, nr = 0;
@@ -415,6 +436,8 @@ __global__ void __launch_bounds__(1024) k_plan(DelDev d0, DelDev d1, const int32
         if (flips && R >= 2 && !fits) set_err(err, ERRF_TRI_COUNT);
         D.ctr[0] = 0;
         D.ctr[1] = off;
+        D.ctr[2] = 0;    // pocket triangles of both sides
+        D.ctr[3] = 0;
         D.ctr[6] = R;
         D.ctr[7] = (flips && R >= 2 && fits) ? 1 : 0;
         D.ctr[8] = 0;    // set to 1 by the flip kernel that handles the problem
@@ -1066,88 +1089,152 @@ __global__ void __launch_bounds__(EMIT_THREADS) k_star_emit(DelDev d0, DelDev d1
     }
 }
 
-// The two hull pockets of one problem, walked at once by lanes 0 of warps 0
-// and 1, each on its own copy of the chain (in `sh` when R <= smem_rows,
-// else in D.chain); the right side writes behind the left one's room (at
-// most R-2 triangles) and is moved down when both are done.  Sets ctr[0].
-__device__ void pocket_block(const DelDev& D, const int32_t* __restrict__ row_off, int nrows, int smem_rows,
-                             int32_t* sh) {
-    __shared__ int npk[2];
-    const int R = D.ctr[6], off = D.ctr[1];
-    const bool in_smem = R <= smem_rows;
-    const int cap = in_smem ? smem_rows : nrows;
+// The two hull pockets of one problem (the triangles of fill_pockets, in its
+// order), every point on its own.  In the stack walk a point j is pushed onto
+// pred(j), the point above it whose direction from j is outermost (the
+// nearest of collinear ones), and pred(j) stays beneath it; j is popped by
+// the first later point i that lies strictly outside the line pred(j) -> j
+// (the chain being convex, such an i has popped everything above j before),
+// which makes the triangle (pred(j), j, i).  Triangles come in order of i
+// and, for one i, of falling j: a triangle's place is the number of smaller
+// keys (i, -j).  pocket_points finds every row's pred and key, POCKET_LANES
+// lanes a point, in blocks of k_strips; pocket_triangles places them in
+// blocks of the next kernel, which also sets the triangle count ctr[0].
+// Bound by latency (a chain of compares per point).  The walk itself, one
+// thread a side, took k_strips to 120 us at 2880x1988 (398 rows), all points
+// in one block 63; now 13.
+constexpr int POCKET_LANES = 8;
+struct PocketRows {                     // per side and row, in D.chain
+    int32_t *key, *pred, *idx;
+    __device__ PocketRows(const DelDev& D, int nrows, int side)
+        : key(D.chain + side * nrows), pred(D.chain + (2 + side) * nrows), idx(D.chain + (4 + side) * nrows) {}
+};
+// The points of block `part`; sh: the coordinates of both sides' rows.
+__device__ void pocket_points(const DelDev& D, const int32_t* __restrict__ row_off, int nrows, int part, int32_t* sh) {
+    const int R = D.ctr[6], lane = threadIdx.x & 31, pl = threadIdx.x % POCKET_LANES;
+    const int it = (part * int(blockDim.x) + int(threadIdx.x)) / POCKET_LANES;
+    if (part * int(blockDim.x) >= 2 * R * POCKET_LANES) return;
     for (int e = threadIdx.x; e < 2 * R; e += blockDim.x) {
-        const int side = e >= R, s = e - side * R;
-        int32_t* ci = (in_smem ? sh : D.chain) + side * 7 * cap;
-        const int r = D.ne[s];
-        const int i = D.srt[row_off[r] + (side ? D.rcnt[r] - 1 : 0)];
-        ci[s] = i; ci[cap + s] = D.x[i]; ci[2 * cap + s] = D.y[i];
+        const int side = e >= R, s = e - side * R, r = D.ne[s];
+        const int pos = row_off[r] + (side ? D.rcnt[r] - 1 : 0);
+        sh[e] = int32_t(D.sxy[pos]);
+        if (part == 0) PocketRows(D, nrows, side).idx[s] = D.srt[pos];
     }
     __syncthreads();
-    if ((threadIdx.x & 31) == 0 && threadIdx.x < 64) {
-        const int side = threadIdx.x >> 5;
-        int32_t* ci = (in_smem ? sh : D.chain) + side * 7 * cap;
-        npk[side] = fill_pockets(ci, ci + cap, ci + 2 * cap, R, side ? -1 : +1, ci + 3 * cap,
-                                 D.tri + 3 * size_t(off + side * R));
+    const int e = imin(it, 2 * R - 1), side = e >= R, j = e - side * R;
+    const int32_t* xy = sh + side * R;
+    const int sg = side ? -1 : 1;
+    const uint32_t c = uint32_t(xy[j]);
+    int pred = -1;
+    int32_t px = 0, ph = 0;                 // pred's offset (mirrored x) and height above j
+#pragma unroll 4
+    for (int a = pl; a < j; a += POCKET_LANES) {
+        const int32_t x = sg * dx_p(uint32_t(xy[a]), c), h = -dy_p(uint32_t(xy[a]), c);
+        if (pred < 0 || x * ph <= px * h) { pred = a; px = x; ph = h; }
     }
+#pragma unroll
+    for (int o = 1; o < POCKET_LANES; o <<= 1) {
+        const int qa = __shfl_xor_sync(0xffffffffu, pred, o);
+        const int32_t qx = __shfl_xor_sync(0xffffffffu, px, o), qh = __shfl_xor_sync(0xffffffffu, ph, o);
+        const int32_t l = qx * ph, g = px * qh;
+        if (qa >= 0 && (pred < 0 || l < g || (l == g && qa > pred))) { pred = qa; px = qx; ph = qh; }
+    }
+    // orient(pred, j, i) on the outer side, relative to j: pred is at (px, -ph)
+    int i = R;
+    for (int i0 = j + 1; __any_sync(0xffffffffu, pred >= 0 && i == R && i0 < R); i0 += POCKET_LANES) {
+        const int q = i0 + pl;
+        bool out = false;
+        if (pred >= 0 && q < R) {
+            const int32_t x = sg * dx_p(uint32_t(xy[q]), c), y = dy_p(uint32_t(xy[q]), c);
+            out = -px * y - ph * x > 0;
+        }
+        const unsigned all = __ballot_sync(0xffffffffu, out) >> (lane & ~(POCKET_LANES - 1));
+        const unsigned m = all & ((1u << POCKET_LANES) - 1u);
+        if (m && i == R) i = i0 + __ffs(m) - 1;
+    }
+    if (pl != 0 || it >= 2 * R) return;
+    const PocketRows P(D, nrows, side);
+    P.pred[j] = pred;
+    P.key[j] = i < R ? (i << 13 | (8191 - j)) : INT_MAX;
+    if (i < R) atomicAdd(&D.ctr[2 + side], 1);
+}
+// Each thread group places its point's triangle; sh: both sides' keys.
+__device__ void pocket_triangles(const DelDev& D, int nrows, int part, int32_t* sh) {
+    const int R = D.ctr[6], pl = threadIdx.x % POCKET_LANES;
+    const int it = (part * int(blockDim.x) + int(threadIdx.x)) / POCKET_LANES;
+    if (part * int(blockDim.x) >= 2 * R * POCKET_LANES) return;
+    for (int e = threadIdx.x; e < 2 * R; e += blockDim.x) sh[e] = D.chain[(e >= R) * nrows + e - (e >= R ? R : 0)];
     __syncthreads();
-    const int k0 = npk[0], k1 = npk[1];
-    // move the right side's triangles from off+R to off+k0 (k0 <= R-2, so
-    // a forward copy in rounds of one block never overwrites unread data)
-    for (int b0 = 0; b0 < 3 * k1; b0 += blockDim.x) {
-        const int j = b0 + threadIdx.x;
-        int32_t v = 0;
-        if (j < 3 * k1) v = D.tri[3 * size_t(off + R) + j];
-        __syncthreads();
-        if (j < 3 * k1) D.tri[3 * size_t(off + k0) + j] = v;
-        __syncthreads();
-    }
-    if (threadIdx.x == 0) D.ctr[0] = off + k0 + k1;
+    const int e = imin(it, 2 * R - 1), side = e >= R, j = e - side * R;
+    const int32_t mine = sh[e];
+    int k = 0;
+#pragma unroll 4
+    for (int q = pl; q < R; q += POCKET_LANES) k += sh[side * R + q] < mine;
+#pragma unroll
+    for (int o = 1; o < POCKET_LANES; o <<= 1) k += __shfl_xor_sync(0xffffffffu, k, o);
+    if (it >= 2 * R || mine == INT_MAX || pl != 0) return;
+    const PocketRows P(D, nrows, side);
+    const int32_t ia = P.idx[P.pred[j]], ib = P.idx[j], ii = P.idx[mine >> 13];
+    int32_t* t = D.tri + 3 * (size_t(D.ctr[1]) + (side ? D.ctr[2] : 0) + k);
+    t[0] = ia;
+    t[1] = side ? ii : ib;
+    t[2] = side ? ib : ii;
 }
 
-// Blocks [0, gridDim.x - 1): one thread per sorted point of a non-empty
-// row: the point's triangle in the strip below its row (as the upper row)
-// and in the strip above (as the lower row), placed by merge path.  The last
-// block walks the problem's two hull pockets meanwhile.
-__global__ void k_strips(DelDev d0, DelDev d1, const int32_t* __restrict__ row_off, int nrows, int nmax,
-                         int smem_rows) {
+// Block s < R: the points of non-empty row s, each placing its triangle in
+// the strip below the row (as the upper row) and in the strip above (as the
+// lower row) by merge path (strip_tri_upper, strip_tri_lower).  The x of the
+// two neighbouring rows are staged in shared memory, so the binary searches
+// do not chase loads (a thread finding its row and both places through
+// global memory: some fifty dependent loads).  The blocks from nrows on
+// find the hull pockets' points meanwhile.
+constexpr int STRIP_THREADS = 512;
+__global__ void __launch_bounds__(STRIP_THREADS) k_strips(DelDev d0, DelDev d1, const int32_t* __restrict__ row_off,
+                                                          int nrows) {
     grid_dep_wait();
     extern __shared__ int32_t sh[];
     const DelDev& D = blockIdx.y ? d1 : d0;
     if (D.ctr[7] == 0) return;
-    if (blockIdx.x == gridDim.x - 1) {
-        pocket_block(D, row_off, nrows, smem_rows, sh);
+    if (int(blockIdx.x) >= nrows) {
+        pocket_points(D, row_off, nrows, blockIdx.x - nrows, sh);
         return;
     }
-    const int R = D.ctr[6];
-    Pts P{D.x, D.y};
-    const int nb = gridDim.x - 1;
-    for (int g = blockIdx.x * blockDim.x + threadIdx.x; g < nmax; g += nb * blockDim.x) {
-        // g walks the support index space; map it to (row, position) through the row offsets
-        int lo = 0, hi = R;    // find the non-empty row whose range holds g
-        // rows are in support-index order, so binary search ne by row_off
+    const int R = D.ctr[6], s = blockIdx.x;
+    if (s >= R) return;
+    const int r = D.ne[s], b = row_off[r], n = D.rcnt[r];
+    const int ra = s > 0 ? D.ne[s - 1] : -1, rb = s + 1 < R ? D.ne[s + 1] : -1;
+    const int ba = ra >= 0 ? row_off[ra] : 0, na = ra >= 0 ? D.rcnt[ra] : 0;
+    const int bb = rb >= 0 ? row_off[rb] : 0, nb = rb >= 0 ? D.rcnt[rb] : 0;
+    int32_t* xa = sh;
+    int32_t* xb = sh + SORT_CAP;
+    for (int i = threadIdx.x; i < na; i += STRIP_THREADS) xa[i] = px_of(D.sxy[ba + i]);
+    for (int i = threadIdx.x; i < nb; i += STRIP_THREADS) xb[i] = px_of(D.sxy[bb + i]);
+    __syncthreads();
+    // how many of the sorted x[0..cnt) lie below v (or at it)
+    auto below = [](const int32_t* x, int cnt, int32_t v) {
+        int lo = 0, hi = cnt;
         while (lo < hi) {
-            int mid = (lo + hi) >> 1;
-            if (row_off[D.ne[mid] + 1] <= g) lo = mid + 1;
+            const int mid = (lo + hi) >> 1;
+            if (x[mid] < v) lo = mid + 1;
             else hi = mid;
         }
-        if (lo >= R) continue;
-        int r = D.ne[lo];
-        int k = g - row_off[r];
-        if (k < 1 || k >= D.rcnt[r]) continue;
-        const int32_t* A_row = D.srt + row_off[r];
-        int32_t tri[3];
-        if (lo + 1 < R) {       // as the upper row of strip lo
-            int rb = D.ne[lo + 1];
-            int pos = strip_tri_upper(P, A_row, D.srt + row_off[rb], D.rcnt[rb], k, tri);
-            int32_t* o = D.tri + 3 * size_t(D.soff[lo] + pos);
-            o[0] = tri[0]; o[1] = tri[1]; o[2] = tri[2];
+        return lo;
+    };
+    for (int k = 1 + threadIdx.x; k < n; k += STRIP_THREADS) {
+        const int x = px_of(D.sxy[b + k]), ik = D.srt[b + k], ip = D.srt[b + k - 1];
+        if (rb >= 0) {          // as the upper row of strip s: points below strictly left of x
+            const int j = imax(below(xb, nb, x) - 1, 0);
+            int32_t* o = D.tri + 3 * (size_t(D.soff[s]) + (k - 1) + j);
+            o[0] = ip;
+            o[1] = ik;
+            o[2] = D.srt[bb + j];
         }
-        if (lo >= 1) {          // as the lower row of strip lo-1
-            int ra = D.ne[lo - 1];
-            int pos = strip_tri_lower(P, D.srt + row_off[ra], D.rcnt[ra], A_row, k, tri);
-            int32_t* o = D.tri + 3 * size_t(D.soff[lo - 1] + pos);
-            o[0] = tri[0]; o[1] = tri[1]; o[2] = tri[2];
+        if (ra >= 0) {          // as the lower row of strip s - 1: points above at or left of x
+            const int i = imax(below(xa, na, x + 1) - 1, 0);
+            int32_t* o = D.tri + 3 * (size_t(D.soff[s - 1]) + i + (k - 1));
+            o[0] = D.srt[ba + i];
+            o[1] = ik;
+            o[2] = ip;
         }
     }
 }
@@ -1159,11 +1246,20 @@ __device__ __forceinline__ uint32_t hash_cap(int T) {
     return c;
 }
 
-__global__ void k_hash_clear(DelDev d0, DelDev d1) {
+// The last pocket_blocks blocks place the hull pockets' triangles.
+constexpr int CLEAR_THREADS = 256;
+__global__ void __launch_bounds__(CLEAR_THREADS) k_hash_clear(DelDev d0, DelDev d1, int nrows, int pocket_blocks) {
     grid_dep_wait();
+    extern __shared__ int32_t sh[];
     const DelDev& D = blockIdx.y ? d1 : d0;
-    uint32_t cap = hash_cap(D.ctr[0]);
-    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < cap && i < D.Hmax; i += gridDim.x * blockDim.x) {
+    const int T = D.ctr[7] ? D.ctr[1] + D.ctr[2] + D.ctr[3] : 0, clear = gridDim.x - pocket_blocks;
+    if (blockIdx.x == 0 && threadIdx.x == 0) D.ctr[0] = T;
+    if (int(blockIdx.x) >= clear) {
+        if (T) pocket_triangles(D, nrows, blockIdx.x - clear, sh);
+        return;
+    }
+    uint32_t cap = hash_cap(T);
+    for (uint32_t i = blockIdx.x * CLEAR_THREADS + threadIdx.x; i < cap && i < D.Hmax; i += clear * CLEAR_THREADS) {
         D.hkey[i] = HASH_EMPTY;
         D.hcnt[i] = 0;
     }
@@ -1859,15 +1955,14 @@ cudaError_t launch_delaunay(DelDev& d0, DelDev& d1, const int32_t* row_off, int 
         if (nlaunch) *nlaunch += 5;
         return cudaGetLastError();
     }
-    // the pocket walk's chain and stack (2 sides x (index, x, y, 4-int stack
-    // records) = 56 bytes a row) in shared memory up to 32 KiB; every block
-    // of k_strips carries it
-    const int smem_rows = imin(nrows, (32 * 1024) / 56);
-    const size_t smem = size_t(smem_rows) * 56;
-    int blocks = 4 * num_sms;
-    launch_k(k_strips, dim3(imax(1, imin(blocks, (nmax + 255) / 256)) + 1, 2), 256, smem, st, d0, d1, row_off,
-             nrows, nmax, smem_rows);
-    launch_k(k_hash_clear, dim3(blocks, 2), 256, 0, st, d0, d1);
+    // shared memory: two rows' coordinates, or the pockets' rows
+    const size_t smem = std::max(size_t(2) * nrows, size_t(2) * SORT_CAP) * sizeof(int32_t);
+    const int blocks = 4 * num_sms;
+    auto pockets = [&](int threads) { return (2 * nrows * POCKET_LANES + threads - 1) / threads; };
+    allow_smem(k_strips);
+    launch_k(k_strips, dim3(nrows + pockets(STRIP_THREADS), 2), STRIP_THREADS, smem, st, d0, d1, row_off, nrows);
+    launch_k(k_hash_clear, dim3(blocks + pockets(CLEAR_THREADS), 2), CLEAR_THREADS, size_t(2) * nrows * sizeof(int32_t),
+             st, d0, d1, nrows, pockets(CLEAR_THREADS));
     launch_k(k_hash_insert, dim3(blocks, 2), 256, 0, st, d0, d1, err);
     launch_k(k_link, dim3(blocks, 2), 256, 0, st, d0, d1, err);
     int launched = 6;

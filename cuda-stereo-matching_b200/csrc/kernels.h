@@ -15,7 +15,7 @@ struct DelDev {
     int32_t* rcnt;         // [rows] unique points per row
     int32_t* ne;           // [rows] non-empty rows
     int32_t* soff;         // [rows] strip triangle offsets
-    int32_t* chain;        // [14*rows] pocket walk scratch (2 sides) when it does not fit in shared memory
+    int32_t* chain;        // [6*rows] hull pockets: key, predecessor and point of each row, both sides
     int32_t* tri;          // [3*Tmax]
     int32_t* opp;          // [3*Tmax]
     uint32_t* txy;         // [3*Tmax] packed corner coordinates (global flip kernel)
@@ -28,7 +28,7 @@ struct DelDev {
     int32_t* cwl;          // cluster kernel: per-CTA worklists  [16 * 2 * 6 * 4096]
     int32_t* ccand;        // cluster kernel: per-CTA proposals  [16 * 2 * 6 * 4096]
     int32_t* cflips;       // cluster kernel: per-CTA flips      [16 * 6 * 4096]
-    int32_t* ctr;          // [16]: 0 triangles, 1 strip triangles, 4 flip rounds, 5 flips,
+    int32_t* ctr;          // [16]: 0 triangles, 1 strip and 2, 3 pocket triangles, 4 flip rounds, 5 flips,
                            //       6 non-empty rows, 8 handled by the cluster kernel, 9 points,
                            //       10 points of far, 11 star pool cursor, 12 unused (0),
                            //       13 window doublings that prove the stars
