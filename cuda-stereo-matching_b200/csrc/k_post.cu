@@ -187,8 +187,8 @@ __device__ __forceinline__ float lr_checked(float d, const float* __restrict__ o
     return fabsf(other_row[int(uw)] - d) > thr ? -1.0f : d;
 }
 
-// A CTA of 32 x 8 threads per 32x32 tile, each thread taking the tile rows
-// ty, ty + 8, ty + 16, ty + 24 (a warp holds one tile row at a time).  Bound
+// A CTA of 32 x ROWS threads per 32x32 tile, each thread taking the tile rows
+// ty, ty + ROWS, .. (a warp holds one tile row at a time).  Bound
 // by instruction issue and, on small images, by its chain of barriers, so
 // the nodes of the tile's forest are runs (connected pixels of one row, named
 // by their first pixel) and every decision about runs is made on ballots:
@@ -207,13 +207,16 @@ __device__ __forceinline__ float lr_checked(float d, const float* __restrict__ o
 // connected pair.
 // Check, tiles and borders as three kernels with a node per pixel: 3.7 + 15.6
 // + 9.0 us at 1242x375, 32 + 113 + 31 at 2880x1988; this kernel 21 and 136
-// (eight CTAs per SM; five: 25 and 182).
-constexpr int SPK_ROWS = 8;
-constexpr int SPK_RPT = SPK_T / SPK_ROWS;
-template <bool LR>
-__global__ void __launch_bounds__(SPK_T * SPK_ROWS, 8) k_spk_tile(PostViews pv, LrInput lr, int W, int H, float thr,
-                                                               unsigned* err) {
+// (eight CTAs per SM; five: 25 and 182).  While all tiles fit the SMs at once,
+// taller CTAs shorten the chain, as a warp does not go through four rows'
+// unions and finds one after the other: a row per warp (ROWS = 32) up to two
+// tiles per SM (160x120: 16.1 -> 12.4 us), two rows up to four (450x375: 18.3
+// -> 15.7).
+template <bool LR, int SPK_ROWS>
+__global__ void __launch_bounds__(SPK_T * SPK_ROWS, 64 / SPK_ROWS)
+    k_spk_tile(PostViews pv, LrInput lr, int W, int H, float thr, unsigned* err) {
     grid_dep_wait();
+    constexpr int SPK_RPT = SPK_T / SPK_ROWS;
     __shared__ float S[SPK_T][SPK_T];
     __shared__ int L[SPK_T * SPK_T];            // forest, at run heads only
     __shared__ int C[SPK_T * SPK_T];            // pixel counts, at tile-local roots
@@ -779,8 +782,13 @@ cudaError_t launch_post(PostViews pv, const LrInput& lr, int nviews, const Geom&
     const bool fuse = p.ipol_gap_width <= PGMAX && (p.ipol_gap_width > 0 || adaptive_mean || median);
     if (p.speckle_size > 0) {
         const dim3 tiles((W + SPK_T - 1) / SPK_T, (H + SPK_T - 1) / SPK_T, nviews);
-        launch_k(lr.d0 ? k_spk_tile<true> : k_spk_tile<false>, tiles, dim3(SPK_T, SPK_ROWS), 0, st, pv, lr, W, H,
-                 p.speckle_sim_threshold, err);
+        const int per_sm = (int(tiles.x * tiles.y * tiles.z) + num_sms - 1) / num_sms;
+        const int rows = per_sm <= 2 ? 32 : (per_sm <= 4 ? 16 : 8);
+        const dim3 threads(SPK_T, rows);
+        auto kern = rows == 32 ? (lr.d0 ? k_spk_tile<true, 32> : k_spk_tile<false, 32>)
+                  : rows == 16 ? (lr.d0 ? k_spk_tile<true, 16> : k_spk_tile<false, 16>)
+                               : (lr.d0 ? k_spk_tile<true, 8> : k_spk_tile<false, 8>);
+        launch_k(kern, tiles, threads, 0, st, pv, lr, W, H, p.speckle_sim_threshold, err);
         const int gn = imax(1, imin(8 * 1024, (n + 255) / 256));
         // the roots list is far shorter than the image: a grid of one CTA per
         // SM walks it (idle CTAs cost their launch; measured against four)
