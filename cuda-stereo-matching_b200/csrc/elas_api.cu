@@ -62,6 +62,7 @@ struct elas_handle {
     int32_t *can_lr = nullptr, *can = nullptr, *row_cnt = nullptr, *row_off = nullptr;
     int32_t *uvd = nullptr, *x0 = nullptr, *x1 = nullptr, *y = nullptr;
     uint32_t *gtmp0 = nullptr, *gtmp1 = nullptr, *grid0 = nullptr, *grid1 = nullptr;
+    int16_t *list0 = nullptr, *list1 = nullptr;
     DelDev del[2]{};
     uint32_t *prior0 = nullptr, *prior1 = nullptr;
     void* rast = nullptr;   // per-triangle plane/edge set-up of both views
@@ -260,6 +261,8 @@ size_t layout(elas_handle* h, const Geom& g, char* base) {
     h->gtmp1 = (uint32_t*)take(cells * 4);
     h->grid0 = (uint32_t*)take(cells * 4);
     h->grid1 = (uint32_t*)take(cells * 4);
+    h->list0 = (int16_t*)take(size_t(g.gw) * g.gh * CELL_LIST * 2);
+    h->list1 = (int16_t*)take(size_t(g.gw) * g.gh * CELL_LIST * 2);
     for (int k = 0; k < 2; ++k) {
         DelDev& D = h->del[k];
         D.srt = (int32_t*)take(nmax * 4);
@@ -403,8 +406,8 @@ int dense_threads_for(elas_handle* h, const Geom& g, const DevParams& dp, cudaSt
         float shape_ms = 1e30f;
         for (int rep = 0; rep < 3; ++rep) {
             CK(cudaEventRecord(e0, st));
-            CK(launch_dense(h->desc0, h->desc1, h->prior0, h->prior1, h->grid0, h->grid1, h->raw0, h->raw1, g, dp,
-                            prior_shift(g, dp), h->err, st, shape, sub));
+            CK(launch_dense(h->desc0, h->desc1, h->prior0, h->prior1, h->grid0, h->grid1, h->list0, h->list1,
+                            h->raw0, h->raw1, g, dp, prior_shift(g, dp), h->err, st, shape, sub));
             CK(cudaEventRecord(e1, st));
             CK(cudaEventSynchronize(e1));
             float ms = 0;
@@ -559,7 +562,7 @@ int run_pipeline(elas_handle* h, const uint8_t* img0, const uint8_t* img1, float
         if (!h->side_join) CK(cudaEventCreateWithFlags(&h->side_join, cudaEventDisableTiming));
         CK(cudaEventRecordWithFlags(h->side_fork, st, 0));
         CK(cudaStreamWaitEvent(h->side, h->side_fork, 0));
-        CK(launch_grid(h->can, h->gtmp0, h->gtmp1, h->grid0, h->grid1, g, h->side, &n));
+        CK(launch_grid(h->can, h->gtmp0, h->gtmp1, h->grid0, h->grid1, h->list0, h->list1, g, h->side, &n));
         if (!tiled) {
             CK(cudaMemsetAsync(h->prior0, 0, size_t(W) * H * sizeof(uint32_t), h->side));
             CK(cudaMemsetAsync(h->prior1, 0, size_t(W) * H * sizeof(uint32_t), h->side));
@@ -568,7 +571,7 @@ int run_pipeline(elas_handle* h, const uint8_t* img0, const uint8_t* img1, float
         }
         CK(cudaEventRecordWithFlags(h->side_join, h->side, 0));
     } else {
-        CK(launch_grid(h->can, h->gtmp0, h->gtmp1, h->grid0, h->grid1, g, st, &n));
+        CK(launch_grid(h->can, h->gtmp0, h->gtmp1, h->grid0, h->grid1, h->list0, h->list1, g, st, &n));
     }
     CK(mark(ELAS_TIME_DELAUNAY));
     const bool flips = (h->test_flags & (ELAS_TEST_DELAUNAY_FLIPS | ELAS_TEST_FLIP_GLOBAL)) != 0 ||
@@ -588,8 +591,9 @@ int run_pipeline(elas_handle* h, const uint8_t* img0, const uint8_t* img1, float
     rc = dense_threads_for(h, g, dp, st, &n, &shape);
     if (rc != ELAS_OK) return rc;
     CK(mark(ELAS_TIME_DENSE));
-    CK(launch_dense(h->desc0, h->desc1, h->prior0, h->prior1, h->grid0, h->grid1, h->raw0, h->raw1, g, dp,
-                    prior_shift(g, dp), h->err, st, shape, sub, (h->test_flags & ELAS_TEST_DENSE_BITSET) != 0));
+    CK(launch_dense(h->desc0, h->desc1, h->prior0, h->prior1, h->grid0, h->grid1, h->list0, h->list1,
+                    h->raw0, h->raw1, g, dp, prior_shift(g, dp), h->err, st, shape, sub,
+                    (h->test_flags & ELAS_TEST_DENSE_BITSET) != 0));
     n += 1;
     CK(mark(ELAS_TIME_LR));
     // The post-filters start from the checked maps and write the outputs in

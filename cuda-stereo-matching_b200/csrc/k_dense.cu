@@ -374,10 +374,6 @@ __global__ void __launch_bounds__(256) k_prior_tiles(const Raster* __restrict__ 
     }
 }
 
-// Candidate-list entries per grid cell kept in shared memory; cells with
-// more candidates walk their bitset instead.
-constexpr int LMAX = 48;
-
 // Energy update with the reference's strict '<' (the first minimum in
 // evaluation order wins).
 // Both passes (the cell list, then the plane window) walk their
@@ -390,29 +386,38 @@ __device__ __forceinline__ int pk_ed(int e, int d) { return e * 4096 + d; }
 __device__ __forceinline__ void take_min(int e, int d, int& best) { best = min(best, pk_ed(e, d)); }
 
 // blockIdx.x = row, blockIdx.y = view (0 left, 1 right).  The other view's
-// descriptor row arrives by bulk copy (TMA) while the CTA expands the
-// candidate lists of the row's grid cells into shared memory.
+// descriptor row and the candidate lists of the row's grid cells arrive by
+// bulk copy (TMA).
+//
+// Instruction issue bounds it (82% of the issue slots while a 2880x1988
+// pair's rows run; 127 us): per candidate a 16-byte shared load, four
+// absolute-difference sums, the address and the packed minimum.  40
+// registers keep three CTAs of 512 threads on an SM (without the bound 50,
+// and two); the CTA's size is timed per shape by the caller.
 //
 // Per pixel u the reference evaluates the cell's sorted list, skipping the
 // plane window [d_plane - r, d_plane + r] and every d whose warped column
 // leaves [3, W - 3), then the window with the penalty added.  Here:
 //   * the warped-column test is one bound on d (dlim below): the left view
 //     needs d <= u - 3, the right view d <= W - 4 - u, every other bound
-//     holds for 3 < u < W - 3; the list is ascending, so the walk stops at
-//     the first d > dlim;
+//     holds for 3 < u < W - 3; the list is ascending, so what lies beyond
+//     dlim is cut from its end before the walk (a list's number is even,
+//     with its last disparity twice, which changes no minimum);
 //   * when every window penalty is negative (the usual parameters), the
 //     window entries need no skipping in the list walk: the window pass
 //     re-evaluates each of them with a strictly lower energy, so it ends
 //     at the same (value, first index) as the reference's walk;
-//   * RFIX > 0 unrolls the window for plane_radius == RFIX;
+//   * RFIX > 0 unrolls the window for plane_radius == RFIX, without a test
+//     per disparity where all of it is allowed;
 //   * the own descriptor and the prior of the thread's next pixel are
 //     loaded before the current pixel is matched.
 template <int RFIX>
-__global__ void __launch_bounds__(1024) k_dense(const uint4* __restrict__ desc0, const uint4* __restrict__ desc1,
-                                               const uint32_t* __restrict__ prior0, const uint32_t* __restrict__ prior1,
-                                               const uint32_t* __restrict__ grid0, const uint32_t* __restrict__ grid1,
-                                               float* __restrict__ disp0, float* __restrict__ disp1, Geom g,
-                                               DevParams p, int pshift, int sub, int lcap, unsigned* err) {
+__global__ void __maxnreg__(40) k_dense(const uint4* __restrict__ desc0, const uint4* __restrict__ desc1,
+                                         const uint32_t* __restrict__ prior0, const uint32_t* __restrict__ prior1,
+                                         const uint32_t* __restrict__ grid0, const uint32_t* __restrict__ grid1,
+                                         const int16_t* __restrict__ list0, const int16_t* __restrict__ list1,
+                                         float* __restrict__ disp0, float* __restrict__ disp1, Geom g, DevParams p,
+                                         int pshift, int sub, int lcap, unsigned* err) {
     grid_dep_wait();
     extern __shared__ __align__(128) uint8_t sm[];
     __shared__ uint64_t bar;
@@ -429,30 +434,17 @@ __global__ void __launch_bounds__(1024) k_dense(const uint4* __restrict__ desc0,
     }
     uint4* row = reinterpret_cast<uint4*>(sm);
     int16_t* lst = reinterpret_cast<int16_t*>(sm + size_t(W) * 16);
-    uint8_t* lcnt = reinterpret_cast<uint8_t*>(lst + size_t(g.gw) * LMAX);
+    const int gy = floordiv(v, g.gs);
     const uint4* self = (right ? desc1 : desc0) + size_t(v) * W;
     const uint4* other = (right ? desc0 : desc1) + size_t(v) * W;
     const uint32_t* prior = (right ? prior1 : prior0) + size_t(v) * W;
     const uint32_t* grid = right ? grid1 : grid0;
     if (tid == 0) {
         mbar_init(&bar, 1);
-        mbar_expect_tx(&bar, unsigned(W) * 16u);
+        const unsigned lbytes = unsigned(g.gw) * CELL_LIST * 2;
+        mbar_expect_tx(&bar, unsigned(W) * 16u + lbytes);
         bulk_g2s_chunked(row, other, unsigned(W) * 16u, &bar);
-    }
-    const int gy = floordiv(v, g.gs);
-    for (int c = tid; c < g.gw; c += NT) {
-        const uint32_t* cell = grid + (size_t(gy) * g.gw + c) * g.words;
-        int n = 0;
-        for (int w = 0; w < g.words; ++w) {
-            uint32_t bits = cell[w];
-            while (bits) {
-                int d = 32 * w + __ffs(bits) - 1;
-                bits &= bits - 1;
-                if (n < lcap) lst[c * LMAX + n] = int16_t(d);
-                ++n;
-            }
-        }
-        lcnt[c] = uint8_t(n > lcap ? 255 : n);
+        bulk_g2s_chunked(lst, (right ? list1 : list0) + size_t(gy) * g.gw * CELL_LIST, lbytes, &bar);
     }
     // first pixel of this thread and its prefetch
     int o = tid, u = o << sub;
@@ -490,30 +482,34 @@ __global__ void __launch_bounds__(1024) k_dense(const uint4* __restrict__ desc0,
             const int dpmin = imax(dp - r, 0);
             const int dpmax = imin(dp + r, g.D);
             int best_l = PK_NONE, best_w = PK_NONE;
-            const int n = lcnt[c];
-            if (n != 255) {
-                const int16_t* Ls = lst + c * LMAX;
+            const int16_t* Ls = lst + c * CELL_LIST;
+            int n = Ls[CELL_LIST - 1];
+            if (n <= lcap) {
                 int i = 0;
+                while (n > 0 && Ls[n - 1] > dlim) --n;
                 if (p.window_negative) {
-                    const uint32_t* L2 = reinterpret_cast<const uint32_t*>(Ls);
-                    for (; i + 1 < n; i += 2) {
-                        const uint32_t pr = L2[i >> 1];
+                    const auto pair = [&](uint32_t pr) {
                         const int da = int(pr & 0xffffu), db = int(pr >> 16);
-                        if (db > dlim) break;
                         const int ea = sad16(I1, row[u + dir * da]);
                         const int eb = sad16(I1, row[u + dir * db]);
-                        take_min(ea, da, best_l);
-                        take_min(eb, db, best_l);
+                        best_l = min(best_l, min(pk_ed(ea, da), pk_ed(eb, db)));
+                    };
+                    for (; i + 3 < n; i += 4) {
+                        const uint2 q = *reinterpret_cast<const uint2*>(Ls + i);
+                        pair(q.x);
+                        pair(q.y);
                     }
-                    for (; i < n; ++i) {
+                    if (i + 1 < n) {
+                        pair(*reinterpret_cast<const uint32_t*>(Ls + i));
+                        i += 2;
+                    }
+                    if (i < n) {
                         const int d = Ls[i];
-                        if (d > dlim) break;
                         take_min(sad16(I1, row[u + dir * d]), d, best_l);
                     }
                 } else {
                     for (; i < n; ++i) {
                         const int d = Ls[i];
-                        if (d > dlim) break;
                         if (d >= dpmin && d <= dpmax) continue;
                         take_min(sad16(I1, row[u + dir * d]), d, best_l);
                     }
@@ -532,7 +528,12 @@ __global__ void __launch_bounds__(1024) k_dense(const uint4* __restrict__ desc0,
                     }
                 }
             }
-            if (RFIX > 0) {
+            if (RFIX > 0 && dp >= RFIX && dp + RFIX <= imin(g.D, dlim)) {
+                const uint4* at = row + (u + dir * dp);
+#pragma unroll
+                for (int k = -RFIX; k <= RFIX; ++k)
+                    take_min(sad16(I1, at[k], p.penalty[k < 0 ? -k : k]), dp + dir * k, best_w);
+            } else if (RFIX > 0) {
 #pragma unroll
                 for (int k = -RFIX; k <= RFIX; ++k) {
                     const int d = dp + k;
@@ -622,26 +623,26 @@ cudaError_t launch_prior(const int32_t* tri0, const int32_t* tri1, const int32_t
 
 size_t raster_bytes() { return sizeof(Raster); }
 
-size_t dense_smem_bytes(const Geom& g) { return size_t(g.W) * 16 + size_t(g.gw) * (LMAX * 2 + 1); }
+size_t dense_smem_bytes(const Geom& g) { return size_t(g.W) * 16 + size_t(g.gw) * CELL_LIST * 2; }
 
 cudaError_t launch_dense(const uint4* desc0, const uint4* desc1, const uint32_t* prior0, const uint32_t* prior1,
-                         const uint32_t* grid0, const uint32_t* grid1, float* disp0, float* disp1, const Geom& g,
-                         const DevParams& p, int pshift, unsigned* err, cudaStream_t st, int threads, int sub,
-                         bool force_bitset) {
-    // list capacity per cell (0 sends every non-empty cell to the bitset walk)
-    const int lcap = force_bitset ? 0 : LMAX;
+                         const uint32_t* grid0, const uint32_t* grid1, const int16_t* list0, const int16_t* list1,
+                         float* disp0, float* disp1, const Geom& g, const DevParams& p, int pshift, unsigned* err,
+                         cudaStream_t st, int threads, int sub, bool force_bitset) {
+    // candidates a cell's list may hold (0 sends every non-empty cell to the bitset walk)
+    const int lcap = force_bitset ? 0 : CELL_LIST_MAX;
     size_t smem = dense_smem_bytes(g);
     if (threads <= 0) threads = 512;
     threads = imin(threads, (((g.W >> sub) + 31) / 32) * 32);
     const dim3 grid(g.H >> sub, 2);
     if (p.plane_radius == 2) {
         allow_smem(k_dense<2>);
-        launch_k(k_dense<2>, grid, threads, smem, st, desc0, desc1, prior0, prior1, grid0, grid1, disp0, disp1, g, p,
-                                                pshift, sub, lcap, err);
+        launch_k(k_dense<2>, grid, threads, smem, st, desc0, desc1, prior0, prior1, grid0, grid1, list0, list1, disp0,
+                 disp1, g, p, pshift, sub, lcap, err);
     } else {
         allow_smem(k_dense<0>);
-        launch_k(k_dense<0>, grid, threads, smem, st, desc0, desc1, prior0, prior1, grid0, grid1, disp0, disp1, g, p,
-                                                pshift, sub, lcap, err);
+        launch_k(k_dense<0>, grid, threads, smem, st, desc0, desc1, prior0, prior1, grid0, grid1, list0, list1, disp0,
+                 disp1, g, p, pshift, sub, lcap, err);
     }
     return cudaGetLastError();
 }

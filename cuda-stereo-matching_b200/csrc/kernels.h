@@ -77,8 +77,13 @@ cudaError_t launch_support(const uint4* desc0, const uint4* desc1, int32_t* can_
 cudaError_t launch_compact(const int32_t* can, const int32_t* row_cnt, int32_t* row_off, int32_t* uvd, int32_t* x0,
                            int32_t* x1, int32_t* y, const Geom& g, cudaStream_t st, int corners, int* nlaunch);
 
+// A grid cell's candidate list for the dense step: CELL_LIST 16-bit slots (a
+// multiple of 16 bytes, for the bulk copies), the first CELL_LIST_MAX for
+// the disparities, the last one for their number, which is larger than
+// CELL_LIST_MAX where the list does not hold the cell (its bitset does).
+constexpr int CELL_LIST = 48, CELL_LIST_MAX = CELL_LIST - 2;
 cudaError_t launch_grid(const int32_t* can, uint32_t* tmp0, uint32_t* tmp1, uint32_t* grid0, uint32_t* grid1,
-                        const Geom& g, cudaStream_t st, int* nlaunch);
+                        int16_t* list0, int16_t* list1, const Geom& g, cudaStream_t st, int* nlaunch);
 
 // Default: every point's star found directly (k_star).  flips: row strips
 // and Lawson edge flips instead; then force_global flips every problem with
@@ -131,8 +136,9 @@ size_t raster_bytes();
 
 size_t dense_smem_bytes(const Geom& g);
 cudaError_t launch_dense(const uint4* desc0, const uint4* desc1, const uint32_t* prior0, const uint32_t* prior1,
-                         const uint32_t* grid0, const uint32_t* grid1, float* disp0, float* disp1, const Geom& g,
-                         const DevParams& p, int pshift, unsigned* err, cudaStream_t st, int threads, int sub = 0,
+                         const uint32_t* grid0, const uint32_t* grid1, const int16_t* list0, const int16_t* list1,
+                         float* disp0, float* disp1, const Geom& g, const DevParams& p, int pshift, unsigned* err,
+                         cudaStream_t st, int threads, int sub = 0,
                          bool force_bitset = false);
 
 // L/R check into o0/o1 and, where given, also into c0 and c1 (arguments

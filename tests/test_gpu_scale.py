@@ -192,6 +192,22 @@ def test_forced_dense_bitset_walk(elas, preset, seed):
     assert np.array_equal(g["disp_right"].reshape(-1), ref[1])
 
 
+@pytest.mark.parametrize("disp_max", [31, 255, 256, 511, 512, 1100])
+def test_candidate_lists_at_word_counts(elas, disp_max):
+    """Candidate lists made by 8, 16 and 32 threads per cell and by several
+    passes of 32, against the oracle and the cells' bitsets."""
+    L, R, _, _ = eb.synth_pair(3, 71, width=700, height=83, disp_max=min(disp_max, 300))
+    p = eb.params_config(disp_max)
+    _, _, g = run_and_compare(elas, L, R, p, check_triangle=False)
+    elas.set_test_mode(eb.Elas.TEST_DENSE_BITSET)
+    try:
+        _, _, b = run_and_compare(elas, L, R, p, check_triangle=False)
+    finally:
+        elas.set_test_mode(0)
+    for k in ("disp_left", "disp_right"):
+        assert np.array_equal(g[k], b[k])
+
+
 @pytest.mark.parametrize("preset,seed,flag", [(1, 61, "TEST_PRIOR_TILED"), (2, 62, "TEST_PRIOR_DIRECT"),
                                                (1, 63, "TEST_PRIOR_TILED TEST_PRIOR_SMALL_BINS"),
                                                (2, 64, "TEST_PRIOR_SMALL_BINS")])
