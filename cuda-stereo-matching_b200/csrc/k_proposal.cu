@@ -71,21 +71,26 @@ __global__ void k_bf16_to_f32(const __nv_bfloat16* __restrict__ in, float* __res
 
 // ---------------------------------------------------------------------------
 // Training convolution (fp32).  Bound by the FP32 pipes (9216 FMAs a cell),
-// so the design keeps their operands in registers: a CTA computes an 8 x 32
-// cell tile, a thread 8 cells of one tile row x 4 output channels.  Per
-// four input channels of a tap it loads 8 + 4 16-byte words from shared
-// memory for 128 FMAs (a thread per output needed two loads per FMA and
-// ran at a tenth of the peak).  The input tile is padded to 36 floats a cell:
-// the four cell groups of a warp then read distinct banks, and the weight
-// words are shared by them.  CTAs are persistent (two per SM), so the
-// weights are staged once.  Sums run over taps, then input channels, in
-// order, as one chain per output.  `mask` (nullable) multiplies each input
-// value by (mask > 0): the ReLU derivative when this kernel computes the
-// gradient of the layer input.
-// 32 images of 93 x 310 cells: 1726 us -> 440 us a layer.
-constexpr int CT_H = 8, CT_W = 32, CT_STRIDE = CH + 4, CT_THREADS = 256;
-constexpr size_t CONV_F32_SMEM = sizeof(float) * (TAPS * CH * CH + (CT_H + 2) * (CT_W + 2) * CT_STRIDE);
-static_assert(CT_THREADS * 32 == CT_H * CT_W * CH && CT_THREADS / 32 == CT_H, "a warp per tile row");
+// so two of them go in one instruction (twice 32 bits, rounded as two
+// separate ones) and their operands stay in registers: a thread computes 16
+// cells x 4 output channels, as eight pairs of cells eight rows apart, and
+// loads 16 + 4 words from shared memory per input channel for 64 FMAs (8
+// cells x 4 channels, one FMA an instruction: 12 words for 32 FMAs, 440 us a
+// layer; 16 x 8, half as many warps: 457).  A group of 256 threads takes a
+// 16 x 32 cell tile, held in shared memory with the two rows of a pair side
+// by side, so that a pair's values arrive in one register pair at every tap;
+// CT_PITCH values a cell let the cells of a warp read distinct banks.  One
+// CTA per SM holds the weights and two such groups, each with a tile and a
+// barrier of its own: one computes while the other stages.  Sums run over
+// taps, then input channels, in order, as one chain per output.  `mask`
+// (nullable) multiplies each input value by (mask > 0): the ReLU derivative
+// when this kernel computes the gradient of the layer input.
+// 32 images of 93 x 310 cells: 1726 us -> 361 us a layer (the FMAs alone: 252).
+constexpr int CT_H = 16, CT_W = 32, CT_PITCH = CH + 2, CT_GROUP = 256, CT_GROUPS = 2;
+constexpr int CT_THREADS = CT_GROUP * CT_GROUPS, CT_PAIRS = CT_H / 2 + 2;      // row pairs with the halo
+constexpr int CT_TILE = CT_PAIRS * (CT_W + 2) * CT_PITCH;                       // float2 of one tile
+constexpr size_t CONV_F32_SMEM = sizeof(float) * (TAPS * CH * CH + CT_GROUPS * CT_TILE * 2);
+static_assert(CT_GROUP / 32 == CT_H / 2 && CT_W == 32 && CH == 32, "a warp per row pair");
 
 // Four channels of one cell; vec: the base is 16-byte aligned.
 __device__ __forceinline__ float4 load4(const float* p, bool vec) {
@@ -96,7 +101,26 @@ __device__ __forceinline__ float4 masked4(float4 v, float4 m) {
                        m.w > 0.0f ? v.w : 0.0f);
 }
 
-__global__ void __launch_bounds__(CT_THREADS, 2) k_conv_f32(const float* __restrict__ x,
+// Two FP32 values in a register pair: one instruction multiplies and adds both.
+__device__ __forceinline__ uint64_t pack2(float lo, float hi) {
+    uint64_t r;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(lo), "f"(hi));
+    return r;
+}
+__device__ __forceinline__ float2 unpack2(uint64_t v) {
+    float2 r;
+    asm("mov.b64 {%0, %1}, %2;" : "=f"(r.x), "=f"(r.y) : "l"(v));
+    return r;
+}
+__device__ __forceinline__ void fma2(uint64_t& acc, uint64_t a, uint64_t b) {
+    asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(acc) : "l"(a), "l"(b));
+}
+
+__device__ __forceinline__ void group_sync(int group) {
+    asm volatile("bar.sync %0, %1;" ::"r"(group + 1), "n"(CT_GROUP) : "memory");
+}
+
+__global__ void __launch_bounds__(CT_THREADS, 1) k_conv_f32(const float* __restrict__ x,
                                                             const float* __restrict__ mask,
                                                             const float* __restrict__ w, const float* __restrict__ b,
                                                             float* __restrict__ y, int nimg, int Hd, int Wd, int relu,
@@ -104,73 +128,99 @@ __global__ void __launch_bounds__(CT_THREADS, 2) k_conv_f32(const float* __restr
     grid_dep_wait();
     extern __shared__ __align__(16) float conv_sm[];
     float* sw = conv_sm;                        // [TAPS][ci][co]
-    float* sx = conv_sm + TAPS * CH * CH;       // [CT_H + 2][CT_W + 2][CT_STRIDE]
-    const int tid = threadIdx.x, cog = tid & 7, cg = (tid >> 3) & 3, row = tid >> 5;
-    for (int i = tid; i < TAPS * CH * CH; i += CT_THREADS) sw[i] = w[i];
-    float bias[4];
-#pragma unroll
-    for (int c = 0; c < 4; ++c) bias[c] = b ? b[4 * cog + c] : 0.0f;
+    const int group = threadIdx.x / CT_GROUP, tid = threadIdx.x % CT_GROUP;
+    // [CT_PAIRS][CT_W + 2][CT_PITCH]
+    float2* sx = reinterpret_cast<float2*>(conv_sm + TAPS * CH * CH) + group * CT_TILE;
+    const int cog = tid & 7, cg = (tid >> 3) & 3, rp = tid >> 5;
+    for (int i = threadIdx.x; i < TAPS * CH * CH; i += CT_THREADS) sw[i] = w[i];
+    __syncthreads();
     const int tx = (Wd + CT_W - 1) / CT_W, ty = (Hd + CT_H - 1) / CT_H;
     const long long ntiles = (long long)nimg * tx * ty;
-    for (long long tile = blockIdx.x; tile < ntiles; tile += gridDim.x) {
+    for (long long tile = blockIdx.x + (long long)group * gridDim.x; tile < ntiles;
+         tile += CT_GROUPS * (long long)gridDim.x) {
         const int n = int(tile / (tx * ty)), q = int(tile % (tx * ty));
         const int r0 = q / tx * CT_H, c0 = q % tx * CT_W;
-        __syncthreads();
-        for (int i = tid; i < (CT_H + 2) * (CT_W + 2) * (CH / 4); i += CT_THREADS) {
-            const int k = i % (CH / 4), j = (i / (CH / 4)) % (CT_W + 2), r = i / (CH / 4 * (CT_W + 2));
-            const int yy = r0 + r - 1, xx = c0 + j - 1;
-            float4 v = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-            if (yy >= 0 && yy < Hd && xx >= 0 && xx < Wd) {
-                const size_t at = ((size_t(n) * Hd + yy) * Wd + xx) * CH + 4 * k;
-                v = load4(x + at, vec);
-                if (mask) v = masked4(v, load4(mask + at, vec));
+        group_sync(group);              // the tile before has been read
+        {
+            const int k = tid % (CH / 4);
+            int r = 0, j = tid / (CH / 4);
+            const auto word = [&](int yy, int xx) {
+                float4 v = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+                if (yy >= 0 && yy < Hd && xx >= 0 && xx < Wd) {
+                    const size_t at = ((size_t(n) * Hd + yy) * Wd + xx) * CH + 4 * k;
+                    v = load4(x + at, vec);
+                    if (mask) v = masked4(v, load4(mask + at, vec));
+                }
+                return v;
+            };
+#pragma unroll 4
+            for (int i = tid; i < CT_PAIRS * (CT_W + 2) * (CH / 4); i += CT_GROUP) {
+                const int yy = r0 + r - 1, xx = c0 + j - 1;
+                const float4 lo = word(yy, xx), hi = word(yy + CT_H / 2, xx);
+                float4* o = reinterpret_cast<float4*>(sx + (r * (CT_W + 2) + j) * CT_PITCH + 4 * k);
+                o[0] = make_float4(lo.x, hi.x, lo.y, hi.y);
+                o[1] = make_float4(lo.z, hi.z, lo.w, hi.w);
+                j += CT_GROUP / (CH / 4);
+                if (j >= CT_W + 2) { j -= CT_W + 2; ++r; }
             }
-            *reinterpret_cast<float4*>(sx + (r * (CT_W + 2) + j) * CT_STRIDE + 4 * k) = v;
         }
-        __syncthreads();
-        // cells cg, cg + 4, ... of the tile row, channels 4 cog ..
-        float acc[8][4];
+        group_sync(group);
+        // row pair rp, columns cg, cg + 4, ..., channels 4 cog ..
+        uint64_t acc[8][4];
 #pragma unroll
-        for (int i = 0; i < 8; ++i)
+        for (int c = 0; c < 4; ++c) {
+            const float bc = b ? b[4 * cog + c] : 0.0f;
 #pragma unroll
-            for (int c = 0; c < 4; ++c) acc[i][c] = bias[c];
+            for (int i = 0; i < 8; ++i) acc[i][c] = pack2(bc, bc);
+        }
 #pragma unroll 1
         for (int t = 0; t < TAPS; ++t) {
-            const float* xs = sx + ((row + t / 3) * (CT_W + 2) + cg + t % 3) * CT_STRIDE;
+            const float2* xs = sx + ((rp + t / 3) * (CT_W + 2) + cg + t % 3) * CT_PITCH;
             const float* ws = sw + t * CH * CH + 4 * cog;
-#pragma unroll 2
-            for (int ci = 0; ci < CH; ci += 4) {
-                float4 wv[4], xv[8];
+// unrolled in full: short loops moved registers about (421 in place of 361 us)
 #pragma unroll
-                for (int k = 0; k < 4; ++k) wv[k] = *reinterpret_cast<const float4*>(ws + (ci + k) * CH);
+            for (int ci = 0; ci < CH; ci += 2) {
+                ulonglong2 xv[8];
+                float4 wv[2];
 #pragma unroll
-                for (int i = 0; i < 8; ++i) xv[i] = *reinterpret_cast<const float4*>(xs + 4 * i * CT_STRIDE + ci);
+                for (int k = 0; k < 2; ++k) wv[k] = *reinterpret_cast<const float4*>(ws + (ci + k) * CH);
 #pragma unroll
-                for (int k = 0; k < 4; ++k)
+                for (int i = 0; i < 8; ++i) xv[i] = *reinterpret_cast<const ulonglong2*>(xs + 4 * i * CT_PITCH + ci);
 #pragma unroll
-                    for (int i = 0; i < 8; ++i) {
-                        const float a = k == 0 ? xv[i].x : k == 1 ? xv[i].y : k == 2 ? xv[i].z : xv[i].w;
-                        acc[i][0] = fmaf(a, wv[k].x, acc[i][0]);
-                        acc[i][1] = fmaf(a, wv[k].y, acc[i][1]);
-                        acc[i][2] = fmaf(a, wv[k].z, acc[i][2]);
-                        acc[i][3] = fmaf(a, wv[k].w, acc[i][3]);
-                    }
+                for (int k = 0; k < 2; ++k) {
+                    const uint64_t w2[4] = {pack2(wv[k].x, wv[k].x), pack2(wv[k].y, wv[k].y),
+                                            pack2(wv[k].z, wv[k].z), pack2(wv[k].w, wv[k].w)};
+#pragma unroll
+                    for (int c = 0; c < 4; ++c)
+#pragma unroll
+                        for (int i = 0; i < 8; ++i) fma2(acc[i][c], k ? xv[i].y : xv[i].x, w2[c]);
+                }
             }
         }
-        if (r0 + row < Hd) {
 #pragma unroll
-            for (int i = 0; i < 8; ++i) {
-                const int xo = c0 + cg + 4 * i;
-                if (xo >= Wd) continue;
-                float* o = y + ((size_t(n) * Hd + r0 + row) * Wd + xo) * CH + 4 * cog;
-                if (relu)
+        for (int i = 0; i < 8; ++i) {
+            const int xo = c0 + cg + 4 * i;
+            if (xo >= Wd) continue;
+            float2 v[4];
 #pragma unroll
-                    for (int c = 0; c < 4; ++c) acc[i][c] = fmaxf(acc[i][c], 0.0f);
+            for (int c = 0; c < 4; ++c) {
+                v[c] = unpack2(acc[i][c]);
+                if (relu) v[c] = make_float2(fmaxf(v[c].x, 0.0f), fmaxf(v[c].y, 0.0f));
+            }
+#pragma unroll
+            for (int half = 0; half < 2; ++half) {
+                const int yy = r0 + rp + half * (CT_H / 2);
+                if (yy >= Hd) continue;
+                float* o = y + ((size_t(n) * Hd + yy) * Wd + xo) * CH + 4 * cog;
+                const float4 q4 = half ? make_float4(v[0].y, v[1].y, v[2].y, v[3].y)
+                                       : make_float4(v[0].x, v[1].x, v[2].x, v[3].x);
                 if (vec) {
-                    *reinterpret_cast<float4*>(o) = make_float4(acc[i][0], acc[i][1], acc[i][2], acc[i][3]);
+                    *reinterpret_cast<float4*>(o) = q4;
                 } else {
-#pragma unroll
-                    for (int c = 0; c < 4; ++c) o[c] = acc[i][c];
+                    o[0] = q4.x;
+                    o[1] = q4.y;
+                    o[2] = q4.z;
+                    o[3] = q4.w;
                 }
             }
         }
@@ -189,16 +239,17 @@ __global__ void k_flip_weights(const float* __restrict__ w, float* __restrict__ 
 
 // Weight and bias gradients: dW[t][ci][co] += sum_cells x[cell + off_t][ci] * g[cell][co],
 // db[co] += sum g[cell][co], with g = dy * (y > 0) when `y` is given.  Bound
-// by the FP32 pipes like the convolution: 64 threads hold all 9 x 32 x 32
+// by the FP32 pipes like the convolution, two FMAs an instruction: 64 threads hold all 9 x 32 x 32
 // sums in registers (4 ci x 4 co x 9 taps each) and walk along a row of
 // cells; a step loads the three new input words of the 3 x 3 window and one
-// gradient word, 16 bytes each, for 144 FMAs.  A CTA runs four such groups,
+// gradient word, 16 bytes each and a step ahead, for 144 FMAs.  A CTA runs four such groups,
 // one per row of a 4 x 32 cell tile; the next tile arrives by cp.async
 // meanwhile (the registers leave room for one CTA per SM, so nothing else
 // would cover its latency).  CTAs are persistent: the four groups' sums are
 // added in shared memory once, at the end, so dW receives one atomic per
 // weight and CTA (a CTA per 8-row band used to add 26 times as many).
-// 32 images of 93 x 310 cells: 964 us -> 441 us a layer.
+// 32 images of 93 x 310 cells: 964 us -> 370 us a layer (one FMA an
+// instruction and a division per staged word: 441).
 constexpr int WG_H = 4, WG_W = 32, WG_THREADS = 256;
 constexpr int WG_X = (WG_H + 2) * (WG_W + 2) * CH, WG_G = WG_H * WG_W * CH;      // floats of the two tiles
 constexpr int WG_SUMS = TAPS * CH * CH + CH;
@@ -228,32 +279,38 @@ __global__ void __launch_bounds__(WG_THREADS, 1) k_conv_wgrad(const float* __res
     grid_dep_wait();
     extern __shared__ __align__(16) float wg_sm[];
     const int tid = threadIdx.x, cog = tid & 7, cig = (tid >> 3) & 7, row = tid >> 6;
-    float acc[TAPS][4][4];              // [tap][ci][co]
+    uint64_t acc[TAPS][2][4];           // [tap][ci pair][co]
     float bacc[4] = {0.0f, 0.0f, 0.0f, 0.0f};
 #pragma unroll
     for (int t = 0; t < TAPS; ++t)
 #pragma unroll
-        for (int i = 0; i < 4; ++i)
+        for (int i = 0; i < 2; ++i)
 #pragma unroll
-            for (int c = 0; c < 4; ++c) acc[t][i][c] = 0.0f;
+            for (int c = 0; c < 4; ++c) acc[t][i][c] = 0;
     const int tx = (Wd + WG_W - 1) / WG_W, ty = (Hd + WG_H - 1) / WG_H;
     const long long ntiles = (long long)nimg * tx * ty;
     // tile buffer: inputs [WG_H + 2][WG_W + 2][CH], then dy and y [WG_H][WG_W][CH]
     auto stage = [&](long long tile, float* buf) {
         const int n = int(tile / (tx * ty)), q = int(tile % (tx * ty));
         const int r0 = q / tx * WG_H, c0 = q % tx * WG_W;
-        for (int i = tid; i < WG_X / 4; i += WG_THREADS) {
-            const int k = i % (CH / 4), j = (i / (CH / 4)) % (WG_W + 2), r = i / (CH / 4 * (WG_W + 2));
-            const int yy = r0 + r - 1, xx = c0 + j - 1;
+        // a word of 32 columns' 8 per thread, row by row; the two last columns' words by 96 threads
+        const int k = tid % (CH / 4), j = tid / (CH / 4);
+        const auto copy_x = [&](int r, int col) {
+            const int yy = r0 + r - 1, xx = c0 + col - 1;
             const bool ok = yy >= 0 && yy < Hd && xx >= 0 && xx < Wd;
-            copy4_async(buf + 4 * i, ok ? x + ((size_t(n) * Hd + yy) * Wd + xx) * CH + 4 * k : x, ok, vec);
-        }
-        for (int i = tid; i < WG_G / 4; i += WG_THREADS) {
-            const int k = i % (CH / 4), j = (i / (CH / 4)) % WG_W, r = i / (CH / 4 * WG_W);
+            copy4_async(buf + (r * (WG_W + 2) + col) * CH + 4 * k,
+                        ok ? x + ((size_t(n) * Hd + yy) * Wd + xx) * CH + 4 * k : x, ok, vec);
+        };
+#pragma unroll
+        for (int r = 0; r < WG_H + 2; ++r) copy_x(r, j);
+        if (j < 2 * (WG_H + 2)) copy_x(j >> 1, WG_W + (j & 1));
+#pragma unroll
+        for (int r = 0; r < WG_H; ++r) {
             const bool ok = r0 + r < Hd && c0 + j < Wd;
             const size_t at = ok ? ((size_t(n) * Hd + r0 + r) * Wd + c0 + j) * CH + 4 * k : 0;
-            copy4_async(buf + WG_X + 4 * i, dy + at, ok, vec);
-            if (y) copy4_async(buf + WG_X + WG_G + 4 * i, y + at, ok, vec);
+            float* g = buf + WG_X + (r * WG_W + j) * CH + 4 * k;
+            copy4_async(g, dy + at, ok, vec);
+            if (y) copy4_async(g + WG_G, y + at, ok, vec);
         }
         asm volatile("cp.async.commit_group;" ::: "memory");
     };
@@ -271,53 +328,49 @@ __global__ void __launch_bounds__(WG_THREADS, 1) k_conv_wgrad(const float* __res
         const float* sg = sx + WG_X;
         const float* xr = sx + row * (WG_W + 2) * CH + 4 * cig;
         const float* gr = sg + row * WG_W * CH + 4 * cog;
-        float4 win[3][3];               // the 3 x 3 window's inputs, columns rotating by position
+        // columns j .. j + 2 of the window and j + 3, on its way; column c lies in win[.][c % 4]
+        float4 win[3][4];
+        const auto load_g = [&](int j) {
+            const float4 g = *reinterpret_cast<const float4*>(gr + j * CH);
+            return y ? masked4(g, *reinterpret_cast<const float4*>(gr + WG_G + j * CH)) : g;
+        };
 #pragma unroll
         for (int r = 0; r < 3; ++r)
 #pragma unroll
-            for (int c = 0; c < 2; ++c)
+            for (int c = 0; c < 3; ++c)
                 win[r][c] = *reinterpret_cast<const float4*>(xr + (r * (WG_W + 2) + c) * CH);
-        // one cell; A, B, C: which columns of win hold the window's left, middle and right
-        auto cell = [&](int j, auto ca, auto cb, auto cc) {
-            constexpr int A = decltype(ca)::value, B = decltype(cb)::value, C = decltype(cc)::value;
+        float4 g_next = load_g(0);
+#pragma unroll 2
+        for (int j0 = 0; j0 < WG_W; j0 += 4)
 #pragma unroll
-            for (int r = 0; r < 3; ++r)
-                win[r][C] = *reinterpret_cast<const float4*>(xr + (r * (WG_W + 2) + j + 2) * CH);
-            float4 g = *reinterpret_cast<const float4*>(gr + j * CH);
-            if (y) g = masked4(g, *reinterpret_cast<const float4*>(gr + WG_G + j * CH));
+            for (int p = 0; p < 4; ++p) {
+                const int j = j0 + p;
+                const float4 g = g_next;
+                const uint64_t g2[4] = {pack2(g.x, g.x), pack2(g.y, g.y), pack2(g.z, g.z), pack2(g.w, g.w)};
+                // (past the row's end: a word of the next row, not used)
 #pragma unroll
-            for (int r = 0; r < 3; ++r)
+                for (int r = 0; r < 3; ++r)
+                    win[r][(p + 3) & 3] = *reinterpret_cast<const float4*>(xr + (r * (WG_W + 2) + j + 3) * CH);
+                g_next = load_g(min(j + 1, WG_W - 1));
 #pragma unroll
-                for (int c = 0; c < 3; ++c) {
-                    const float4 v = c == 0 ? win[r][A] : c == 1 ? win[r][B] : win[r][C];
-                    float(&a)[4][4] = acc[3 * r + c];
+                for (int r = 0; r < 3; ++r)
 #pragma unroll
-                    for (int i = 0; i < 4; ++i) {
-                        const float vi = i == 0 ? v.x : i == 1 ? v.y : i == 2 ? v.z : v.w;
-                        a[i][0] = fmaf(vi, g.x, a[i][0]);
-                        a[i][1] = fmaf(vi, g.y, a[i][1]);
-                        a[i][2] = fmaf(vi, g.z, a[i][2]);
-                        a[i][3] = fmaf(vi, g.w, a[i][3]);
+                    for (int c = 0; c < 3; ++c) {
+                        const float4 v = win[r][(p + c) & 3];
+                        const uint64_t v01 = pack2(v.x, v.y), v23 = pack2(v.z, v.w);
+#pragma unroll
+                        for (int k = 0; k < 4; ++k) {
+                            fma2(acc[3 * r + c][0][k], v01, g2[k]);
+                            fma2(acc[3 * r + c][1][k], v23, g2[k]);
+                        }
                     }
+                if (cig == 0) {
+                    bacc[0] += g.x;
+                    bacc[1] += g.y;
+                    bacc[2] += g.z;
+                    bacc[3] += g.w;
                 }
-            if (cig == 0) {
-                bacc[0] += g.x;
-                bacc[1] += g.y;
-                bacc[2] += g.z;
-                bacc[3] += g.w;
             }
-        };
-        using I0 = std::integral_constant<int, 0>;
-        using I1 = std::integral_constant<int, 1>;
-        using I2 = std::integral_constant<int, 2>;
-#pragma unroll 1
-        for (int j = 0; j < 30; j += 3) {
-            cell(j, I0{}, I1{}, I2{});
-            cell(j + 1, I1{}, I2{}, I0{});
-            cell(j + 2, I2{}, I0{}, I1{});
-        }
-        cell(30, I0{}, I1{}, I2{});
-        cell(31, I1{}, I2{}, I0{});
         __syncthreads();                // the buffer is free for the tile after next
     }
     // the four groups' sums, group by group, into shared memory, then one atomic per weight
@@ -329,7 +382,13 @@ __global__ void __launch_bounds__(WG_THREADS, 1) k_conv_wgrad(const float* __res
 #pragma unroll
             for (int i = 0; i < 4; ++i) {
                 float4* o = reinterpret_cast<float4*>(wg_sm + (t * CH + 4 * cig + i) * CH + 4 * cog);
-                float4 v = make_float4(acc[t][i][0], acc[t][i][1], acc[t][i][2], acc[t][i][3]);
+                float v4[4];
+#pragma unroll
+                for (int c = 0; c < 4; ++c) {
+                    const float2 pr = unpack2(acc[t][i >> 1][c]);
+                    v4[c] = i & 1 ? pr.y : pr.x;
+                }
+                float4 v = make_float4(v4[0], v4[1], v4[2], v4[3]);
                 if (g) {
                     const float4 p = *o;
                     v = make_float4(p.x + v.x, p.y + v.y, p.z + v.z, p.w + v.w);
@@ -347,7 +406,8 @@ __global__ void __launch_bounds__(WG_THREADS, 1) k_conv_wgrad(const float* __res
     for (int i = tid; i < TAPS * CH * CH; i += WG_THREADS) atomicAdd(&dw[i], wg_sm[i]);
     if (tid < CH) atomicAdd(&db[tid], wg_sm[TAPS * CH * CH + tid]);
 }
-static_assert(WG_W == 32, "the cell loop is written out for 32 cells");
+static_assert(WG_W * (CH / 4) == WG_THREADS, "a thread stages one word of each row");
+static_assert(WG_W % 4 == 0, "four cells a turn of the window's columns");
 
 // Correlation scores, softmax cross-entropy and the feature gradients, one
 // warp per label (pair, cx, cy, bin) in turn.  Bound by the L2 atomics of
@@ -530,7 +590,7 @@ cudaError_t launch_conv_f32(const float* x, const float* mask, const float* w, c
                             int Hd, int Wd, int relu, cudaStream_t st) {
     allow_smem(k_conv_f32);
     const long long tiles = (long long)nimg * ((Wd + CT_W - 1) / CT_W) * ((Hd + CT_H - 1) / CT_H);
-    k_conv_f32<<<tile_grid(tiles, 2 * sm_count()), CT_THREADS, CONV_F32_SMEM, st>>>(
+    k_conv_f32<<<tile_grid(tiles, sm_count()), CT_THREADS, CONV_F32_SMEM, st>>>(
         x, mask, w, b, y, nimg, Hd, Wd, relu, aligned16({x, mask, y}));
     return cudaGetLastError();
 }

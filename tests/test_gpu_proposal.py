@@ -206,10 +206,12 @@ def test_topk_bins_match_float64_scores(preset, seed):
 
 
 @pytest.mark.parametrize("shift", [0, 1])
-@pytest.mark.parametrize("nimg,hd,wd", [(1, 1, 1), (2, 8, 32), (3, 9, 33), (2, 5, 31), (1, 17, 65)])
+@pytest.mark.parametrize("nimg,hd,wd", [(1, 1, 1), (2, 8, 32), (3, 9, 33), (2, 5, 31), (1, 17, 65),
+                                        (7, 100, 200)])
 def test_training_convolutions_at_tile_edges(torch, nimg, hd, wd, shift):
     """Forward, input, weight and bias gradients of one layer around the
-    kernels' tile sizes (8 x 32 and 4 x 32 cells) and with buffers off a
+    kernels' tile sizes (16 x 32 and 4 x 32 cells), with more tiles than the
+    GPU takes at once, and with buffers off a
     16-byte boundary (shift floats), against float64.  A sum of n products
     in fp32, in any order, is off by at most n * 2^-23 of the sum of their
     magnitudes."""
