@@ -5,14 +5,14 @@
 // long serial scanline loops.  Here one thread per triangle solves the plane
 // (same double Gauss-Jordan as kerSolve, :321-375) and sets up the edges.
 // Two ways to paint, chosen by image size (both give the same bytes):
-//   * direct: a warp per triangle, lanes over its pixels, atomics straight
-//     into the zeroed prior (one launch after the memset, each warp setting
-//     its triangle up itself; the faster one for small images);
+//   * direct: a warp per piece of a triangle, lanes over its pixels, atomics
+//     straight into the zeroed prior (one launch after the memset, each CTA
+//     setting its triangles up itself; the faster one for small images);
 //   * tiled: the set-up also finds the 64x32 prior tiles a triangle's pixels
 //     can fall in and drops the triangle into each tile's fixed bin (the
 //     slot its count's atomic returns; no scan), and one CTA per tile paints
 //     it in shared memory and writes it once (no memset, no global atomics
-//     on the prior; the faster one from about a megapixel up).
+//     on the prior; the faster one from about three megapixels up).
 // A pixel covered by more than one triangle (rounding at shared vertices)
 // must keep the last triangle in list order, as a sequential rasteriser
 // would; both paint with a 32-bit atomicMax of (triangle+1) << pshift |
@@ -301,31 +301,61 @@ __device__ __forceinline__ void paint_warp(const Raster& R, int wu0, int wu1, in
     }
 }
 
-// Direct paint: one warp per (view, triangle), which first sets the
-// triangle up itself (every lane the same operations on the same loads, so
-// no per-triangle record goes through memory and no set-up launch runs);
+// Direct paint: a CTA takes every gridDim-th triangle of both views' lists,
+// up to 32 at a time; a lane of its first warp sets each of them up in
+// shared memory, and its warps share out their RASTER_W x RASTER_H pieces;
 // every pixel keeps the last covering triangle through atomicMax on the
-// packed value in the zeroed prior.
-__global__ void __launch_bounds__(256) k_prior_raster(const int32_t* __restrict__ tri0,
-                                                      const int32_t* __restrict__ tri1,
-                                                      const int32_t* __restrict__ ctr0,
-                                                      const int32_t* __restrict__ ctr1,
-                                                      const int32_t* __restrict__ can, const int32_t* __restrict__ uvd,
-                                                      uint32_t* prior0, uint32_t* prior1, Geom g, int pshift,
-                                                      int dcap) {
+// packed value in the zeroed prior.  What it waits for is the largest
+// triangles (neighbours at the hull, so consecutive in the list) and the
+// double-precision solve's chain: a warp per triangle that sets it up and
+// paints all of it took 17.5 us at 1242x375, 33 with the default parameters
+// and 11 at 450x375; now 11.5, 13.8 and 8.0 (pieces of 32 or 64 columns: 13;
+// CTAs of 64 threads: 17.5).
+constexpr int RASTER_THREADS = 128, RASTER_CTAS_PER_SM = 8, RASTER_W = 16, RASTER_H = 64;
+__global__ void __launch_bounds__(RASTER_THREADS, RASTER_CTAS_PER_SM)
+    k_prior_raster(const int32_t* __restrict__ tri0, const int32_t* __restrict__ tri1,
+                   const int32_t* __restrict__ ctr0, const int32_t* __restrict__ ctr1,
+                   const int32_t* __restrict__ can, const int32_t* __restrict__ uvd, uint32_t* prior0,
+                   uint32_t* prior1, Geom g, int pshift, int dcap) {
     grid_dep_wait();
-    const int lane = threadIdx.x & 31;
-    const int T0 = ctr0[0], T1 = ctr1[0];
-    const int nw = (gridDim.x * blockDim.x) >> 5;
-    for (int i = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; i < T0 + T1; i += nw) {
-        const bool right = i >= T0;
-        const int t = right ? i - T0 : i;
-        Raster R;
-        setup_triangle((right ? tri1 : tri0) + 3 * size_t(t), can, uvd, g.cw, g.step, right, R);
-        const uint32_t tag = uint32_t(t + 1) << pshift;
-        uint32_t* prior = right ? prior1 : prior0;
-        paint_warp(R, 0, g.W, 0, g.H, lane, dcap,
-                   [&](int u, int v, uint32_t d) { atomicMax(&prior[size_t(v) * g.W + u], tag | d); });
+    __shared__ Raster sr[32];
+    constexpr int WARPS = RASTER_THREADS / 32;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int T0 = ctr0[0], T = T0 + ctr1[0];
+    const int ctas = gridDim.x;
+    for (int base = blockIdx.x; base < T; base += 32 * ctas) {
+        const int n = imin((T - base + ctas - 1) / ctas, 32);
+        if (int(threadIdx.x) < n) {
+            const int i = base + int(threadIdx.x) * ctas;
+            const bool right = i >= T0;
+            Raster R;
+            setup_triangle((right ? tri1 : tri0) + 3 * size_t(right ? i - T0 : i), can, uvd, g.cw, g.step, right, R);
+            int r0 = g.H, r1 = -1;
+            part_rows(R, 0, g.W, g.H, r0, r1);
+            part_rows(R, 1, g.W, g.H, r0, r1);
+            R.ty0 = r0;
+            R.ty1 = r1;
+            sr[threadIdx.x] = R;
+        }
+        __syncthreads();
+        // triangles of many columns by all warps, the others by a warp each
+        for (int k = 0; k < n; ++k) {
+            const int i = base + k * ctas;
+            const bool right = i >= T0;
+            const uint32_t tag = uint32_t((right ? i - T0 : i) + 1) << pshift;
+            uint32_t* prior = right ? prior1 : prior0;
+            const Raster& R = sr[k];
+            const int u0 = imax(int(R.A_u), 0), v0 = R.ty0;
+            const int nx = (imin(int(R.C_u), g.W) - u0 + RASTER_W - 1) / RASTER_W;
+            const int ny = (R.ty1 - v0 + RASTER_H) / RASTER_H;
+            if (nx <= 0 || ny <= 0) continue;
+            for (int c = nx * ny == 1 ? (k + warp) % WARPS : warp; c < nx * ny; c += WARPS) {
+                const int wu = u0 + c % nx * RASTER_W, wv = v0 + c / nx * RASTER_H;
+                paint_warp(R, wu, imin(wu + RASTER_W, g.W), wv, imin(wv + RASTER_H, g.H), lane, dcap,
+                           [&](int u, int v, uint32_t d) { atomicMax(&prior[size_t(v) * g.W + u], tag | d); });
+            }
+        }
+        __syncthreads();
     }
 }
 
@@ -606,7 +636,7 @@ cudaError_t launch_prior(const int32_t* tri0, const int32_t* tri1, const int32_t
             cudaMemsetAsync(prior0, 0, n, st);
             cudaMemsetAsync(prior1, 0, n, st);
         }
-        launch_k(k_prior_raster, imax(1, imin(16 * num_sms, (2 * Tmax + 7) / 8)), 256, 0, st, tri0, tri1, ctr0, ctr1,
+        launch_k(k_prior_raster, imax(1, imin(RASTER_CTAS_PER_SM * num_sms, 2 * Tmax)), RASTER_THREADS, 0, st, tri0, tri1, ctr0, ctr1,
                  can, uvd, prior0, prior1, g, pshift, dcap);
         if (nlaunch) *nlaunch += 1;
         return cudaGetLastError();

@@ -125,9 +125,10 @@ cudaError_t launch_prior(const int32_t* tri0, const int32_t* tri1, const int32_t
                          uint32_t* prior0, uint32_t* prior1, const Geom& g, int pshift, int dcap, int num_sms,
                          unsigned* err, cudaStream_t st, int* nlaunch, bool tiled, bool zeroed = false,
                          int bin_cap = PT_BIN);
-// Images from this many pixels up take the tiled prior paint (measured:
-// the direct paint is faster at 1242x375, the tiled one at 2880x1988).
-constexpr long long PRIOR_TILED_MIN_PIXELS = 1LL << 20;
+// Images from this many pixels up take the tiled prior paint, whose cost
+// grows more slowly (direct and tiled: 29 and 36 us at 1920x1080, 91 and 74
+// at 2880x1988, so they cross at some 3.5 million pixels).
+constexpr long long PRIOR_TILED_MIN_PIXELS = 3LL << 20;
 // Images up to this many pixels take the star construction of the
 // Delaunay triangulations, larger ones the strips and flips (measured: the
 // stars are faster at 1242x375, the flips at 2880x1988).

@@ -184,9 +184,9 @@ int elas_b200_set_graphs(elas_handle* h, int enable);
  *                           bitset, the path otherwise taken only by cells
  *                           with more candidates than the per-row list holds;
  *   ELAS_TEST_PRIOR_TILED   the plane prior is painted tile by tile in shared
- *                           memory (otherwise from 2^20 pixels up);
+ *                           memory (otherwise from 3 * 2^20 pixels up);
  *   ELAS_TEST_PRIOR_DIRECT  the plane prior is painted with global atomics
- *                           (otherwise below 2^20 pixels); not together with
+ *                           (otherwise below 3 * 2^20 pixels); not together with
  *                           ELAS_TEST_PRIOR_TILED;
  *   ELAS_TEST_PRIOR_SMALL_BINS the tiled paint keeps 2 triangles per tile in
  *                           each tile's bin (otherwise 128), so that most go
