@@ -302,8 +302,41 @@ HD void flip_relink(M& m, int t, int n, const int32_t* res) {
         m.set_opp(x, r);
         if (r >= 0) m.set_opp(r, x);
     }
-    m.set_opp(3 * t + 2, m.opp(3 * t + 2) & ~FINAL);
-    m.set_opp(3 * n + 2, m.opp(3 * n + 2) & ~FINAL);
+    m.set_opp(3 * t + 2, 3 * n + 2);
+    m.set_opp(3 * n + 2, 3 * t + 2);
+}
+
+// flip_resolve_slot for the four outer slots of a flipped pair, step by
+// step, so that the four chains of loads overlap.  q: the pair's vertices
+// c, a, d, b (t' = (c, a, d), n' = (d, b, c)), whose order is that of the
+// outer edges: slot k runs from q[k] to q[k + 1].
+template <class M>
+HD void flip_resolve4(const M& m, int t, int n, const int32_t (&q)[4], uint32_t round, int T, int32_t (&r)[4]) {
+    int mt[4];
+    bool moved[4];
+    for (int k = 0; k < 4; ++k) r[k] = m.opp(outer_slot(t, n, k));
+    for (int k = 0; k < 4; ++k) {
+        mt[k] = r[k] < 0 ? t : r[k] / 3;
+        r[k] = r[k] < 0 ? -1 : (mt[k] >= T ? -2 : r[k]);
+        moved[k] = false;
+        if (r[k] >= 0) moved[k] = m.fround(mt[k]) == int32_t(round);
+    }
+    if (!(moved[0] || moved[1] || moved[2] || moved[3])) return;
+    int mt2[4];
+    for (int k = 0; k < 4; ++k) mt2[k] = moved[k] ? m.opp(3 * mt[k] + 2) : -1;
+    for (int k = 0; k < 4; ++k) {
+        mt2[k] = mt2[k] < 0 ? T : (mt2[k] & ~FINAL) / 3;
+        if (!moved[k]) continue;
+        r[k] = -2;
+        if (mt2[k] >= T) continue;
+        const int a = q[k], b = q[(k + 1) & 3];
+        const int u0 = m.v(mt[k], 0), u1 = m.v(mt[k], 1), u2 = m.v(mt[k], 2);
+        const int w0 = m.v(mt2[k], 0), w1 = m.v(mt2[k], 1), w2 = m.v(mt2[k], 2);
+        if (w1 == b && w2 == a) r[k] = 3 * mt2[k] + 1;
+        if (w0 == b && w1 == a) r[k] = 3 * mt2[k];
+        if (u1 == b && u2 == a) r[k] = 3 * mt[k] + 1;
+        if (u0 == b && u1 == a) r[k] = 3 * mt[k];
+    }
 }
 
 // Flat storage: plain arrays (global memory on the device, host memory in

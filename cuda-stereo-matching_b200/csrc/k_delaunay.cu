@@ -1432,35 +1432,69 @@ constexpr int WL_PER_CTA = 6 * SLICE_MAX;           // worklist entries per CTA 
 constexpr int CAND_PER_CTA = 6 * SLICE_MAX;         // proposals per CTA and round
 constexpr int FLIP_PER_CTA = SLICE_MAX;             // flipped pairs per CTA and round
 constexpr int CL_MARK = 3 * SLICE_MAX / 32;         // words of a per-round half-edge bitset
+constexpr int CL_CAND = 864, CL_FLIP = 768;         // entries of a round's lists kept in shared memory
 // shared memory: the triangle slice (48 bytes a triangle), two push bitsets
-// and the round-0 staging rings (64 entries per warp)
-constexpr size_t CL_SMEM = size_t(SLICE_MAX) * 48 + size_t(8) * CL_MARK + size_t(4) * 64 * (CL_THREADS / 32);
+// and the heads of the round lists
+constexpr size_t CL_SMEM = size_t(SLICE_MAX) * 48 + size_t(8) * CL_MARK + size_t(16) * CL_CAND + size_t(24) * CL_FLIP;
+static_assert(CL_SMEM + 256 <= 227 * 1024, "one CTA's shared memory");
+// round 0 stages each warp's owned half-edges (64 entries) in the flip list's
+// shared part, which is unused until the first flips
+static_assert(6 * CL_FLIP >= 64 * (CL_THREADS / 32), "round-0 staging does not fit");
+
+// Shared-memory addresses of the cluster (32 bits): a word of CTA `rank`,
+// its loads, stores and atomics.  (Through generic 64-bit pointers the rounds
+// of k_flip_smem took 281 us at 2880x1988, so 271.)
+__device__ __forceinline__ uint32_t cl_map(uint32_t addr, int rank) {
+    uint32_t r;
+    asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(addr), "r"(rank));
+    return r;
+}
+__device__ __forceinline__ uint32_t cl_ld(uint32_t a) {
+    uint32_t v;
+    asm volatile("ld.shared::cluster.u32 %0, [%1];" : "=r"(v) : "r"(a) : "memory");
+    return v;
+}
+__device__ __forceinline__ void cl_st(uint32_t a, uint32_t v) {
+    asm volatile("st.shared::cluster.u32 [%0], %1;" ::"r"(a), "r"(v) : "memory");
+}
+__device__ __forceinline__ void cl_min(uint32_t a, uint32_t v) {
+    asm volatile("red.relaxed.cluster.shared::cluster.min.u32 [%0], %1;" ::"r"(a), "r"(v) : "memory");
+}
+__device__ __forceinline__ uint32_t cl_or(uint32_t a, uint32_t v) {
+    uint32_t o;
+    asm volatile("atom.relaxed.cluster.shared::cluster.or.b32 %0, [%1], %2;" : "=r"(o) : "r"(a), "r"(v) : "memory");
+    return o;
+}
+__device__ __forceinline__ int cl_add(uint32_t a, int v) {
+    int o;
+    asm volatile("atom.relaxed.cluster.shared::cluster.add.s32 %0, [%1], %2;" : "=r"(o) : "r"(a), "r"(v) : "memory");
+    return o;
+}
 
 struct ClusterTri {
-    int32_t* lv;      // [3*SLICE_MAX] in this CTA's shared memory
-    uint32_t* lxy;    // [3*SLICE_MAX]
-    int32_t* lopp;    // [3*SLICE_MAX]
-    uint32_t* llock;  // [SLICE_MAX]
-    int32_t* lround;  // [SLICE_MAX]
+    uint32_t lv, lxy, lopp, llock, lround;   // addresses in the own CTA: vertices, coordinates and links
+                                             // [3 * SLICE_MAX], locks and flip rounds [SLICE_MAX]
     int shift, mask;
-    template <class X>
-    __device__ __forceinline__ X* at(X* base, int t) const {
-        return cg::this_cluster().map_shared_rank(base, unsigned(t >> shift));
+    // word 3 t + k of an array of three words a triangle, word t of one
+    __device__ __forceinline__ uint32_t at3(uint32_t base, int t, int k) const {
+        return cl_map(base + 4u * uint32_t(3 * (t & mask) + k), t >> shift);
     }
-    __device__ int v(int t, int k) const { return at(lv, t)[3 * (t & mask) + k]; }
-    __device__ uint32_t xy(int t, int k) const { return at(lxy, t)[3 * (t & mask) + k]; }
-    __device__ int opp(int h) const { int t = h / 3; return at(lopp, t)[3 * (t & mask) + h - 3 * t]; }
-    __device__ uint32_t lock(int t) const { return *((volatile uint32_t*)at(llock, t) + (t & mask)); }
-    __device__ int32_t fround(int t) const { return at(lround, t)[t & mask]; }
-    __device__ void lock_min(int t, uint32_t p) { atomicMin(at(llock, t) + (t & mask), p); }
+    __device__ __forceinline__ uint32_t at1(uint32_t base, int t) const {
+        return cl_map(base + 4u * uint32_t(t & mask), t >> shift);
+    }
+    __device__ int v(int t, int k) const { return int(cl_ld(at3(lv, t, k))); }
+    __device__ uint32_t xy(int t, int k) const { return cl_ld(at3(lxy, t, k)); }
+    __device__ int opp(int h) const { int t = h / 3; return int(cl_ld(at3(lopp, t, h - 3 * t))); }
+    __device__ uint32_t lock(int t) const { return cl_ld(at1(llock, t)); }
+    __device__ int32_t fround(int t) const { return int32_t(cl_ld(at1(lround, t))); }
+    __device__ void lock_min(int t, uint32_t p) { cl_min(at1(llock, t), p); }
     __device__ void set_v(int t, int a, int b, int c, uint32_t pa, uint32_t pb, uint32_t pc) {
-        int32_t* V = at(lv, t) + 3 * (t & mask);
-        uint32_t* X = at(lxy, t) + 3 * (t & mask);
-        V[0] = a; V[1] = b; V[2] = c;
-        X[0] = pa; X[1] = pb; X[2] = pc;
+        const uint32_t V = at3(lv, t, 0), X = at3(lxy, t, 0);
+        cl_st(V, a); cl_st(V + 4, b); cl_st(V + 8, c);
+        cl_st(X, pa); cl_st(X + 4, pb); cl_st(X + 8, pc);
     }
-    __device__ void set_opp(int h, int o) { int t = h / 3; at(lopp, t)[3 * (t & mask) + h - 3 * t] = o; }
-    __device__ void set_fround(int t, int32_t r) { at(lround, t)[t & mask] = r; }
+    __device__ void set_opp(int h, int o) { int t = h / 3; cl_st(at3(lopp, t, h - 3 * t), uint32_t(o)); }
+    __device__ void set_fround(int t, int32_t r) { cl_st(at1(lround, t), uint32_t(r)); }
 };
 
 // Point-table accessor for a problem that fits one SM: corner coordinates
@@ -1733,6 +1767,13 @@ struct ClusterSync {
 // proposal is queued at the CTA that owns its lower half-edge, so a CTA
 // flips at most its own triangles in a round (f < FLIP_PER_CTA), and that
 // CTA releases the proposal's locks in the next round.
+//
+// Latency bounds it: some twenty rounds, most of them with a few hundred
+// proposals or fewer, of three chains of remote accesses (about 300 cycles
+// each, a barrier 750).  So the lists' heads lie in shared memory, the four
+// edges of a pair go through each step of C1 together, on the pair's own
+// four vertices, and a warp's lanes read the CTAs' counts once: 367 -> 271 us
+// at 2880x1988.
 __global__ void __launch_bounds__(CL_THREADS) k_flip_smem(DelDev d0, DelDev d1, int csize, int max_rounds,
                                                           unsigned* err) {
     grid_dep_wait();
@@ -1749,47 +1790,56 @@ __global__ void __launch_bounds__(CL_THREADS) k_flip_smem(DelDev d0, DelDev d1, 
     int shift = 6;
     while ((csize << shift) < T) ++shift;
     ClusterTri m;
-    m.lv = reinterpret_cast<int32_t*>(csm);
-    m.lxy = reinterpret_cast<uint32_t*>(m.lv + 3 * SLICE_MAX);
-    m.lopp = reinterpret_cast<int32_t*>(m.lxy + 3 * SLICE_MAX);
-    uint32_t* const lock0 = reinterpret_cast<uint32_t*>(m.lopp + 3 * SLICE_MAX);
+    // the own slice
+    int32_t* const lv = reinterpret_cast<int32_t*>(csm);
+    uint32_t* const lxy = reinterpret_cast<uint32_t*>(lv + 3 * SLICE_MAX);
+    int32_t* const lopp = reinterpret_cast<int32_t*>(lxy + 3 * SLICE_MAX);
+    uint32_t* const lock0 = reinterpret_cast<uint32_t*>(lopp + 3 * SLICE_MAX);
     uint32_t* const lock1 = lock0 + SLICE_MAX;
-    m.lround = reinterpret_cast<int32_t*>(lock1 + SLICE_MAX);
-    uint32_t* const mark0 = reinterpret_cast<uint32_t*>(m.lround + SLICE_MAX);
+    int32_t* const lround = reinterpret_cast<int32_t*>(lock1 + SLICE_MAX);
+    uint32_t* const mark0 = reinterpret_cast<uint32_t*>(lround + SLICE_MAX);
+    m.lv = smem_u32(lv);
+    m.lxy = smem_u32(lxy);
+    m.lopp = smem_u32(lopp);
+    m.lround = smem_u32(lround);
     uint32_t* const mark1 = mark0 + CL_MARK;
-    int32_t* const ring = reinterpret_cast<int32_t*>(mark1 + CL_MARK);
+    int32_t* const heads = reinterpret_cast<int32_t*>(mark1 + CL_MARK);
     m.shift = shift;
     m.mask = (1 << shift) - 1;
     const int t0 = rank << shift, t1 = min(T, (rank + 1) << shift);
     const int tid = threadIdx.x;
     for (int t = t0 + tid; t < t1; t += CL_THREADS) {
-        int l = t - t0;
-        for (int k = 0; k < 3; ++k) {
-            int v = D.tri[3 * t + k];
-            m.lv[3 * l + k] = v;
-            m.lxy[3 * l + k] = pack_xy(D.x[v], D.y[v]);
-            m.lopp[3 * l + k] = D.opp[3 * t + k];
-        }
+        const int l = t - t0;
+        int v[3], o[3];
+        uint32_t xy[3];
+#pragma unroll
+        for (int k = 0; k < 3; ++k) { v[k] = D.tri[3 * t + k]; o[k] = D.opp[3 * t + k]; }
+#pragma unroll
+        for (int k = 0; k < 3; ++k) xy[k] = pack_xy(D.x[v[k]], D.y[v[k]]);
+#pragma unroll
+        for (int k = 0; k < 3; ++k) { lv[3 * l + k] = v[k]; lxy[3 * l + k] = xy[k]; lopp[3 * l + k] = o[k]; }
         lock0[l] = LOCK_FREE;
         lock1[l] = LOCK_FREE;
-        m.lround[l] = -1;
+        lround[l] = -1;
     }
     if (tid == 0) { n_cand[0] = 0; n_cand[1] = 0; n_flip = 0; }
-    // the proposal lists of CTA r, by round parity, in global memory
-    auto cand_list = [&](int parity, int r) -> int32_t* {
-        return parity ? D.cwl + size_t(r) * 2 * WL_PER_CTA : D.ccand + size_t(r) * 2 * CAND_PER_CTA;
+    // the proposal lists of CTA r, by round parity, and the own flip list
+    auto cand_list = [&](int parity, int r) -> List2 {
+        int32_t* g = parity ? D.cwl + size_t(r) * 2 * WL_PER_CTA : D.ccand + size_t(r) * 2 * CAND_PER_CTA;
+        return List2{sync.remote(heads + parity * 2 * CL_CAND, r), g, CL_CAND, CAND_PER_CTA - CL_CAND, 2};
     };
-    int32_t* const flips = D.cflips + size_t(rank) * 6 * FLIP_PER_CTA;
+    const List2 flips{heads + 4 * CL_CAND, D.cflips + size_t(rank) * 6 * FLIP_PER_CTA, CL_FLIP, FLIP_PER_CTA - CL_FLIP,
+                      6};
     sync();
     // round 0's proposals: every interior edge of the own slice once
-    m.llock = lock0;
+    m.llock = smem_u32(lock0);
     {
-        int32_t* const c0 = cand_list(0, rank);
+        const List2 c0 = cand_list(0, rank);
         auto add0 = [&](int hh, int nn) {
             int idx = agg_inc(&n_cand[0]);
-            if (idx < CAND_PER_CTA) { c0[2 * idx] = hh; c0[2 * idx + 1] = nn; }
+            if (idx < CAND_PER_CTA) { int32_t* c = c0.slot(idx); c[0] = hh; c[1] = nn; }
         };
-        propose_owned(3 * t0, 3 * t1, ring + 64 * (tid >> 5), [&](int h) { return m.opp(h); }, [&](int h) {
+        propose_owned(3 * t0, 3 * t1, flips.s + 64 * (tid >> 5), [&](int h) { return m.opp(h); }, [&](int h) {
             if (!flip_propose(m, h, T, 0u, false, add0)) set_err(err, ERRF_BOUNDS);
         });
     }
@@ -1798,19 +1848,15 @@ __global__ void __launch_bounds__(CL_THREADS) k_flip_smem(DelDev d0, DelDev d1, 
     bool converged = false;
     for (; round < max_rounds; ++round) {
         const int cur = round & 1, nxt = cur ^ 1;
-        int32_t* const cand_cur = cand_list(cur, rank);
-        int32_t* const cand_old = cand_list(nxt, rank);   // the previous round's list, until C1 refills it
-        uint32_t* const lock_cur = cur ? lock1 : lock0;
-        uint32_t* const lock_nxt = cur ? lock0 : lock1;
+        const List2 cand_cur = cand_list(cur, rank);
+        const List2 cand_old = cand_list(nxt, rank);   // the previous round's list, until C1 refills it
+        const uint32_t lock_nxt = smem_u32(cur ? lock0 : lock1);
         uint32_t* const mark_nxt = cur ? mark0 : mark1;
         // every CTA's count is final since the last barrier, so all CTAs take the same decision
-        int total = 0;
-        bool over = false;
-        for (int r = 0; r < csize; ++r) {
-            const int c = *sync.remote(&n_cand[cur], r);
-            total += c;
-            over |= c > CAND_PER_CTA;
-        }
+        // (each warp's lanes read one count each)
+        const int lane = tid & 31, theirs = lane < csize ? *sync.remote(&n_cand[cur], lane) : 0;
+        const int total = __reduce_add_sync(0xffffffffu, theirs);
+        const bool over = __any_sync(0xffffffffu, theirs > CAND_PER_CTA);
         if (over) {
             if (tid == 0) set_err(err, ERRF_BOUNDS);
             break;
@@ -1818,74 +1864,120 @@ __global__ void __launch_bounds__(CL_THREADS) k_flip_smem(DelDev d0, DelDev d1, 
         if (total == 0) { converged = true; break; }
         const int nc = n_cand[cur];
         // B: flip the winners (own triangles); release the previous round's locks; clear the next bitset
-        m.llock = lock_cur;
+        m.llock = smem_u32(cur ? lock1 : lock0);
         for (int c = tid; c < nc; c += CL_THREADS) {
-            int h = cand_cur[2 * c], n = cand_cur[2 * c + 1];
+            const int32_t* cc = cand_cur.slot(c);
+            const int h = cc[0], n = cc[1];
             if (flip_apply(m, h, n, uint32_t(round))) {
-                int f = agg_inc(&n_flip);
-                if (f < FLIP_PER_CTA) { flips[6 * f] = h / 3; flips[6 * f + 1] = n; }
+                const int f = agg_inc(&n_flip);
+                if (f < FLIP_PER_CTA) { int32_t* q = flips.slot(f); q[0] = h / 3; q[1] = n; }
             }
         }
         for (int c = tid; c < nc_prev; c += CL_THREADS) {
-            const int t = cand_old[2 * c] / 3, n = cand_old[2 * c + 1];
-            *(m.at(lock_nxt, t) + (t & m.mask)) = LOCK_FREE;
-            *(m.at(lock_nxt, n) + (n & m.mask)) = LOCK_FREE;
+            const int32_t* cc = cand_old.slot(c);
+            const int t = cc[0] / 3, n = cc[1];
+            cl_st(m.at1(lock_nxt, t), LOCK_FREE);
+            cl_st(m.at1(lock_nxt, n), LOCK_FREE);
         }
         for (int i = tid; i < CL_MARK; i += CL_THREADS) mark_nxt[i] = 0u;
         sync();
         const int nf = min(n_flip, FLIP_PER_CTA);
         // a proposal for the next round, queued at the CTA owning its lower half-edge h
         auto add_next = [&](int h, int n, uint32_t p) {
-            atomicMin(m.at(lock_nxt, h / 3) + ((h / 3) & m.mask), p);
-            atomicMin(m.at(lock_nxt, n) + (n & m.mask), p);
+            cl_min(m.at1(lock_nxt, h / 3), p);
+            cl_min(m.at1(lock_nxt, n), p);
             const int owner = (h / 3) >> shift;
             int idx = agg_inc_keyed(sync.remote(&n_cand[nxt], owner));
             if (idx < CAND_PER_CTA) {
-                int32_t* e = cand_list(nxt, owner) + 2 * idx;
+                int32_t* e = cand_list(nxt, owner).slot(idx);
                 e[0] = h;
                 e[1] = n;
             }
         };
         // C1: resolve the outer neighbours (read only); propose the outer edges
         for (int f = tid; f < nf; f += CL_THREADS) {
-            int32_t* q = flips + 6 * f;
+            int32_t* q = flips.slot(f);
             const int t = q[0], n = q[1];
-            int r[4], c[4], tw[4];
-#pragma unroll
-            for (int k = 0; k < 4; ++k) {
-                r[k] = flip_resolve_slot(m, outer_slot(t, n, k), uint32_t(round), T);
-                if (r[k] == -2) { set_err(err, ERRF_BOUNDS); r[k] = -1; }
-            }
-#pragma unroll
-            for (int k = 0; k < 4; ++k) q[2 + k] = r[k];
+            // the pair's vertices in the order of its outer edges: c, a, d, b
+            const int32_t id[4] = {m.v(t, 0), m.v(t, 1), m.v(t, 2), m.v(n, 1)};
+            const uint32_t xy[4] = {m.xy(t, 0), m.xy(t, 1), m.xy(t, 2), m.xy(n, 1)};
+            int32_t r[4];
+            flip_resolve4(m, t, n, id, uint32_t(round), T, r);
+            int c[4], tw[4], vd[4];
+            uint32_t xd[4];
             unsigned claimed = 0;
 #pragma unroll
             for (int k = 0; k < 4; ++k) {
+                if (r[k] == -2) { set_err(err, ERRF_BOUNDS); r[k] = -1; }
+                q[2 + k] = r[k];
                 const int x = outer_slot(t, n, k);
-                // a hull edge (r < 0) tests against its own triangle, is never claimed, and is masked out
+                // a hull edge (r < 0) is never claimed
                 c[k] = r[k] >= 0 ? min(x, r[k]) : x;
-                tw[k] = r[k] >= 0 ? (c[k] == x ? r[k] : x) : x;
+                tw[k] = r[k] >= 0 ? max(x, r[k]) : x;
+                // the vertex beyond the edge
+                const int o = r[k] >= 0 ? r[k] : x, to = o / 3, so = o % 3;
+                vd[k] = m.v(to, so == 0 ? 2 : so - 1);
+                xd[k] = m.xy(to, so == 0 ? 2 : so - 1);
+            }
+#pragma unroll
+            for (int k = 0; k < 4; ++k) {
                 // the edge's bit lives at the CTA that owns its lower half-edge
                 const int owner = (c[k] / 3) >> shift;
                 const int lb = c[k] - 3 * (owner << shift);
                 const uint32_t bit = 1u << (lb & 31);
-                if (r[k] >= 0 && !(atomicOr(sync.remote(mark_nxt, owner) + (lb >> 5), bit) & bit)) claimed |= 1u << k;
+                if (r[k] >= 0 && !(cl_or(cl_map(smem_u32(mark_nxt) + 4u * uint32_t(lb >> 5), owner), bit) & bit)) claimed |= 1u << k;
             }
-            unsigned flippable = 0;
+            // edge_flippable from the pair's side (the determinant and the
+            // perturbation are the same from either side)
+            unsigned want = 0;
 #pragma unroll
-            for (int k = 0; k < 4; ++k) flippable |= edge_flippable(m, c[k], tw[k]) ? 1u << k : 0u;
-            const unsigned want = claimed & flippable;
+            for (int k = 0; k < 4; ++k) {
+                const int k1 = (k + 1) & 3, kc = k == 0 || k == 3 ? 2 : 0;
+                if (inside_sos_p(id[k], xy[k], id[k1], xy[k1], id[kc], xy[kc], vd[k], xd[k])) want |= 1u << k;
+            }
+            want &= claimed;
+            // add_next for the four edges, step by step
+            const unsigned act = __activemask();
+            int base[4], lead[4], before[4];
 #pragma unroll
-            for (int k = 0; k < 4; ++k)
-                if (want & (1u << k)) add_next(c[k], tw[k] / 3, prio(uint32_t(c[k]), uint32_t(round + 1)));
+            for (int k = 0; k < 4; ++k) {
+                const int owner = (c[k] / 3) >> shift;
+                const bool w = want >> k & 1u;
+                const unsigned peers = __match_any_sync(act, w ? owner : -1);
+                lead[k] = __ffs(peers) - 1;
+                before[k] = __popc(peers & ((1u << lane) - 1u));
+                base[k] = 0;
+                if (w && lane == lead[k]) base[k] = cl_add(cl_map(smem_u32(&n_cand[nxt]), owner), __popc(peers));
+            }
+#pragma unroll
+            for (int k = 0; k < 4; ++k) {
+                if (!(want >> k & 1u)) continue;
+                const uint32_t p = prio(uint32_t(c[k]), uint32_t(round + 1));
+                cl_min(m.at1(lock_nxt, c[k] / 3), p);
+                cl_min(m.at1(lock_nxt, tw[k] / 3), p);
+            }
+#pragma unroll
+            for (int k = 0; k < 4; ++k) {
+                const int idx = __shfl_sync(act, base[k], lead[k]) + before[k];
+                if ((want >> k & 1u) && idx < CAND_PER_CTA) {
+                    int32_t* e = cand_list(nxt, (c[k] / 3) >> shift).slot(idx);
+                    e[0] = c[k];
+                    e[1] = tw[k] / 3;
+                }
+            }
         }
         sync();
         // C2: relink; re-propose the own proposals that lost (no outer edge of a flipped pair)
         if (tid == 0) { n_flip = 0; n_cand[cur] = 0; }   // both were read before the last barrier
-        for (int f = tid; f < nf; f += CL_THREADS) flip_relink(m, flips[6 * f], flips[6 * f + 1], flips + 6 * f + 2);
+        for (int f = tid; f < nf; f += CL_THREADS) {
+            const int32_t* q = flips.slot(f);
+            flip_relink(m, q[0], q[1], q + 2);
+        }
         for (int c = tid; c < nc; c += CL_THREADS) {
-            const int h = cand_cur[2 * c], n = cand_cur[2 * c + 1], t = h / 3;
-            if (m.fround(t) != round && m.fround(n) != round) add_next(h, n, prio(uint32_t(h), uint32_t(round + 1)));
+            const int32_t* cc = cand_cur.slot(c);
+            const int h = cc[0], n = cc[1], t = h / 3;
+            const int rt = m.fround(t), rn = m.fround(n);
+            if (rt != round && rn != round) add_next(h, n, prio(uint32_t(h), uint32_t(round + 1)));
         }
         flips_total += nf;
         nc_prev = nc;
@@ -1894,7 +1986,7 @@ __global__ void __launch_bounds__(CL_THREADS) k_flip_smem(DelDev d0, DelDev d1, 
     // write back this CTA's slice
     for (int t = t0 + tid; t < t1; t += CL_THREADS) {
         const int l = t - t0;
-        int32_t v[3] = {m.lv[3 * l], m.lv[3 * l + 1], m.lv[3 * l + 2]};
+        int32_t v[3] = {lv[3 * l], lv[3 * l + 1], lv[3 * l + 2]};
         normalise(v);
         for (int k = 0; k < 3; ++k) D.tri[3 * t + k] = v[k];
     }
