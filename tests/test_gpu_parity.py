@@ -164,6 +164,19 @@ def test_wide_gap_sizes(elas, width, height, gap, speckle, median):
     run_and_compare(elas, L, R, p, check_triangle=False)
 
 
+@pytest.mark.parametrize("width,height,window,threshold", [(170, 45, 0, 5), (165, 330, 3, 0), (331, 167, 7, 5000),
+                                                           (160, 120, 5, -1), (1300, 640, 60, 5)])
+def test_support_filters_at_window_sizes(elas, width, height, window, threshold):
+    """The lattice filters at windows of other half widths than 5 (60: too
+    large for shared memory), thresholds that none or all points meet, and
+    columns and rows of one point up to several words."""
+    L, R, _, _ = eb.synth_pair(3, 47, width=width, height=height, disp_max=32)
+    p = eb.params_config(32)
+    p.incon_window_size = window
+    p.incon_threshold = threshold
+    run_and_compare(elas, L, R, p, check_triangle=False)
+
+
 def test_constructor_default_parameters(elas):
     """Elas::parameters() defaults (support_threshold 0.95, gamma 5, sradius 3,
     ipol_gap_width 5000, median on)."""
