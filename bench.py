@@ -283,9 +283,14 @@ def time_e2e(e, L, R, steps, torch, flush, warmup=3):
     return total, {"h2d_bytes_per_step": 2 * W * H, "d2h_bytes_per_step": 2 * W * H * 4}
 
 
+NO_TRIANGLE = "the reference's Triangle was not built (the oracle needs it for whole pairs)"
+
+
 def cpu_baseline(L, R, p, budget_s=12.0):
     import oracle
 
+    if not oracle.have_triangle():
+        return {"unavailable": NO_TRIANGLE}
     threads = os.cpu_count() or 1
     oracle.process(L, R, p, threads=threads)   # warm-up
     n, t0 = 0, time.perf_counter()
@@ -525,6 +530,9 @@ def run_reference(args):
         return
     import oracle   # the generator and presets come from the oracle library: no product library is loaded
 
+    if not oracle.have_triangle():
+        print(json.dumps({"impl": "reference", "unavailable": NO_TRIANGLE}))
+        return
     W, H, D = oracle.synth_dims(PRESET)
     L, R, _, _ = oracle.synth_pair(PRESET, 1000)
     p = oracle.params_config(D)
