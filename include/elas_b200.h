@@ -160,9 +160,9 @@ int elas_b200_process_batch_device(elas_handle* h, int n,
 
 /* Capture and replay as CUDA graphs (1, default) or run eagerly (0): batches,
  * and single pairs through elas_b200_process / _process_device, whose second
- * call with the same buffers, size, parameters and settings is captured (on
- * the handle's own stream) and whose later calls replay the graph.  A caller
- * that is itself capturing a stream gets plain launches. */
+ * call with the same size, parameters and settings is captured (on the
+ * handle's own stream) and whose later calls replay the graph with their own
+ * buffers.  A caller that is itself capturing a stream gets plain launches. */
 int elas_b200_set_graphs(elas_handle* h, int enable);
 
 /* Fallback switches, for tests of paths that the usual inputs never reach.
