@@ -460,3 +460,14 @@ extern "C" long long emu_orient_p(const int32_t* xy) {
 extern "C" long long emu_incircle_p(const int32_t* xy) {
     return incircle_p(pack_xy(xy[0], xy[1]), pack_xy(xy[2], xy[3]), pack_xy(xy[4], xy[5]), pack_xy(xy[6], xy[7]));
 }
+
+// star_better and star_better_left on one edge p->q and two points a, b
+// (xy: x, y of p, q, a, b; id: their indices): -1 where a or b is not
+// strictly left of the edge, else whether the two agree.
+extern "C" int emu_star_better_agree(const int32_t* xy, const int32_t* id) {
+    uint32_t c[4];
+    for (int k = 0; k < 4; ++k) c[k] = pack_xy(xy[2 * k], xy[2 * k + 1]);
+    if (!star_side(c[0], c[1], c[2], 1) || !star_side(c[0], c[1], c[3], 1)) return -1;
+    return star_better(id[0], c[0], id[1], c[1], id[2], c[2], id[3], c[3], 1) ==
+           star_better_left(id[0], c[0], id[1], c[1], id[2], c[2], id[3], c[3]);
+}

@@ -246,3 +246,21 @@ def test_three_phase_rounds_equal_worklist_rounds(emu_lib):
         t1, s1 = emu_triangulate(emu_lib, xy, row_of, phased=True)
         assert np.array_equal(t0, t1)
         assert tuple(s0) == tuple(s1)
+
+
+@pytest.mark.parametrize("xr,yr", [(3, 3), (12, 40), (14000, 16383)])
+def test_star_order_on_the_left_agrees_with_the_general_one(emu_lib, xr, yr):
+    """star_better_left against star_better on small grids (many co-circular
+    points, every order of the indices) and up to the size limits."""
+    rng = np.random.default_rng(xr)
+    seen = 0
+    for _ in range(20000):
+        xy = np.empty((4, 2), np.int32)
+        xy[:, 0], xy[:, 1] = rng.integers(0, xr + 1, 4), rng.integers(0, yr + 1, 4)
+        if len({tuple(q) for q in xy.tolist()}) < 4:
+            continue
+        ids = rng.permutation(4).astype(np.int32)
+        r = emu_lib.emu_star_better_agree(xy.ctypes.data_as(ctypes.c_void_p), ids.ctypes.data_as(ctypes.c_void_p))
+        assert r != 0, (xy.tolist(), ids.tolist())
+        seen += r == 1
+    assert seen > 500
