@@ -54,6 +54,7 @@ struct elas_handle {
     // workspace arena
     void* arena = nullptr;
     size_t arena_bytes = 0;
+    int64_t workspace_version = 0;    // bumped whenever a buffer of the arena or the proposal is allocated anew
     Geom g{};          // geometry of the last call
     bool have_last = false;
 
@@ -333,6 +334,7 @@ size_t layout(elas_handle* h, const Geom& g, char* base) {
 int ensure_workspace(elas_handle* h, const Geom& g) {
     size_t need = layout(h, g, nullptr);
     if (need > h->arena_bytes) {
+        ++h->workspace_version;
         if (h->arena) {
             CK(cudaDeviceSynchronize());
             CK(cudaFree(h->arena));
@@ -432,6 +434,7 @@ int ensure_pn(elas_handle* h, const Geom& g) {
     const size_t elems = size_t(2) * (g.H / 4) * (g.W / 4) * pn::CH;
     const size_t cands = size_t(g.cw) * g.ch;
     if (elems > h->pn_map_elems) {
+        ++h->workspace_version;
         CK(cudaDeviceSynchronize());
         __nv_bfloat16** bufs[4] = {&h->pn_in, &h->pn_a0, &h->pn_a1, &h->pn_out};
         for (auto b : bufs) {
@@ -443,6 +446,7 @@ int ensure_pn(elas_handle* h, const Geom& g) {
         h->pn_map_elems = elems;
     }
     if (cands > h->pn_cands) {
+        ++h->workspace_version;
         CK(cudaDeviceSynchronize());
         if (h->pn_bins) cudaFree(h->pn_bins);
         h->pn_bins = nullptr;
@@ -1139,9 +1143,10 @@ int elas_b200_process_batch_device(elas_handle* h, int n, const uint8_t* const* 
     rc = ensure_slots(h, n);
     if (rc != ELAS_OK) return fail(h, rc, "creating batch workers failed");
     cudaStream_t st = stream ? (cudaStream_t)stream : h->own_stream;
-    // what a captured graph depends on: sizes, disparity ranges, buffers, parameters
-    std::vector<int64_t> sig;
-    sig.push_back(n);
+    // what a captured graph depends on: sizes, disparity ranges, buffers,
+    // parameters, proposal weights, and the workers' workspaces (another
+    // batch in between may have allocated those anew)
+    std::vector<int64_t> sig = {n, h->prop ? 1 : 0, h->prop_version};
     for (int i = 0; i < n; ++i) {
         sig.push_back(dims[2 * i]);
         sig.push_back(dims[2 * i + 1]);
@@ -1157,6 +1162,12 @@ int elas_b200_process_batch_device(elas_handle* h, int n, const uint8_t* const* 
     sig.push_back(int64_t(st));
     sig.push_back(h->test_flags);
     sig.push_back(h->flip_round_limit);
+    const size_t fixed = sig.size();
+    auto add_workspaces = [&] {
+        sig.resize(fixed);
+        for (int i = 0; i < n; ++i) sig.push_back(h->slots[i]->workspace_version);
+    };
+    add_workspaces();
     if (h->use_graphs && h->graph_exec && sig == h->graph_sig) {
         CK(cudaGraphLaunch(h->graph_exec, st));
     } else {
@@ -1176,6 +1187,7 @@ int elas_b200_process_batch_device(elas_handle* h, int n, const uint8_t* const* 
             e = cudaGraphInstantiate(&h->graph_exec, graph, 0);
             cudaGraphDestroy(graph);
             if (e != cudaSuccess) { h->graph_exec = nullptr; return cuda_fail(h, e, "cudaGraphInstantiate"); }
+            add_workspaces();           // as the eager run left them
             h->graph_sig = sig;
         }
     }

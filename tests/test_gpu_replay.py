@@ -1,0 +1,83 @@
+"""Replayed CUDA graphs against fresh runs: whatever happens to a handle
+between two calls with the same sizes, buffers and parameters, a replay must
+give what a handle without a graph gives."""
+import numpy as np
+import pytest
+
+import elas_b200 as eb
+
+pytestmark = pytest.mark.gpu
+
+
+class Batch:
+    """Device buffers of a batch, its inputs, and the call on them."""
+
+    def __init__(self, shapes, seed):
+        import torch
+
+        self.torch = torch
+        self.dims, self.dmax = [(w, h) for w, h, _ in shapes], [d for _, _, d in shapes]
+        self.images = [eb.synth_pair(3, seed + i, width=w, height=h, disp_max=d, gt=False)[:2]
+                       for i, (w, h, d) in enumerate(shapes)]
+        self.bufs = [[torch.from_numpy(x).cuda() for x in p] + [torch.empty((h, w), device="cuda") for _ in range(2)]
+                     for p, (w, h, _) in zip(self.images, shapes)]
+
+    def run(self, e):
+        for b in self.bufs:
+            b[2].fill_(7.0)
+            b[3].fill_(7.0)
+        self.torch.cuda.synchronize()
+        e.process_batch_device(*[[b[k].data_ptr() for b in self.bufs] for k in range(4)], self.dims, self.dmax)
+        self.torch.cuda.synchronize()
+        return [b[k].cpu().numpy() for b in self.bufs for k in (2, 3)]
+
+
+def singles(batch, weights=None):
+    out = []
+    for (L, R), d in zip(batch.images, batch.dmax):
+        e = eb.Elas(eb.params_config(d))
+        e.set_graphs(False)
+        e.set_proposal(weights)
+        out += e.process(L, R)
+        e.close()
+    return out
+
+
+def same(a, b):
+    return all(np.array_equal(x, y) for x, y in zip(a, b))
+
+
+def test_batch_replays_follow_the_proposal():
+    """A batch that was captured without the learned proposal, called again
+    with it, with other weights and without it."""
+    import proposal_oracle as po
+
+    batch = Batch([(640, 480, 128), (480, 272, 128)], 310)
+    sets = [None, eb.load_proposal(), po.init_params(2), None]
+    e = eb.Elas(eb.params_config(128))
+    try:
+        expected = {}
+        for k, w in enumerate(sets):
+            e.set_proposal(w)
+            ref = expected[k] = singles(batch, w)
+            for _ in range(3):                  # eager and captured, then replayed twice
+                assert same(batch.run(e), ref), k
+        assert not same(expected[0], expected[1])       # the proposal does change these maps
+    finally:
+        e.close()
+
+
+def test_batch_replays_after_larger_batches():
+    """A captured batch called again after batches of larger pairs, host and
+    device, have made the workers allocate other workspaces."""
+    small, large = Batch([(160, 120, 47), (200, 144, 63)], 330), Batch([(640, 480, 128), (800, 600, 255)], 340)
+    ref_small, ref_large = singles(small), singles(large)
+    e = eb.Elas(eb.params_config(64))
+    try:
+        assert same(small.run(e), ref_small) and same(small.run(e), ref_small)
+        o1, o2 = e.process_batch([p[0] for p in large.images], [p[1] for p in large.images], large.dmax)
+        assert same([x for p in zip(o1, o2) for x in p], ref_large)
+        assert same(small.run(e), ref_small) and same(small.run(e), ref_small)
+        assert same(large.run(e), ref_large) and same(small.run(e), ref_small)
+    finally:
+        e.close()
