@@ -721,10 +721,8 @@ int run_pipeline_graphed(elas_handle* h, const uint8_t* img0, const uint8_t* img
     }
     // images on 16-byte boundaries take another descriptor kernel
     const int64_t aligned = ((reinterpret_cast<uintptr_t>(img0) | reinterpret_cast<uintptr_t>(img1)) & 15) == 0;
-    std::vector<int64_t> sig = {aligned, W, H, int64_t(h->arena), int64_t(h->arena_bytes), int64_t(h->pn_in),
-                                int64_t(h->pn_bins),
-                                int64_t(h->pn_stats), h->timing ? 1 : 0, h->prop ? 1 : 0, h->prop_version,
-                                h->test_flags, h->flip_round_limit};
+    std::vector<int64_t> sig = {aligned, W, H, h->workspace_version, h->timing ? 1 : 0, h->prop ? 1 : 0,
+                                h->prop_version, h->test_flags, h->flip_round_limit};
     int64_t pw[sizeof(elas_params) / 8 + 1] = {};
     std::memcpy(pw, &h->params, sizeof(elas_params));
     for (int64_t x : pw) sig.push_back(x);

@@ -81,3 +81,28 @@ def test_batch_replays_after_larger_batches():
         assert same(large.run(e), ref_large) and same(small.run(e), ref_small)
     finally:
         e.close()
+
+
+def test_pair_replays_after_the_network_maps_were_reallocated():
+    """A captured pair with the proposal called again after elas_b200_pn_infer
+    on larger maps has made the handle allocate its feature maps anew."""
+    import torch
+
+    W, H, D = 160, 120, 47
+    weights = eb.load_proposal()
+    e, other = eb.Elas(eb.params_config(D)), eb.Elas(eb.params_config(D))
+    other.set_graphs(False)
+    for h in (e, other):
+        h.set_proposal(weights)
+    try:
+        for k, (hd, wd) in enumerate([(0, 0), (40, 50), (150, 200), (500, 600)]):
+            if hd:
+                x = torch.zeros((2, hd, wd, 32), dtype=torch.bfloat16, device="cuda")
+                e.pn_infer(x.data_ptr(), torch.empty_like(x).data_ptr(), hd, wd)
+            L, R = eb.synth_pair(3, 350 + k, width=W, height=H, disp_max=D, gt=False)[:2]
+            ref = other.process(L, R)
+            for _ in range(3):
+                assert same(e.process(L, R), ref), k
+    finally:
+        e.close()
+        other.close()
