@@ -1168,6 +1168,7 @@ int elas_b200_process_batch_device(elas_handle* h, int n, const uint8_t* const* 
     add_workspaces();
     if (h->use_graphs && h->graph_exec && sig == h->graph_sig) {
         CK(cudaGraphLaunch(h->graph_exec, st));
+        h->last_batch = n;
     } else {
         // eager run: sizes every workspace, tunes the dense shape, produces the result
         rc = issue_batch(h, n, d_lefts, d_rights, d_disp_lefts, d_disp_rights, dims, disp_max_per_pair, false, st);

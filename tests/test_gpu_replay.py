@@ -106,3 +106,21 @@ def test_pair_replays_after_the_network_maps_were_reallocated():
     finally:
         e.close()
         other.close()
+
+
+def test_batch_latency_belongs_to_the_last_batch():
+    """elas_b200_batch_latency after a replay that follows a batch of another
+    length: the replayed batch's pairs."""
+    three, one = Batch([(160, 120, 47)] * 3, 360), Batch([(96, 64, 31)], 370)
+    e = eb.Elas(eb.params_config(64))
+    try:
+        three.run(e)
+        three.run(e)
+        L, R = one.images[0]
+        e.process_batch([L], [R], one.dmax)
+        assert len(e.batch_latency(3)) == 1
+        three.run(e)
+        lat = e.batch_latency(3)
+        assert len(lat) == 3 and (lat > 0).all()
+    finally:
+        e.close()
