@@ -656,7 +656,8 @@ void drop_single_graph(elas_handle* h) {
 
 // Point the captured pair at these buffers: the nodes that take them get new
 // arguments (a microsecond or two on the host, only when a buffer changed),
-// which launches already under way do not see.
+// which launches already under way do not see.  After a failure some nodes
+// may have the new buffers and others the old ones: the graph must go.
 int bind_buffers(elas_handle* h, const PairBuffers& io) {
     const PairNodes& nd = h->single_nodes;
     PairBuffers& now = h->single_io;
@@ -676,6 +677,7 @@ int bind_buffers(elas_handle* h, const PairBuffers& io) {
         CK(cudaGraphExecKernelNodeSetParams(h->single_exec, nd.desc, &p));
     }
     if (io.out0 != now.out0 || io.out1 != now.out1) {
+        if (h->test_flags & ELAS_TEST_REBIND_FAILS) return fail(h, ELAS_ERR_CUDA, "rebinding made to fail");
         float *o0 = io.out0, *o1 = io.out1;
         if (nd.lr && (nd.lr_out[0] || nd.lr_out[1])) {
             CK(fetch(nd.lr, LR_ARGS));
@@ -728,8 +730,11 @@ int run_pipeline_graphed(elas_handle* h, const uint8_t* img0, const uint8_t* img
     for (int64_t x : pw) sig.push_back(x);
     const PairBuffers io{img0, img1, out0, out1};
     if (h->single_exec && sig == h->single_sig) {
-        rc = bind_buffers(h, io);
-        if (rc != ELAS_OK) return rc;
+        if (bind_buffers(h, io) != ELAS_OK) {
+            cudaGetLastError();         // not this run's
+            drop_single_graph(h);       // the next call captures another one
+            return run_pipeline(h, img0, img1, out0, out1, W, H, st);
+        }
         CK(cudaGraphLaunch(h->single_exec, st));
         h->g = g;   // what run_pipeline leaves behind for the stage dumps
         h->pn_used = h->prop && H >= 4 && W >= 4 && g.cw > 0 && g.ch > 0;
@@ -1198,7 +1203,7 @@ int elas_b200_set_test_mode(elas_handle* h, int32_t flags, int32_t flip_round_li
     if (!h) return ELAS_ERR_INVALID_ARG;
     const int32_t known = ELAS_TEST_FLIP_GLOBAL | ELAS_TEST_DENSE_BITSET | ELAS_TEST_PRIOR_TILED |
                           ELAS_TEST_PRIOR_DIRECT | ELAS_TEST_DELAUNAY_FLIPS | ELAS_TEST_DELAUNAY_STARS |
-                          ELAS_TEST_PRIOR_SMALL_BINS;
+                          ELAS_TEST_PRIOR_SMALL_BINS | ELAS_TEST_REBIND_FAILS;
     if ((flags & ~known) != 0 || flip_round_limit < 0)
         return fail(h, ELAS_ERR_INVALID_ARG, "unknown test flag or negative round limit");
     if ((flags & ELAS_TEST_DELAUNAY_STARS) &&

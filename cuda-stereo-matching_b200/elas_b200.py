@@ -293,6 +293,7 @@ class Elas:
     TEST_DELAUNAY_FLIPS = 16  # triangulations from row strips and edge flips at every size
     TEST_DELAUNAY_STARS = 32  # triangulations found star by star at every size
     TEST_PRIOR_SMALL_BINS = 256  # tiled prior paint with 2-entry tile bins (the overflow list used)
+    TEST_REBIND_FAILS = 512   # a captured pair cannot be given other output buffers
 
     def set_test_mode(self, flags=0, flip_round_limit=0):
         """Force fallback paths (results unchanged) and/or cap the flip rounds

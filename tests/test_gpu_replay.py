@@ -124,3 +124,32 @@ def test_batch_latency_belongs_to_the_last_batch():
         assert len(lat) == 3 and (lat > 0).all()
     finally:
         e.close()
+
+
+def test_pair_survives_a_failed_rebind():
+    """A captured pair whose images could be rebound but not its outputs: that
+    call and the later ones, on the first and the other buffers, give their
+    own images' maps in their own outputs."""
+    import torch
+
+    W, H, D = 160, 120, 47
+    e, other = eb.Elas(eb.params_config(D)), eb.Elas(eb.params_config(D))
+    e.set_test_mode(eb.Elas.TEST_REBIND_FAILS)
+    other.set_graphs(False)
+    pairs = [eb.synth_pair(3, 380 + k, width=W, height=H, disp_max=D, gt=False)[:2] for k in range(2)]
+    refs = [other.process(L, R) for L, R in pairs]
+    sets = [[torch.from_numpy(x).cuda() for x in p] + [torch.empty((H, W), device="cuda") for _ in range(2)]
+            for p in pairs]
+    try:
+        for k, i in enumerate([0, 0, 0, 1, 0, 0, 1, 1, 1, 0]):     # eager, captured, replayed, refused, ...
+            for b in sets:
+                b[2].fill_(7.0)
+                b[3].fill_(7.0)
+            torch.cuda.synchronize()
+            e.process_device(*[x.data_ptr() for x in sets[i]], W, H)
+            torch.cuda.synchronize()
+            assert same([x.cpu().numpy() for x in sets[i][2:]], refs[i]), k
+            assert bool((sets[1 - i][2] == 7.0).all()), k
+    finally:
+        e.close()
+        other.close()
