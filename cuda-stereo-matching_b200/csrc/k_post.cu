@@ -328,7 +328,9 @@ __global__ void __launch_bounds__(SPK_T * SPK_ROWS, 64 / SPK_ROWS)
         before = atomicAdd(&tick[(vertical ? 0 : txn * tyn) + by * txn + bx], 1);
         __threadfence();                // the other tile's labels after it
     }
-    if (__shfl_sync(0xffffffffu, before, 0) == 0) return;       // the other tile is yet to end
+    before = __shfl_sync(0xffffffffu, before, 0);
+    __syncwarp();                       // ... in every lane (the shuffle orders no memory)
+    if (before == 0) return;            // the other tile is yet to end
     const int xa = vertical ? bx * SPK_T + SPK_T - 1 : bx * SPK_T + tx;
     const int ya = vertical ? by * SPK_T + tx : by * SPK_T + SPK_T - 1;
     int a = -1, b = -1;
