@@ -227,6 +227,54 @@ __global__ void __launch_bounds__(CT_THREADS, 1) k_conv_f32(const float* __restr
     }
 }
 
+// The same convolution, the same sums in the same order, for small maps: a
+// block takes ROW_SEG cells of one image row x 32 output channels (lane =
+// output channel, warp = cell), with the three input rows of the segment (and
+// a one-cell halo) and all weights in shared memory.  A thread has one
+// output, so a map of a few thousand cells still spreads over every SM,
+// where k_conv_f32's tiles would leave most of them idle and one group would
+// take 31-33 us for the first of them.
+constexpr int ROW_SEG = 32;
+constexpr size_t CONV_ROWS_SMEM = sizeof(float) * (TAPS * CH * CH + 3 * (ROW_SEG + 2) * CH);
+
+__global__ void __launch_bounds__(ROW_SEG * CH) k_conv_f32_rows(const float* __restrict__ x,
+                                                                const float* __restrict__ mask,
+                                                                const float* __restrict__ w,
+                                                                const float* __restrict__ b, float* __restrict__ y,
+                                                                int Hd, int Wd, int relu) {
+    grid_dep_wait();
+    extern __shared__ float row_sm[];
+    float* sw = row_sm;                                                   // [TAPS][ci][co]
+    float(*sx)[ROW_SEG + 2][CH] = reinterpret_cast<float(*)[ROW_SEG + 2][CH]>(row_sm + TAPS * CH * CH);
+    const int n = blockIdx.z, row = blockIdx.y, x0 = blockIdx.x * ROW_SEG;
+    const int co = threadIdx.x & 31, cell = threadIdx.x >> 5;
+    for (int i = threadIdx.x; i < TAPS * CH * CH; i += blockDim.x) sw[i] = w[i];
+    for (int i = threadIdx.x; i < 3 * (ROW_SEG + 2) * CH; i += blockDim.x) {
+        const int c = i % CH, j = (i / CH) % (ROW_SEG + 2), r = i / (CH * (ROW_SEG + 2));
+        const int yy = row + r - 1, xx = x0 + j - 1;
+        float v = 0.0f;
+        if (yy >= 0 && yy < Hd && xx >= 0 && xx < Wd) {
+            const size_t at = ((size_t(n) * Hd + yy) * Wd + xx) * CH + c;
+            v = x[at];
+            if (mask && !(mask[at] > 0.0f)) v = 0.0f;
+        }
+        sx[r][j][c] = v;
+    }
+    __syncthreads();
+    const int xo = x0 + cell;
+    if (xo >= Wd) return;
+    float acc = b ? b[co] : 0.0f;
+#pragma unroll
+    for (int t = 0; t < TAPS; ++t) {
+        const float* xs = sx[t / 3][cell + t % 3];
+        const float* ws = sw + t * CH * CH + co;
+#pragma unroll 8
+        for (int ci = 0; ci < CH; ++ci) acc = fmaf(xs[ci], ws[ci * CH], acc);
+    }
+    if (relu) acc = fmaxf(acc, 0.0f);
+    y[((size_t(n) * Hd + row) * Wd + xo) * CH + co] = acc;
+}
+
 // Wt[8 - t][co][ci] = W[t][ci][co]: the gradient of a layer input is the
 // same convolution of the output gradient with these weights.
 __global__ void k_flip_weights(const float* __restrict__ w, float* __restrict__ wt) {
@@ -588,10 +636,20 @@ int tile_grid(long long tiles, int ctas) { return int(tiles < ctas ? tiles : cta
 
 cudaError_t launch_conv_f32(const float* x, const float* mask, const float* w, const float* b, float* y, int nimg,
                             int Hd, int Wd, int relu, cudaStream_t st) {
+    const int sms = sm_count();
+    // 83 cells an SM (12284): rows of 1 x 16 x 32, 2 x 60 x 80 and 10 x 20 x
+    // 64 cells take 13, 29 and 29 us, tiles 33 of all three; 2 x 93 x 80
+    // (14880 cells) 39 and 33, 2 x 93 x 310 115 and 33
+    if ((long long)nimg * Hd * Wd <= 83LL * sms) {
+        allow_smem(k_conv_f32_rows);
+        k_conv_f32_rows<<<dim3((Wd + ROW_SEG - 1) / ROW_SEG, Hd, nimg), ROW_SEG * CH, CONV_ROWS_SMEM, st>>>(
+            x, mask, w, b, y, Hd, Wd, relu);
+        return cudaGetLastError();
+    }
     allow_smem(k_conv_f32);
     const long long tiles = (long long)nimg * ((Wd + CT_W - 1) / CT_W) * ((Hd + CT_H - 1) / CT_H);
-    k_conv_f32<<<tile_grid(tiles, sm_count()), CT_THREADS, CONV_F32_SMEM, st>>>(
-        x, mask, w, b, y, nimg, Hd, Wd, relu, aligned16({x, mask, y}));
+    k_conv_f32<<<tile_grid(tiles, sms), CT_THREADS, CONV_F32_SMEM, st>>>(x, mask, w, b, y, nimg, Hd, Wd, relu,
+                                                                         aligned16({x, mask, y}));
     return cudaGetLastError();
 }
 

@@ -257,3 +257,62 @@ def test_training_convolutions_at_tile_edges(torch, nimg, hd, wd, shift):
     assert bool(((gw.cpu().double().view(w.shape) - wgrad(xd, g)).abs()
                  <= cells * 2.0 ** -23 * wgrad(xd.abs(), g.abs())).all())
     assert bool(((gb.cpu().double() - g.sum((0, 1, 2))).abs() <= cells * 2.0 ** -23 * g.abs().sum((0, 1, 2))).all())
+
+
+def _conv_pair(torch, nimg, hd, wd, shift, groups):
+    """Forward map and input gradient of `nimg` images, `groups` equal calls
+    after one another on parts of the same buffers."""
+    gen = torch.Generator().manual_seed(100 * hd + wd + shift)
+    ch, taps = po.CH, po.TAPS
+
+    def buf(t):
+        b = torch.zeros(t.numel() + 4, device="cuda")[shift:shift + t.numel()]
+        b.copy_(t.reshape(-1))
+        return b
+
+    x, dy = (buf(torch.randn((nimg, hd, wd, ch), generator=gen)) for _ in range(2))
+    w, b = buf(torch.randn((taps, ch, ch), generator=gen) * 0.1), buf(torch.randn(ch, generator=gen))
+    y, dx = torch.full_like(x, 9.0), torch.full_like(x, 9.0)
+    gw, gb, scratch = buf(torch.zeros(taps * ch * ch)), buf(torch.zeros(ch)), buf(torch.zeros(taps * ch * ch))
+    n = nimg // groups
+    part = 4 * n * hd * wd * ch                 # bytes
+    for k in range(groups):
+        at = [t.data_ptr() + k * part for t in (x, y, dy, dx)]
+        eb.pn_conv_forward(at[0], w.data_ptr(), b.data_ptr(), at[1], n, hd, wd, True)
+        eb.pn_conv_backward(at[0], at[1], w.data_ptr(), at[2], at[3], gw.data_ptr(), gb.data_ptr(),
+                            scratch.data_ptr(), n, hd, wd, True)
+    torch.cuda.synchronize()
+    return y, dx
+
+
+@pytest.mark.parametrize("shift", [0, 1])
+@pytest.mark.parametrize("nimg,hd,wd", [(12800, 1, 1), (60, 8, 32), (30, 16, 32), (50, 9, 33), (90, 5, 31), (12, 17, 65),
+                                        (2, 37, 332)])
+def test_training_convolutions_equal_over_the_dispatch(torch, nimg, hd, wd, shift):
+    """The same images in one call, large enough for the tile kernel, and in
+    small calls, which the row kernel takes (37 x 332 cells: the most it
+    takes on 148 SMs): the same bits, as both add in the same order."""
+    assert nimg * hd * wd > 12284 and nimg * hd * wd // 2 <= 12284
+    for a, b in zip(_conv_pair(torch, nimg, hd, wd, shift, 1), _conv_pair(torch, nimg, hd, wd, shift, 2)):
+        assert torch.equal(a, b), int((a != b).sum())
+
+
+def test_small_training_convolutions_take_less_time(torch):
+    """A layer on 1 x 16 x 32 cells takes less than 0.6 of the time of one on
+    73 times as many (2 x 60 x 310), each the fastest of 20 times 20 calls."""
+    ms = []
+    for nimg, hd, wd in [(1, 16, 32), (2, 60, 310)]:
+        n = nimg * hd * wd * po.CH
+        x, y = torch.zeros(n, device="cuda"), torch.zeros(n, device="cuda")
+        w, b = torch.zeros(po.TAPS * po.CH * po.CH, device="cuda"), torch.zeros(po.CH, device="cuda")
+        times = []
+        for _ in range(20):
+            t0, t1 = (torch.cuda.Event(enable_timing=True) for _ in range(2))
+            t0.record()
+            for _ in range(20):
+                eb.pn_conv_forward(x.data_ptr(), w.data_ptr(), b.data_ptr(), y.data_ptr(), nimg, hd, wd, True)
+            t1.record()
+            torch.cuda.synchronize()
+            times.append(t0.elapsed_time(t1))
+        ms.append(min(times))
+    assert ms[0] < 0.6 * ms[1], ms
