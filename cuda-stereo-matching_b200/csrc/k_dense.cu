@@ -7,7 +7,7 @@
 // Two ways to paint, chosen by image size (both give the same bytes):
 //   * direct: a warp per piece of a triangle, lanes over its pixels, atomics
 //     straight into the zeroed prior (one launch after the memset, each CTA
-//     setting its triangles up itself; the faster one for small images);
+//     setting its triangles up itself; the faster one up to some megapixels);
 //   * tiled: the set-up also finds the 64x32 prior tiles a triangle's pixels
 //     can fall in and drops the triangle into each tile's fixed bin (the
 //     slot its count's atomic returns; no scan), and one CTA per tile paints
@@ -30,6 +30,7 @@
 // bitset walked in ascending order (the reference's sorted int list),
 // skipping the plane window, then the plane window with the penalty added.
 // Strict '<' keeps the first minimum in that order, as the reference does.
+#include <algorithm>
 #include <cuda_runtime.h>
 #include "common.cuh"
 #include "launch.cuh"
@@ -301,17 +302,25 @@ __device__ __forceinline__ void paint_warp(const Raster& R, int wu0, int wu1, in
     }
 }
 
-// Direct paint: a CTA takes every gridDim-th triangle of both views' lists,
-// up to 32 at a time; a lane of its first warp sets each of them up in
-// shared memory, and its warps share out their RASTER_W x RASTER_H pieces;
-// every pixel keeps the last covering triangle through atomicMax on the
-// packed value in the zeroed prior.  What it waits for is the largest
-// triangles (neighbours at the hull, so consecutive in the list) and the
-// double-precision solve's chain: a warp per triangle that sets it up and
-// paints all of it took 17.5 us at 1242x375, 33 with the default parameters
-// and 11 at 450x375; now 11.5, 13.8 and 8.0 (pieces of 32 or 64 columns: 13;
-// CTAs of 64 threads: 17.5).
+// Direct paint: groups of CTAs take the triangles of both views' lists in
+// turn, up to 32 at a time; in each CTA a lane of the first warp sets each
+// of them up in shared memory, and the group's warps share out the
+// RASTER_W x RASTER_H pieces of all of them; every pixel keeps the last
+// covering triangle through atomicMax on the packed value in the zeroed
+// prior.  What it waits for is the largest triangles (neighbours at the hull,
+// so consecutive in the list) and the double-precision solve's chain, which
+// takes as long for 32 triangles as for one.  So a group has as many CTAs (a
+// power of two) as let each set up one batch of 32 (fewer, larger triangles:
+// more CTAs share them), but no more than leave each warp some eight pieces
+// of a triangle that covers the whole image (RASTER_SHARE pixels a CTA).  A
+// warp per triangle that sets it up and paints all of it took 17.5 us at
+// 1242x375 and 33 with the default parameters; a CTA per triangle 11.6, 13.7
+// and 29 at 1920x1080, but 420 there where the corner points' triangles
+// cover a textureless image; now 9.9, 10.8, 23 and 37 (groups at every image
+// size: 160x120 6.3 in place of 4.9; pieces of 32 or 64 columns: 13 at
+// 1242x375; CTAs of 64 threads: 17.5).
 constexpr int RASTER_THREADS = 128, RASTER_CTAS_PER_SM = 8, RASTER_W = 16, RASTER_H = 64;
+constexpr int RASTER_SHARE = 8 * RASTER_THREADS / 32 * RASTER_W * RASTER_H;
 __global__ void __launch_bounds__(RASTER_THREADS, RASTER_CTAS_PER_SM)
     k_prior_raster(const int32_t* __restrict__ tri0, const int32_t* __restrict__ tri1,
                    const int32_t* __restrict__ ctr0, const int32_t* __restrict__ ctr1,
@@ -319,41 +328,57 @@ __global__ void __launch_bounds__(RASTER_THREADS, RASTER_CTAS_PER_SM)
                    uint32_t* prior1, Geom g, int pshift, int dcap) {
     grid_dep_wait();
     __shared__ Raster sr[32];
+    __shared__ int first[32];           // pieces of the triangles before
+    __shared__ int pieces;
     constexpr int WARPS = RASTER_THREADS / 32;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int T0 = ctr0[0], T = T0 + ctr1[0];
     const int ctas = gridDim.x;
-    for (int base = blockIdx.x; base < T; base += 32 * ctas) {
-        const int n = imin((T - base + ctas - 1) / ctas, 32);
-        if (int(threadIdx.x) < n) {
-            const int i = base + int(threadIdx.x) * ctas;
-            const bool right = i >= T0;
-            Raster R;
-            setup_triangle((right ? tri1 : tri0) + 3 * size_t(right ? i - T0 : i), can, uvd, g.cw, g.step, right, R);
-            int r0 = g.H, r1 = -1;
-            part_rows(R, 0, g.W, g.H, r0, r1);
-            part_rows(R, 1, g.W, g.H, r0, r1);
-            R.ty0 = r0;
-            R.ty1 = r1;
-            sr[threadIdx.x] = R;
+    int sh = 0;                         // 2^sh CTAs a group
+    while ((2 << sh) <= g.W * g.H / RASTER_SHARE && (T << sh) <= 16 * ctas && (2 << sh) <= ctas) ++sh;
+    const int groups = ctas >> sh, group = blockIdx.x >> sh;
+    if (group >= groups) return;
+    for (int base = group; base < T; base += 32 * groups) {
+        const int n = imin((T - base + groups - 1) / groups, 32);
+        if (warp == 0) {
+            int count = 0;
+            if (lane < n) {
+                const int i = base + lane * groups;
+                const bool right = i >= T0;
+                Raster R;
+                setup_triangle((right ? tri1 : tri0) + 3 * size_t(right ? i - T0 : i), can, uvd, g.cw, g.step, right,
+                               R);
+                int r0 = g.H, r1 = -1;
+                part_rows(R, 0, g.W, g.H, r0, r1);
+                part_rows(R, 1, g.W, g.H, r0, r1);
+                // pieces in a row and in all, from column tx1 and row ty0 on
+                R.tx1 = imax(int(R.A_u), 0);
+                R.tx0 = imax((imin(int(R.C_u), g.W) - R.tx1 + RASTER_W - 1) / RASTER_W, 0);
+                R.ty0 = r0;
+                count = R.tx0 * imax((r1 - r0 + RASTER_H) / RASTER_H, 0);
+                sr[lane] = R;
+            }
+            int upto = count;
+#pragma unroll
+            for (int o = 1; o < 32; o <<= 1) {
+                const int y = __shfl_up_sync(0xffffffffu, upto, o);
+                if (lane >= o) upto += y;
+            }
+            first[lane] = upto - count;
+            if (lane == 31) pieces = upto;
         }
         __syncthreads();
-        // triangles of many columns by all warps, the others by a warp each
-        for (int k = 0; k < n; ++k) {
-            const int i = base + k * ctas;
+        const int total = pieces, before = first[lane];
+        for (int p = (int(blockIdx.x) & ((1 << sh) - 1)) * WARPS + warp; p < total; p += WARPS << sh) {
+            const int k = __popc(__ballot_sync(0xffffffffu, before <= p)) - 1;     // the piece's triangle
+            const int c = p - __shfl_sync(0xffffffffu, before, k), i = base + k * groups;
             const bool right = i >= T0;
             const uint32_t tag = uint32_t((right ? i - T0 : i) + 1) << pshift;
             uint32_t* prior = right ? prior1 : prior0;
             const Raster& R = sr[k];
-            const int u0 = imax(int(R.A_u), 0), v0 = R.ty0;
-            const int nx = (imin(int(R.C_u), g.W) - u0 + RASTER_W - 1) / RASTER_W;
-            const int ny = (R.ty1 - v0 + RASTER_H) / RASTER_H;
-            if (nx <= 0 || ny <= 0) continue;
-            for (int c = nx * ny == 1 ? (k + warp) % WARPS : warp; c < nx * ny; c += WARPS) {
-                const int wu = u0 + c % nx * RASTER_W, wv = v0 + c / nx * RASTER_H;
-                paint_warp(R, wu, imin(wu + RASTER_W, g.W), wv, imin(wv + RASTER_H, g.H), lane, dcap,
-                           [&](int u, int v, uint32_t d) { atomicMax(&prior[size_t(v) * g.W + u], tag | d); });
-            }
+            const int wu = R.tx1 + c % R.tx0 * RASTER_W, wv = R.ty0 + c / R.tx0 * RASTER_H;
+            paint_warp(R, wu, imin(wu + RASTER_W, g.W), wv, imin(wv + RASTER_H, g.H), lane, dcap,
+                       [&](int u, int v, uint32_t d) { atomicMax(&prior[size_t(v) * g.W + u], tag | d); });
         }
         __syncthreads();
     }
@@ -636,8 +661,9 @@ cudaError_t launch_prior(const int32_t* tri0, const int32_t* tri1, const int32_t
             cudaMemsetAsync(prior0, 0, n, st);
             cudaMemsetAsync(prior1, 0, n, st);
         }
-        launch_k(k_prior_raster, imax(1, imin(RASTER_CTAS_PER_SM * num_sms, 2 * Tmax)), RASTER_THREADS, 0, st, tri0, tri1, ctr0, ctr1,
-                 can, uvd, prior0, prior1, g, pshift, dcap);
+        const long long most = 2LL * Tmax * imax(1, g.W * g.H / RASTER_SHARE);      // CTAs that can have work
+        launch_k(k_prior_raster, int(std::min(most, (long long)RASTER_CTAS_PER_SM * num_sms)), RASTER_THREADS, 0, st,
+                 tri0, tri1, ctr0, ctr1, can, uvd, prior0, prior1, g, pshift, dcap);
         if (nlaunch) *nlaunch += 1;
         return cudaGetLastError();
     }

@@ -126,8 +126,9 @@ cudaError_t launch_prior(const int32_t* tri0, const int32_t* tri1, const int32_t
                          unsigned* err, cudaStream_t st, int* nlaunch, bool tiled, bool zeroed = false,
                          int bin_cap = PT_BIN);
 // Images from this many pixels up take the tiled prior paint, whose cost
-// grows more slowly (direct and tiled: 29 and 36 us at 1920x1080, 91 and 74
-// at 2880x1988, so they cross at some 3.5 million pixels).
+// grows more slowly with the number of triangles (prior stage, direct and
+// tiled: 33 and 39 us at 1920x1080; at 2400x1500 49 and 57 or, on a scene
+// with more support points, 84 and 60; 119 and 82 at 2880x1988).
 constexpr long long PRIOR_TILED_MIN_PIXELS = 3LL << 20;
 // Images up to this many pixels take the star construction of the
 // Delaunay triangulations, larger ones the strips and flips.  The line was

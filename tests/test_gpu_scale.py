@@ -232,6 +232,69 @@ def test_forced_prior_paint(elas, preset, seed, flag):
     assert np.array_equal(got[0], ref[0]) and np.array_equal(got[1], ref[1])
 
 
+def _sparse_pair(kind, W, H):
+    """A textureless pair, or one with a textured square in the middle."""
+    L = np.full((H, W), 90, np.uint8)
+    R = L.copy()
+    if kind == "square":
+        s, y, x = min(W, H) // 4, H // 2, W // 2
+        t = np.random.default_rng(5).integers(0, 256, (s, s), dtype=np.uint8)
+        L[y:y + s, x:x + s] = t
+        R[y:y + s, x - 6:x - 6 + s] = t
+    return L, R
+
+
+@pytest.mark.parametrize("kind", ["flat", "square"])
+@pytest.mark.parametrize("width,height,step", [(64, 48, 5), (450, 375, 5), (1920, 1080, 5), (1920, 1080, 400),
+                                               (2000, 2400, 999)])
+def test_direct_prior_paint_of_large_triangles(elas, kind, width, height, step):
+    """The corner points' triangles over (almost) textureless images, where
+    several CTAs share a triangle, and lattices of hardly any point: the
+    direct paint against the tiled one, both views."""
+    L, R = _sparse_pair(kind, width, height)
+    p = eb.params_config(63)
+    p.add_corners, p.candidate_stepsize = True, step
+    elas.set_params(p)
+    got = []
+    try:
+        for flag in (eb.Elas.TEST_PRIOR_DIRECT, eb.Elas.TEST_PRIOR_TILED):
+            elas.set_test_mode(flag)
+            elas.process(L, R)
+            got.append([elas.stage(k).view(np.int32).copy() for k in ("prior_left", "prior_right")])
+    finally:
+        elas.set_test_mode(0)
+    for a, b in zip(*got):
+        assert np.array_equal(a, b)
+
+
+def test_large_triangles_do_not_hold_the_prior_up(elas):
+    """Two triangles cover a textureless 1920x1080 view: the paint that this
+    size takes needs at most twice the time of the tiled one (fastest of 10)."""
+    import torch
+
+    W, H = 1920, 1080
+    L, R = (torch.from_numpy(x).cuda() for x in _sparse_pair("flat", W, H))
+    o1, o2 = (torch.empty((H, W), device="cuda") for _ in range(2))
+    p = eb.params_config(127)
+    p.add_corners = True
+    elas.set_params(p)
+    elas.set_timing(True)
+    best = []
+    try:
+        for flag in (0, eb.Elas.TEST_PRIOR_TILED):
+            elas.set_test_mode(flag)
+            times = []
+            for _ in range(10):
+                elas.process_device(L.data_ptr(), R.data_ptr(), o1.data_ptr(), o2.data_ptr(), W, H)
+                torch.cuda.synchronize()
+                times.append(elas.timing()["prior"])
+            best.append(min(times))
+    finally:
+        elas.set_test_mode(0)
+        elas.set_timing(False)
+    assert best[0] <= 2 * best[1], best
+
+
 def test_flip_round_limit_returns_timeout(elas):
     """A one-round cap on edge flipping: the call reports ELAS_ERR_TIMEOUT
     (the bounded device loop gave up), and the same handle then runs the
