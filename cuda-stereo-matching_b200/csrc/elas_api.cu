@@ -371,6 +371,8 @@ int check_dims(elas_handle* h, const int32_t* dims, int& W, int& H) {
     if (W > 14000 || H > 16384) return fail(h, ELAS_ERR_UNSUPPORTED, "images wider than 14000 or taller than 16384");
     if (W / h->params.candidate_stepsize > 2048)
         return fail(h, ELAS_ERR_UNSUPPORTED, "more than 2048 candidates per lattice row");
+    if (H / h->params.candidate_stepsize > LATTICE_ROWS_MAX)
+        return fail(h, ELAS_ERR_UNSUPPORTED, "more than " + std::to_string(LATTICE_ROWS_MAX) + " lattice rows");
     {
         Geom g = geom_of(W, H, h->params);
         DevParams dp = dev_params(h->params);

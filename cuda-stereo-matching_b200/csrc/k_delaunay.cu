@@ -384,6 +384,8 @@ __device__ void star_setup(const DelDev& D, const int32_t* roff, const int32_t* 
 // within Tmax); the strips and pockets are then built by k_strips, which
 // also sets the triangle count ctr[0].
 constexpr int PLAN_ARRAYS = 9;
+static_assert(size_t(PLAN_ARRAYS) * sizeof(int32_t) * (LATTICE_ROWS_MAX + 1) + 1024 <= SMEM_PER_CTA,
+              "the rows of the tallest lattice and the corners' row fit");
 __global__ void __launch_bounds__(1024) k_plan(DelDev d0, DelDev d1, const int32_t* __restrict__ row_off,
                                                int nrows, RowGeom rg, int flips, unsigned* err) {
     grid_dep_wait();
@@ -1155,6 +1157,7 @@ __device__ void pocket_points(const DelDev& D, const int32_t* __restrict__ row_o
     if (pl != 0 || it >= 2 * R) return;
     const PocketRows P(D, nrows, side);
     P.pred[j] = pred;
+    static_assert(LATTICE_ROWS_MAX + 1 <= 8192, "a row takes 13 bits");
     P.key[j] = i < R ? (i << 13 | (8191 - j)) : INT_MAX;
     if (i < R) atomicAdd(&D.ctr[2 + side], 1);
 }

@@ -711,7 +711,9 @@ __device__ void redundant_line(int* a, const uint8_t* code, int len, int lane) {
 // CTA.  (A warp per column with strided loads and an atomic per point:
 // 1242x375 5.7 us, 2880x1988 15.1; now 4.8 and 10.0.)
 constexpr int COL_LINES = 8;
-__host__ __device__ inline int col_pitch(int ch) { return (ch + 27) / 32 * 32 + 4; }    // >= ch, 4 modulo 32 banks
+__host__ __device__ inline constexpr int col_pitch(int ch) { return (ch + 27) / 32 * 32 + 4; }  // >= ch, 4 modulo 32 banks
+inline constexpr size_t redundant_smem(int ch) { return size_t(COL_LINES) * col_pitch(ch) * (sizeof(int) + 1); }
+static_assert(redundant_smem(LATTICE_ROWS_MAX) <= SMEM_PER_CTA, "the tallest lattice's columns fit");
 __global__ void __launch_bounds__(1024) k_redundant(int32_t* __restrict__ can, Geom g, int32_t* __restrict__ row_cnt) {
     grid_dep_wait();
     extern __shared__ int lines[];              // [COL_LINES][pitch], then the code bytes
@@ -1079,10 +1081,10 @@ cudaError_t launch_support(const uint4* desc0, const uint4* desc1, int32_t* can_
             else go(k_incon_rows<false, 1>, sm);
         }
         allow_smem(k_redundant);
-        const size_t smv = size_t(COL_LINES) * col_pitch(g.ch) * (sizeof(int) + 1);
         // warps in multiples of COL_LINES, up to one pass over the columns
         const int col_threads = imin(1024, (g.ch + 31) / 32 * 32 * COL_LINES);
-        launch_k(k_redundant, (g.cw + COL_LINES - 1) / COL_LINES, col_threads, smv, st, can, g, row_cnt);
+        launch_k(k_redundant, (g.cw + COL_LINES - 1) / COL_LINES, col_threads, redundant_smem(g.ch), st, can, g,
+                 row_cnt);
     }
     (void)can_tmp;
     return cudaGetLastError();

@@ -65,6 +65,12 @@ constexpr int DESCRIPTOR_ARGS = 7;     // of its kernel: the images come first
 cudaError_t launch_descriptor(const uint8_t* img0, const uint8_t* img1, uint4* desc0, uint4* desc1,
                               int W, int H, const PairZero& z, cudaStream_t st);
 
+// Rows of the candidate lattice that the column filter and the row plan of
+// the triangulations hold in one CTA's shared memory (40 and 36 bytes a
+// row); taller lattices are refused before anything is launched.
+constexpr int LATTICE_ROWS_MAX = 5796;
+constexpr size_t SMEM_PER_CTA = 227 * 1024;
+
 // bins (nullable): packed learned search sets per candidate; then stats[0]
 // counts candidates the proposal settled and stats[1] those that fell back
 // to the full sweep.

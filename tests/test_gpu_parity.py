@@ -177,6 +177,28 @@ def test_support_filters_at_window_sizes(elas, width, height, window, threshold)
     run_and_compare(elas, L, R, p, check_triangle=False)
 
 
+@pytest.mark.parametrize("height,step", [(5796, 1), (11593, 2)])
+def test_tallest_lattice(elas, height, step):
+    """The most lattice rows that are taken (5796), with and without the
+    corner points' row, triangulated either way, against the oracle; one more
+    is refused."""
+    L, R, _, _ = eb.synth_pair(3, 53, width=64, height=height, disp_max=15)
+    p = eb.params_config(15)
+    p.candidate_stepsize = step
+    for corners in (False, True):
+        p.add_corners = corners
+        try:
+            for flags in (eb.Elas.TEST_DELAUNAY_STARS, eb.Elas.TEST_DELAUNAY_FLIPS):
+                elas.set_test_mode(flags)
+                run_and_compare(elas, L, R, p, check_triangle=False)
+        finally:
+            elas.set_test_mode(0)
+    big = np.zeros((step * 5797, 64), np.uint8)
+    with pytest.raises(eb.ElasError) as refused:
+        elas.process(big, big)
+    assert refused.value.status == 2
+
+
 def test_constructor_default_parameters(elas):
     """Elas::parameters() defaults (support_threshold 0.95, gamma 5, sradius 3,
     ipol_gap_width 5000, median on)."""
