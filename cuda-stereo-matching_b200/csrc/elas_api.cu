@@ -605,10 +605,11 @@ int run_pipeline(elas_handle* h, const uint8_t* img0, const uint8_t* img1, float
     // The post-filters start from the checked maps and write the outputs in
     // their last pass; a view without post-filters gets them from the check
     // itself.  With speckle removal on both views the check is made by its
-    // first kernel (the L/R stage mark then covers nothing).
+    // first kernel, except with stage timing on, where it stays a stage of
+    // its own.
     const int nviews = p.postprocess_only_left ? 1 : 2;
     const bool post = post_any(dp, p.filter_median, p.filter_adaptive_mean);
-    const bool lr_in_post = dp.speckle_size > 0 && nviews == 2;
+    const bool lr_in_post = dp.speckle_size > 0 && nviews == 2 && !h->timing;
     float* outs[2] = {out0, out1};
     if (!lr_in_post) {
         CK(launch_lr(h->raw0, h->raw1, h->lr0, h->lr1, post ? nullptr : outs[0],
