@@ -32,6 +32,7 @@
 #include <cstring>
 #include <dlfcn.h>
 #include <string>
+#include <tuple>
 #include <vector>
 #ifdef _OPENMP
 #include <omp.h>
@@ -673,8 +674,11 @@ int orc_triangulate_ref(const float* xy, int n, int32_t* tris, int cap) {
 // ---------------------------------------------------------------------------
 // Full pipeline, host sequencing of Elas::process (src/Elas.cu:19-120).
 // tri_left/tri_right: if non-null, these triangle lists are used (e.g. the
-// CUDA library's) instead of Triangle's.  `dumps` (nullable) receives
+// CUDA library's) instead of Triangle's or, where Triangle is not loaded,
+// orc_delaunay's.  `dumps` (nullable) receives
 // intermediate stages; `post` selects whether post-filters run.
+int orc_delaunay(const int32_t* P, int n, int32_t* tris, int cap);
+
 struct orc_dumps {
     uint8_t* desc_left; uint8_t* desc_right;
     int32_t* can_lr; int32_t* can;
@@ -743,23 +747,25 @@ int orc_process(const uint8_t* L, const uint8_t* R, int W, int H, const elas_par
     const int32_t* tr = tri_right;
     int ntl = n_tri_left, ntr = n_tri_right;
     if (!tl || !tr) {
-        std::vector<float> xy0(size_t(2) * std::max(n, 1)), xy1(xy0.size());
-        for (int i = 0; i < n; ++i) {
-            xy0[2 * i] = float(uvd[3 * i]);
-            xy0[2 * i + 1] = float(uvd[3 * i + 1]);
-            xy1[2 * i] = float(uvd[3 * i] - uvd[3 * i + 2]);
-            xy1[2 * i + 1] = float(uvd[3 * i + 1]);
-        }
         int cap = 2 * n + 16;
+        auto triangulate = [&](bool right, std::vector<int32_t>& t) {
+            std::vector<int32_t> xy(size_t(2) * std::max(n, 1));
+            for (int i = 0; i < n; ++i) {
+                xy[2 * i] = uvd[3 * i] - (right ? uvd[3 * i + 2] : 0);
+                xy[2 * i + 1] = uvd[3 * i + 1];
+            }
+            t.resize(size_t(3) * cap);
+            if (!g_ref_tri) return orc_delaunay(xy.data(), n, t.data(), cap);
+            const std::vector<float> f(xy.begin(), xy.end());
+            return orc_triangulate_ref(f.data(), n, t.data(), cap);
+        };
         if (!tl) {
-            t0.resize(size_t(3) * cap);
-            ntl = orc_triangulate_ref(xy0.data(), n, t0.data(), cap);
+            ntl = triangulate(false, t0);
             if (ntl < 0) return -ntl;
             tl = t0.data();
         }
         if (!tr) {
-            t1.resize(size_t(3) * cap);
-            ntr = orc_triangulate_ref(xy1.data(), n, t1.data(), cap);
+            ntr = triangulate(true, t1);
             if (ntr < 0) return -ntr;
             tr = t1.data();
         }
@@ -846,6 +852,116 @@ static bool inside_sos(const int32_t* P, int a, int b, int c, int d) {
 
 int orc_inside_sos(const int32_t* P, int a, int b, int c, int d) { return inside_sos(P, a, b, c, d); }
 long long orc_incircle(const int32_t* P, int a, int b, int c, int d) { return incircle(P, a, b, c, d); }
+
+// The Delaunay triangulation under that perturbation, for whole pairs where
+// Triangle is not there: the points in (x, y) order (the lowest index of a
+// repeated point), each joined to the hull edges that it sees, then Lawson
+// flips of every edge that fails inside_sos.  Writes the triangles, each
+// counter-clockwise from its smallest vertex, in ascending order; returns
+// their number or -status.
+int orc_delaunay(const int32_t* P, int n, int32_t* tris, int cap) {
+    std::vector<int> order(n);
+    for (int i = 0; i < n; ++i) order[i] = i;
+    std::sort(order.begin(), order.end(), [&](int a, int b) {
+        return std::make_tuple(P[2 * a], P[2 * a + 1], a) < std::make_tuple(P[2 * b], P[2 * b + 1], b);
+    });
+    order.erase(std::unique(order.begin(), order.end(),
+                            [&](int a, int b) { return P[2 * a] == P[2 * b] && P[2 * a + 1] == P[2 * b + 1]; }),
+                order.end());
+    const int m = int(order.size());
+    int line = 2;                       // the first points on one line
+    while (line < m && orient(P, order[0], order[1], order[line]) == 0) ++line;
+    if (m < 3 || line == m) return 0;
+    // half-edge h of triangle h / 3 runs from org[h] to org of the next one; twin -1: on the hull
+    std::vector<int> org, twin, dirty;
+    auto next = [](int h) { return h % 3 == 2 ? h - 2 : h + 1; };
+    auto link = [&](int a, int b) {
+        if (a >= 0) twin[a] = b;
+        if (b >= 0) twin[b] = a;
+    };
+    auto add = [&](int a, int b, int c) {
+        const int h = int(org.size());
+        org.insert(org.end(), {a, b, c});
+        twin.insert(twin.end(), {-1, -1, -1});
+        return h;
+    };
+    // the hull, counter-clockwise: each vertex's successor, predecessor and half-edge to the successor
+    std::vector<int> hs(n, -1), hp(n, -1), he(n, -1);
+    auto join = [&](int a, int b, int h) { hs[a] = b; hp[b] = a; he[a] = h; };
+    {
+        const int p = order[line];
+        const bool left = orient(P, order[0], order[1], p) > 0;
+        int before = -1;
+        for (int i = 0; i + 1 < line; ++i) {
+            // a -> b counter-clockwise as seen from p
+            const int a = left ? order[i] : order[line - 1 - i], b = left ? order[i + 1] : order[line - 2 - i];
+            const int h = add(a, b, p);
+            join(a, b, h);
+            if (before >= 0) link(before + 1, h + 2);
+            else join(p, a, h + 2);
+            before = h;
+            dirty.push_back(h + 2);
+        }
+        join(left ? order[line - 1] : order[0], p, before + 1);
+    }
+    int last = order[line];
+    for (int i = line + 1; i < m; ++i) {
+        const int p = order[i];
+        // the last point is on the hull and is seen from p; so are its neighbours up to a tangent
+        int lo = last, hi = last;       // hull edges lo -> .. -> hi are seen
+        while (orient(P, hi, hs[hi], p) < 0) hi = hs[hi];
+        while (orient(P, hp[lo], lo, p) < 0) lo = hp[lo];
+        int before = -1, first = -1;
+        for (int a = lo; a != hi;) {
+            const int b = hs[a], h = add(b, a, p);
+            link(h, he[a]);
+            if (before >= 0) link(before + 2, h + 1);
+            else first = h + 1;
+            before = h;
+            dirty.push_back(h);
+            a = b;
+        }
+        join(lo, p, first);
+        join(p, hi, before + 2);
+        last = p;
+        // flips until every edge passes
+        while (!dirty.empty()) {
+            const int h = dirty.back();
+            dirty.pop_back();
+            const int t = twin[h];
+            if (t < 0) continue;
+            const int a = org[h], b = org[next(h)], c = org[next(next(h))], d = org[next(next(t))];
+            if (!inside_sos(P, a, b, c, d)) continue;
+            // (a, b, c) and (b, a, d) become (c, a, d) at h and (d, b, c) at t
+            const int hn = next(h), hq = next(hn), tn = next(t), tq = next(tn);
+            const int bc = twin[hn], ad = twin[tn];
+            link(h, ad);                // a -> d
+            org[h] = a;
+            org[hn] = d;
+            org[hq] = c;
+            link(t, bc);                // b -> c
+            org[t] = b;
+            org[tn] = c;
+            org[tq] = d;
+            link(hn, tn);               // d -> c and c -> d
+            if (ad < 0) he[a] = h;
+            if (bc < 0) he[b] = t;
+            if (twin[hq] < 0) he[c] = hq;
+            if (twin[tq] < 0) he[d] = tq;
+            dirty.insert(dirty.end(), {h, hq, t, tq});
+        }
+    }
+    std::vector<std::array<int, 3>> out(org.size() / 3);
+    for (size_t t = 0; t < out.size(); ++t) {
+        int* v = &org[3 * t];
+        std::rotate(v, std::min_element(v, v + 3), v + 3);
+        out[t] = {v[0], v[1], v[2]};
+    }
+    if (int(out.size()) > cap) return -ELAS_ERR_INTERNAL;
+    std::sort(out.begin(), out.end());
+    for (size_t t = 0; t < out.size(); ++t) std::copy(out[t].begin(), out[t].end(), tris + 3 * t);
+    return int(out.size());
+}
 
 // stats[0] triangles, [1] non-positive orientation, [2] edges used by more
 // than two triangles or twice in one direction, [3] interior edges failing

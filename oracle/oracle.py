@@ -204,6 +204,20 @@ def triangulate_ref(xy):
     return out[:t].copy()
 
 
+def delaunay(xy):
+    """The oracle's own exact triangulation of int32 points (n, 2) under the
+    symbolic perturbation, which whole pairs use where the reference's
+    Triangle is not built."""
+    xy = np.ascontiguousarray(xy, np.int32)
+    n = xy.shape[0]
+    cap = 2 * n + 16
+    out = np.empty((cap, 3), np.int32)
+    t = lib().orc_delaunay(P(xy), n, P(out), cap)
+    if t < 0:
+        raise RuntimeError(f"oracle triangulation failed with status {-t}")
+    return out[:t].copy()
+
+
 def prior(can, uvd, tris, right, W, H, step):
     can = np.ascontiguousarray(can, np.int32)
     uvd = np.ascontiguousarray(uvd, np.int32)
@@ -241,7 +255,9 @@ def penalty(dd, p):
 
 
 def process(left, right, p, tri_left=None, tri_right=None, dumps=False, threads=0):
-    """Full CPU pipeline.  Returns (D1, D2, stages dict or None)."""
+    """Full CPU pipeline on the given triangle lists or else on the
+    reference's Triangle's (the oracle's own where that is not built).
+    Returns (D1, D2, stages dict or None)."""
     left = np.ascontiguousarray(left, np.uint8)
     right = np.ascontiguousarray(right, np.uint8)
     H, W = left.shape

@@ -195,3 +195,40 @@ def test_add_corners_support_list():
     d = [nearest(0, 0), nearest(W - 1, 0), nearest(0, H - 1), nearest(W - 1, H - 1)]
     assert sb[:3].tolist() == [[0, 0, d[0]], [W - 1, 0, d[1]], [W - 1 + d[1], 0, d[1]]]
     assert sb[-3:].tolist() == [[0, H - 1, d[2]], [W - 1, H - 1, d[3]], [W - 1 + d[3], H - 1, d[3]]]
+
+
+def test_own_triangulation_is_the_perturbed_delaunay_one():
+    """The oracle's triangulation, which whole pairs use where Triangle is not
+    built: the exact check on lattices (co-circular everywhere), random and
+    repeated points, points on lines, and fewer than three."""
+    rng = np.random.default_rng(7)
+    cases = [np.stack(np.meshgrid(np.arange(w) * 5, np.arange(h) * 5), -1).reshape(-1, 2) for w, h in
+             [(2, 2), (9, 7), (1, 8), (8, 1)]]
+    cases += [rng.integers(0, k, (n, 2)) for k, n in [(4, 30), (60, 40), (1000, 500), (16000, 2000)]]
+    cases += [np.array([[0, 0], [5, 5], [10, 10], [15, 15], [3, 9], [9, 3], [40, 40]]), np.zeros((5, 2)),
+              np.array([[0, 0], [3, 1]]), np.zeros((0, 2))]
+    for xy in cases:
+        for points in (xy, rng.permutation(xy)):
+            points = np.ascontiguousarray(points, np.int32)
+            t = oracle.delaunay(points)
+            if len(points):
+                ok, stats = oracle.delaunay_check(points, t)
+                assert ok, (points[:10], stats)
+            if oracle.have_triangle() and len(points) >= 3:
+                ref = oracle.triangulate_ref(points.astype(np.float32))
+                assert ref.shape == t.shape and oracle.tri_compare(points, t, ref)[4] == 0
+
+
+def test_whole_pair_on_its_own_triangulation():
+    """A pair with the oracle's own triangle lists given equals one where the
+    oracle finds the triangulations itself (unless Triangle does)."""
+    L, R, _, _ = eb.synth_pair(0, 4)
+    p = eb.params_config(63)
+    D1, D2, st = oracle.process(L, R, p, dumps=True)
+    own = [oracle.delaunay(oracle.support_points(st["support"], k)) for k in (0, 1)]
+    for t, k in zip(own, ("tri_left", "tri_right")):
+        assert t.shape == st[k].shape
+        if not oracle.have_triangle():
+            assert np.array_equal(t, st[k])
+    E1, E2, _ = oracle.process(L, R, p, tri_left=st["tri_left"], tri_right=st["tri_right"])
+    assert np.array_equal(D1, E1) and np.array_equal(D2, E2)
