@@ -497,6 +497,56 @@ def test_stars_match_host_emulation(elas, emu_lib, preset):
         assert (ctr[right, 12], ctr[right, 13]) == (st[0], st[1]), (right, ctr[right], st)
 
 
+def _disc_pair(W, H, radius, d):
+    """A textured disc at disparity d on grey."""
+    y, x = np.mgrid[:H, :W]
+    t = np.random.default_rng(3).integers(0, 256, (H, W + d), dtype=np.uint8)
+    L, R = np.full((H, W), 90, np.uint8), np.full((H, W), 90, np.uint8)
+    m, ms = ((x + k - W // 2) ** 2 + (y - H // 2) ** 2 <= radius * radius for k in (0, d))
+    L[m], R[ms] = t[:, :W][m], t[:, d:][ms]
+    return L, R
+
+
+@pytest.mark.parametrize("kind,step", [("disc", 5), ("dense", 1), ("dense", 2), ("sparse", 40)])
+def test_stars_of_many_and_few_neighbours(elas, emu_lib, kind, step):
+    """The star kernels' own paths, list order included, against the host
+    emulation, with corner points: a disc that the corners see from afar
+    (stars that are handed on, more owned triangles than a point's slot
+    holds, more neighbours than the record takes), lattices whose windows hold
+    more points than a warp's registers, and a handful of points (windows
+    that grow to the whole box)."""
+    from test_delaunay_cpu import emu_star
+
+    if kind == "disc":
+        W, H = 1200, 900
+        L, R = _disc_pair(W, H, 400, 6)
+    else:
+        W, H = 320, 240
+        L, R, _, _ = eb.synth_pair(3, 31, width=W, height=H, disp_max=31)
+    p = eb.params_config(31)
+    p.add_corners, p.candidate_stepsize = True, step
+    elas.set_params(p)
+    elas.process(L, R)
+    uvd = elas.stage("support").view(np.int32).reshape(-1, 3)
+    ctr = elas.stage("del_counters").view(np.int32).reshape(2, 16)
+    row_of = np.where(uvd[:, 1] == H - 1, H // step, uvd[:, 1] // step)
+    for right, key in ((0, "tri_left"), (1, "tri_right")):
+        xy = oracle.support_points(uvd, right)
+        tris, st = emu_star(emu_lib, xy, row_of)
+        assert np.array_equal(elas.stage(key).view(np.int32).reshape(-1, 3), tris), key
+        assert ctr[right, 13] == st[1]
+        if kind == "disc":
+            owned, degree = np.bincount(tris[:, 0]), np.bincount(tris.reshape(-1))
+            assert ctr[right, 10] > 0 and owned.max() > 12 and degree.max() >= 32
+        elif kind == "dense":
+            # the window's half-size: the largest r in [16, 128] with 4 r^2 n <= 49 box areas
+            area = int(np.prod(xy.max(0) - xy.min(0) + 1))
+            r = max(q for q in range(16, 129) if q == 16 or 4 * q * q * len(xy) <= 49 * area)
+            assert max((np.abs(xy - c).max(1) <= r).sum() for c in xy) > 64
+        else:
+            assert len(uvd) < 40
+
+
 @pytest.mark.parametrize("preset", [1, 2])
 def test_flip_rounds_match_host_emulation(elas, emu_lib, preset):
     """The flip construction (forced): the flip kernels (one SM at 1242x375,
