@@ -3,7 +3,8 @@
 // Replaces the reference's CPU round trip through Shewchuk's Triangle
 // (Elas::computeDelaunyTrianguation, src/Elas.cu:282-328).
 //
-// Algorithm (all steps data-parallel except two short serial chains):
+// Two constructions of the same triangulation: stars (below, PXY_NONE on),
+// and strips with edge flips, all steps data-parallel:
 //  1. Per candidate row, sort the row's points by x and drop duplicated
 //     coordinates (the lowest support index of a group is kept; Triangle
 //     keeps the first of its randomised sort, src/triangle.cpp divconqdelaunay).
@@ -12,7 +13,8 @@
 //     point finds its own triangle by a binary search in the other row
 //     (merge path), so the strips are built fully in parallel.
 //  3. Fill the pockets between the rows' first (last) points and the convex
-//     hull with the monotone-chain stack walk.
+//     hull with the triangles of the monotone-chain stack walk, each point
+//     finding its own.
 //  4. Build edge adjacency with an open-addressing hash of undirected edges.
 //  5. Lawson edge flipping in rounds driven by a worklist: round 0 tests
 //     every interior edge; later rounds test only the four outer edges of
@@ -32,7 +34,8 @@
 // wherever no four points are co-circular.
 //
 // Everything here is __host__ __device__ so the same code runs in a
-// sequential host emulation used by the CPU tests.
+// sequential host emulation used by the CPU tests, which adds sequential
+// forms of its own of the parallel steps.
 #pragma once
 
 #include <cmath>
@@ -41,92 +44,6 @@
 
 namespace elas {
 namespace del {
-
-struct Pts {
-    const int32_t* x;
-    const int32_t* y;
-};
-
-// Strip between an upper row A[0..m) and a lower row B[0..n), both sorted
-// by strictly increasing x: walking the merge of A[1..m) and B[1..n) by x
-// (A first on equal x), each element advances its row by one point and
-// creates one counter-clockwise triangle.  These two functions give the
-// triangle of one element and its position in the strip, so every point
-// can emit its triangles independently.
-//
-// Number of elements of the sorted X[0..n) with x < v (strict) or x <= v.
-HD int count_below(Pts P, const int32_t* X, int n, int32_t v, bool inclusive) {
-    int lo = 0, hi = n;
-    while (lo < hi) {
-        int mid = (lo + hi) >> 1;
-        int32_t x = P.x[X[mid]];
-        if (inclusive ? (x <= v) : (x < v)) lo = mid + 1;
-        else hi = mid;
-    }
-    return lo;
-}
-
-// Element A[k], 1 <= k < m: triangle (A[k-1], A[k], B[j]); returns its position.
-HD int strip_tri_upper(Pts P, const int32_t* A, const int32_t* B, int n, int k, int32_t* tri) {
-    int cl = count_below(P, B, n, P.x[A[k]], false);
-    int j = cl > 0 ? cl - 1 : 0;
-    tri[0] = A[k - 1]; tri[1] = A[k]; tri[2] = B[j];
-    return (k - 1) + j;
-}
-
-// Element B[k], 1 <= k < n: triangle (A[i], B[k], B[k-1]); returns its position.
-HD int strip_tri_lower(Pts P, const int32_t* A, int m, const int32_t* B, int k, int32_t* tri) {
-    int cl = count_below(P, A, m, P.x[B[k]], true);
-    int i = cl > 0 ? cl - 1 : 0;
-    tri[0] = A[i]; tri[1] = B[k]; tri[2] = B[k - 1];
-    return i + (k - 1);
-}
-
-// Fill the pocket between a boundary chain (one point per non-empty row,
-// top to bottom: point index ci[k] at (cx[k], cy[k])) and its convex hull.
-// side = +1 for the left chain (first points), -1 for the right chain
-// (last points).  `stack` has room for 4 * len ints: an entry is the
-// record (point index, x, y, -) of a chain point, so a pop reads one
-// 16-byte record.  The next chain point is loaded one step ahead.  Returns
-// the number of counter-clockwise triangles written.
-HD int fill_pockets(const int32_t* ci, const int32_t* cx, const int32_t* cy, int len, int side, int32_t* stack,
-                    int32_t* tri) {
-    // the two top stack entries are kept in registers: (a, b) = stack[sp-2], stack[sp-1]
-    int sp = 0, k = 0;
-    // orientations are exact in int32 within the library's coordinate range
-    // (|dx| <= 18094, |dy| <= 16383, see orient_p)
-    int32_t ia = 0, ib = 0;
-    int32_t ax = 0, ay = 0, bx = 0, by = 0;
-    int32_t nx = len > 0 ? cx[0] : 0, ny = len > 0 ? cy[0] : 0, ni = len > 0 ? ci[0] : 0;
-    for (int i = 0; i < len; ++i) {
-        const int32_t x = nx, y = ny;
-        const int32_t ii = ni;
-        if (i + 1 < len) { nx = cx[i + 1]; ny = cy[i + 1]; ni = ci[i + 1]; }
-        while (sp >= 2) {
-            const int32_t o = (bx - ax) * (y - ay) - (by - ay) * (x - ax);
-            if (side > 0 ? (o > 0) : (o < 0)) {
-                tri[3 * k] = ia;
-                tri[3 * k + 1] = side > 0 ? ib : ii;
-                tri[3 * k + 2] = side > 0 ? ii : ib;
-                ++k;
-                --sp;
-                ib = ia; bx = ax; by = ay;
-                if (sp >= 2) {
-                    const int32_t* q = stack + 4 * (sp - 2);
-                    ia = q[0]; ax = q[1]; ay = q[2];
-                }
-            } else {
-                break;
-            }
-        }
-        int32_t* e = stack + 4 * sp;
-        e[0] = ii; e[1] = x; e[2] = y; e[3] = 0;
-        ++sp;
-        ia = ib; ax = bx; ay = by;
-        ib = ii; bx = x; by = y;
-    }
-    return k;
-}
 
 HD uint32_t hash64(uint64_t k) {
     k ^= k >> 33;
@@ -377,21 +294,14 @@ struct FlatTri {
 // strict total order on the points of one side (the perturbed incircle
 // determinant is antisymmetric in a and b).  The minimum of that order is the
 // next neighbour; a side with no point marks a hull edge.  The walk goes
-// counter-clockwise until it returns to q0 (an interior point) or meets the
-// hull, and then clockwise from q0 to the hull on the other side.
+// counter-clockwise until it returns to q0.  A point of the hull boundary
+// starts at its successor on the boundary (counter-clockwise, the interior
+// on the left) instead and walks until it reaches its predecessor.
 
 constexpr uint32_t PXY_NONE = 0xFFFFFFFFu;   // a dropped duplicate point
 
-// For the edge p->q and two points a, b on the walk's side, is b the better
-// next neighbour (inside the circle through p, q and a)?  side > 0: left of
-// p->q, triangle (p, q, a) counter-clockwise; side < 0: right, triangle
-// (p, a, q).
-HD bool star_better(int ip, uint32_t pp, int iq, uint32_t pq, int ia, uint32_t pa, int ib, uint32_t pb, int side) {
-    return side > 0 ? inside_sos_p(ip, pp, iq, pq, ia, pa, ib, pb) : inside_sos_p(ip, pp, ia, pa, iq, pq, ib, pb);
-}
-
-// star_better for side > 0 with a and b known to lie strictly left of p->q,
-// by the centres of their circles on the bisector of p and q: with u = q - p
+// That order for a and b known to lie strictly left of p->q: is b the better
+// next neighbour (inside_sos_p(p, q, a, b))?  By the centres of their circles on the bisector of p and q: with u = q - p
 // a point s (relative to p) has its centre at t = (|s|^2 - u.s) / cross(u, s)
 // (up to a common scale), and b is inside a's circle when its t is smaller.
 // Numerators stay below 2^31 and denominators below 2^30 at the coordinate
@@ -412,47 +322,16 @@ HD bool star_better_left(int ip, uint32_t pp, int iq, uint32_t pq, int ia, uint3
     return (m == ip ? orient_p(pb, pq, pa) : orient_p(pp, pb, pa)) < 0;
 }
 
-// Is b strictly on the walk's side of p->q?
-HD bool star_side(uint32_t pp, uint32_t pq, uint32_t pb, int side) {
-    const int64_t o = orient_p(pp, pq, pb);
-    return side > 0 ? o > 0 : o < 0;
-}
-
 // Does every point inside the circle through p, q and r lie in the square
 // |x - px|, |y - py| <= R?  Points exist only in the box [bx0, bx1] x
 // [by0, by1] (all points of the problem), so only the part of the circle
 // inside the box counts: its extent is bounded through the circle's chords
-// at the box edges nearest the centre.  Every point outside the square is
-// at least R + 1 away from p in x or in y, which leaves a pixel of margin
-// for the rounding of the centre and the chords (the centre's numerators
-// and denominator are exact integers in double).  *need: the square that
-// would pass.
-HD bool circle_within(uint32_t pp, uint32_t pq, uint32_t pr, int R, const int32_t* box, int* need) {
-    const double qx = dx_p(pq, pp), qy = dy_p(pq, pp), rx = dx_p(pr, pp), ry = dy_p(pr, pp);
-    const double d = 2.0 * (qx * ry - qy * rx);
-    const double q2 = qx * qx + qy * qy, r2 = rx * rx + ry * ry;
-    const double cx = (ry * q2 - qy * r2) / d, cy = (qx * r2 - rx * q2) / d;
-    const double rho2 = cx * cx + cy * cy;
-    // the box relative to p
-    const double bx0 = box[0] - px_of(pp), by0 = box[1] - py_of(pp), bx1 = box[2] - px_of(pp), by1 = box[3] - py_of(pp);
-    const double ey = fmin(fmax(cy, by0), by1) - cy, ex = fmin(fmax(cx, bx0), bx1) - cx;
-    double ext = 0.0;
-    if (ey * ey < rho2 && ex * ex < rho2) {
-        const double h = sqrt(rho2 - ey * ey), v = sqrt(rho2 - ex * ex);
-        const double x0 = fmax(cx - h, bx0), x1 = fmin(cx + h, bx1);
-        const double y0 = fmax(cy - v, by0), y1 = fmin(cy + v, by1);
-        ext = fmax(fmax(-x0, x1), fmax(-y0, y1));
-    }
-    if (need) *need = ext < 1e9 ? int(ext) + 2 : (1 << 30);
-    return ext <= double(R);
-}
-
-// circle_within's answer without its extent, by comparisons only: every
-// quantity scaled by D = |2 cross(q - p, r - p)| (the centre's numerators,
-// the box, R), so no division and no square root.  The centre numerators
-// and the scaled box are exact integers in double; the squared terms
-// (below 2^93) carry a relative rounding of 2^-53, which moves a decision
-// by far less than the pixel of margin circle_within relies on.
+// at the box edges nearest the centre.  By comparisons only: every quantity
+// is scaled by D = |2 cross(q - p, r - p)| (the centre's numerators, the box,
+// R), so no division and no square root.  The centre numerators and the
+// scaled box are exact integers in double; the squared terms (below 2^93)
+// carry a relative rounding of 2^-53, and every point outside the square is
+// at least R + 1 away from p in x or in y, a pixel of margin.
 HD bool circle_inside(uint32_t pp, uint32_t pq, uint32_t pr, int R, const int32_t* box) {
     const double qx = dx_p(pq, pp), qy = dy_p(pq, pp), rx = dx_p(pr, pp), ry = dy_p(pr, pp);
     const double d2x = 2.0 * (qx * ry - qy * rx);
@@ -481,10 +360,9 @@ HD bool circle_inside(uint32_t pp, uint32_t pq, uint32_t pr, int R, const int32_
 // box of all points (which also proves a hull edge).  A search over growing
 // squares starts at half-size R0 and doubles it until its answer is
 // certain; the number of doublings a star needs is therefore a property of
-// the star, whatever points were looked at to find it.  The sequential
-// emulation searches that way (its window keeps every point, STAR_CAP); the
-// device finds the star from fewer points and counts the same doublings.
-constexpr int STAR_CAP = 1 << 30;
+// the star, whatever points were looked at to find it.  The tests' sequential
+// emulation searches that way; the device finds the star from fewer points
+// and counts the same doublings.
 
 // The window's half-size R0 of a problem: 3.5 mean point spacings (the
 // square root of the box area per point), within [16, 128] pixels: the
@@ -498,249 +376,14 @@ HD int star_r0(const int32_t* box, int n) {
         if (r + st <= 128 && 4LL * (r + st) * (r + st) * (n > 0 ? n : 1) <= 49 * area) r += st;
     return r;
 }
-constexpr int STAR_NB = 256;      // neighbours of one point on each side of its start
-
-// Half-size of the next square after one of half-size R held no candidate.
-HD int star_square(int R) { return R < (1 << 20) ? 2 * R : R; }
-
-// The rows [y0, y1] and, per row y, the columns [x0, x1] of a region:
-// a square of half-size R around (px, py), or the circle (centre (cx, cy),
-// squared radius rho2, absolute coordinates) with a pixel of margin; both
-// clipped to the box.  An empty range has y0 > y1 or x0 > x1.
-struct StarRegion {
-    bool circle;
-    double cx, cy, rho2;
-    int32_t sx0, sx1;     // square columns
-    int32_t y0, y1;
-    // optional half-plane (a square searched for a next neighbour): only
-    // the points strictly on side `side` of the line through (hx, hy) with
-    // direction (ux, uy) count, kept with a pixel of margin
-    int32_t hx, hy, ux, uy, side;
-    // optional hole (a ring, the square minus a smaller one): rows
-    // [ky0, ky1] lose the columns [kx0, kx1]
-    int32_t kx0, kx1, ky0, ky1;
-    bool hole;
-    // The columns of row y as up to two ranges [x0, x1], [x2, x3] (empty
-    // when the first bound exceeds the second).
-    HD void cols2(int32_t y, const int32_t* box, int32_t* x0, int32_t* x1, int32_t* x2, int32_t* x3) const {
-        cols(y, box, x0, x1);
-        *x2 = 1;
-        *x3 = 0;
-        if (hole && y >= ky0 && y <= ky1) {
-            *x2 = imax(*x0, kx1 + 1);
-            *x3 = *x1;
-            *x1 = imin(*x1, kx0 - 1);
-        }
-    }
-    HD void cols(int32_t y, const int32_t* box, int32_t* x0, int32_t* x1) const {
-        if (!circle) {
-            *x0 = sx0;
-            *x1 = sx1;
-            if (side != 0) {
-                if (uy == 0) {
-                    if (int64_t(ux) * (y - hy) * side <= 0) *x0 = *x1 + 1;
-                } else {
-                    const double xl = double(hx) + double(ux) * double(y - hy) / double(uy);
-                    if ((uy > 0) == (side > 0))
-                        *x1 = int32_t(fmax(fmin(double(*x1), ceil(xl) + 1.0), double(*x0) - 1.0));
-                    else
-                        *x0 = int32_t(fmin(fmax(double(*x0), floor(xl) - 1.0), double(*x1) + 1.0));
-                }
-            }
-            return;
-        }
-        // half-chord at row y, plus a pixel for the rounding of the centre
-        // and radius (both far below a pixel at these coordinates)
-        const double dy = double(y) - cy;
-        const double h = sqrt(fmax(rho2 - dy * dy, 0.0)) + 1.0;
-        // clamped into the box (an empty range stays empty) before the
-        // conversion: a near-degenerate circle's centre can lie far outside
-        *x0 = int32_t(fmin(fmax(floor(cx - h) - 1.0, double(box[0])), double(box[2]) + 1.0));
-        *x1 = int32_t(fmax(fmin(ceil(cx + h) + 1.0, double(box[2])), double(box[0]) - 1.0));
-    }
-};
-
-HD StarRegion star_square_region(uint32_t pp, int R, const int32_t* box) {
-    StarRegion g;
-    g.circle = false;
-    g.cx = g.cy = g.rho2 = 0.0;
-    g.hx = g.hy = g.ux = g.uy = g.side = 0;
-    g.kx0 = g.kx1 = g.ky0 = g.ky1 = 0;
-    g.hole = false;
-    const int32_t px = px_of(pp), py = py_of(pp);
-    g.sx0 = imax(px - R, box[0]);
-    g.sx1 = imin(px + R, box[2]);
-    g.y0 = imax(py - R, box[1]);
-    g.y1 = imin(py + R, box[3]);
-    return g;
-}
-
-// The ring between the squares of half-sizes R and 2R around p.
-HD StarRegion star_ring_region(uint32_t pp, int R, const int32_t* box) {
-    StarRegion g = star_square_region(pp, 2 * R, box);
-    const int32_t px = px_of(pp), py = py_of(pp);
-    g.hole = true;
-    g.kx0 = px - R;
-    g.kx1 = px + R;
-    g.ky0 = py - R;
-    g.ky1 = py + R;
-    return g;
-}
-
-// The square of half-size R around p restricted to side `side` of p->q.
-HD StarRegion star_half_region(uint32_t pp, uint32_t pq, int side, int R, const int32_t* box) {
-    StarRegion g = star_square_region(pp, R, box);
-    g.hx = px_of(pp);
-    g.hy = py_of(pp);
-    g.ux = dx_p(pq, pp);
-    g.uy = dy_p(pq, pp);
-    g.side = side;
-    return g;
-}
-
-// The circle through p, q and r (any order), clipped to the box.
-HD StarRegion star_circle_region(uint32_t pp, uint32_t pq, uint32_t pr, const int32_t* box) {
-    const double qx = dx_p(pq, pp), qy = dy_p(pq, pp), rx = dx_p(pr, pp), ry = dy_p(pr, pp);
-    const double d = 2.0 * (qx * ry - qy * rx);
-    const double q2 = qx * qx + qy * qy, r2 = rx * rx + ry * ry;
-    const double cx = (ry * q2 - qy * r2) / d, cy = (qx * r2 - rx * q2) / d;
-    StarRegion g;
-    g.circle = true;
-    g.hx = g.hy = g.ux = g.uy = g.side = 0;
-    g.kx0 = g.kx1 = g.ky0 = g.ky1 = 0;
-    g.hole = false;
-    g.cx = cx + px_of(pp);
-    g.cy = cy + py_of(pp);
-    g.rho2 = cx * cx + cy * cy;
-    g.sx0 = g.sx1 = 0;
-    const double rho = sqrt(g.rho2);
-    g.y0 = int32_t(fmax(floor(g.cy - rho) - 1.0, double(box[1])));
-    g.y1 = int32_t(fmin(ceil(g.cy + rho) + 1.0, double(box[3])));
-    return g;
-}
-
-// Walk the star.  An interior point (hn < 0) starts at nearest(), p's
-// nearest neighbour, and walks counter-clockwise until it is back there.  A
-// point of the hull boundary starts at hn, its successor on the boundary
-// (counter-clockwise, the interior on the left), and walks until it reaches
-// hp, its predecessor.  next(q, side) returns the next neighbour after q on
-// that side (-1: none, so p->q is a hull edge; -2: the search failed).
-// The neighbours are appended to ccw (counter-clockwise) and, should an
-// interior point meet the hull (all points collinear), to cw (clockwise from
-// the start); star_at gives them in counter-clockwise order.  Returns false
-// if a search failed or a list would pass cap.
-template <class Nearest, class Next>
-HD bool star_walk(int hn, int hp, Nearest nearest, Next next, int32_t* ccw, int32_t* cw, int cap, int* m, int* k,
-                  bool* closed) {
-    *m = 0;
-    *k = 0;
-    *closed = false;
-    const int q0 = hn >= 0 ? hn : nearest();
-    if (q0 < 0) return q0 == -1;
-    ccw[(*m)++] = q0;
-    int q = q0;
-    for (;;) {
-        const int r = next(q, +1);
-        if (r == -2) return false;
-        if (r < 0) break;
-        if (r == q0) {
-            *closed = hn < 0;
-            return hn < 0;
-        }
-        if (*m >= cap) return false;
-        ccw[(*m)++] = r;
-        if (r == hp) return true;
-        q = r;
-    }
-    if (hn >= 0) return true;
-    q = q0;
-    for (;;) {
-        const int r = next(q, -1);
-        if (r == -2) return false;
-        if (r < 0) break;
-        if (*k >= cap) return false;
-        cw[(*k)++] = r;
-        q = r;
-    }
-    return true;
-}
+constexpr int STAR_NB = 256;      // neighbours of one point
 
 // The hull boundary, counter-clockwise (the interior on the left of each
 // step), from the rows' extreme points: the top row left to right, the
 // right chain down, the bottom row right to left, the left chain up.  The
-// chains are the rows' last (first) points with the concave ones removed by
-// the monotone stack walk; collinear points stay, as every point on the
-// boundary is a vertex of the triangulation.  xy[s] holds the packed
-// coordinates of the leftmost (side 0) or rightmost (side 1) point of
-// non-empty row s (of R, top to bottom).  Writes the chain as row positions
-// (top to bottom; room for R) and its length.
-HD void hull_chain(int side, int R, const uint32_t* xy, int32_t* st, int* len) {
-    int sp = 0;
-    uint32_t a = 0, b = 0;     // the stack's top two points
-    for (int s = 0; s < R; ++s) {
-        const uint32_t x = xy[s];
-        while (sp >= 2) {
-            const int64_t o = orient_p(a, b, x);
-            if (side ? o < 0 : o > 0) {
-                --sp;
-                b = a;
-                if (sp >= 2) a = xy[st[sp - 2]];
-            } else {
-                break;
-            }
-        }
-        st[sp++] = s;
-        a = b;
-        b = x;
-    }
-    *len = sp;
-}
-
-// The same chain, decided point by point (for a parallel build): row i's
-// point is dropped by the stack walk exactly when it lies strictly inside
-// the segment of two other chain points j < i < k (strictly right of L_j ->
-// L_k for the left chain, left of it for the right chain).  With
-// coordinates relative to point i and x mirrored for the right chain, that
-// holds iff min_{j<i} x_j / -y_j + min_{k>i} x_k / y_k < 0 (the rows above
-// have y < 0, those below y > 0); both minima and their sum are compared
-// as exact fractions.  |x| <= 18094 and 0 < y <= 16383 (the coordinate
-// limits of orient_p), so every cross product is below 2^29 and the final
-// sum below 2^30: exact in int32.
-HD bool hull_on_chain(int side, int R, const uint32_t* xy, int i) {
-    if (i == 0 || i == R - 1) return true;
-    const uint32_t c = xy[i];
-    const int sg = side ? -1 : 1;
-    // each minimum over four interleaved partial minima (independent chains)
-    int32_t n[2][4], d[2][4];
-    for (int h = 0; h < 2; ++h)
-        for (int u = 0; u < 4; ++u) {
-            n[h][u] = 1;
-            d[h][u] = 0;     // +infinity: 1/0 compares above every fraction below
-        }
-    auto fold = [&](int h, int u, uint32_t v, int dsign) {
-        const int32_t x = sg * dx_p(v, c), dd = dsign * dy_p(v, c);
-        if (d[h][u] == 0 || x * d[h][u] < n[h][u] * dd) {
-            n[h][u] = x;
-            d[h][u] = dd;
-        }
-    };
-    int j = 0;
-    for (; j + 4 <= i; j += 4)
-        for (int u = 0; u < 4; ++u) fold(0, u, xy[j + u], -1);
-    for (; j < i; ++j) fold(0, 0, xy[j], -1);
-    int k = i + 1;
-    for (; k + 4 <= R; k += 4)
-        for (int u = 0; u < 4; ++u) fold(1, u, xy[k + u], 1);
-    for (; k < R; ++k) fold(1, 0, xy[k], 1);
-    int32_t sn = n[0][0], sd = d[0][0], tn = n[1][0], td = d[1][0];
-    for (int u = 1; u < 4; ++u) {
-        if (d[0][u] != 0 && n[0][u] * sd < sn * d[0][u]) { sn = n[0][u]; sd = d[0][u]; }
-        if (d[1][u] != 0 && n[1][u] * td < tn * d[1][u]) { tn = n[1][u]; td = d[1][u]; }
-    }
-    return sn * td + tn * sd >= 0;
-}
-
-// Position j of the boundary cycle (hull_chain's layout): top row (tl
+// chains are the rows' last (first) points, top to bottom, without the
+// concave ones; collinear points stay, as every point on the boundary is a
+// vertex of the triangulation.  Position j of that cycle: top row (tl
 // points) left to right, right chain rows 1..nr-1, bottom row (bl points)
 // right to left from its second last, left chain rows nl-2..1.  Returns
 // (row position, index within that row); the cycle has
@@ -758,13 +401,6 @@ HD void hull_cycle_at(int j, int R, int tl, int bl, const int32_t* lstk, int nl,
     j -= bl - 1;
     *row = lstk[nl - 2 - j];
     *pos = 0;
-}
-
-// Neighbour i in counter-clockwise order: the clockwise part reversed, then
-// the counter-clockwise part.
-HD int32_t star_at(const int32_t* ccw, int m, const int32_t* cw, int k, int i) {
-    (void)m;
-    return i < k ? cw[k - 1 - i] : ccw[i - k];
 }
 
 // Triangles of a star of deg neighbours: (p, nb(i), nb(i+1)), wrapping when

@@ -265,9 +265,15 @@ struct RowGeom {
 // of all points (box[0..3]) and the window half-size (box[4], star_r0), and
 // the hull boundary (hnext / hprev of every boundary point).  roff and cnt:
 // the rows' offsets and unique counts, also in shared memory.  The rows'
-// extreme points are staged in shared memory; HULL_LANES lanes decide one of
-// them together (hull_on_chain's two minima over the other rows, each lane
-// a share of the rows, then merged), both chains at once: first against the
+// extreme points are staged in shared memory.  Point i leaves its chain
+// exactly when it lies strictly inside the segment of two other chain points
+// above and below it (strictly right of it on the left chain, left on the
+// right one).  With coordinates relative to i, x mirrored for the right
+// chain, that holds iff min_{above} x / -y + min_{below} x / y < 0.  |x| <=
+// 18094 and |y| <= 16383 (the limits of orient_p), so every cross product
+// is below 2^29 and the final sum below 2^30: exact in int32.  HULL_LANES
+// lanes decide one point together (the two minima over the other rows, each
+// lane a share of them, then merged), both chains at once: first against the
 // HULL_GROUP rows around it, then what is left (a third) against what is
 // left, as a point inside the hull is inside the hull of the points that
 // their own groups keep.  One SM does this, bound by instruction issue:
@@ -313,7 +319,7 @@ __device__ void star_setup(const DelDev& D, const int32_t* roff, const int32_t* 
     if (R < 2) return;
     // flag[i]: bit 0 on the left chain, bit 16 on the right one
     const int hl = tid % HULL_LANES;
-    // hull_on_chain for row i of a side against n rows, row(k) the k-th
+    // whether row i stays on a side's chain against n rows, row(k) the k-th
     auto on_chain = [&](int side, int i, int n, auto row) {
         const uint32_t* xy = side ? xyl : xyf;
         const uint32_t c = xy[i];
@@ -454,7 +460,7 @@ __global__ void __launch_bounds__(1024) k_plan(DelDev d0, DelDev d1, const int32
 }
 
 // ---------------------------------------------------------------------------
-// Star construction (delaunay_core.h, star_walk): every point's Delaunay
+// Star construction (delaunay_core.h, "Stars"): every point's Delaunay
 // neighbours are found directly, with no initial triangulation and no
 // flips.  Every search is a minimum under a strict total order, so its
 // answer does not depend on how threads split the candidates, nor on which
@@ -1091,8 +1097,9 @@ __global__ void __launch_bounds__(EMIT_THREADS) k_star_emit(DelDev d0, DelDev d1
     }
 }
 
-// The two hull pockets of one problem (the triangles of fill_pockets, in its
-// order), every point on its own.  In the stack walk a point j is pushed onto
+// The two hull pockets of one problem: the triangles, in its order, of the
+// monotone-chain stack walk over the rows' first (last) points, every point
+// on its own.  In the walk a point j is pushed onto
 // pred(j), the point above it whose direction from j is outermost (the
 // nearest of collinear ones), and pred(j) stays beneath it; j is popped by
 // the first later point i that lies strictly outside the line pred(j) -> j
@@ -1185,8 +1192,11 @@ __device__ void pocket_triangles(const DelDev& D, int nrows, int part, int32_t* 
 }
 
 // Block s < R: the points of non-empty row s, each placing its triangle in
-// the strip below the row (as the upper row) and in the strip above (as the
-// lower row) by merge path (strip_tri_upper, strip_tri_lower).  The x of the
+// the strip below the row (as the upper row A) and in the strip above (as
+// the lower row B).  Walking the merge of A[1..m) and B[1..n) by x (A first
+// on equal x), each element advances its row by one point and creates one
+// counter-clockwise triangle, whose other row's point and place in the strip
+// a search finds for each element on its own (merge path).  The x of the
 // two neighbouring rows are staged in shared memory, so the binary searches
 // do not chase loads (a thread finding its row and both places through
 // global memory: some fifty dependent loads).  The blocks from nrows on

@@ -12,6 +12,241 @@
 
 #include "../../cuda-stereo-matching_b200/csrc/delaunay_core.h"
 
+// Sequential forms of steps that the device's kernels make in parallel.
+namespace elas {
+namespace del {
+
+struct Pts {
+    const int32_t* x;
+    const int32_t* y;
+};
+
+// Strip between an upper row A[0..m) and a lower row B[0..n), both sorted
+// by strictly increasing x: walking the merge of A[1..m) and B[1..n) by x
+// (A first on equal x), each element advances its row by one point and
+// creates one counter-clockwise triangle.  These two functions give the
+// triangle of one element and its position in the strip, so every point
+// can emit its triangles independently.
+//
+// Number of elements of the sorted X[0..n) with x < v (strict) or x <= v.
+HD int count_below(Pts P, const int32_t* X, int n, int32_t v, bool inclusive) {
+    int lo = 0, hi = n;
+    while (lo < hi) {
+        int mid = (lo + hi) >> 1;
+        int32_t x = P.x[X[mid]];
+        if (inclusive ? (x <= v) : (x < v)) lo = mid + 1;
+        else hi = mid;
+    }
+    return lo;
+}
+
+// Element A[k], 1 <= k < m: triangle (A[k-1], A[k], B[j]); returns its position.
+HD int strip_tri_upper(Pts P, const int32_t* A, const int32_t* B, int n, int k, int32_t* tri) {
+    int cl = count_below(P, B, n, P.x[A[k]], false);
+    int j = cl > 0 ? cl - 1 : 0;
+    tri[0] = A[k - 1]; tri[1] = A[k]; tri[2] = B[j];
+    return (k - 1) + j;
+}
+
+// Element B[k], 1 <= k < n: triangle (A[i], B[k], B[k-1]); returns its position.
+HD int strip_tri_lower(Pts P, const int32_t* A, int m, const int32_t* B, int k, int32_t* tri) {
+    int cl = count_below(P, A, m, P.x[B[k]], true);
+    int i = cl > 0 ? cl - 1 : 0;
+    tri[0] = A[i]; tri[1] = B[k]; tri[2] = B[k - 1];
+    return i + (k - 1);
+}
+
+// Fill the pocket between a boundary chain (one point per non-empty row,
+// top to bottom: point index ci[k] at (cx[k], cy[k])) and its convex hull.
+// side = +1 for the left chain (first points), -1 for the right chain
+// (last points).  `stack` has room for 4 * len ints: an entry is the
+// record (point index, x, y, -) of a chain point, so a pop reads one
+// 16-byte record.  The next chain point is loaded one step ahead.  Returns
+// the number of counter-clockwise triangles written.
+HD int fill_pockets(const int32_t* ci, const int32_t* cx, const int32_t* cy, int len, int side, int32_t* stack,
+                    int32_t* tri) {
+    // the two top stack entries are kept in registers: (a, b) = stack[sp-2], stack[sp-1]
+    int sp = 0, k = 0;
+    // orientations are exact in int32 within the library's coordinate range
+    // (|dx| <= 18094, |dy| <= 16383, see orient_p)
+    int32_t ia = 0, ib = 0;
+    int32_t ax = 0, ay = 0, bx = 0, by = 0;
+    int32_t nx = len > 0 ? cx[0] : 0, ny = len > 0 ? cy[0] : 0, ni = len > 0 ? ci[0] : 0;
+    for (int i = 0; i < len; ++i) {
+        const int32_t x = nx, y = ny;
+        const int32_t ii = ni;
+        if (i + 1 < len) { nx = cx[i + 1]; ny = cy[i + 1]; ni = ci[i + 1]; }
+        while (sp >= 2) {
+            const int32_t o = (bx - ax) * (y - ay) - (by - ay) * (x - ax);
+            if (side > 0 ? (o > 0) : (o < 0)) {
+                tri[3 * k] = ia;
+                tri[3 * k + 1] = side > 0 ? ib : ii;
+                tri[3 * k + 2] = side > 0 ? ii : ib;
+                ++k;
+                --sp;
+                ib = ia; bx = ax; by = ay;
+                if (sp >= 2) {
+                    const int32_t* q = stack + 4 * (sp - 2);
+                    ia = q[0]; ax = q[1]; ay = q[2];
+                }
+            } else {
+                break;
+            }
+        }
+        int32_t* e = stack + 4 * sp;
+        e[0] = ii; e[1] = x; e[2] = y; e[3] = 0;
+        ++sp;
+        ia = ib; ax = bx; ay = by;
+        ib = ii; bx = x; by = y;
+    }
+    return k;
+}
+
+// For the edge p->q and two points a, b on the walk's side, is b the better
+// next neighbour (inside the circle through p, q and a)?  side > 0: left of
+// p->q, triangle (p, q, a) counter-clockwise; side < 0: right, triangle
+// (p, a, q).
+HD bool star_better(int ip, uint32_t pp, int iq, uint32_t pq, int ia, uint32_t pa, int ib, uint32_t pb, int side) {
+    return side > 0 ? inside_sos_p(ip, pp, iq, pq, ia, pa, ib, pb) : inside_sos_p(ip, pp, ia, pa, iq, pq, ib, pb);
+}
+
+// Is b strictly on the walk's side of p->q?
+HD bool star_side(uint32_t pp, uint32_t pq, uint32_t pb, int side) {
+    const int64_t o = orient_p(pp, pq, pb);
+    return side > 0 ? o > 0 : o < 0;
+}
+
+// Walk the star.  An interior point (hn < 0) starts at nearest(), p's
+// nearest neighbour, and walks counter-clockwise until it is back there.  A
+// point of the hull boundary starts at hn, its successor on the boundary
+// (counter-clockwise, the interior on the left), and walks until it reaches
+// hp, its predecessor.  next(q, side) returns the next neighbour after q on
+// that side (-1: none, so p->q is a hull edge; -2: the search failed).
+// The neighbours are appended to ccw (counter-clockwise) and, should an
+// interior point meet the hull (all points collinear), to cw (clockwise from
+// the start); star_at gives them in counter-clockwise order.  Returns false
+// if a search failed or a list would pass cap.
+template <class Nearest, class Next>
+HD bool star_walk(int hn, int hp, Nearest nearest, Next next, int32_t* ccw, int32_t* cw, int cap, int* m, int* k,
+                  bool* closed) {
+    *m = 0;
+    *k = 0;
+    *closed = false;
+    const int q0 = hn >= 0 ? hn : nearest();
+    if (q0 < 0) return q0 == -1;
+    ccw[(*m)++] = q0;
+    int q = q0;
+    for (;;) {
+        const int r = next(q, +1);
+        if (r == -2) return false;
+        if (r < 0) break;
+        if (r == q0) {
+            *closed = hn < 0;
+            return hn < 0;
+        }
+        if (*m >= cap) return false;
+        ccw[(*m)++] = r;
+        if (r == hp) return true;
+        q = r;
+    }
+    if (hn >= 0) return true;
+    q = q0;
+    for (;;) {
+        const int r = next(q, -1);
+        if (r == -2) return false;
+        if (r < 0) break;
+        if (*k >= cap) return false;
+        cw[(*k)++] = r;
+        q = r;
+    }
+    return true;
+}
+
+// The hull boundary, counter-clockwise (the interior on the left of each
+// step), from the rows' extreme points: the top row left to right, the
+// right chain down, the bottom row right to left, the left chain up.  The
+// chains are the rows' last (first) points with the concave ones removed by
+// the monotone stack walk; collinear points stay, as every point on the
+// boundary is a vertex of the triangulation.  xy[s] holds the packed
+// coordinates of the leftmost (side 0) or rightmost (side 1) point of
+// non-empty row s (of R, top to bottom).  Writes the chain as row positions
+// (top to bottom; room for R) and its length.
+HD void hull_chain(int side, int R, const uint32_t* xy, int32_t* st, int* len) {
+    int sp = 0;
+    uint32_t a = 0, b = 0;     // the stack's top two points
+    for (int s = 0; s < R; ++s) {
+        const uint32_t x = xy[s];
+        while (sp >= 2) {
+            const int64_t o = orient_p(a, b, x);
+            if (side ? o < 0 : o > 0) {
+                --sp;
+                b = a;
+                if (sp >= 2) a = xy[st[sp - 2]];
+            } else {
+                break;
+            }
+        }
+        st[sp++] = s;
+        a = b;
+        b = x;
+    }
+    *len = sp;
+}
+
+// The same chain, decided point by point (for a parallel build): row i's
+// point is dropped by the stack walk exactly when it lies strictly inside
+// the segment of two other chain points j < i < k (strictly right of L_j ->
+// L_k for the left chain, left of it for the right chain).  With
+// coordinates relative to point i and x mirrored for the right chain, that
+// holds iff min_{j<i} x_j / -y_j + min_{k>i} x_k / y_k < 0 (the rows above
+// have y < 0, those below y > 0); both minima and their sum are compared
+// as exact fractions.  |x| <= 18094 and 0 < y <= 16383 (the coordinate
+// limits of orient_p), so every cross product is below 2^29 and the final
+// sum below 2^30: exact in int32.
+HD bool hull_on_chain(int side, int R, const uint32_t* xy, int i) {
+    if (i == 0 || i == R - 1) return true;
+    const uint32_t c = xy[i];
+    const int sg = side ? -1 : 1;
+    // each minimum over four interleaved partial minima (independent chains)
+    int32_t n[2][4], d[2][4];
+    for (int h = 0; h < 2; ++h)
+        for (int u = 0; u < 4; ++u) {
+            n[h][u] = 1;
+            d[h][u] = 0;     // +infinity: 1/0 compares above every fraction below
+        }
+    auto fold = [&](int h, int u, uint32_t v, int dsign) {
+        const int32_t x = sg * dx_p(v, c), dd = dsign * dy_p(v, c);
+        if (d[h][u] == 0 || x * d[h][u] < n[h][u] * dd) {
+            n[h][u] = x;
+            d[h][u] = dd;
+        }
+    };
+    int j = 0;
+    for (; j + 4 <= i; j += 4)
+        for (int u = 0; u < 4; ++u) fold(0, u, xy[j + u], -1);
+    for (; j < i; ++j) fold(0, 0, xy[j], -1);
+    int k = i + 1;
+    for (; k + 4 <= R; k += 4)
+        for (int u = 0; u < 4; ++u) fold(1, u, xy[k + u], 1);
+    for (; k < R; ++k) fold(1, 0, xy[k], 1);
+    int32_t sn = n[0][0], sd = d[0][0], tn = n[1][0], td = d[1][0];
+    for (int u = 1; u < 4; ++u) {
+        if (d[0][u] != 0 && n[0][u] * sd < sn * d[0][u]) { sn = n[0][u]; sd = d[0][u]; }
+        if (d[1][u] != 0 && n[1][u] * td < tn * d[1][u]) { tn = n[1][u]; td = d[1][u]; }
+    }
+    return sn * td + tn * sd >= 0;
+}
+
+// Neighbour i in counter-clockwise order: the clockwise part reversed, then
+// the counter-clockwise part.
+HD int32_t star_at(const int32_t* ccw, int m, const int32_t* cw, int k, int i) {
+    (void)m;
+    return i < k ? cw[k - 1 - i] : ccw[i - k];
+}
+
+}  // namespace del
+}  // namespace elas
+
 using namespace elas::del;
 
 // px, py: n points; row_off: nrows+1 offsets of the points of each lattice
@@ -236,12 +471,12 @@ extern "C" int emu_delaunay_phased(const int32_t* px, const int32_t* py, int n, 
     return emu_core(px, py, n, row_off, nrows, tris_out, cap, stats, 1);
 }
 
-// Star construction (k_hull, k_star, k_star_scan, k_star_emit),
-// sequentially: the same rows, hull boundary, windows, walk and owner rule,
-// one point after another, each search a plain loop under the star order.  Triangles come out in point
-// order, as on the device.  stats (nullable): [0] phase-2 searches, [1]
-// squares grown, [2] candidates examined outside the staged windows.
-// Returns the triangle count, or -1.
+// Star construction (k_plan, k_star, k_star_far, k_star_emit), sequentially:
+// the same rows, hull boundary, star order and owner rule, one point after
+// another, each search over squares that grow until its answer is certain.
+// Triangles come out in point order, as on the device.  stats (nullable): [0]
+// 0, [1] squares grown, [2] candidates examined.  Returns the triangle count,
+// or -1.
 extern "C" int emu_delaunay_star(const int32_t* px, const int32_t* py, int n, const int32_t* row_off, int nrows,
                                  int32_t* tris_out, int cap, long long* stats) {
     // rows sorted by (x, index), repeated x dropped (k_rowsort)
@@ -263,7 +498,7 @@ extern "C" int emu_delaunay_star(const int32_t* px, const int32_t* py, int n, co
     std::vector<int> ne;
     for (int r = 0; r < nrows; ++r)
         if (rcnt[r] > 0) ne.push_back(r);
-    // hull boundary and the box of all points (k_hull)
+    // hull boundary and the box of all points (k_plan)
     std::vector<int32_t> hnext(std::max(n, 1), -1), hprev(std::max(n, 1), -1);
     int32_t box[4] = {0, 0, 0, 0};
     const int R = int(ne.size());
@@ -302,26 +537,10 @@ extern "C" int emu_delaunay_star(const int32_t* px, const int32_t* py, int n, co
             hprev[at(j)] = at(j == 0 ? C - 1 : j - 1);
         }
     }
-    long long circles = 0, squares = 0, evals = 0;
+    long long squares = 0, evals = 0;
     const int R0 = star_r0(box, n);
     std::vector<int32_t> tri, ccw(STAR_NB), cw(STAR_NB);
     std::vector<std::pair<int32_t, uint32_t>> win;
-    // every point of a region, row by row (the device splits them over lanes)
-    auto each_in = [&](const StarRegion& g, auto&& take) {
-        for (int r : ne) {
-            const int32_t y = py[row_off[r]];
-            if (y < g.y0 || y > g.y1) continue;
-            int32_t x0, x1, x2, x3;
-            g.cols2(y, box, &x0, &x1, &x2, &x3);
-            for (int j = row_off[r]; j < row_off[r] + rcnt[r]; ++j) {
-                const int32_t x = px_of(sxy[j]);
-                if ((x >= x0 && x <= x1) || (x >= x2 && x <= x3)) {
-                    ++evals;
-                    take(srt[j], sxy[j]);
-                }
-            }
-        }
-    };
     for (int p = 0; p < n; ++p) {
         const uint32_t pp = pxy[p];
         if (pp == PXY_NONE) continue;
@@ -329,29 +548,31 @@ extern "C" int emu_delaunay_star(const int32_t* px, const int32_t* py, int n, co
         auto covers = [&](int Rs) {
             return x0 - Rs <= box[0] && x0 + Rs >= box[2] && y0 - Rs <= box[1] && y0 + Rs >= box[3];
         };
-        // the window: staged once, grown (persisting for the point's later
-        // searches) while its rings fit STAR_CAP
+        // the points of the square of half-size Rs around p that are not in the one of half-size hole
+        auto each_in = [&](int Rs, int hole, auto&& take) {
+            for (int r : ne) {
+                const int dy = std::abs(py[row_off[r]] - y0);
+                if (dy > Rs) continue;
+                for (int j = row_off[r]; j < row_off[r] + rcnt[r]; ++j) {
+                    const int dx = std::abs(px_of(sxy[j]) - x0);
+                    if (dx <= Rs && (dx > hole || dy > hole)) {
+                        ++evals;
+                        take(srt[j], sxy[j]);
+                    }
+                }
+            }
+        };
+        // the window, which grows for the point's later searches
         win.clear();
-        each_in(star_square_region(pp, R0, box), [&](int32_t s2, uint32_t sx) { win.push_back({s2, sx}); });
-        const bool staged = win.size() <= size_t(STAR_CAP);
         int Rw = R0;
-        bool ring_full = !staged;
-        // one window growth, its ring's points given to take; false once
-        // the rings no longer fit (the ring was still searched)
+        each_in(Rw, -1, [&](int32_t s2, uint32_t sx) { win.push_back({s2, sx}); });
         auto grow = [&](auto&& take) {
             ++squares;
-            const size_t K0 = win.size();
-            each_in(star_ring_region(pp, Rw, box), [&](int32_t s2, uint32_t sx) {
+            each_in(2 * Rw, Rw, [&](int32_t s2, uint32_t sx) {
                 take(s2, sx);
                 win.push_back({s2, sx});
             });
-            if (win.size() > size_t(STAR_CAP)) {
-                win.resize(K0);
-                ring_full = true;
-                return false;
-            }
             Rw *= 2;
-            return true;
         };
         auto nearest = [&]() -> int {
             unsigned long long best = ~0ull;
@@ -361,27 +582,9 @@ extern "C" int emu_delaunay_star(const int32_t* px, const int32_t* py, int n, co
                 best = std::min<unsigned long long>(best, uint64_t(uint32_t(dx * dx + dy * dy)) << 32 | uint32_t(s2));
             };
             for (auto& c : win) take(c.first, c.second);
-            for (int Rs = Rw;;) {
-                const uint64_t d2 = best >> 32;
-                if (best != ~0ull && d2 <= uint64_t(Rs) * uint64_t(Rs)) return int(uint32_t(best));
-                if (covers(Rs)) return best == ~0ull ? -1 : int(uint32_t(best));
-                if (Rs == Rw && !ring_full) {
-                    if (!grow(take)) Rs *= 2;
-                    else Rs = Rw;
-                    continue;
-                }
-                if (best != ~0ull) {
-                    // the nearest lies within distance sqrt(d2): the square of that half-size
-                    int d = int(std::sqrt(double(d2)));
-                    while (uint64_t(d) * uint64_t(d) < d2) ++d;
-                    ++circles;
-                    best = ~0ull;
-                    each_in(star_square_region(pp, d, box), take);
-                    return int(uint32_t(best));
-                }
-                Rs = star_square(Rs);
-                ++squares;
-                each_in(star_square_region(pp, Rs, box), take);
+            for (;; grow(take)) {
+                if (best != ~0ull && (best >> 32) <= uint64_t(Rw) * uint64_t(Rw)) return int(uint32_t(best));
+                if (covers(Rw)) return best == ~0ull ? -1 : int(uint32_t(best));
             }
         };
         auto next = [&](int q, int side) -> int {
@@ -396,25 +599,8 @@ extern "C" int emu_delaunay_star(const int32_t* px, const int32_t* py, int n, co
                 }
             };
             for (auto& c : win) take(c.first, c.second);
-            for (int Rs = Rw;;) {
-                if (bi >= 0 && circle_inside(pp, pq, bxy, Rs, box)) return bi;
-                if (covers(Rs)) return bi;
-                if (Rs == Rw && !ring_full) {
-                    if (!grow(take)) Rs *= 2;
-                    else Rs = Rw;
-                    continue;
-                }
-                int need = 0;
-                if (bi >= 0) circle_within(pp, pq, bxy, Rs, box, &need);
-                if (bi >= 0 && need <= 2 * Rs) {
-                    ++circles;
-                    each_in(star_circle_region(pp, pq, bxy, box), take);
-                    return bi;
-                }
-                Rs = star_square(Rs);
-                ++squares;
-                each_in(star_half_region(pp, pq, side, Rs, box), take);
-            }
+            for (;; grow(take))
+                if ((bi >= 0 && circle_inside(pp, pq, bxy, Rw, box)) || covers(Rw)) return bi;
         };
         int m = 0, k = 0;
         bool closed = false;
@@ -433,12 +619,12 @@ extern "C" int emu_delaunay_star(const int32_t* px, const int32_t* py, int n, co
     }
     const int T = int(tri.size() / 3);
     if (T <= cap) std::memcpy(tris_out, tri.data(), sizeof(int32_t) * tri.size());
-    if (stats) { stats[0] = circles; stats[1] = squares; stats[2] = evals; }
+    if (stats) { stats[0] = 0; stats[1] = squares; stats[2] = evals; }
     return T;
 }
 
-// hull_chain (the stack walk) and hull_on_chain (the per-point test of the
-// device) on one chain: returns 1 if they keep the same points.
+// hull_chain (the stack walk) and hull_on_chain (the test that the device
+// makes in two levels, rows of a group and then what they leave) on one chain: returns 1 if they keep the same points.
 extern "C" int emu_hull_agree(const int32_t* xs, const int32_t* ys, int R, int side) {
     std::vector<uint32_t> xy(std::max(R, 1));
     for (int i = 0; i < R; ++i) xy[i] = pack_xy(xs[i], ys[i]);
