@@ -472,6 +472,7 @@ int set_proposal_weights(elas_handle* h, const float* params, int n) {
             return fail(h, ELAS_ERR_OOM, "proposal weights");
         CK(cudaMemset(h->pn_stats, 0, 4 * sizeof(int32_t)));
     }
+    CK(cudaDeviceSynchronize());    // calls in flight keep the weights they were made with
     CK(pn::upload_weights(params, h->pw, nullptr));
     h->prop_params.assign(params, params + n);
     h->prop = true;

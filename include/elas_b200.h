@@ -232,7 +232,8 @@ int elas_b200_dense_shape(const elas_handle* h, int32_t width, int32_t disp_max)
 #define ELAS_PN_PARAMS 36992
 
 /* Enable the proposal with these parameters (n == ELAS_PN_PARAMS) or
- * disable it (n == 0). */
+ * disable it (n == 0).  Enabling waits for the device: calls in flight keep
+ * the parameters that they were made with. */
 int elas_b200_set_proposal(elas_handle* h, const float* params, int32_t n);
 
 /* Candidates of the last call settled by the proposal (out[0]) and sent to

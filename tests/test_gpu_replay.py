@@ -153,3 +153,35 @@ def test_pair_survives_a_failed_rebind():
     finally:
         e.close()
         other.close()
+
+
+def test_new_weights_wait_for_calls_in_flight():
+    """elas_b200_set_proposal while pairs on a stream of their own are still
+    running: those keep the weights that they were called with."""
+    import torch
+
+    import proposal_oracle as po
+
+    W, H, D = 2880, 1988, 255
+    L, R = eb.synth_pair(2, 390, width=W, height=H, disp_max=D, gt=False)[:2]
+    first, second = eb.load_proposal(), po.init_params(2)
+    e = eb.Elas(eb.params_config(D))
+    try:
+        refs = []
+        for w in (first, second):
+            e.set_proposal(w)
+            refs.append(e.process(L, R))
+        assert not same(*refs)
+        st = torch.cuda.Stream()
+        images = [torch.from_numpy(x).cuda() for x in (L, R)]
+        outs = [[torch.empty((H, W), device="cuda") for _ in range(2)] for _ in range(8)]
+        torch.cuda.synchronize()
+        for k, o in enumerate(outs):            # new weights after every pair, none waited for
+            e.set_proposal((first, second)[k % 2])
+            e.process_device(*[x.data_ptr() for x in images + o], W, H, stream=st.cuda_stream)
+        e.set_proposal(first)
+        torch.cuda.synchronize()
+        for k, o in enumerate(outs):
+            assert same([x.cpu().numpy() for x in o], refs[k % 2]), k
+    finally:
+        e.close()
