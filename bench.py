@@ -283,7 +283,7 @@ def time_e2e(e, L, R, steps, torch, flush, warmup=3):
     return total, {"h2d_bytes_per_step": 2 * W * H, "d2h_bytes_per_step": 2 * W * H * 4}
 
 
-NO_TRIANGLE = "the reference's Triangle was not built (the oracle needs it for whole pairs)"
+NO_TRIANGLE = "the reference's Triangle was not built (the timed CPU pipeline runs on it)"
 
 
 def cpu_baseline(L, R, p, budget_s=12.0):

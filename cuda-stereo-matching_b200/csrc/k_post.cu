@@ -532,8 +532,10 @@ __device__ __forceinline__ float med9(const Tri& p, const Tri& q, const Tri& r) 
 // columns, four strips of R rows (the mean's region is 64 x 4 R: whole
 // warps).
 //
-// Bound by instruction issue and the shared-memory pipe, so each stage keeps
-// what neighbouring pixels share in registers:
+// Bound by latency and instruction issue (56 % of the issue slots with three
+// CTAs per SM; the first stall is the load stage's chain of map and label,
+// size slot and segment size), so each stage keeps what neighbouring pixels
+// share in registers:
 //   load    a warp loads whole rows and, as it knows their valid pixels from
 //           ballots, fills the row gaps at once: run lengths come from the
 //           bits on either side.  Fills are written in place (only invalid

@@ -139,9 +139,9 @@ constexpr long long PRIOR_TILED_MIN_PIXELS = 3LL << 20;
 // Images up to this many pixels take the star construction of the
 // Delaunay triangulations, larger ones the strips and flips.  The line was
 // drawn at the crossover of earlier constructions (now the stars are faster
-// on both sides: a pair takes 158 against 256 us at 1242x375, 1265 against
-// 1448 at 2880x1988), and stays: the list orders differ, and a pixel that
-// two triangles cover keeps the last one.
+// on both sides: a pair of the synthetic scene 3 takes 158 against 256 us at
+// 1242x375, 1265 against 1448 at 2880x1988), and stays: the list orders
+// differ, and a pixel that two triangles cover keeps the last one.
 constexpr long long DELAUNAY_STARS_MAX_PIXELS = 1LL << 21;
 size_t raster_bytes();
 

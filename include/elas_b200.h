@@ -125,7 +125,8 @@ int elas_b200_process(elas_handle* h, const uint8_t* left, const uint8_t* right,
                       void* stream);
 
 /* Same computation on caller-owned device buffers; asynchronous on `stream`
- * (no host synchronisation except the one-off workspace growth). */
+ * (no host synchronisation except the one-off workspace growth).  A handle's
+ * calls share its workspace: the caller orders calls on different streams. */
 int elas_b200_process_device(elas_handle* h, const uint8_t* d_left, const uint8_t* d_right,
                              float* d_disp_left, float* d_disp_right, const int32_t* dims,
                              void* stream);
@@ -146,8 +147,9 @@ int elas_b200_process_batch(elas_handle* h, int n,
  * Batched form on device buffers (pointer arrays in host memory).  Pair i
  * runs on its own worker (workspace + stream); the whole batch -- fork, n
  * pipelines, join -- is captured once into a CUDA graph and later calls with
- * the same sizes, disparity ranges, buffers, parameters and stream replay it
- * with a single graph launch.  The first call of a new signature runs
+ * the same sizes, disparity ranges, buffers, parameters, proposal and stream
+ * replay it with a single graph launch (unless other batches in between made
+ * the workers allocate larger workspaces).  The first call of a new signature runs
  * eagerly (sizing workspaces, tuning the dense kernel) and then captures.
  * stream NULL: an internal stream, and the call returns when done.
  * No counterpart in the reference (one pair per call, src/Elas.cu:19).
