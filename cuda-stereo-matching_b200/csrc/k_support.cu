@@ -25,6 +25,7 @@
 // which is what the warp computes; the oracle restates the reference's
 // lane-by-lane merge literally and the tests compare the two.
 #include <cuda_runtime.h>
+#include <type_traits>
 #include "common.cuh"
 #include "launch.cuh"
 #include "kernels.h"
@@ -746,34 +747,44 @@ __global__ void __launch_bounds__(1024) k_redundant(int32_t* __restrict__ can, G
 // candidate row computes the row's inconsistency filter (reading the
 // unfiltered lattice) into shared memory, warp 0 runs the row's
 // redundancy recurrence there, and the row is written once.  The window's
-// lattice rows are staged in shared memory first (STAGED; windows too tall
-// for it read the lattice in place), and PARTS neighbouring lanes share a
+// lattice rows are staged in shared memory first (windows too tall for it
+// read the lattice in place: IN_PLACE), and PARTS neighbouring lanes share a
 // candidate, each counting every PARTS-th window row; the counts are summed
 // across the lanes.  Narrow lattices (few candidates per row, too few CTAs
 // to fill the GPU) take 4 lanes per candidate, wide ones 1.
-// The staged window is padded by its half width, and what is no point lies
-// out of every threshold's reach, so that a count is a load, a subtraction
-// and a compare, unrolled for the usual half width of 5; the codes of the
-// recurrence come from all threads (1242x375: 10.4 -> 7.2 us,
-// 2880x1988: 28 -> 17.3).
+// In the staged window what is no point lies out of every threshold's reach,
+// and while it is no wider than the lattice it is padded by its half width
+// (PADDED), so that a count is a load, a subtraction and a compare, unrolled
+// for the usual half width of 5; the codes of the recurrence come from all
+// threads (1242x375: 10.4 -> 7.2 us, 2880x1988: 28 -> 17.3).  A wider window,
+// or one that fits only without its padding, is clipped to the lattice
+// (CLIPPED; half width 100: a pair of noise at 320x240 92 us padded, 70
+// clipped, at 1242x375 218 in place, 137 clipped).
 constexpr size_t INCON_STAGE_MAX = 96 * 1024;   // shared-memory bytes up to which the window is staged
 constexpr int INCON_NONE = -(1 << 30);
-template <bool STAGED, int PARTS>
+enum InconWindow { IN_PLACE, CLIPPED, PADDED };
+template <InconWindow WIN, int PARTS>
 __global__ void k_incon_rows(const int32_t* __restrict__ cin, int32_t* __restrict__ cout, Geom g, DevParams p,
                              int32_t* __restrict__ row_cnt) {
     grid_dep_wait();
     if (threadIdx.x == 0) row_cnt[blockIdx.x] = 0;     // counted by the vertical redundancy pass
-    extern __shared__ int sm[];             // [window rows x (cw + 2 ws) ints when STAGED], cw ints, cw code bytes
+    constexpr bool STAGED = WIN != IN_PLACE;
+    extern __shared__ int sm[];             // [window rows x pitch ints when STAGED], cw ints, cw code bytes
     const int ws = p.incon_window, y = blockIdx.x;
     const int ylo = max(0, y - ws), yhi = min(g.ch - 1, y + ws), nr = yhi - ylo + 1;
-    const int pitch = g.cw + 2 * ws;
+    const int pad = WIN == PADDED ? ws : 0, pitch = g.cw + 2 * pad;
     int* row = sm + (STAGED ? nr * pitch : 0);
     uint8_t* code = reinterpret_cast<uint8_t*>(row + g.cw);
     const int* in = cin + size_t(ylo) * g.cw;          // the window's rows, from ylo
     if (STAGED) {
         for (int i = threadIdx.x; i < nr * pitch; i += blockDim.x) {
-            const int r = i / pitch, x = i - r * pitch - ws;
-            const int d = x >= 0 && x < g.cw ? in[r * g.cw + x] : -1;
+            int d;
+            if (WIN == PADDED) {
+                const int r = i / pitch, x = i - r * pitch - ws;
+                d = x >= 0 && x < g.cw ? in[r * g.cw + x] : -1;
+            } else {
+                d = in[i];
+            }
             sm[i] = d < 0 ? INCON_NONE : d;
         }
         __syncthreads();
@@ -784,13 +795,20 @@ __global__ void k_incon_rows(const int32_t* __restrict__ cin, int32_t* __restric
     const int part = threadIdx.x % PARTS, per = blockDim.x / PARTS;
     for (int x0 = 0; x0 < g.cw; x0 += per) {   // every lane of a warp takes the same trips (the shuffles)
         const int x = x0 + int(threadIdx.x) / PARTS;
-        const int d = x >= g.cw ? -1 : STAGED ? max(sm[(y - ylo) * pitch + x + ws], -1) : in[(y - ylo) * g.cw + x];
+        const int d = x >= g.cw ? -1 : STAGED ? max(sm[(y - ylo) * pitch + x + pad], -1) : in[(y - ylo) * g.cw + x];
         const bool check = d >= 0 && y < g.cw;
         int support = 0;
         if (STAGED) {
             if (check) {
                 const int dt = thr >= 0 ? d + thr : INCON_NONE / 2;
-                if (ws == 5) {
+                if (WIN == CLIPPED) {
+                    const int xa = max(0, x - ws), nx = min(g.cw - 1, x + ws) - xa + 1;
+                    for (int r = part; r < nr; r += PARTS) {
+                        const int* w = sm + r * pitch + xa;
+#pragma unroll 8
+                        for (int j = 0; j < nx; ++j) support += unsigned(dt - w[j]) <= lim;
+                    }
+                } else if (ws == 5) {
                     for (int r = part; r < nr; r += PARTS) {
                         const int* w = sm + r * pitch + x;
 #pragma unroll
@@ -1063,23 +1081,26 @@ cudaError_t launch_support(const uint4* desc0, const uint4* desc1, int32_t* can_
     {
         const size_t sm = size_t(g.cw) * (sizeof(int) + 1);
         const long long ww = 2LL * p.incon_window;
-        const size_t wsm = size_t(ww + 1 < g.ch ? ww + 1 : g.ch) * size_t(g.cw + ww) * sizeof(int);
+        const size_t wrows = size_t(ww + 1 < g.ch ? ww + 1 : g.ch);
+        auto win_smem = [&](long long pad) { return sm + wrows * size_t(g.cw + pad) * sizeof(int); };
         const int parts = g.cw <= 256 ? 4 : (g.cw <= 512 ? 2 : 1);
         const int threads = imin(1024, imax(32, ((parts * g.cw + 31) / 32) * 32));
-        const bool staged = sm + wsm <= INCON_STAGE_MAX;
         auto go = [&](auto kern, size_t bytes) {
             allow_smem(kern);
             launch_k(kern, g.ch, threads, bytes, st, can_lr, can, g, p, row_cnt);
         };
-        if (staged) {
-            if (parts == 4) go(k_incon_rows<true, 4>, sm + wsm);
-            else if (parts == 2) go(k_incon_rows<true, 2>, sm + wsm);
-            else go(k_incon_rows<true, 1>, sm + wsm);
-        } else {
-            if (parts == 4) go(k_incon_rows<false, 4>, sm);
-            else if (parts == 2) go(k_incon_rows<false, 2>, sm);
-            else go(k_incon_rows<false, 1>, sm);
-        }
+        auto win = [&](auto w, size_t bytes) {
+            constexpr InconWindow WIN = decltype(w)::value;
+            if (parts == 4) go(k_incon_rows<WIN, 4>, bytes);
+            else if (parts == 2) go(k_incon_rows<WIN, 2>, bytes);
+            else go(k_incon_rows<WIN, 1>, bytes);
+        };
+        if (ww + 1 <= g.cw && win_smem(ww) <= INCON_STAGE_MAX)
+            win(std::integral_constant<InconWindow, PADDED>{}, win_smem(ww));
+        else if (win_smem(0) <= INCON_STAGE_MAX)
+            win(std::integral_constant<InconWindow, CLIPPED>{}, win_smem(0));
+        else
+            win(std::integral_constant<InconWindow, IN_PLACE>{}, sm);
         allow_smem(k_redundant);
         // warps in multiples of COL_LINES, up to one pass over the columns
         const int col_threads = imin(1024, (g.ch + 31) / 32 * 32 * COL_LINES);

@@ -177,6 +177,45 @@ def test_support_filters_at_window_sizes(elas, width, height, window, threshold)
     run_and_compare(elas, L, R, p, check_triangle=False)
 
 
+@pytest.mark.parametrize("width,height,window", [(320, 240, 31), (320, 240, 32), (640, 480, 63), (640, 480, 64),
+                                                 (160, 120, 1000), (1242, 375, 41), (1300, 900, 100)])
+def test_inconsistency_windows_wider_than_the_lattice(elas, width, height, window):
+    """The window staged with its padding, clipped to the lattice (wider than
+    it, or too large with the padding) and read in place (1300 x 900)."""
+    L, R, _, _ = eb.synth_pair(3, 49, width=width, height=height, disp_max=32)
+    p = eb.params_config(32)
+    p.incon_window_size, p.incon_min_support = window, 40
+    run_and_compare(elas, L, R, p, check_triangle=False)
+
+
+def test_wide_inconsistency_window_takes_no_longer(elas):
+    """A window that covers the whole lattice from everywhere (half width 100
+    on 128 x 96 points) counts hardly more points than one of half width 60:
+    the support stage takes at most 1.25 times as long (fastest of 10)."""
+    import torch
+
+    W, H = 640, 480
+    rng = np.random.default_rng(6)
+    L, R = (torch.from_numpy(rng.integers(0, 256, (H, W), dtype=np.uint8)).cuda() for _ in range(2))
+    o1, o2 = (torch.empty((H, W), device="cuda") for _ in range(2))
+    best = []
+    elas.set_timing(True)
+    try:
+        for window in (60, 100):
+            p = eb.params_config(128, post=False)
+            p.incon_window_size = window
+            elas.set_params(p)
+            times = []
+            for _ in range(10):
+                elas.process_device(L.data_ptr(), R.data_ptr(), o1.data_ptr(), o2.data_ptr(), W, H)
+                torch.cuda.synchronize()
+                times.append(elas.timing()["support"])
+            best.append(min(times))
+    finally:
+        elas.set_timing(False)
+    assert best[1] <= 1.25 * best[0], best
+
+
 @pytest.mark.parametrize("height,step", [(5796, 1), (11593, 2)])
 def test_tallest_lattice(elas, height, step):
     """The most lattice rows that are taken (5796), with and without the
