@@ -1080,14 +1080,16 @@ cudaError_t launch_support(const uint4* desc0, const uint4* desc1, int32_t* can_
     }
     {
         const size_t sm = size_t(g.cw) * (sizeof(int) + 1);
-        const long long ww = 2LL * p.incon_window;
+        DevParams q = p;
+        q.incon_window = imin(p.incon_window, imax(g.cw, g.ch));    // beyond, the same window (and no overflow)
+        const long long ww = 2LL * q.incon_window;
         const size_t wrows = size_t(ww + 1 < g.ch ? ww + 1 : g.ch);
         auto win_smem = [&](long long pad) { return sm + wrows * size_t(g.cw + pad) * sizeof(int); };
         const int parts = g.cw <= 256 ? 4 : (g.cw <= 512 ? 2 : 1);
         const int threads = imin(1024, imax(32, ((parts * g.cw + 31) / 32) * 32));
         auto go = [&](auto kern, size_t bytes) {
             allow_smem(kern);
-            launch_k(kern, g.ch, threads, bytes, st, can_lr, can, g, p, row_cnt);
+            launch_k(kern, g.ch, threads, bytes, st, can_lr, can, g, q, row_cnt);
         };
         auto win = [&](auto w, size_t bytes) {
             constexpr InconWindow WIN = decltype(w)::value;

@@ -611,3 +611,18 @@ def test_flip_rounds_match_host_emulation(elas, emu_lib, preset):
         assert (ctr[right, 4], ctr[right, 5]) == (st[0], st[1]), (right, ctr[right], st)
         ok, stats = oracle.delaunay_check(xy, elas.stage(key).view(np.int32).reshape(-1, 3))
         assert ok, (key, stats)
+
+
+def test_largest_inconsistency_window(elas):
+    """A half width of 2^31 - 1, which parameters may hold, means the whole
+    lattice, as one of 5000 does."""
+    L, R, _, _ = eb.synth_pair(3, 57, width=200, height=160, disp_max=32)
+    p = eb.params_config(32)
+    p.incon_min_support = 30
+    got = []
+    for window in (5000, 2 ** 31 - 1):
+        p.incon_window_size = window
+        elas.set_params(p)
+        elas.process(L, R)
+        got.append(elas.stage("can").copy())
+    assert np.array_equal(*got) and (got[0].view(np.int32) >= 0).any()
